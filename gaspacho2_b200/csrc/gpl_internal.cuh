@@ -52,6 +52,21 @@ struct DevBuf {
 // Operands, partial sums and TMA descriptors of the tensor-core contractions (k_tc.cu).
 // Column-pair FP64 GEMM state (k_dgemm.cu): the pair list (a <= b over the dense columns),
 // 1/Omega, the gathered Psi^{-1} pairs per gene and a range of V rows.
+// Integer form of the column-pair products (k_crt.cu): cells per range of both products, the scales
+// of the operand rows (genes, pairs, cells: 2^s and 2^-s of each) and the parts of the pair buffer.
+struct CrtState {
+  bool on = false;
+  int Jp = 0, Pp = 0, Jk = 0;     // genes and pairs padded to tiles, genes padded to K chunks
+  int gram_cells = 0, grad_cells = 0;  // 0: that product stays with the DMMA form
+  size_t bytes = 0;
+  double* scales = nullptr;
+  int *flag = nullptr, *err = nullptr;  // operands out of range (the DMMA form runs); a wait gave up
+  int8_t *g_a = nullptr, *g_b = nullptr, *v_a = nullptr, *v_b = nullptr;
+  uint8_t *g_out = nullptr, *v_out = nullptr;
+  double* g_acc = nullptr;
+  CUtensorMap map_ga, map_gb, map_va, map_vb;
+};
+
 struct PairState {
   bool ready = false, wide = false;  // wide: a cell's V row exceeds k_v_to_u's shared memory
   int n_pairs = 0, pairs_pad = 0, cpad = 0, v_cells = 0;
@@ -59,6 +74,7 @@ struct PairState {
   int2* pairs = nullptr;
   double *rOm = nullptr, *Sp = nullptr, *V = nullptr;
   double* Gacc = nullptr;  // pairs x genes Gram accumulator when the cells need several ranges
+  CrtState crt;            // the integer form, where it is the faster one
 };
 
 struct TcState {
@@ -326,6 +342,15 @@ int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratc
 int dgen_unwhiten(Ctx* c, const double* Gt, double* Tt, const double* Lw);  // Psi_DD = L G L^T + DeltaInv
 int dgen_whiten_inverse(Ctx* c, const double* Lw, double* Tt, double* St);  // S~ = L^T S_DD L per gene
 int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D);  // U from the V rows of cells [c0, c1)
+int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* gate);  // given V, gated
+// k_crt.cu (the pair products on the INT8 tensor cores)
+void crt_plan(Ctx* c, size_t cap);
+int crt_prepare(Ctx* c);
+void crt_release(Ctx* c);
+int launch_crt_gram(Ctx* c);
+int launch_crt_uq(Ctx* c);
+int crt_error_flag(Ctx* c);
+bool tc_map_u8(CUtensorMap* m, void* ptr, uint64_t cols, uint64_t rows);  // 128 x 128 byte boxes, swizzled
 int launch_tc_gram(Ctx* c);               // dense block of every Psi_j on tensor cores
 int launch_tc_grad(Ctx* c);               // U = sum_j O_ij S_j[DD] d_i on tensor cores
 int tc_error_flag(Ctx* c);                // GPL_ERR_TIMEOUT if a tensor-core kernel gave up waiting

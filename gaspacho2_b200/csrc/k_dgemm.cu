@@ -89,8 +89,10 @@ constexpr int kProdCells = 8;
 
 __global__ void __launch_bounds__(256) k_pair_products(int ldN, int n_d, int c0, int c1, int n_pairs, int pairs_pad,
                                                        const int2* __restrict__ pairs, const double* __restrict__ D,
-                                                       const double* __restrict__ rOm, double* __restrict__ A) {
+                                                       const double* __restrict__ rOm, double* __restrict__ A,
+                                                       const int* __restrict__ gate) {
   extern __shared__ double dsh[];  // [n_d][kProdCells] then rOm[kProdCells]
+  if (gate && *gate == 0) return;
   const int i0 = c0 + blockIdx.x * kProdCells;
   const int nc = min(kProdCells, c1 - i0);
   for (int e = threadIdx.x; e < n_d * kProdCells; e += blockDim.x) {
@@ -125,8 +127,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_pair_gram(int N, int ldN, int J, int P, int c0, int c1, int pairs_pad, int n_pairs, int mode,
                 const double* __restrict__ A, const int2* __restrict__ pairs, const int* __restrict__ dcol,
                 const double* __restrict__ W, const double* __restrict__ Dinv, double* __restrict__ Psi,
-                double* __restrict__ Gacc, int group_m) {
+                double* __restrict__ Gacc, int group_m, const int* __restrict__ gate) {
   extern __shared__ __align__(16) double smem_d[];
+  if (gate && *gate == 0) return;
   double* As = smem_d;              // [3][BK][SA]   pair products (pairs contiguous)
   double* Bs = As + 3 * BK * SA;    // [3][BN][SBT]  weights (cells contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -218,7 +221,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Psi_j[mk, ml] = Psi_j[ml, mk] = Gacc[p * J + j] + DeltaInv[mk, ml] after several ranges
 __global__ void k_pair_scatter(int J, int P, int n_pairs, const int2* __restrict__ pairs,
                                const int* __restrict__ dcol, const double* __restrict__ Gacc,
-                               const double* __restrict__ Dinv, double* __restrict__ Psi) {
+                               const double* __restrict__ Dinv, double* __restrict__ Psi,
+                               const int* __restrict__ gate) {
+  if (gate && *gate == 0) return;
   const int p = blockIdx.x;
   const int2 q = pairs[p];
   const size_t mk = dcol[q.x], ml = dcol[q.y];
@@ -255,8 +260,10 @@ __global__ void k_gather_spair(int J, int P, int n_pairs, int pairs_pad, const i
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_pair_v(int N, int ldN, int J, int c0, int c1, int pairs_pad, const double* __restrict__ W,
-             const double* __restrict__ Sp, const double* __restrict__ rOm, double* __restrict__ V, int group_m) {
+             const double* __restrict__ Sp, const double* __restrict__ rOm, double* __restrict__ V, int group_m,
+             const int* __restrict__ gate) {
   extern __shared__ __align__(16) double smem_d[];
+  if (gate && *gate == 0) return;
   double* As = smem_d;                // [3][BK][SA]  W rows (cells contiguous)
   double* Bs = smem_d + 3 * BK * SA;  // [3][BK][SBN] S pairs (pairs contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -330,8 +337,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 // shared memory; pair(a, b) = a*n_d - a*(a-1)/2 + (b - a) (row-major upper triangle).
 __global__ void __launch_bounds__(256) k_v_to_u(int N, int ldN, int n_d, int n_pairs, int pairs_pad, int c0,
                                                 int c1, const double* __restrict__ D,
-                                                const double* __restrict__ V, double* __restrict__ U) {
+                                                const double* __restrict__ V, double* __restrict__ U,
+                                                const int* __restrict__ gate) {
   extern __shared__ __align__(16) double vs[];
+  if (gate && *gate == 0) return;
   double* ds = vs + pairs_pad;  // D row of the cell
   for (int i = c0 + blockIdx.x; i < c1 && i < N; i += gridDim.x) {
     const double* vr = V + (size_t)(i - c0) * pairs_pad;
@@ -356,8 +365,9 @@ __global__ void __launch_bounds__(256) k_v_to_u(int N, int ldN, int n_d, int n_p
 // the cell is staged; identical operations in identical order.
 __global__ void __launch_bounds__(256) k_v_to_u_wide(int N, int ldN, int n_d, int pairs_pad, int c0, int c1,
                                                      const double* __restrict__ D, const double* __restrict__ V,
-                                                     double* __restrict__ U) {
+                                                     double* __restrict__ U, const int* __restrict__ gate) {
   extern __shared__ __align__(16) double ds[];  // D row of the cell
+  if (gate && *gate == 0) return;
   for (int i = c0 + blockIdx.x; i < c1 && i < N; i += gridDim.x) {
     const double* vr = V + (size_t)(i - c0) * pairs_pad;
     for (int e = threadIdx.x; e < n_d; e += blockDim.x) ds[e] = D[(size_t)e * ldN + i];
@@ -399,10 +409,13 @@ int pair_prepare(Ctx* c) {
   // more dense columns than k_v_to_u stages per cell: k_v_to_u_wide reads the V rows from
   // global memory instead
   s.wide = s.smem_vu > 200 * 1024;
+  // the integer form (k_crt.cu) keeps its operands in the same buffer
+  crt_plan(c, (size_t)8 << 30);
+  const size_t v_bytes = std::max(sizeof(double) * (size_t)s.v_cells * s.pairs_pad, s.crt.bytes);
   if (cudaMalloc((void**)&s.pairs, sizeof(int2) * pairs.size()) != cudaSuccess ||
       cudaMalloc((void**)&s.rOm, sizeof(double) * s.cpad) != cudaSuccess ||
       cudaMalloc((void**)&s.Sp, sizeof(double) * (size_t)c->J * s.pairs_pad) != cudaSuccess ||
-      cudaMalloc((void**)&s.V, sizeof(double) * (size_t)s.v_cells * s.pairs_pad) != cudaSuccess) {
+      cudaMalloc((void**)&s.V, v_bytes) != cudaSuccess) {
     cudaGetLastError();
     pair_release(c);
     c->err = "device allocation failed: pair GEMM buffers";
@@ -419,6 +432,11 @@ int pair_prepare(Ctx* c) {
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_gram));
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_v, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_v));
   if (!s.wide) GPL_TRY(c, cudaFuncSetAttribute(k_v_to_u, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_vu));
+  const int rc = crt_prepare(c);
+  if (rc) {
+    pair_release(c);
+    return rc;
+  }
   s.ready = true;
   return GPL_OK;
 }
@@ -426,6 +444,7 @@ int pair_prepare(Ctx* c) {
 void pair_release(Ctx* c) {
   graph_reset(c);
   PairState& s = c->pr;
+  crt_release(c);
   void* bufs[] = {s.pairs, s.rOm, s.Sp, s.V, s.Gacc};
   for (void* p : bufs)
     if (p) cudaFree(p);
@@ -455,26 +474,30 @@ int launch_pair_gram(Ctx* c) {
   PairState& s = c->pr;
   if ((rc = launch_recip(c))) return rc;
   ProfScope ps(c, "gram");
+  // the integer form, where it is planned; the kernels below then run only if it found operands out of
+  // its range (gate), as they do for non-finite values
+  const int* gate = s.crt.gram_cells ? s.crt.flag : nullptr;
+  if (gate && (rc = launch_crt_gram(c))) return rc;
   const bool one = s.v_cells >= c->N;
   for (int c0 = 0; c0 < c->N; c0 += s.v_cells) {
     const int c1 = std::min(c->N, c0 + s.v_cells);
     const int smem_p = (int)sizeof(double) * (c->n_d + 1) * kProdCells;
     k_pair_products<<<div_up(c1 - c0, kProdCells), 256, smem_p, c->stream>>>(
-        c->ldN, c->n_d, c0, c1, s.n_pairs, s.pairs_pad, s.pairs, c->Dm, s.rOm, s.V);
+        c->ldN, c->n_d, c0, c1, s.n_pairs, s.pairs_pad, s.pairs, c->Dm, s.rOm, s.V, gate);
     GPL_LAUNCHED(c, "k_pair_products");
     const int mode = one ? kGramPsi : (c0 == 0 ? kGramSet : kGramAdd);
     const int g = div_up(s.n_pairs, BM) * div_up(c->J, BN);
     Tunable* tu = nullptr;
-    const int gm = tune_pick(c, "pair_gram", {8, 12, 16}, kGroupM, &tu);
+    const int gm = gate ? kGroupM : tune_pick(c, "pair_gram", {8, 12, 16}, kGroupM, &tu);
     TuneScope ts(c, one ? tu : nullptr);
     k_pair_gram<<<g, kThreads, s.smem_gram, c->stream>>>(c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs,
                                                         mode, s.V, s.pairs, c->dcol_d, c->W, c->DeltaInv, c->Psi,
-                                                        s.Gacc, gm);
+                                                        s.Gacc, gm, gate);
     GPL_LAUNCHED(c, "k_pair_gram");
   }
   if (!one) {
     k_pair_scatter<<<s.n_pairs, 256, 0, c->stream>>>(c->J, c->P, s.n_pairs, s.pairs, c->dcol_d, s.Gacc,
-                                                    c->DeltaInv, c->Psi);
+                                                    c->DeltaInv, c->Psi, gate);
     GPL_LAUNCHED(c, "k_pair_scatter");
   }
   return GPL_OK;
@@ -492,34 +515,41 @@ int launch_pair_uq(Ctx* c) {
                                              s.Sp);
     GPL_LAUNCHED(c, "k_gather_spair");
   }
+  const int* gate = s.crt.grad_cells ? s.crt.flag : nullptr;  // as in launch_pair_gram
+  if (gate && (rc = launch_crt_uq(c))) return rc;
   for (int c0 = 0; c0 < c->N; c0 += s.v_cells) {
     const int c1 = std::min(c->N, c0 + s.v_cells);
     {
       ProfScope ps(c, "uq");
       const int g = div_up(c1 - c0, BM) * (s.pairs_pad / BN);
       Tunable* tu = nullptr;
-      const int gm = tune_pick(c, "pair_v", {8, 12, 16}, kGroupM, &tu);
+      const int gm = gate ? kGroupM : tune_pick(c, "pair_v", {8, 12, 16}, kGroupM, &tu);
       TuneScope ts(c, c1 - c0 == c->N ? tu : nullptr);
       k_pair_v<<<g, kThreads, s.smem_v, c->stream>>>(c->N, c->ldN, c->J, c0, c1, s.pairs_pad, c->W, s.Sp, s.rOm,
-                                                     s.V, gm);
+                                                     s.V, gm, gate);
       GPL_LAUNCHED(c, "k_pair_v");
     }
-    if ((rc = launch_v_to_u_cells(c, c0, c1, c->Dm))) return rc;
+    if ((rc = launch_v_to_u_rows(c, c0, c1, c->Dm, s.V, gate))) return rc;
   }
   return GPL_OK;
 }
 
 int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D) {
+  return launch_v_to_u_rows(c, c0, c1, D, c->pr.V, nullptr);
+}
+
+int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* gate) {
   PairState& s = c->pr;
   ProfScope ps(c, "v_to_u");
   const int grid = std::min(c1 - c0, 148 * 8);
   if (s.wide) {
     k_v_to_u_wide<<<grid, 256, sizeof(double) * c->n_d, c->stream>>>(c->N, c->ldN, c->n_d, s.pairs_pad, c0, c1, D,
-                                                                    s.V, c->U);
+                                                                    V, c->U, gate);
     GPL_LAUNCHED(c, "k_v_to_u_wide");
     return GPL_OK;
   }
-  k_v_to_u<<<grid, 256, s.smem_vu, c->stream>>>(c->N, c->ldN, c->n_d, s.n_pairs, s.pairs_pad, c0, c1, D, s.V, c->U);
+  k_v_to_u<<<grid, 256, s.smem_vu, c->stream>>>(c->N, c->ldN, c->n_d, s.n_pairs, s.pairs_pad, c0, c1, D, V, c->U,
+                                                gate);
   GPL_LAUNCHED(c, "k_v_to_u");
   return GPL_OK;
 }

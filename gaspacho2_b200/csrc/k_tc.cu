@@ -633,6 +633,19 @@ static bool make_map(CUtensorMap* m, void* ptr, uint64_t cols, uint64_t rows, ui
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// 2-D byte map over a row-major [rows][cols] array, box (128 bytes, 128 rows), 128-byte swizzle
+bool tc_map_u8(CUtensorMap* m, void* ptr, uint64_t cols, uint64_t rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols};
+  const cuuint32_t box[2] = {128, 128};
+  const cuuint32_t estr[2] = {1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <class T>
 static int tc_alloc(Ctx* c, T** p, size_t n, const char* what) {
   if (cudaMalloc((void**)p, sizeof(T) * (n ? n : 1)) != cudaSuccess) {
@@ -881,6 +894,9 @@ int launch_tc_grad(Ctx* c) {
   return c->tc_check ? tc_check_flag(c) : GPL_OK;
 }
 
-int tc_error_flag(Ctx* c) { return c->tc.ready ? tc_check_flag(c) : GPL_OK; }
+int tc_error_flag(Ctx* c) {
+  const int rc = crt_error_flag(c);
+  return rc == GPL_OK && c->tc.ready ? tc_check_flag(c) : rc;
+}
 
 }  // namespace gpl

@@ -91,7 +91,8 @@ GPL_API int gpl_set_precision(gpl_ctx* ctx, int precision);
  *                       gradient's predictions, the refinement) on the FP64 tensor cores (1,
  *                       default) or as an FFMA tile GEMM (0); the two differ by rounding
  *   "pair_range_cells"  cells per range of the FP64 pair GEMMs (0, default: as many as 8 GiB
- *                       of pair products holds; smaller values exercise the multi-range path)
+ *                       of operands holds; smaller values exercise the multi-range path, values
+ *                       below 256 the FP64 multiply-add form of both products)
  *   "graph"             1: each objective evaluation and each gradient after it (in gpl_fit,
  *                       gpl_fit_outer, gpl_objective, gpl_evaluate, gpl_evaluate_device) runs as
  *                       a CUDA graph, captured on its first use and replayed after (one launch
