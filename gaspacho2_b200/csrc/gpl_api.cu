@@ -208,7 +208,7 @@ static int irls(Ctx* c, int jtr_max, int* n_sweeps) {
 
 static int objective_after_irls(Ctx* c, double* lk) {
   GPL_RUN(launch_oinvt(c));
-  GPL_RUN(launch_chol_single(c, c->DeltaInv, c->P));
+  GPL_RUN(launch_chol_prior(c));
   GPL_RUN(launch_zt_u(c, 0));
   GPL_RUN(launch_lkhd_genes(c));
   GPL_RUN(launch_collect_lkhd(c, c->N, 0));
@@ -221,7 +221,7 @@ static int objective_launch(Ctx* c, int slot) {
   GPL_RUN(launch_expand_delta(c));
   GPL_RUN(launch_gram(c, false));
   GPL_RUN(launch_chol_batched(c, c->Psi, c->P, c->J, (int64_t)c->P * c->P));
-  GPL_RUN(launch_chol_single(c, c->DeltaInv, c->P));
+  GPL_RUN(launch_chol_prior(c));
   GPL_RUN(launch_zt_u(c, 0));
   GPL_RUN(launch_lkhd_genes(c));
   GPL_RUN(launch_collect_lkhd(c, c->N, slot));

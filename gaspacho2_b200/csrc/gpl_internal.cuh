@@ -323,8 +323,10 @@ int launch_inverse_panels(Ctx* c);       // the same in 32-column panels with DM
 int launch_irls_tail(Ctx* c, int jtr, int ctas_per_sm);  // persistent per-gene IRLS tail; GPL_ERR_ARG:
                                                           // P beyond the panel Cholesky's range
 int launch_inverse_single(Ctx* c, const double* L, int n, double* tmp, double* out);
-int launch_cholinv_exact(Ctx* c, const double* L, int n, double* out);  // cholsl order, no FMA
-cudaError_t launch_chol_exact_raw(cudaStream_t st, double* A, int n);  // the launch's own status
+int launch_cholinv(Ctx* c, const double* L, int n, double* out);  // (L L^T)^{-1}, k_kmats.cu
+// choldc's order on one matrix whose first `diag` rows are diagonal; the launch's own status
+cudaError_t launch_chol_exact_raw(cudaStream_t st, double* A, int n, int diag = 0);
+int launch_chol_prior(Ctx* c);           // DeltaInv (blockdiag(diagonal, Kmm / delta_GP)) in place
 int launch_kernel_mats_raw(cudaStream_t st, int N, int M, int Q, const double* X, const double* T,
                            const double* rho, double* Knm, double* KinvKmn, double* titsias, double* Lwork);
 // k_tc.cu (precision form)
@@ -336,6 +338,7 @@ int recip_omega(Ctx* c, const double** rOm);  // 1/Omega (0 past N), refreshed o
 int dgen_zt_u(Ctx* c, int mode, const double* u, double* out);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);
 int dgen_c1_tn(Ctx* c);                   // GPL_ERR_ARG when the dense columns exceed one tile
 int dgen_group_sums(Ctx* c, int mode);
+int dgen_unweighted_gram(Ctx* c);         // the dense block of Psi_0 with every weight 1 (GLM initialisation)
 int dgen_hk(Ctx* c);
 int dgen_weighted_colsums(Ctx* c, const double* G2, int n2, double* out);  // out[j + c*J] = sum_i W_ij G2[c][i]
 int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch);  // device G (N x L) -> S (J x L)

@@ -2,17 +2,10 @@
 // cholPsi :683-692, cholDeltaInv :695-700, cholKmm kernel_funcs.cu:139-143, solvePsi
 // ggplvm.cu:46-53, choldc/cholsl chol.cu:19-97, initPsi init.cu:125-181).
 //
-//   k_gram      dense x dense block of Psi_j = Z^T diag(W_j / Omega) Z + DeltaInv over the
-//               dense model columns (the categorical rows come from the group sums), all
-//               genes, scattered to the model-column positions. A CTA owns a 32x32
-//               block pair (upper triangle of blocks) for 8 genes and streams every cell:
-//               Z column blocks and the weights for a 32-cell chunk go to shared memory,
-//               each thread accumulates a 4x8 tile for one gene in registers.
-//               Roofline: FP64 FMA, N*J*P^2/2 multiply-adds.
-//   k_chol      batched in-place Cholesky, one CTA per matrix, left-looking by columns:
-//               the update of column j reads row j of the factor (broadcast) and the rows
-//               below it (coalesced). A non-positive pivot zero-fills the matrix, as
-//               choldc does.
+//   k_chol_exact  one matrix in choldc's operation order (Kmm, the prior, the GLM Gram).
+//   k_chol      one matrix wider than that kernel's row slots, left-looking by columns: the
+//               update of column j reads row j of the factor (broadcast) and the rows below it
+//               (coalesced). A non-positive pivot zero-fills the matrix, as choldc does.
 //   k_solve     batched (L L^T) x = b, one warp per system: forward substitution column-
 //               oriented (coalesced), back substitution as warp dot products.
 //   k_trtri     V = L^{-1} (row-major scratch), one thread per column of V.
@@ -20,85 +13,6 @@
 #include "gpl_internal.cuh"
 
 namespace gpl {
-
-namespace {
-constexpr int GB = 32;   // column block
-constexpr int GG = 8;    // genes per CTA
-constexpr int GC = 32;   // cells per chunk
-}  // namespace
-
-__global__ void __launch_bounds__(256) k_gram(int N, int ldN, int n_d, int P, int J, const double* __restrict__ Z,
-                                              const int* __restrict__ dcol, const double* __restrict__ W,
-                                              const double* __restrict__ Omega, const double* __restrict__ Dinv,
-                                              double* __restrict__ Psi, int unweighted) {
-  __shared__ double sk[GC][GB + 1];
-  __shared__ double sl[GC][GB + 1];
-  __shared__ double sw[GC][GG];
-  // blockIdx.x enumerates block pairs (kb <= lb) of the upper triangle
-  int lbi = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
-  while ((lbi + 1) * (lbi + 2) / 2 <= (int)blockIdx.x) lbi++;
-  while (lbi * (lbi + 1) / 2 > (int)blockIdx.x) lbi--;
-  const int kbi = (int)blockIdx.x - lbi * (lbi + 1) / 2;
-  const int kb = kbi * GB, lb = lbi * GB;
-  const int j0 = blockIdx.y * GG;
-  const int tid = threadIdx.x;
-  const int g = tid >> 5, kq = (tid & 31) >> 2, lq = tid & 3;
-  double acc[4][8];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 8; b++) acc[a][b] = 0.0;
-
-  for (int i0 = 0; i0 < N; i0 += GC) {
-    // load 32 cells x 32 columns of each block (cell fastest in memory)
-    for (int e = tid; e < GC * GB; e += 256) {
-      const int r = e & (GC - 1), col = e >> 5;
-      const int i = i0 + r;
-      const int ck = kb + col, cl = lb + col;
-      sk[r][col] = (i < N && ck < n_d) ? Z[(size_t)ck * ldN + i] : 0.0;
-      sl[r][col] = (i < N && cl < n_d) ? Z[(size_t)cl * ldN + i] : 0.0;
-    }
-    {
-      const int r = tid & (GC - 1), gg = tid >> 5;
-      const int i = i0 + r, j = j0 + gg;
-      double w = 0.0;
-      if (i < N && j < J) w = unweighted ? 1.0 : W[(size_t)j * ldN + i] / Omega[i];
-      sw[r][gg] = w;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int r = 0; r < GC; r++) {
-      const double w = sw[r][g];
-      double a[4], b[8];
-#pragma unroll
-      for (int x = 0; x < 4; x++) a[x] = sk[r][kq * 4 + x] * w;
-#pragma unroll
-      for (int y = 0; y < 8; y++) b[y] = sl[r][lq * 8 + y];
-#pragma unroll
-      for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 8; y++) acc[x][y] = fma(a[x], b[y], acc[x][y]);
-    }
-    __syncthreads();
-  }
-  const int j = j0 + g;
-  if (j >= J) return;
-  double* Pj = Psi + (size_t)j * P * P;
-#pragma unroll
-  for (int x = 0; x < 4; x++) {
-    const int k = kb + kq * 4 + x;
-    if (k >= n_d) continue;
-#pragma unroll
-    for (int y = 0; y < 8; y++) {
-      const int l = lb + lq * 8 + y;
-      if (l >= n_d || k > l) continue;
-      const size_t mk = dcol[k], ml = dcol[l];  // model columns, mk <= ml
-      const double v = acc[x][y] + Dinv[mk + ml * P];
-      Pj[mk + ml * P] = v;
-      Pj[ml + mk * P] = v;
-    }
-  }
-}
 
 // Left-looking Cholesky of n x n matrices A_b = A + b*stride (col-major, ld n). The input is
 // read from the upper triangle (src_upper) or the lower one; the factor overwrites the
@@ -143,53 +57,86 @@ __global__ void __launch_bounds__(256) k_chol(double* __restrict__ A, int n, int
 // correctly rounded on both). Used for the small, often ill-conditioned matrices: Kmm (no
 // jitter in the reference), the prior precision DeltaInv and the GLM initialisation Gram.
 // Reads the upper triangle, writes the factor into the lower one; zero-fills on a
-// non-positive pivot. One CTA.
-__global__ void __launch_bounds__(256) k_chol_exact(double* __restrict__ a, int n) {
-  __shared__ int fail;
-  if (threadIdx.x == 0) fail = 0;
+// non-positive pivot. One CTA: the bound is the dependent chain of n^2/2 subtractions. The factor's
+// columns k >= k0 stay in shared memory (packed, rows j >= k contiguous), the ones that do not fit
+// are read back from global memory at the end of each chain. At n = 128: 0.58 ms from global
+// memory throughout, 0.18 ms so.
+// The first `diag` rows hold nothing off the diagonal (the prior's covariate part): their factor is
+// the square root of the diagonal, the products they contribute to later rows are exact zeros and
+// are left out, unless a diagonal entry is not finite.
+constexpr int kCholThreads = 256;
+__global__ void __launch_bounds__(kCholThreads) k_chol_exact(double* __restrict__ a, int n, int diag, int k0) {
+  extern __shared__ double ls[];  // column k >= k0, row j at off(k) + j
+  __shared__ int fail, odd;
+  __shared__ double piv;
+  const int tid = threadIdx.x;
+  if (tid == 0) fail = odd = 0;
   __syncthreads();
-  for (int i = 0; i < n; i++) {
-    // sums for j = i .. n-1 (j = i is the pivot)
-    double sums[4];
-    int cnt = 0;
-    for (int j = i + threadIdx.x; j < n && cnt < 4; j += blockDim.x, cnt++) {
-      double sum = a[i + (size_t)j * n];
-      for (int k = i - 1; k >= 0; k--) sum = __dsub_rn(sum, __dmul_rn(a[i + (size_t)k * n], a[j + (size_t)k * n]));
-      sums[cnt] = sum;
+  for (int k = tid; k < diag; k += kCholThreads) {
+    const double d = a[k + (size_t)k * n];
+    if (d <= 0.0) fail = 1;
+    if (!isfinite(d)) odd = 1;
+  }
+  __syncthreads();
+  const bool bad = fail != 0;
+  const int i_first = bad ? n : odd ? 0 : diag;
+  if (!bad && !odd)
+    for (int e = tid; e < diag * n; e += kCholThreads) {  // the lower triangle of the diagonal rows' columns
+      const int k = e / n, j = e - k * n;
+      if (j == k) a[e] = __dsqrt_rn(a[e]);
+      else if (j > k) a[e] = 0.0;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (sums[0] <= 0.0) fail = 1;
-      else a[i + (size_t)i * n] = __dsqrt_rn(sums[0]);
+  __syncthreads();
+  const int k_low = odd ? 0 : diag;  // first column whose products are taken
+  auto off = [&](int k) { return (k - k0) * n - (k * (k - 1) / 2 - k0 * (k0 - 1) / 2) - k; };
+  // a thread keeps its columns j = tid, tid + 256, ..; the next row's entries are loaded one row ahead
+  double sums[4], next[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const int j = tid + c * kCholThreads;
+    next[c] = i_first < n && j >= i_first && j < n ? a[i_first + (size_t)j * n] : 0.0;
+  }
+  for (int i = i_first; i < n; i++) {
+    // sums for j = i .. n-1 (j = i is the pivot)
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int j = tid + c * kCholThreads;
+      if (j < i || j >= n) continue;
+      double sum = next[c];
+      next[c] = j > i ? a[i + 1 + (size_t)j * n] : 0.0;
+      int k = i - 1;
+      const int ks = max(k0, k_low);
+      const double *li = ls + (k >= ks ? off(k) + i : 0), *lj = li + (j - i);
+#pragma unroll 8
+      for (; k >= ks; k--) {
+        sum = __dsub_rn(sum, __dmul_rn(*li, *lj));
+        li -= n - k;  // off(k - 1) = off(k) - (n - k)
+        lj -= n - k;
+      }
+#pragma unroll 8
+      for (; k >= k_low; k--) sum = __dsub_rn(sum, __dmul_rn(a[i + (size_t)k * n], a[j + (size_t)k * n]));
+      sums[c] = sum;
+      if (j == i) {
+        if (sum <= 0.0) fail = 1;
+        else piv = __dsqrt_rn(sum);
+      }
     }
     __syncthreads();
     if (fail) break;
-    const double lii = a[i + (size_t)i * n];
-    cnt = 0;
-    for (int j = i + threadIdx.x; j < n && cnt < 4; j += blockDim.x, cnt++)
-      if (j > i) a[j + (size_t)i * n] = __ddiv_rn(sums[cnt], lii);
+    const double lii = piv;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const int j = tid + c * kCholThreads;
+      if (j < i || j >= n) continue;
+      const double v = j > i ? __ddiv_rn(sums[c], lii) : lii;
+      a[j + (size_t)i * n] = v;
+      if (i >= k0) ls[off(i) + j] = v;
+    }
     __syncthreads();
   }
+  __syncthreads();
   if (fail)
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) a[e] = 0.0;
-}
-
-// Columns of (L L^T)^{-1} in cholsl's order (chol.cu:45-56), thread per column, no
-// contraction: the Kmm^{-1} of getC2 (ggplvm.cu:93-95). Y is an n x n scratch (col-major).
-__global__ void k_cholinv_exact(const double* __restrict__ a, int n, double* __restrict__ Y) {
-  for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n; col += gridDim.x * blockDim.x) {
-    double* x = Y + (size_t)col * n;
-    for (int i = 0; i < n; i++) {
-      double sum = (i == col) ? 1.0 : 0.0;
-      for (int k = i - 1; k >= 0; k--) sum = __dsub_rn(sum, __dmul_rn(a[i + (size_t)k * n], x[k]));
-      x[i] = __ddiv_rn(sum, a[i + (size_t)i * n]);
-    }
-    for (int i = n - 1; i >= 0; i--) {
-      double sum = x[i];
-      for (int k = i + 1; k < n; k++) sum = __dsub_rn(sum, __dmul_rn(a[k + (size_t)i * n], x[k]));
-      x[i] = __ddiv_rn(sum, a[i + (size_t)i * n]);
-    }
-  }
+    for (int e = tid; e < n * n; e += kCholThreads) a[e] = 0.0;
 }
 
 // (L L^T) x = b for `batch` systems, one warp each; y in shared memory.
@@ -254,21 +201,15 @@ __global__ void k_lauum(const double* __restrict__ Vrm, int n, int64_t stride, d
 }
 
 int launch_gram(Ctx* c, bool unweighted) {
-  const int nb = div_up(c->n_d, GB);
-  const int npairs = nb * (nb + 1) / 2;
   const int J = unweighted ? 1 : c->J;
-  int rc = GPL_ERR_ARG;
-  if (!unweighted) rc = c->precision == GPL_PREC_BF16X3 ? launch_tc_gram(c) : launch_pair_gram(c);
-  if (rc != GPL_OK && !(rc == GPL_ERR_ARG && (unweighted || c->precision == GPL_PREC_FP64))) return rc;
-  if (rc == GPL_ERR_ARG) {
-    // the unweighted Gram of one gene (GLM initialisation), or more dense columns than the
-    // staged pair contraction holds
+  int rc;
+  if (unweighted) {  // the Gram of the GLM initialisation, one for all genes
     ProfScope ps(c, "gram");
-    dim3 g(npairs, div_up(J, GG));
-    k_gram<<<g, 256, 0, c->stream>>>(c->N, c->ldN, c->n_d, c->P, J, c->Dm, c->dcol_d, c->W, c->Omega, c->DeltaInv,
-                                     c->Psi, unweighted ? 1 : 0);
-    GPL_LAUNCHED(c, "k_gram");
+    rc = dgen_unweighted_gram(c);
+  } else {
+    rc = c->precision == GPL_PREC_BF16X3 ? launch_tc_gram(c) : launch_pair_gram(c);
   }
+  if (rc != GPL_OK) return rc;
   rc = launch_group_sums(c, unweighted ? 1 : 0);
   if (rc) return rc;
   return launch_assemble_psi(c, J);
@@ -276,36 +217,39 @@ int launch_gram(Ctx* c, bool unweighted) {
 
 int launch_chol_batched(Ctx* c, double* A, int n, int batch, int64_t stride) {
   ProfScope ps(c, "chol");
-  {
-    const int rc = launch_potrf_panels(c, A, n, batch, stride);
-    if (rc != GPL_ERR_ARG) return rc;  // GPL_ERR_ARG: n beyond the panel kernel's checked range
-  }
-  k_chol<<<batch, 256, 0, c->stream>>>(A, n, stride, 0);
-  GPL_LAUNCHED(c, "k_chol");
-  return GPL_OK;
+  return launch_potrf_panels(c, A, n, batch, stride);
 }
 
 int launch_chol_single(Ctx* c, double* A, int n) {
   ProfScope ps(c, "chol_small");
-  if (n > 4 * 256) {  // wider than the exact kernel's per-thread row slots
+  if (n > 4 * kCholThreads) {  // wider than the exact kernel's per-thread row slots
     k_chol<<<1, 256, 0, c->stream>>>(A, n, 0, 1);
     GPL_LAUNCHED(c, "k_chol");
     return GPL_OK;
   }
-  k_chol_exact<<<1, 256, 0, c->stream>>>(A, n);
-  GPL_LAUNCHED(c, "k_chol_exact");
+  c->launches++;
+  GPL_TRY(c, launch_chol_exact_raw(c->stream, A, n));
   return GPL_OK;
 }
 
-cudaError_t launch_chol_exact_raw(cudaStream_t st, double* A, int n) {
-  void* args[] = {&A, &n};
-  return cudaLaunchKernel((const void*)k_chol_exact, dim3(1), dim3(256), args, 0, st);
+int launch_chol_prior(Ctx* c) {
+  if (c->P > 4 * kCholThreads) return launch_chol_single(c, c->DeltaInv, c->P);
+  ProfScope ps(c, "chol_small");
+  c->launches++;
+  GPL_TRY(c, launch_chol_exact_raw(c->stream, c->DeltaInv, c->P, c->nh[c->p - 1]));
+  return GPL_OK;
 }
 
-int launch_cholinv_exact(Ctx* c, const double* L, int n, double* out) {
-  k_cholinv_exact<<<div_up(n, 64), 64, 0, c->stream>>>(L, n, out);
-  GPL_LAUNCHED(c, "k_cholinv_exact");
-  return GPL_OK;
+cudaError_t launch_chol_exact_raw(cudaStream_t st, double* A, int n, int diag) {
+  constexpr size_t most = 224 * 1024;
+  int k0 = diag;  // the diagonal rows' columns are not read
+  while ((size_t)(n - k0) * (n - k0 + 1) / 2 * sizeof(double) > most) k0++;
+  const size_t smem = (size_t)(n - k0) * (n - k0 + 1) / 2 * sizeof(double);
+  const cudaError_t e = cudaFuncSetAttribute((const void*)k_chol_exact, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)most);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&A, &n, &diag, &k0};
+  return cudaLaunchKernel((const void*)k_chol_exact, dim3(1), dim3(kCholThreads), args, smem, st);
 }
 
 int launch_solve_batched(Ctx* c, const double* L, int n, int64_t lstride, const double* B, int64_t bstride,

@@ -5,11 +5,9 @@
 //                lv >= 0 only latent dimension lv enters (the DE driver's per-dimension models).
 //                Bound: N*M*Q transcendental work, ~2% of one objective evaluation.
 //   k_kmm        Kmm (upper, unit diagonal, zero lower) and its copy Kinv.
-//   k_kinvkmn    per cell: x = Kmm^{-1} k_n by two triangular solves against the factor in
-//                Kinv's lower triangle (cholslg order), titsias_n = (1 - k_n . x)/2.
-//                One thread per cell; the factor is read by every thread at the same
-//                address (broadcast), the solution lives in a cell-fastest scratch so the
-//                per-step loads coalesce.
+//   k_kmm_solve  per cell: x = Kmm^{-1} k_n against the factor in Kinv's lower triangle (cholslg),
+//                titsias_n = (1 - k_n . x)/2; also Kmm^{-1} itself. A cell per thread, 32-row blocks
+//                of the solution in registers.
 //   k_expand     DeltaInv = blockdiag(1/delta_k I, Kmm/delta_GP), upper + diagonal.
 #include <algorithm>
 
@@ -73,27 +71,152 @@ __global__ void k_gp_null(int N, int ldN, int M, double* __restrict__ Knm, doubl
   if (i < M * M) K[i] = Kinv[i] = (i % M == i / M) ? 1.0 : 0.0;
 }
 
-// Two triangular solves per cell with the lower factor L (n x n, col-major) held in the
-// lower triangle of Kinv; Knm and the solution Y are cell-fastest (ld ldN).
-__global__ void k_kinvkmn(int N, int ldN, int M, const double* __restrict__ L, const double* __restrict__ Knm,
-                          double* __restrict__ Y, double* __restrict__ titsias) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  // cholslg's order (chol.cu:86-97) without contracted multiply-adds: Kmm has no jitter in
-  // the reference and is often nearly singular, so the solve keeps the reference's rounding
-  for (int r = 0; r < M; r++) {
-    double sum = Knm[i + (size_t)r * ldN];
-    for (int k = r - 1; k >= 0; k--) sum = __dsub_rn(sum, __dmul_rn(L[r + k * M], Y[i + (size_t)k * ldN]));
-    Y[i + (size_t)r * ldN] = __ddiv_rn(sum, L[r + r * M]);
-  }
-  for (int r = M - 1; r >= 0; r--) {
-    double sum = Y[i + (size_t)r * ldN];
-    for (int k = r + 1; k < M; k++) sum = __dsub_rn(sum, __dmul_rn(L[k + r * M], Y[i + (size_t)k * ldN]));
-    Y[i + (size_t)r * ldN] = __ddiv_rn(sum, L[r + r * M]);
-  }
+// x_i = (L L^T)^{-1} b_i for many right-hand sides (one per cell), L the lower factor in A's lower
+// triangle (M x M, column-major): a cell per thread, 32 rows of its solution in registers, so that two
+// multiply-adds come from one broadcast load of L and every finished Y is read once per later block
+// of rows instead of once per row. Bound: N M^2 FP64 operations; a row-at-a-time substitution re-read
+// Y through L2 for every multiply-add (13 GB at N = 100,000, M = 128). kUnit: b_i = the i-th unit
+// vector (Kmm^{-1} of getC2, ggplvm.cu:93-95, the solution's column i at Y + i * ldY); else b_i =
+// column i of Knm^T, and titsias_i = (1 - k_i . x_i)/2.
+// kExact (M <= 32, one block): the sums keep cholslg's order (chol.cu:86-97) without contracted
+// multiply-adds, so that with few inducing points, where Kmm (no jitter in the reference) is often
+// nearly singular, the solution has the reference's bits. Otherwise multiply-adds in ascending order
+// and reciprocals of the diagonal: the error against extended precision is the row-at-a-time form's
+// (it is set by the factor, which keeps choldc's order): 2.7e-12 of the solution at cond(Kmm) = 5e5
+// against 3.0e-12, 1e-13 at 1e4 for both. At N = 100,000, M = 128: 1.58 -> 0.43 ms.
+constexpr int kSolveCells = 64, kSolveAhead = 8;
+template <bool kUnit, bool kExact>
+__global__ void __launch_bounds__(kSolveCells, 8)
+    k_kmm_solve(int N, int64_t ldN, int M, const double* __restrict__ A, const double* __restrict__ B, double* Y,
+                double* __restrict__ titsias) {
+  __shared__ __align__(16) double Ls[2][32][32];  // [k][row of the block]
+  __shared__ double Rd[32];
+  const int tid = threadIdx.x;
+  const int i = blockIdx.x * kSolveCells + tid;
+  const bool on = i < N;
+  // element (row r, cell i) of Y; threads past N follow cell N - 1 and store nothing
+  const size_t rs = kUnit ? 1 : (size_t)ldN, cs = kUnit ? (size_t)ldN : 1;
+  double* y = Y + (size_t)min(i, N - 1) * cs;
+  const double* b = kUnit ? nullptr : B + min(i, N - 1);
+  const int nb = (M + 31) / 32;
   double d = 0.0;
-  for (int k = 0; k < M; k++) d = __dadd_rn(d, __dmul_rn(Knm[i + (size_t)k * ldN], Y[i + (size_t)k * ldN]));
-  titsias[i] = (1.0 - d) / 2.0;
+
+  for (int pass = 0; pass < 2; pass++) {
+    for (int q = 0; q < nb; q++) {
+      const int ib = pass == 0 ? q : nb - 1 - q;
+      const int r0 = ib * 32, nr = min(32, M - r0);
+      // rows of L (forward) or columns of L (backward) of this block against the finished ones
+      const int kbeg = pass == 0 ? 0 : r0 + 32, kend = pass == 0 ? r0 : M;
+      auto stage = [&](int k0, int buf) {
+        for (int e = tid; e < 1024; e += kSolveCells) {
+          const int r = pass == 0 ? e & 31 : e >> 5, k = pass == 0 ? e >> 5 : e & 31;
+          const bool in = k0 + k < kend && r < nr;
+          const size_t at = pass == 0 ? (size_t)(r0 + r) + (size_t)(k0 + k) * M : (size_t)(k0 + k) + (size_t)(r0 + r) * M;
+          Ls[buf][k][r] = in ? A[at] : 0.0;
+        }
+      };
+      // eight finished values, zeros from kend on
+      auto ahead = [&](int k0, double (&v)[kSolveAhead]) {
+#pragma unroll
+        for (int u = 0; u < kSolveAhead; u++) v[u] = k0 + u < kend ? y[(size_t)(k0 + u) * rs] : 0.0;
+      };
+      double x[32];
+#pragma unroll
+      for (int r = 0; r < 32; r++) {
+        if (pass == 0) x[r] = r >= nr ? 0.0 : kUnit ? (r0 + r == i ? 1.0 : 0.0) : b[(size_t)(r0 + r) * ldN];
+        else x[r] = r < nr ? y[(size_t)(r0 + r) * rs] : 0.0;
+      }
+      int buf = 0;
+      double next[kSolveAhead];
+      if (kbeg < kend) {
+        stage(kbeg, 0);
+        ahead(kbeg, next);
+      }
+      for (int k0 = kbeg; k0 < kend; k0 += 32, buf ^= 1) {
+        __syncthreads();
+        if (k0 + 32 < kend) stage(k0 + 32, buf ^ 1);
+#pragma unroll 1
+        for (int k = 0; k < 32; k += kSolveAhead) {
+          double v[kSolveAhead];
+#pragma unroll
+          for (int u = 0; u < kSolveAhead; u++) v[u] = next[u];
+          ahead(k0 + k + kSolveAhead, next);
+#pragma unroll
+          for (int u = 0; u < kSolveAhead; u++) {
+            const double2* l = reinterpret_cast<const double2*>(Ls[buf][k + u]);
+#pragma unroll
+            for (int r = 0; r < 16; r++) {
+              const double2 w = l[r];
+              x[2 * r] = fma(-w.x, v[u], x[2 * r]);
+              x[2 * r + 1] = fma(-w.y, v[u], x[2 * r + 1]);
+            }
+          }
+        }
+      }
+      // the 32 x 32 diagonal block: Ls[0][k][r] = L[r][k], k < r (forward), or L[k][r], k > r (backward)
+      __syncthreads();
+      for (int e = tid; e < 1024; e += kSolveCells) {
+        const int r = pass == 0 ? e & 31 : e >> 5, k = pass == 0 ? e >> 5 : e & 31;
+        const bool in = r < nr && k < nr && (pass == 0 ? r > k : k > r);
+        const size_t at = pass == 0 ? (size_t)(r0 + r) + (size_t)(r0 + k) * M : (size_t)(r0 + k) + (size_t)(r0 + r) * M;
+        Ls[0][k][r] = in ? A[at] : 0.0;
+      }
+      if (tid < 32) {
+        const double v = tid < nr ? A[(size_t)(r0 + tid) * (M + 1)] : 1.0;
+        Rd[tid] = kExact ? v : 1.0 / v;
+      }
+      __syncthreads();
+      if (kExact && pass == 0) {
+#pragma unroll
+        for (int r = 0; r < 32; r++) {
+          if (r < nr) {
+#pragma unroll
+            for (int k = r - 1; k >= 0; k--) x[r] = __dsub_rn(x[r], __dmul_rn(Ls[0][k][r], x[k]));
+            x[r] = __ddiv_rn(x[r], Rd[r]);
+          }
+        }
+      } else if (kExact) {
+#pragma unroll
+        for (int r = 31; r >= 0; r--) {
+          if (r < nr) {
+#pragma unroll
+            for (int k = r + 1; k < 32; k++)
+              if (k < nr) x[r] = __dsub_rn(x[r], __dmul_rn(Ls[0][k][r], x[k]));
+            x[r] = __ddiv_rn(x[r], Rd[r]);
+          }
+        }
+      } else if (pass == 0) {
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+          x[k] *= Rd[k];
+#pragma unroll
+          for (int r = k + 1; r < 32; r++) x[r] = fma(-Ls[0][k][r], x[k], x[r]);
+        }
+      } else {
+#pragma unroll
+        for (int k = 31; k >= 0; k--) {
+          x[k] *= Rd[k];
+#pragma unroll
+          for (int r = 0; r < k; r++) x[r] = fma(-Ls[0][k][r], x[k], x[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 32; r++)
+        if (r < nr && on) y[(size_t)(r0 + r) * rs] = x[r];
+      __syncthreads();  // Ls is refilled
+    }
+  }
+  if (!kUnit && on) {
+    for (int k = 0; k < M; k++) d = __dadd_rn(d, __dmul_rn(b[(size_t)k * ldN], y[(size_t)k * rs]));
+    titsias[i] = (1.0 - d) / 2.0;
+  }
+}
+
+int launch_cholinv(Ctx* c, const double* L, int n, double* out) {
+  auto fn = n <= 32 ? k_kmm_solve<true, true> : k_kmm_solve<true, false>;
+  fn<<<div_up(n, kSolveCells), kSolveCells, 0, c->stream>>>(n, n, n, L, nullptr, out, nullptr);
+  GPL_LAUNCHED(c, "k_kmm_solve");
+  return GPL_OK;
 }
 
 __global__ void k_expand(int P, int p, int g0, int M, const int* __restrict__ mk, const double* __restrict__ delta,
@@ -133,8 +256,10 @@ int launch_kernel_mats_lv(Ctx* c, int lv) {
   int rc = launch_chol_single(c, c->Kinv, c->M);
   if (rc) return rc;
   ProfScope ps(c, "kinvkmn");
-  k_kinvkmn<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn, c->titsias);
-  GPL_LAUNCHED(c, "k_kinvkmn");
+  auto fn = c->M <= 32 ? k_kmm_solve<false, true> : k_kmm_solve<false, false>;
+  fn<<<div_up(c->N, kSolveCells), kSolveCells, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
+                                                               c->titsias);
+  GPL_LAUNCHED(c, "k_kmm_solve");
   return GPL_OK;
 }
 
@@ -165,8 +290,10 @@ int launch_kernel_mats_raw(cudaStream_t st, int N, int M, int Q, const double* X
   e = launch_chol_exact_raw(st, Lwork, M);
   if (e != cudaSuccess) return (int)e;
   const double* L = Lwork;
-  void* a_kk[] = {&N, &ldN, &M, &L, &Knm, &KinvKmn, &titsias};
-  e = cudaLaunchKernel((const void*)k_kinvkmn, dim3(div_up(N, 128)), dim3(128), a_kk, 0, st);
+  int64_t ld = N;
+  void* a_kk[] = {&N, &ld, &M, &L, &Knm, &KinvKmn, &titsias};
+  auto fn = M <= 32 ? k_kmm_solve<false, true> : k_kmm_solve<false, false>;
+  e = cudaLaunchKernel((const void*)fn, dim3(div_up(N, kSolveCells)), dim3(kSolveCells), a_kk, 0, st);
   return (int)e;
 }
 

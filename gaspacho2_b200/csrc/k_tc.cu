@@ -798,7 +798,7 @@ int launch_tc_gram(Ctx* c) {
     dim3 g(div_up(c->n_d, 128), c->n_d);
     k_gather_dinv<<<g, 128, 0, c->stream>>>(c->n_d, c->P, c->dcol_d, c->DeltaInv, t.Lw);
     GPL_LAUNCHED(c, "k_gather_dinv");
-    launch_chol_exact_raw(c->stream, t.Lw, c->n_d);
+    launch_chol_exact_raw(c->stream, t.Lw, c->n_d, c->dg0);
     GPL_LAUNCHED(c, "k_chol_exact");
     k_whiten_rows<<<t.cpad / 128, 128, t.smem_whiten, c->stream>>>(c->N, c->ldN, c->n_d, t.cpad, c->Dm, t.Lw,
                                                                     t.DtC, t.DwC);
