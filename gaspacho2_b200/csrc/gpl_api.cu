@@ -107,7 +107,7 @@ static void free_state(Ctx* c) {
                   c->X,      c->T,      c->rho,     c->phi,     c->ls,     c->lkhds,  c->lkhd_dev, c->grad,
                   c->grad0,  c->ss,     c->SS,      c->XX,      c->gdtmp,  c->C1,     c->C2,     c->grtmp,
                   c->KmmInv, c->bvec,   c->sol,     c->red,     c->lb_work, c->mc_d,  c->mv_d,   c->mk_d,
-                  c->nh_d,   c->rres,   c->bx,      c->rphi,    c->e0,      c->zeta};
+                  c->nh_d,   c->rres,   c->bx,      c->rphi,    c->e0,      c->zeta,  c->state_sums};
   for (void* p : bufs)
     if (p) cudaFree(p);
   c->Z = c->W = c->Nu = c->Psi = c->PsiInv = c->Beta = c->tBeta = c->scratch = c->U = nullptr;
@@ -115,7 +115,7 @@ static void free_state(Ctx* c) {
   c->rho = c->phi = c->ls = c->lkhds = c->lkhd_dev = c->grad = c->grad0 = c->ss = c->SS = c->XX = nullptr;
   c->gdtmp = c->C1 = c->C2 = c->grtmp = c->KmmInv = c->bvec = c->sol = c->red = c->lb_work = nullptr;
   c->mc_d = c->mv_d = c->mk_d = c->nh_d = nullptr;
-  c->rres = c->bx = c->rphi = c->e0 = c->zeta = nullptr;
+  c->rres = c->bx = c->rphi = c->e0 = c->zeta = c->state_sums = nullptr;
   c->have_design = false;
 }
 
@@ -1011,7 +1011,8 @@ int gpl_load_design(gpl_ctx* h, int N, int n_var, const int32_t* cv, const int32
   GPL_RUN(dalloc(c, &c->ss, (size_t)c->tot_max + Q, "ss"));
   GPL_RUN(dalloc(c, &c->SS, (size_t)c->tot_max * kHist, "SS"));
   GPL_RUN(dalloc(c, &c->XX, (size_t)c->tot_max * kHist, "XX"));
-  GPL_RUN(dalloc(c, &c->gdtmp, (size_t)P * J, "gdtmp"));
+  GPL_RUN(dalloc(c, &c->gdtmp, (size_t)p * J, "gdtmp"));
+  GPL_RUN(dalloc(c, &c->state_sums, 3 * kStateParts, "sums over cells"));
   GPL_RUN(dalloc(c, &c->C1, ldN * M, "C1"));
   GPL_RUN(dalloc(c, &c->cellfac, 3 * ldN, "per-cell factors of W"));
   GPL_RUN(dalloc(c, &c->C2, (size_t)M * M, "C2"));

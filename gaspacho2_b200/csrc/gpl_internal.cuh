@@ -40,6 +40,7 @@ constexpr double kIgap1 = 100;  // inverse-gamma prior shape+1 on Omega (ggplvm.
 constexpr double kIgb = 100;    // inverse-gamma prior scale on Omega (ggplvm.cu:22)
 constexpr int kHist = 10;       // L-BFGS memory (ggplvm.cu:872)
 constexpr int kLkhdSlots = 50000;
+constexpr int kStateParts = 64; // partial sums of each of the shared sums over cells (k_sums.cu)
 
 struct Ctx;
 
@@ -206,6 +207,7 @@ struct Ctx {
   double *Omega = nullptr, *delta = nullptr, *X = nullptr, *T = nullptr, *rho = nullptr, *phi = nullptr;
   double *ls = nullptr, *lkhds = nullptr, *lkhd_dev = nullptr;
   double *grad = nullptr, *grad0 = nullptr, *ss = nullptr, *SS = nullptr, *XX = nullptr;
+  double* state_sums = nullptr;  // 3 x kStateParts: log Omega, 1/Omega, Oinvt titsias
   double *gdtmp = nullptr, *C1 = nullptr, *C2 = nullptr, *grtmp = nullptr, *KmmInv = nullptr;
   double *bvec = nullptr;     // P x J right-hand sides Z^T diag(W/Omega) nu
   double *sol = nullptr;      // P x J solutions Psi^{-1} bvec
@@ -336,7 +338,8 @@ void pair_release(Ctx* c);
 int pair_prepare(Ctx* c);                 // column-pair list, 1/Omega, gathered S pairs, V rows
 int recip_omega(Ctx* c, const double** rOm);  // 1/Omega (0 past N), refreshed on every call
 int dgen_zt_u(Ctx* c, int mode, const double* u, double* out);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);
-int dgen_c1_tn(Ctx* c);                   // GPL_ERR_ARG when the dense columns exceed one tile
+int dgen_c1_tn(Ctx* c);
+int dgen_c2(Ctx* c);                      // C2 (M x M adjoint of Kmm) up to its final combination
 int dgen_group_sums(Ctx* c, int mode);
 int dgen_unweighted_gram(Ctx* c);         // the dense block of Psi_0 with every weight 1 (GLM initialisation)
 int dgen_hk(Ctx* c);
@@ -366,8 +369,13 @@ int init_latent(Ctx* c, int pca_iters, int kmeans_iters, uint64_t seed, double* 
 int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* stats);
 int cell_objective(Ctx* c, const double* X_host, double* obj_host, double* grad_host);
 void tc_release(Ctx* c);
-// k_lkhd.cu
+// k_sums.cu
 int launch_oinvt(Ctx* c);
+int launch_tn_sum(Ctx* c, const double* E, double* out);  // per cell: the gradient's sum over genes
+size_t cell_sums_part(const Ctx* c);      // values of c->part that the sums per cell take
+int launch_state_sums(Ctx* c);            // state_sums at the current Omega, Oinvt and titsias
+int ensure_part(Ctx* c, size_t n);        // the split sums' buffer (c->part), at least n values (k_dgen.cu)
+// k_lkhd.cu
 int launch_beta_phi(Ctx* c, int jtr);
 int launch_lkhd_pois(Ctx* c);
 int launch_lkhd_genes(Ctx* c);

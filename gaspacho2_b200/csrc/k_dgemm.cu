@@ -409,9 +409,12 @@ int pair_prepare(Ctx* c) {
   // more dense columns than k_v_to_u stages per cell: k_v_to_u_wide reads the V rows from
   // global memory instead
   s.wide = s.smem_vu > 200 * 1024;
-  // the integer form (k_crt.cu) keeps its operands in the same buffer
-  crt_plan(c, (size_t)8 << 30);
-  const size_t v_bytes = std::max(sizeof(double) * (size_t)s.v_cells * s.pairs_pad, s.crt.bytes);
+  // the integer form (k_crt.cu) keeps its operands in the same buffer, of 1 GiB at least: with 14 bytes
+  // per operand entry it takes the cells in a few ranges where the DMMA form takes one, which costs it
+  // less than a larger buffer costs a new context (about 10 ms per GiB)
+  const size_t dmma_bytes = sizeof(double) * (size_t)s.v_cells * s.pairs_pad;
+  crt_plan(c, std::max(dmma_bytes, (size_t)1 << 30));
+  const size_t v_bytes = std::max(dmma_bytes, s.crt.bytes);
   if (cudaMalloc((void**)&s.pairs, sizeof(int2) * pairs.size()) != cudaSuccess ||
       cudaMalloc((void**)&s.rOm, sizeof(double) * s.cpad) != cudaSuccess ||
       cudaMalloc((void**)&s.Sp, sizeof(double) * (size_t)c->J * s.pairs_pad) != cudaSuccess ||

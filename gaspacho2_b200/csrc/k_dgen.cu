@@ -22,6 +22,7 @@
 // [k][m] and [k][n] with rows padded to 4 mod 16 doubles (conflict-free fragment loads).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "dmma_common.cuh"
 #include "gpl_internal.cuh"
@@ -350,8 +351,13 @@ static int launch_dgen(Ctx* c, dim3 grid, int m, int n, LA A, LB B, KR kr, Epi e
   return GPL_OK;
 }
 
-static int ensure_part(Ctx* c, size_t n) {
+static size_t part_bound(const Ctx* c);
+
+// The buffer of the split sums. Its first use sizes it for every phase of the context (part_bound), so
+// that later phases neither free nor allocate; a larger request grows it.
+int ensure_part(Ctx* c, size_t n) {
   if (c->part_n >= n) return GPL_OK;
+  n = std::max(n, part_bound(c));
   graph_reset(c);
   if (c->part) cudaFree(c->part);
   c->part = nullptr;
@@ -391,36 +397,47 @@ static int split_count(int tiles, int sms) {
 // (gene tile, cell range z) writes its partial sums to part[z][a][j]. MODE 0: B = W u / Omega
 // (u cells x genes); 1: B = u; 2: B = W g / Omega with g one value per cell. The cell ranges
 // start at even cells, so every 16-byte copy is aligned (ldN is a multiple of 32).
+// The dense columns are taken in row tiles of MT x 16 (grid x): one tile of the least MT in {1, 3, 5, 9}
+// that holds them, 144-row tiles beyond that.
 namespace {
 constexpr int kZtBK = 16, kZtS = kZtBK + 4;  // slice depth; row stride, 4 mod 16 doubles
-constexpr int kZtBM = 144, kZtBN = 128, kZtStages = 3;
-constexpr int kZtStage = kZtBM * kZtS + 2 * kZtBN * kZtS + 2 * kZtBK;  // doubles per stage
-constexpr int kZtSmem = (int)sizeof(double) * kZtStages * kZtStage;
+constexpr int kZtBN = 128, kZtStages = 3;
+constexpr int zt_stage(int mt) { return mt * 16 * kZtS + 2 * kZtBN * kZtS + 2 * kZtBK; }  // doubles per stage
+constexpr int zt_smem(int mt) { return (int)sizeof(double) * kZtStages * zt_stage(mt); }
+// calls f with the row tile's MT as a constant
+template <class F>
+int with_row_tiles(int rows, F f) {
+  if (rows <= 16) return f(std::integral_constant<int, 1>());
+  if (rows <= 48) return f(std::integral_constant<int, 3>());
+  if (rows <= 80) return f(std::integral_constant<int, 5>());
+  return f(std::integral_constant<int, 9>());
+}
 }  // namespace
 
-template <int MODE>
+template <int MODE, int MT>
 __global__ void __launch_bounds__(256, 1)
     k_zt_u(int m, int n, int N, int ldN, int per, const double* __restrict__ D, const double* __restrict__ W,
            const double* __restrict__ U, const double* __restrict__ rOm, double* __restrict__ part) {
   extern __shared__ __align__(16) double zs[];
   const int tid = threadIdx.x, wn = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.y * kZtBN, z = blockIdx.z;
+  constexpr int kRows = MT * 16, kStage = zt_stage(MT);
+  const int m0 = blockIdx.x * kRows, n0 = blockIdx.y * kZtBN, z = blockIdx.z;
   const int kbeg = min(N, z * per), kend = min(N, (z + 1) * per);
   const int nsl = kend > kbeg ? (kend - kbeg + kZtBK - 1) / kZtBK : 0;
 
   // slice s into stage st; a pair of cells past the range is zero-filled (8 bytes of a pair
   // whose second cell is past it), its source clamped into the matrix
   auto load = [&](int s, int st) {
-    double* As = zs + st * kZtStage;
-    double* Ws = As + kZtBM * kZtS;
+    double* As = zs + st * kStage;
+    double* Ws = As + kRows * kZtS;
     double* Us = Ws + kZtBN * kZtS;
     double* Rs = Us + kZtBN * kZtS;
     double* Vs = Rs + kZtBK;
     const int k0 = kbeg + s * kZtBK;
-    for (int ch = tid; ch < kZtBM * (kZtBK / 2); ch += 256) {
+    for (int ch = tid; ch < kRows * (kZtBK / 2); ch += 256) {
       const int r = ch >> 3, kc = (ch & 7) * 2, k = k0 + kc;
-      const int nb = (r < m && k < kend) ? (k + 1 < kend ? 16 : 8) : 0;
-      cp_async16(As + r * kZtS + kc, D + (size_t)min(r, m - 1) * ldN + min(k, ldN - 2), nb);
+      const int nb = (m0 + r < m && k < kend) ? (k + 1 < kend ? 16 : 8) : 0;
+      cp_async16(As + r * kZtS + kc, D + (size_t)min(m0 + r, m - 1) * ldN + min(k, ldN - 2), nb);
     }
 #pragma unroll
     for (int q = 0; q < (kZtBN * (kZtBK / 2)) / 256; q++) {
@@ -438,9 +455,9 @@ __global__ void __launch_bounds__(256, 1)
     }
   };
 
-  double acc[9][2][4];
+  double acc[MT][2][4];
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int y = 0; y < 2; y++)
 #pragma unroll
@@ -454,17 +471,17 @@ __global__ void __launch_bounds__(256, 1)
     __syncthreads();     // and every warp is done with slice s - 1, whose stage is refilled next
     if (s + 2 < nsl) load(s + 2, (s + 2) % kZtStages);
     cp_async_commit();
-    const double* As = zs + (s % kZtStages) * kZtStage;
-    const double* Ws = As + kZtBM * kZtS;
+    const double* As = zs + (s % kZtStages) * kStage;
+    const double* Ws = As + kRows * kZtS;
     const double* Us = Ws + kZtBN * kZtS;
     const double* Rs = Us + kZtBN * kZtS;
     const double* Vs = Rs + kZtBK;
 #pragma unroll
     for (int k4 = 0; k4 < kZtBK / 4; k4++) {
       const int kk = k4 * 4 + t;
-      double a[9][2], b[2];
+      double a[MT][2], b[2];
 #pragma unroll
-      for (int x = 0; x < 9; x++) {
+      for (int x = 0; x < MT; x++) {
         a[x][0] = As[(x * 16 + g) * kZtS + kk];
         a[x][1] = As[(x * 16 + g + 8) * kZtS + kk];
       }
@@ -474,17 +491,17 @@ __global__ void __launch_bounds__(256, 1)
         b[y] = MODE == 1 ? Us[e] : MODE == 0 ? Ws[e] * Rs[kk] * Us[e] : Ws[e] * Rs[kk] * Vs[kk];
       }
 #pragma unroll
-      for (int x = 0; x < 9; x++)
+      for (int x = 0; x < MT; x++)
 #pragma unroll
         for (int y = 0; y < 2; y++) dmma_16x8x4(acc[x][y], a[x][0], a[x][1], b[y]);
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int r = x * 16 + g + 8 * h;
+      const int r = m0 + x * 16 + g + 8 * h;
       if (r >= m) continue;
 #pragma unroll
       for (int y = 0; y < 2; y++)
@@ -496,28 +513,35 @@ __global__ void __launch_bounds__(256, 1)
     }
 }
 
+static int zt_splits(const Ctx* c, int rows) {
+  return split_count(div_up(c->J, kZtBN) * div_up(c->n_d, rows), c->sm_count);
+}
+
 int dgen_zt_u(Ctx* c, int mode, const double* u, double* out) {
-  if (c->n_d > kZtBM) return GPL_ERR_ARG;
+  if (mode == 2 && c->n_d > 144) return GPL_ERR_ARG;
   const double* rOm = nullptr;
   if (mode != 1) {
     int rc = recip_omega(c, &rOm);
     if (rc) return rc;
   }
-  const int tiles = div_up(c->J, kZtBN);
-  const int S = split_count(tiles, c->sm_count);
-  int rc = ensure_part(c, (size_t)S * c->n_d * c->J);
-  if (rc) return rc;
-  int per = (c->N + S - 1) / S;
-  per += per & 1;  // even range starts: aligned 16-byte copies
-  dim3 g(1, tiles, S);
-  auto* fn = mode == 0 ? k_zt_u<0> : mode == 1 ? k_zt_u<1> : k_zt_u<2>;
-  GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kZtSmem));
-  fn<<<g, 256, kZtSmem, c->stream>>>(c->n_d, c->J, c->N, c->ldN, per, c->Dm, c->W, u, rOm, c->part);
-  GPL_LAUNCHED(c, "k_zt_u");
-  dim3 g2(div_up(c->J, 256), c->n_d);
-  k_reduce_bvec<<<g2, 256, 0, c->stream>>>(c->n_d, c->J, c->P, S, c->dcol_d, c->part, out);
-  GPL_LAUNCHED(c, "k_reduce_bvec");
-  return GPL_OK;
+  return with_row_tiles(c->n_d, [&](auto mt) -> int {
+    constexpr int MT = decltype(mt)::value;
+    const int tiles = div_up(c->J, kZtBN), mtiles = div_up(c->n_d, MT * 16);
+    const int S = zt_splits(c, MT * 16);
+    int rc = ensure_part(c, (size_t)S * c->n_d * c->J);
+    if (rc) return rc;
+    int per = (c->N + S - 1) / S;
+    per += per & 1;  // even range starts: aligned 16-byte copies
+    auto* fn = mode == 0 ? k_zt_u<0, MT> : mode == 1 ? k_zt_u<1, MT> : k_zt_u<2, MT>;
+    GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
+    fn<<<dim3(mtiles, tiles, S), 256, zt_smem(MT), c->stream>>>(c->n_d, c->J, c->N, c->ldN, per, c->Dm, c->W, u, rOm,
+                                                               c->part);
+    GPL_LAUNCHED(c, "k_zt_u");
+    dim3 g2(div_up(c->J, 256), c->n_d);
+    k_reduce_bvec<<<g2, 256, 0, c->stream>>>(c->n_d, c->J, c->P, S, c->dcol_d, c->part, out);
+    GPL_LAUNCHED(c, "k_reduce_bvec");
+    return GPL_OK;
+  });
 }
 
 // C1 over S gene ranges (S = 1..4, the count whose CTAs fill their last wave best: 3 at config
@@ -531,13 +555,8 @@ __global__ void k_reduce_parts_ld(int m, int n, int nz, const double* __restrict
   out[r + (size_t)cc * ld] = s;
 }
 
-int dgen_c1_tn(Ctx* c) {
-  using T = TileSq;
-  const double* rOm = nullptr;
-  int rc = recip_omega(c, &rOm);
-  if (rc) return rc;
-  const int g0 = c->nh[c->p - 1];
-  const int tiles = div_up(c->N, T::BM) * div_up(c->M, T::BN);
+static int c1_splits(const Ctx* c) {
+  const int tiles = div_up(c->N, TileSq::BM) * div_up(c->M, TileSq::BN);
   int S = 1;
   double best = 0.0;
   for (int z = 1; z <= 4; z++) {
@@ -547,6 +566,16 @@ int dgen_c1_tn(Ctx* c) {
       S = z;
     }
   }
+  return S;
+}
+
+int dgen_c1_tn(Ctx* c) {
+  using T = TileSq;
+  const double* rOm = nullptr;
+  int rc = recip_omega(c, &rOm);
+  if (rc) return rc;
+  const int g0 = c->nh[c->p - 1];
+  const int S = c1_splits(c);
   LdTn A{c->W, c->Nu, c->scratch, rOm, c->rphi, c->ldN};
   LdTBetaGP B{c->tBeta, c->P, g0};
   if (S == 1) {
@@ -569,27 +598,33 @@ int dgen_c1_tn(Ctx* c) {
 // through a three-stage cp.async pipeline of the raw operands, 8-byte copies (a group starts at
 // any cell): the dense columns [a][cell] from their group-ordered copy, W's group-ordered values
 // [gene][cell] and 1/Omega [cell]; w formed at the fragment loads, the same product in the same
-// order as the register-staged form, so the sums are TileTall's.
-template <int MODE>
+// order as the register-staged form. With few groups the group's cells are split into ns runs of
+// whole slices (grid z = group x ns) whose partial sums part[z][j][a] k_reduce_groups adds in order:
+// 4 groups of 20,000 cells x 2,000 genes (68 columns) took 0.94 ms as 64 blocks, 0.17 ms split.
+template <int MODE, int MT>
 __global__ void __launch_bounds__(256, 1)
-    k_group_sums_dmma(int m, int n, int n_grp, int ldN, const int* __restrict__ gstart, const double* __restrict__ Dg,
-                      const double* __restrict__ Wg, const double* __restrict__ rOmg, double* __restrict__ S) {
+    k_group_sums_dmma(int m, int n, int n_grp, int ns, int ldN, const int* __restrict__ gstart,
+                      const double* __restrict__ Dg, const double* __restrict__ Wg, const double* __restrict__ rOmg,
+                      double* __restrict__ S, double* __restrict__ part) {
   extern __shared__ __align__(16) double zs[];
   const int tid = threadIdx.x, wn = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.y * kZtBN, z = blockIdx.z;
-  const int kbeg = gstart[z], kend = gstart[z + 1];
+  constexpr int kRows = MT * 16, kStage = zt_stage(MT);
+  const int m0 = blockIdx.x * kRows, n0 = blockIdx.y * kZtBN, z = blockIdx.z, grp = z / ns, c = z - grp * ns;
+  const int g0 = gstart[grp], g1 = gstart[grp + 1];
+  const int per = ((g1 - g0 + kZtBK - 1) / kZtBK + ns - 1) / ns * kZtBK;  // cells per run
+  const int kbeg = min(g1, g0 + c * per), kend = min(g1, kbeg + per);
   const int nsl = kend > kbeg ? (kend - kbeg + kZtBK - 1) / kZtBK : 0;
   const int last = max(kend - 1, 0);  // a cell of the matrix, for the sources of zero-fill copies
 
   auto load = [&](int s, int st) {
-    double* As = zs + st * kZtStage;
-    double* Ws = As + kZtBM * kZtS;
+    double* As = zs + st * kStage;
+    double* Ws = As + kRows * kZtS;
     double* Rs = Ws + 2 * kZtBN * kZtS;
     const int k0 = kbeg + s * kZtBK;
-    for (int e = tid; e < kZtBM * kZtBK; e += 256) {
+    for (int e = tid; e < kRows * kZtBK; e += 256) {
       const int r = e >> 4, kc = e & 15, k = k0 + kc;
-      const int nb = (r < m && k < kend) ? 8 : 0;
-      cp_async8(As + r * kZtS + kc, Dg + (size_t)min(r, m - 1) * ldN + min(k, last), nb);
+      const int nb = (m0 + r < m && k < kend) ? 8 : 0;
+      cp_async8(As + r * kZtS + kc, Dg + (size_t)min(m0 + r, m - 1) * ldN + min(k, last), nb);
     }
     if (MODE == 0) {
 #pragma unroll
@@ -605,9 +640,9 @@ __global__ void __launch_bounds__(256, 1)
     }
   };
 
-  double acc[9][2][4];
+  double acc[MT][2][4];
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int y = 0; y < 2; y++)
 #pragma unroll
@@ -621,16 +656,16 @@ __global__ void __launch_bounds__(256, 1)
     __syncthreads();     // and every warp is done with slice s - 1, whose stage is refilled next
     if (s + 2 < nsl) load(s + 2, (s + 2) % kZtStages);
     cp_async_commit();
-    const double* As = zs + (s % kZtStages) * kZtStage;
-    const double* Ws = As + kZtBM * kZtS;
+    const double* As = zs + (s % kZtStages) * kStage;
+    const double* Ws = As + kRows * kZtS;
     const double* Rs = Ws + 2 * kZtBN * kZtS;
     const int live = kend - (kbeg + s * kZtBK);  // cells of this slice in the group
 #pragma unroll
     for (int k4 = 0; k4 < kZtBK / 4; k4++) {
       const int kk = k4 * 4 + t;
-      double a[9][2], b[2];
+      double a[MT][2], b[2];
 #pragma unroll
-      for (int x = 0; x < 9; x++) {
+      for (int x = 0; x < MT; x++) {
         a[x][0] = As[(x * 16 + g) * kZtS + kk];
         a[x][1] = As[(x * 16 + g + 8) * kZtS + kk];
       }
@@ -640,30 +675,48 @@ __global__ void __launch_bounds__(256, 1)
         b[y] = MODE == 0 ? Ws[e] * Rs[kk] : (kk < live && n0 + wn * 16 + y * 8 + g < n ? 1.0 * 1.0 : 0.0);
       }
 #pragma unroll
-      for (int x = 0; x < 9; x++)
+      for (int x = 0; x < MT; x++)
 #pragma unroll
         for (int y = 0; y < 2; y++) dmma_16x8x4(acc[x][y], a[x][0], a[x][1], b[y]);
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int r = x * 16 + g + 8 * h;
+      const int r = m0 + x * 16 + g + 8 * h;
       if (r >= m) continue;
 #pragma unroll
       for (int y = 0; y < 2; y++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           const int j = n0 + wn * 16 + y * 8 + 2 * t + e;
-          if (j < n) S[((size_t)j * n_grp + z) * (m + 1) + r] = acc[x][y][2 * h + e];
+          if (j >= n) continue;
+          if (ns == 1) S[((size_t)j * n_grp + grp) * (m + 1) + r] = acc[x][y][2 * h + e];
+          else part[((size_t)z * n + j) * m + r] = acc[x][y][2 * h + e];
         }
     }
 }
 
+// S[j][g][a] = sum over the runs c of part[g ns + c][j][a]
+__global__ void k_reduce_groups(int m, int n, int n_grp, int ns, const double* __restrict__ part,
+                                double* __restrict__ S) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (int64_t)n * m) return;
+  const int grp = blockIdx.y, j = (int)(e / m), a = (int)(e - (int64_t)j * m);
+  double s = 0.0;
+  for (int c = 0; c < ns; c++) s += part[(size_t)(grp * ns + c) * n * m + e];
+  S[((size_t)j * n_grp + grp) * (m + 1) + a] = s;
+}
+
+static int group_runs(const Ctx* c, int J, int rows) {
+  const int tiles = div_up(J, kZtBN) * div_up(c->n_d, rows) * c->n_grp;
+  // runs of at least 128 cells on average, up to four blocks per SM
+  return std::max(1, std::min(4 * c->sm_count / tiles, c->N / (c->n_grp * 128)));
+}
+
 int dgen_group_sums(Ctx* c, int mode) {
-  if (c->n_d > kZtBM) return GPL_ERR_ARG;
   int rc;
   if (mode == 0) {
     const double* rOm = nullptr;
@@ -672,12 +725,25 @@ int dgen_group_sums(Ctx* c, int mode) {
   }
   if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
   const int J = mode == 1 ? 1 : c->J;
-  dim3 g(1, div_up(J, kZtBN), c->n_grp);
-  auto* fn = mode == 0 ? k_group_sums_dmma<0> : k_group_sums_dmma<1>;
-  GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kZtSmem));
-  fn<<<g, 256, kZtSmem, c->stream>>>(c->n_d, J, c->n_grp, c->ldN, c->gstart_d, c->Dg, c->Wg, c->rOmg, c->gsum);
-  GPL_LAUNCHED(c, "k_group_sums_dmma");
-  return GPL_OK;
+  return with_row_tiles(c->n_d, [&](auto mt) -> int {
+    constexpr int MT = decltype(mt)::value;
+    const int ns = group_runs(c, J, MT * 16);
+    if (ns > 1) {
+      const int rp = ensure_part(c, (size_t)c->n_grp * ns * J * c->n_d);
+      if (rp) return rp;
+    }
+    auto* fn = mode == 0 ? k_group_sums_dmma<0, MT> : k_group_sums_dmma<1, MT>;
+    GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
+    fn<<<dim3(div_up(c->n_d, MT * 16), div_up(J, kZtBN), c->n_grp * ns), 256, zt_smem(MT), c->stream>>>(
+        c->n_d, J, c->n_grp, ns, c->ldN, c->gstart_d, c->Dg, c->Wg, c->rOmg, c->gsum, c->part);
+    GPL_LAUNCHED(c, "k_group_sums_dmma");
+    if (ns > 1) {
+      k_reduce_groups<<<dim3(div_up((int64_t)J * c->n_d, 256), c->n_grp), 256, 0, c->stream>>>(c->n_d, J, c->n_grp, ns,
+                                                                                             c->part, c->gsum);
+      GPL_LAUNCHED(c, "k_reduce_groups");
+    }
+    return GPL_OK;
+  });
 }
 
 // HK[i, a] = sum_j O_ij tab[j][g(i)][a] for the 128 cell slots of each group tile (grid z =
@@ -685,45 +751,52 @@ int dgen_group_sums(Ctx* c, int mode) {
 // the group's table rows tab[j][g][0..ld) ([gene][a]) and W's group-ordered values of the tile's
 // slots ([gene][slot]), by 8-byte copies (neither row starts at an even offset in general);
 // 1/Omega of the slots is read once. The B operand W (1/Omega) is formed at the fragment loads,
-// the same product in the same order as the register-staged form, so the sums are TileTall's.
+// the same product in the same order as the register-staged form. Table rows in tiles of MT x 16
+// (grid x); with few cell tiles, or a last wave that would be nearly empty, the genes are split into
+// ns ranges (grid y) whose partial sums part[s][r][slot] k_reduce_hk adds in order: 157 tiles on 148
+// SMs (20,000 cells, 2,000 genes, 69 rows) took 0.82 ms, 0.27 ms split.
 namespace {
-constexpr int kHkBK = 16, kHkSA = 148, kHkSB = 132, kHkStages = 4;  // row strides 4 mod 16
-constexpr int kHkStage = kHkBK * kHkSA + kHkBK * kHkSB;             // doubles per stage
-constexpr int kHkSmem = (int)sizeof(double) * (kHkStages * kHkStage + 128);
+constexpr int kHkBK = 16, kHkSB = 132, kHkStages = 4;         // row strides 4 mod 16
+constexpr int hk_sa(int mt) { return mt * 16 + 4; }
+constexpr int hk_stage(int mt) { return kHkBK * hk_sa(mt) + kHkBK * kHkSB; }  // doubles per stage
+constexpr int hk_smem(int mt) { return (int)sizeof(double) * (kHkStages * hk_stage(mt) + 128); }
 }  // namespace
 
+template <int MT>
 __global__ void __launch_bounds__(256, 1)
-    k_hk(int ld, int J, int n_grp, int ldN, const double* __restrict__ tab, const int2* __restrict__ tiles,
+    k_hk(int ld, int J, int jper, int n_grp, int ldN, const double* __restrict__ tab, const int2* __restrict__ tiles,
          const double* __restrict__ Wg, const double* __restrict__ rOmg, const int* __restrict__ pos,
-         const int* __restrict__ cells, double* __restrict__ HK) {
+         const int* __restrict__ cells, double* __restrict__ HK, double* __restrict__ part) {
+  constexpr int kRows = MT * 16, kHkSA = hk_sa(MT), kHkStage = hk_stage(MT);
   extern __shared__ __align__(16) double hs[];
   double* Rs = hs + kHkStages * kHkStage;  // [128] 1/Omega of the slots, 0 past the group
   const int tid = threadIdx.x, wn = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int z = blockIdx.z, grp = tiles[z].x;
+  const int m0 = blockIdx.x * kRows, sp = blockIdx.y, z = blockIdx.z, grp = tiles[z].x;
+  const int j_beg = sp * jper, j_end = min(J, j_beg + jper);
   const int myq = pos[(size_t)z * 128 + (tid & 127)];  // this thread's slot in every B copy
   if (tid < 128) Rs[tid] = myq < 0 ? 0.0 : rOmg[myq];
-  const int nsl = (J + kHkBK - 1) / kHkBK;
+  const int nsl = j_end > j_beg ? (j_end - j_beg + kHkBK - 1) / kHkBK : 0;
 
   auto load = [&](int s, int st) {
     double* As = hs + st * kHkStage;
     double* Bs = As + kHkBK * kHkSA;
-    const int k0 = s * kHkBK;
-    for (int e = tid; e < kHkBK * 144; e += 256) {
-      const int k = e / 144, r = e - k * 144, j = k0 + k;
-      const int nb = (r < ld && j < J) ? 8 : 0;
-      cp_async8(As + k * kHkSA + r, tab + ((size_t)min(j, J - 1) * n_grp + grp) * ld + min(r, ld - 1), nb);
+    const int k0 = j_beg + s * kHkBK;
+    for (int e = tid; e < kHkBK * kRows; e += 256) {
+      const int k = e / kRows, r = e - k * kRows, j = k0 + k;
+      const int nb = (m0 + r < ld && j < j_end) ? 8 : 0;
+      cp_async8(As + k * kHkSA + r, tab + ((size_t)min(j, J - 1) * n_grp + grp) * ld + min(m0 + r, ld - 1), nb);
     }
 #pragma unroll
     for (int q = 0; q < (kHkBK * 128) / 256; q++) {
       const int k = (tid >> 7) + 2 * q, j = k0 + k;
-      const int nb = (myq >= 0 && j < J) ? 8 : 0;
+      const int nb = (myq >= 0 && j < j_end) ? 8 : 0;
       cp_async8(Bs + k * kHkSB + (tid & 127), Wg + (size_t)min(j, J - 1) * ldN + max(myq, 0), nb);
     }
   };
 
-  double acc[9][2][4];
+  double acc[MT][2][4];
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int y = 0; y < 2; y++)
 #pragma unroll
@@ -743,9 +816,9 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
     for (int k4 = 0; k4 < kHkBK / 4; k4++) {
       const int kk = k4 * 4 + t;
-      double a[9][2], b[2];
+      double a[MT][2], b[2];
 #pragma unroll
-      for (int x = 0; x < 9; x++) {
+      for (int x = 0; x < MT; x++) {
         a[x][0] = As[kk * kHkSA + x * 16 + g];
         a[x][1] = As[kk * kHkSA + x * 16 + g + 8];
       }
@@ -755,7 +828,7 @@ __global__ void __launch_bounds__(256, 1)
         b[y] = Bs[kk * kHkSB + cs] * Rs[cs];
       }
 #pragma unroll
-      for (int x = 0; x < 9; x++)
+      for (int x = 0; x < MT; x++)
 #pragma unroll
         for (int y = 0; y < 2; y++) dmma_16x8x4(acc[x][y], a[x][0], a[x][1], b[y]);
     }
@@ -763,35 +836,78 @@ __global__ void __launch_bounds__(256, 1)
   cp_async_wait<0>();
   const int* cz = cells + (size_t)z * 128;
 #pragma unroll
-  for (int x = 0; x < 9; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int r = x * 16 + g + 8 * h;
+      const int r = m0 + x * 16 + g + 8 * h;
       if (r >= ld) continue;
 #pragma unroll
       for (int y = 0; y < 2; y++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-          const int i = cz[wn * 16 + y * 8 + 2 * t + e];
-          if (i >= 0) HK[i + (size_t)r * ldN] = acc[x][y][2 * h + e];
+          const int slot = wn * 16 + y * 8 + 2 * t + e, i = cz[slot];
+          if (i < 0) continue;
+          if (gridDim.y == 1) HK[i + (size_t)r * ldN] = acc[x][y][2 * h + e];
+          else part[(((size_t)sp * ld + r) * gridDim.z + z) * 128 + slot] = acc[x][y][2 * h + e];
         }
     }
 }
 
+// HK[cell(slot), r] = sum over the gene ranges s of part[s][r][slot]
+__global__ void k_reduce_hk(int ld, int ns, int slots, int ldN, const int* __restrict__ cells,
+                            const double* __restrict__ part, double* __restrict__ HK) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+  if (q >= slots) return;
+  const int i = cells[q];
+  if (i < 0) return;
+  double v = 0.0;
+  for (int s = 0; s < ns; s++) v += part[((size_t)s * ld + r) * slots + q];
+  HK[i + (size_t)r * ldN] = v;
+}
+
+// the gene ranges (of at least 128 genes) whose blocks fill their last wave best
+static int hk_ranges(const Ctx* c, int rows) {
+  const int tiles = c->n_hk_tiles128 * div_up(c->n_d + 1, rows);
+  int ns = 1;
+  double best = 0.0;
+  for (int s = 1; s <= 16 && (s == 1 || c->J / s >= 128); s++) {
+    const double waves = (double)tiles * s / c->sm_count, fill = waves / std::ceil(waves);
+    if (fill > best + 0.05) {
+      best = fill;
+      ns = s;
+    }
+  }
+  return ns;
+}
+
 int dgen_hk(Ctx* c) {
   const int ld = c->n_d + 1;
-  if (ld > 144) return GPL_ERR_ARG;
   const double* rOm = nullptr;
   int rc = recip_omega(c, &rOm);
   if (rc) return rc;
   if ((rc = launch_group_order(c, rOm, 1, c->rOmg))) return rc;
-  if (c->n_hk_tiles128 == 0) return GPL_OK;
-  GPL_TRY(c, cudaFuncSetAttribute(k_hk, cudaFuncAttributeMaxDynamicSharedMemorySize, kHkSmem));
-  k_hk<<<dim3(1, 1, c->n_hk_tiles128), 256, kHkSmem, c->stream>>>(ld, c->J, c->n_grp, c->ldN, c->gsum,
-                                                                   c->hk_tiles128_d, c->Wg, c->rOmg, c->hk_pos_d,
-                                                                   c->hk_cells_d, c->HK);
-  GPL_LAUNCHED(c, "k_hk");
-  return GPL_OK;
+  const int nt = c->n_hk_tiles128;
+  if (nt == 0) return GPL_OK;
+  return with_row_tiles(ld, [&](auto mt) -> int {
+    constexpr int MT = decltype(mt)::value;
+    const int mtiles = div_up(ld, MT * 16), ns = hk_ranges(c, MT * 16);
+    if (ns > 1) {
+      const int rp = ensure_part(c, (size_t)ns * ld * nt * 128);
+      if (rp) return rp;
+    }
+    const int jper = div_up(div_up(c->J, ns), kHkBK) * kHkBK;
+    GPL_TRY(c, cudaFuncSetAttribute(k_hk<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, hk_smem(MT)));
+    k_hk<MT><<<dim3(mtiles, ns, nt), 256, hk_smem(MT), c->stream>>>(ld, c->J, jper, c->n_grp, c->ldN, c->gsum,
+                                                                    c->hk_tiles128_d, c->Wg, c->rOmg, c->hk_pos_d,
+                                                                    c->hk_cells_d, c->HK, c->part);
+    GPL_LAUNCHED(c, "k_hk");
+    if (ns > 1) {
+      k_reduce_hk<<<dim3(div_up(nt * 128, 256), ld), 256, 0, c->stream>>>(ld, ns, nt * 128, c->ldN, c->hk_cells_d,
+                                                                         c->part, c->HK);
+      GPL_LAUNCHED(c, "k_reduce_hk");
+    }
+    return GPL_OK;
+  });
 }
 
 // Psi_DD,j = L G~_j L^T + DeltaInv_DD for every gene: T_j = G~_j L^T as one GEMM over the stacked
@@ -898,10 +1014,140 @@ __global__ void k_reduce_gram(int n, int P, int nz, const int* __restrict__ dcol
   Psi[ml + mk * P] = s;
 }
 
+// C2 (getC2, ggplvm.cu:57-100): three M x M sums, over the cells (KinvKmn^T diag(Oinvt) KinvKmn), over
+// the genes' coefficients (tilde-beta tilde-beta^T / phi) and over the genes' inverses. The first two
+// are split-K products, the third a sum of J blocks read along their columns; the parts are added in
+// order by k_c2. One block per entry pair re-read two columns of every cell: 13 GB through L2 and
+// 1.86 ms at 100,000 cells, 3,000 genes, M = 128 (0.19 ms so).
+namespace {
+struct LdDcolW {  // B(k = cell, c = column) times the cell's weight
+  static constexpr bool kFastK = true;
+  const double *D, *w;
+  int ldN;
+  struct Raw {
+    double d, w;
+  };
+  __device__ Raw load(int k, int c, int) const { return Raw{D[(size_t)c * ldN + k], w[k]}; }
+  __device__ double finish(const Raw& v) const { return v.d * v.w; }
+};
+struct LdTBetaRow {  // A(r = GP column, k = gene)
+  static constexpr bool kFastK = false;
+  const double* tB;
+  int P, g0;
+  __device__ double operator()(int r, int k, int) const { return tB[g0 + r + (size_t)k * P]; }
+};
+struct LdTBetaPhi {  // B(k = gene, c = GP column) / phi
+  static constexpr bool kFastK = false;
+  const double *tB, *rphi;
+  int P, g0;
+  struct Raw {
+    double b, f;
+  };
+  __device__ Raw load(int k, int c, int) const { return Raw{tB[g0 + c + (size_t)k * P], rphi[k]}; }
+  __device__ double finish(const Raw& v) const { return v.b * v.f; }
+};
+}  // namespace
+
+// part[z][j + k M] = sum over the z-th range of genes of S_g[GP j, GP k], j <= k
+__global__ void k_c2_genes(int J, int jper, int P, int M, int g0, const double* __restrict__ S,
+                           double* __restrict__ part) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= M * M) return;
+  const int k = e / M, j = e - k * M;
+  if (j > k) return;
+  const double* s = S + (size_t)(k + g0) * P + (j + g0);
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  const int a = blockIdx.y * jper, b = min(J, a + jper);
+  int g = a;
+  for (; g + 4 <= b; g += 4)
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] += s[(size_t)(g + u) * P * P];
+  for (; g < b; g++) v[0] += s[(size_t)g * P * P];
+  part[(size_t)blockIdx.y * M * M + e] = (v[0] + v[1]) + (v[2] + v[3]);
+}
+
+__global__ void k_c2(int J, int M, int pvars, int n1, int n2, int n3, const double* __restrict__ p1,
+                     const double* __restrict__ p2, const double* __restrict__ p3, const double* __restrict__ KmmInv,
+                     const double* __restrict__ K, const double* __restrict__ delta, double* __restrict__ C2) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= M * M) return;
+  const int k = e / M, j = e - k * M;
+  if (j > k) return;
+  double s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  for (int z = 0; z < n1; z++) s1 += p1[(size_t)z * M * M + (size_t)j * M + k];
+  for (int z = 0; z < n2; z++) s2 += p2[(size_t)z * M * M + (size_t)j * M + k];
+  for (int z = 0; z < n3; z++) s3 += p3[(size_t)z * M * M + e];
+  const double d = delta[pvars - 1];
+  double v = -kWt * d * s1 / 2.0;
+  v -= s2 / d / 2.0;
+  v -= s3 / d / 2.0;
+  v += ((double)J) * KmmInv[j + k * M] / 2.0;
+  v *= K[j + k * M];
+  C2[j + k * M] = v;
+  if (j < k) C2[k + j * M] = v;
+}
+
+static void c2_parts(const Ctx* c, int* n1, int* n2, int* n3) {
+  const int t = div_up(c->M, TileSq::BM), nb = div_up((int64_t)c->M * c->M, 256);
+  *n1 = std::max(1, std::min(c->sm_count / (t * t), div_up(c->N, 64)));
+  *n2 = std::max(1, std::min(c->sm_count / (t * t), div_up(c->J, 64)));
+  *n3 = std::max(1, std::min(8 * c->sm_count / nb, div_up(c->J, 16)));
+}
+
+int dgen_c2(Ctx* c) {
+  using T = TileSq;
+  const int M = c->M, t = div_up(M, T::BM), g0 = c->nh[c->p - 1];
+  const size_t MM = (size_t)M * M;
+  const int nb = div_up((int64_t)MM, 256);
+  int n1, n2, n3;
+  c2_parts(c, &n1, &n2, &n3);
+  int rc = ensure_part(c, MM * (n1 + n2 + n3));
+  if (rc) return rc;
+  double *p1 = c->part, *p2 = p1 + MM * n1, *p3 = p2 + MM * n2;
+  const double* Oinvt = c->W + (size_t)c->J * c->ldN;
+  if ((rc = launch_dgen<T>(c, dim3(t, t, n1), M, M, LdDrow{c->KinvKmn, c->ldN}, LdDcolW{c->KinvKmn, Oinvt, c->ldN},
+                           KSplit{c->N, div_up(c->N, n1)}, EpPart{p1, M, M}, "k_dgen(c2 cells)")))
+    return rc;
+  if ((rc = launch_dgen<T>(c, dim3(t, t, n2), M, M, LdTBetaRow{c->tBeta, c->P, g0},
+                           LdTBetaPhi{c->tBeta, c->rphi, c->P, g0}, KSplit{c->J, div_up(c->J, n2)}, EpPart{p2, M, M},
+                           "k_dgen(c2 coefficients)")))
+    return rc;
+  k_c2_genes<<<dim3(nb, n3), 256, 0, c->stream>>>(c->J, div_up(c->J, n3), c->P, M, g0, c->PsiInv, p3);
+  GPL_LAUNCHED(c, "k_c2_genes");
+  k_c2<<<nb, 256, 0, c->stream>>>(c->J, M, c->p, n1, n2, n3, p1, p2, p3, c->KmmInv, c->Kmm, c->delta, c->C2);
+  GPL_LAUNCHED(c, "k_c2");
+  return GPL_OK;
+}
+
+static int gram_splits(const Ctx* c) {
+  const int t = div_up(c->n_d, TileSq::BM);
+  return std::max(1, std::min(c->sm_count / (t * t), div_up(c->N, 64)));
+}
+
+// The largest request of the phases of a fit (the score statistics ask for their own).
+static size_t part_bound(const Ctx* c) {
+  const size_t J = c->J, n_d = c->n_d, MM = (size_t)c->M * c->M;
+  int n1, n2, n3;
+  c2_parts(c, &n1, &n2, &n3);
+  size_t n = std::max(MM * (n1 + n2 + n3), (size_t)gram_splits(c) * n_d * n_d);
+  with_row_tiles(c->n_d, [&](auto mt) -> int {
+    n = std::max(n, (size_t)zt_splits(c, 16 * decltype(mt)::value) * n_d * J);
+    if (c->n_grp) n = std::max(n, (size_t)c->n_grp * group_runs(c, c->J, 16 * decltype(mt)::value) * J * n_d);
+    return GPL_OK;
+  });
+  with_row_tiles(c->n_d + 1, [&](auto mt) -> int {
+    const int ns = hk_ranges(c, 16 * decltype(mt)::value);
+    if (ns > 1) n = std::max(n, (size_t)ns * (n_d + 1) * c->n_hk_tiles128 * 128);
+    return GPL_OK;
+  });
+  if (c1_splits(c) > 1) n = std::max(n, (size_t)c1_splits(c) * c->N * c->M);
+  return std::max(n, cell_sums_part(c));
+}
+
 int dgen_unweighted_gram(Ctx* c) {
   using T = TileSq;
   const int n = c->n_d, t = div_up(n, T::BM);
-  const int S = std::max(1, std::min({c->sm_count / (t * t), div_up(c->N, 64), 65535}));
+  const int S = gram_splits(c);
   int rc = ensure_part(c, (size_t)S * n * n);
   if (rc) return rc;
   rc = launch_dgen<T>(c, dim3(t, t, S), n, n, LdDrow{c->Dm, c->ldN}, LdDcol{c->Dm, c->ldN},

@@ -44,33 +44,11 @@ struct LoadBetaDense {  // B(k = dense column, c = gene) = B[dcol[k] + c*P]
   int P, n_d, J;
   __device__ double operator()(int k, int c) const { return (k < n_d && c < J) ? B[dcol[k] + (size_t)c * P] : 0.0; }
 };
-struct LoadOinvNu {  // B(k = cell, c = gene) = W/Omega * Nu
-  static constexpr bool kFastK = true;
-  const double *W, *Nu, *Omega;
-  int ldN, N, J;
-  __device__ double operator()(int k, int c) const {
-    if (k >= N || c >= J) return 0.0;
-    const size_t e = (size_t)c * ldN + k;
-    return W[e] / Omega[k] * Nu[e];
-  }
-};
 struct LoadCellGene {  // B(k = cell, c = gene) = S[c*ldN + k]
   static constexpr bool kFastK = true;
   const double* S;
   int ldN, N, J;
   __device__ double operator()(int k, int c) const { return (k < N && c < J) ? S[(size_t)c * ldN + k] : 0.0; }
-};
-struct LoadTn {  // A(r = cell, k = gene) = tn / phi, tn = O*nu - O*E, O = W/Omega
-  static constexpr bool kFastK = false;
-  const double *W, *Nu, *E, *Omega, *phi;
-  int ldN, N, J;
-  __device__ double operator()(int r, int k) const {
-    if (r >= N || k >= J) return 0.0;
-    const size_t e = (size_t)k * ldN + r;
-    const double o = W[e] / Omega[r];
-    const double tn = o * Nu[e] - o * E[e];
-    return tn / phi[k];
-  }
 };
 struct LoadCellGeneA {  // A(r = cell, k = gene) = S[k*ldN + r]
   static constexpr bool kFastK = false;
@@ -379,24 +357,9 @@ int launch_zt_u(Ctx* c, int mode) { return launch_zt_u_ex(c, mode, mode == 0 ? c
 int launch_zt_u_ex(Ctx* c, int mode, const double* u, double* out) {
   {
     ProfScope ps(c, "zt_u");
-    dim3 g(div_up(c->n_d, TM), div_up(c->J, TN));
-    LoadDt A{c->Dm, c->ldN, c->N, c->n_d};
     const int rc = dgen_zt_u(c, mode, u, out);
-    if (rc != GPL_OK && rc != GPL_ERR_ARG) return rc;
-    if (rc == GPL_ERR_ARG && mode == 2) {
-      c->err = "per-cell Z^T u needs the DMMA form (at most 144 dense columns)";
-      return GPL_ERR_ARG;
-    }
-    if (rc == GPL_ERR_ARG) {  // the FFMA form: more dense columns than one DMMA tile
-      if (mode == 0)
-        k_gemm_store<<<g, 256, 0, c->stream>>>(c->n_d, c->J, c->N, A,
-                                               LoadOinvNu{c->W, u, c->Omega, c->ldN, c->N, c->J}, out,
-                                               (int64_t)c->P, c->dcol_d);
-      else
-        k_gemm_store<<<g, 256, 0, c->stream>>>(c->n_d, c->J, c->N, A, LoadCellGene{u, c->ldN, c->N, c->J}, out,
-                                               (int64_t)c->P, c->dcol_d);
-      GPL_LAUNCHED(c, "k_gemm_store(zt_u)");
-    }
+    if (rc == GPL_ERR_ARG) c->err = "per-cell Z^T u takes at most 144 dense columns";
+    if (rc != GPL_OK) return rc;
   }
   c->zt_u_src = (mode == 2 || (mode == 0 && u != c->Nu)) ? u : nullptr;
   int rc = launch_group_sums(c, mode == 0 ? 3 : mode == 2 ? 4 : 2);
@@ -408,18 +371,7 @@ int launch_zt_u_ex(Ctx* c, int mode, const double* u, double* out) {
 // C1 <- sum_j (tn_ij/phi_j) tBeta_j[GP]   (stored cell-fastest, ld ldN)
 int launch_c1_tn(Ctx* c) {
   ProfScope ps(c, "c1_tn");
-  {
-    const int rc = dgen_c1_tn(c);
-    if (rc != GPL_ERR_ARG) return rc;  // GPL_ERR_ARG: more dense columns than one DMMA tile
-  }
-  const int g0 = c->nh[c->p - 1];
-  dim3 g(div_up(c->N, TM), div_up(c->M, TN));
-  k_gemm_store<<<g, 256, 0, c->stream>>>(c->N, c->M, c->J,
-                                         LoadTn{c->W, c->Nu, c->scratch, c->Omega, c->phi, c->ldN, c->N, c->J},
-                                         LoadTBetaGP{c->tBeta, c->P, g0, c->M, c->J}, c->C1, (int64_t)c->ldN,
-                                         (const int*)nullptr);
-  GPL_LAUNCHED(c, "k_gemm_store(c1_tn)");
-  return GPL_OK;
+  return dgen_c1_tn(c);
 }
 
 }  // namespace gpl

@@ -3,7 +3,6 @@
 // getOinvt :284-294, initBeta init.cu:193-221). All reductions are block-deterministic:
 // a fixed shuffle tree per warp, then the warps in order.
 //
-//   k_oinvt       Oinvt_i = sum_j W_ij / Omega_i (thread per cell, genes in order) -> W column J
 //   k_beta_phi    per gene: damped beta <- (1-r) beta + r Psi^{-1} b, phi from the residual
 //                 quadratic form nu^T (W/Omega) nu - |L^T beta|^2, clamped as the reference
 //   k_lkhd_pois   per gene: sum over matched counts of (log W - delta_GP titsias wt) y, minus sum W
@@ -13,30 +12,6 @@
 #include "gpl_internal.cuh"
 
 namespace gpl {
-
-// sum_j W_ij / Omega_i as (sum_j W_ij) / Omega_i: one division per cell instead of per entry,
-// four independent partial sums (genes j = 4q + r in order within each) to keep loads in flight.
-__global__ void k_oinvt(int N, int ldN, int J, const double* __restrict__ Omega, double* __restrict__ W) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  int j = 0;
-  for (; j + 4 <= J; j += 4) {
-    s0 += W[(size_t)j * ldN + i];
-    s1 += W[(size_t)(j + 1) * ldN + i];
-    s2 += W[(size_t)(j + 2) * ldN + i];
-    s3 += W[(size_t)(j + 3) * ldN + i];
-  }
-  for (; j < J; j++) s0 += W[(size_t)j * ldN + i];
-  W[(size_t)J * ldN + i] = ((s0 + s1) + (s2 + s3)) / Omega[i];
-}
-
-int launch_oinvt(Ctx* c) {
-  ProfScope ps(c, "oinvt");
-  k_oinvt<<<div_up(c->N, 256), 256, 0, c->stream>>>(c->N, c->ldN, c->J, c->Omega, c->W);
-  GPL_LAUNCHED(c, "k_oinvt");
-  return GPL_OK;
-}
 
 // sol_j = Psi_j^{-1} b_j was solved beforehand.
 __global__ void __launch_bounds__(256) k_beta_phi(int N, int ldN, int P, double r, const double* __restrict__ W,
@@ -225,23 +200,59 @@ int launch_lkhd_pois(Ctx* c) {
   return GPL_OK;
 }
 
+// A product of positive normal numbers as mantissa and exponent: its logarithm costs one log() per
+// thread in place of one per number. Other values (zero, negative, denormal, not finite) go through
+// log() themselves.
+struct LogProduct {
+  double m = 1.0, rest = 0.0;
+  int e = 0;
+  __device__ __forceinline__ void mul(double x) {
+    const int hi = __double2hiint(x), f = hi >> 20;
+    if (f > 0 && f < 2047) {
+      e += f - 1023;
+      m *= __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+    } else {
+      rest += log(x);
+    }
+  }
+  __device__ __forceinline__ void fold() {  // after at most 512 factors in [1, 2)
+    const int hi = __double2hiint(m);
+    e += (hi >> 20) - 1023;
+    m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(m));
+  }
+  __device__ __forceinline__ double value() const { return fma((double)e, 0.693147180559945309417, log(m)) + rest; }
+};
+
 // l_j = -N/2 log phi - sum_i log(Omega/W)/2 - sum_k log L_kk + sum_k log LD_kk
 //       - sum_i nu^2 (W/Omega) / (2 phi) + b^T Psi^{-1} b / (2 phi)
+// with sum_i log Omega from the shared sums. Bound: one read of W and nu; with a log() and two
+// divisions per entry it was bound by their instructions (1.9 ms at 100,000 x 3,000 against 0.85 ms).
 __global__ void __launch_bounds__(256) k_lkhd_genes(int N, int ldN, int P, const double* __restrict__ W,
-                                                    const double* __restrict__ Nu, const double* __restrict__ Omega,
-                                                    const double* __restrict__ Psi, const double* __restrict__ LD,
-                                                    const double* __restrict__ bvec, const double* __restrict__ sol,
-                                                    const double* __restrict__ phi, double* __restrict__ lkhds) {
+                                                    const double* __restrict__ Nu, const double* __restrict__ rOm,
+                                                    const double* __restrict__ sums, const double* __restrict__ Psi,
+                                                    const double* __restrict__ LD, const double* __restrict__ bvec,
+                                                    const double* __restrict__ sol, const double* __restrict__ phi,
+                                                    double* __restrict__ lkhds) {
   __shared__ double sh[32];
   const int j = blockIdx.x;
   const double* Wj = W + (size_t)j * ldN;
   const double* nj = Nu + (size_t)j * ldN;
   const double phij = phi[j];
-  double a = 0.0, q = 0.0;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    const double om = Omega[i], w = Wj[i];
-    a += log(om / w);
-    q += nj[i] * nj[i] * (w / om);
+  LogProduct lw;
+  double q0 = 0.0, q1 = 0.0;
+  for (int i0 = 2 * threadIdx.x; i0 < N; i0 += 64 * 512) {
+#pragma unroll 4
+    for (int i = i0; i < min(N, i0 + 64 * 512); i += 512) {  // up to 128 factors between folds
+      const double2 w = *reinterpret_cast<const double2*>(Wj + i), u = *reinterpret_cast<const double2*>(nj + i);
+      const double2 r = *reinterpret_cast<const double2*>(rOm + i);
+      lw.mul(w.x);
+      q0 += u.x * u.x * (w.x * r.x);
+      if (i + 1 < N) {
+        lw.mul(w.y);
+        q1 += u.y * u.y * (w.y * r.y);
+      }
+    }
+    lw.fold();
   }
   const double* L = Psi + (size_t)j * P * P;
   double ld = 0.0, bx = 0.0;
@@ -249,12 +260,13 @@ __global__ void __launch_bounds__(256) k_lkhd_genes(int N, int ldN, int P, const
     ld += log(LD[k + (size_t)k * P]) - log(L[k + (size_t)k * P]);
     bx += bvec[(size_t)j * P + k] * sol[(size_t)j * P + k];
   }
-  const double sa = block_sum(a, sh);
-  const double sq = block_sum(q, sh);
+  const double slo = block_sum(threadIdx.x < kStateParts ? sums[threadIdx.x] : 0.0, sh);
+  const double slw = block_sum(lw.value(), sh);
+  const double sq = block_sum(q0 + q1, sh);
   const double sld = block_sum(ld, sh);
   const double sbx = block_sum(bx, sh);
   if (threadIdx.x == 0)
-    lkhds[j] = -((double)N) / 2.0 * log(phij) - sa / 2.0 + sld - sq / 2.0 / phij + sbx / 2.0 / phij;
+    lkhds[j] = -((double)N) / 2.0 * log(phij) - (slo - slw) / 2.0 + sld - sq / 2.0 / phij + sbx / 2.0 / phij;
 }
 
 // y_j = bx_j + DeltaInv v_j (DeltaInv as its factor L once cholDeltaInv has run: L (L^T v)), one
@@ -332,9 +344,12 @@ int launch_lkhd_genes(Ctx* c) {
   // x is refined against the FP64 operator (a 1e-6 error in x would survive the cancellation)
   int rc = solve_refined(c, c->bvec, c->sol, true);  // cholDeltaInv has run (ggplvm.cu:1206,1266)
   if (rc) return rc;
+  const double* rOm = nullptr;
+  if ((rc = recip_omega(c, &rOm))) return rc;
   {
     ProfScope ps(c, "lkhd_genes");
-    k_lkhd_genes<<<c->J, 256, 0, c->stream>>>(c->N, c->ldN, c->P, c->W, c->Nu, c->Omega, c->Psi, c->DeltaInv,
+    if ((rc = launch_state_sums(c))) return rc;
+    k_lkhd_genes<<<c->J, 256, 0, c->stream>>>(c->N, c->ldN, c->P, c->W, c->Nu, rOm, c->state_sums, c->Psi, c->DeltaInv,
                                               c->bvec, c->sol, c->phi, c->lkhds);
     GPL_LAUNCHED(c, "k_lkhd_genes");
   }
@@ -342,28 +357,25 @@ int launch_lkhd_genes(Ctx* c) {
   return GPL_OK;
 }
 
-// sum_j l_j - Q-prior - wt delta_GP sum_i Oinvt_i titsias_i - sum_i (igb/Omega_i + iga log Omega_i);
-// Q-prior: N(0, 1) on X and T in dimensions 1..qp-1 (qp = 0 for none). The fit driver:
-// wt = 0.1, igb = iga = 100, qp = 0 (ggplvm.cu:788-815); the variance-component driver: wt = 0,
-// 30, 30 and qp = Q (ggplvm_delta.cu:677-704).
-__global__ void __launch_bounds__(1024) k_collect(int J, int n, int ldN, int pvars, double wt, double igb, double iga,
-                                                  int qp, int M, const double* __restrict__ X,
-                                                  const double* __restrict__ T, const double* __restrict__ lkhds,
-                                                  const double* __restrict__ W, const double* __restrict__ titsias,
-                                                  const double* __restrict__ Omega, const double* __restrict__ delta,
-                                                  double* __restrict__ out) {
+// sum_j l_j - Q-prior - wt delta_GP sum_i Oinvt_i titsias_i - sum_i (igb/Omega_i + iga log Omega_i)
+// from the shared sums (n = 0: the sum of the l_j alone); Q-prior: N(0, 1) on X and T in dimensions
+// 1..qp-1 (qp = 0 for none). The fit driver: wt = 0.1, igb = iga = 100, qp = 0 (ggplvm.cu:788-815);
+// the variance-component driver: wt = 0, 30, 30 and qp = Q (ggplvm_delta.cu:677-704).
+__global__ void __launch_bounds__(1024) k_collect(int J, int n, int pvars, double wt, double igb, double iga, int qp,
+                                                  int M, const double* __restrict__ X, const double* __restrict__ T,
+                                                  const double* __restrict__ lkhds, const double* __restrict__ sums,
+                                                  const double* __restrict__ delta, double* __restrict__ out) {
   __shared__ double sh[32];
   double s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
   for (int k = threadIdx.x; k < J; k += blockDim.x) s1 += lkhds[k];
-  const double* Oinvt = W + (size_t)J * ldN;
-  const double dgp = delta[pvars - 1];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    s2 += wt * dgp * Oinvt[i] * titsias[i];
-    s3 += igb / Omega[i] + iga * log(Omega[i]);
-    for (int k = 1; k < qp; k++) s4 += X[i + (size_t)k * n] * X[i + (size_t)k * n] / 2.0;
+  if (n > 0 && threadIdx.x < kStateParts) {
+    s2 = wt * delta[pvars - 1] * sums[2 * kStateParts + threadIdx.x];
+    s3 = igb * sums[kStateParts + threadIdx.x] + iga * sums[threadIdx.x];
   }
-  for (int i = threadIdx.x; i < M && qp > 1; i += blockDim.x)
-    for (int k = 1; k < qp; k++) s4 += T[i + (size_t)k * M] * T[i + (size_t)k * M] / 2.0;
+  for (int k = 1; k < qp; k++) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s4 += X[i + (size_t)k * n] * X[i + (size_t)k * n] / 2.0;
+    for (int i = threadIdx.x; i < M; i += blockDim.x) s4 += T[i + (size_t)k * M] * T[i + (size_t)k * M] / 2.0;
+  }
   s1 = block_sum(s1, sh);
   s2 = block_sum(s2, sh);
   s3 = block_sum(s3, sh);
@@ -374,9 +386,9 @@ __global__ void __launch_bounds__(1024) k_collect(int J, int n, int ldN, int pva
 int launch_collect_lkhd(Ctx* c, int n_cells, int slot) {
   ProfScope ps(c, "collect");
   const int qp = (c->vcomp && n_cells > 0) ? c->Q : 0;
-  k_collect<<<1, 1024, 0, c->stream>>>(c->J, n_cells, c->ldN, c->p, c->vcomp ? 0.0 : kWt, c->vcomp ? 30.0 : kIgb,
-                                       c->vcomp ? 30.0 : kIgap1, qp, c->M, c->X, c->T, c->lkhds, c->W, c->titsias,
-                                       c->Omega, c->delta, c->lkhd_dev + slot);
+  k_collect<<<1, 1024, 0, c->stream>>>(c->J, n_cells, c->p, c->vcomp ? 0.0 : kWt, c->vcomp ? 30.0 : kIgb,
+                                       c->vcomp ? 30.0 : kIgap1, qp, c->M, c->X, c->T, c->lkhds, c->state_sums,
+                                       c->delta, c->lkhd_dev + slot);
   GPL_LAUNCHED(c, "k_collect");
   return GPL_OK;
 }
