@@ -84,7 +84,7 @@ static void free_state(Ctx* c) {
   tc_release(c);
   pair_release(c);
   void* extra[] = {c->cellfac, c->lvt, c->Dm, c->gsum, c->gT, c->HK, c->dcol_d, c->cv_nh_d, c->cv_nlev_d, c->gid_d, c->glev_d,
-                   c->gcells_d, c->gstart_d, c->codes_d, c->hk_tiles_d, c->hk_tiles128_d, c->part, c->hk_cells_d,
+                   c->gcells_d, c->gstart_d, c->codes_d, c->hk_tiles_d, c->hk_tiles128_d, c->part, c->work, c->hk_cells_d,
                    c->lvl_cc_d, c->lvl_v_d, c->lvl_ptr_d, c->lvl_grp_d, c->hk_pos_d, c->Wg, c->Dg, c->rOmg,
                    c->gpos_d};
   for (void* q : extra)
@@ -92,8 +92,8 @@ static void free_state(Ctx* c) {
   c->hk_tiles128_d = nullptr;
   c->hk_cells_d = nullptr;
   c->n_hk_tiles128 = 0;
-  c->part = nullptr;
-  c->part_n = 0;
+  c->part = c->work = nullptr;
+  c->part_n = c->work_n = 0;
   c->cellfac = c->lvt = c->Dm = c->gsum = c->gT = c->HK = nullptr;
   c->dcol_d = c->cv_nh_d = c->cv_nlev_d = c->gid_d = c->glev_d = c->gcells_d = c->gstart_d = c->codes_d = nullptr;
   c->lvl_cc_d = c->lvl_v_d = c->lvl_ptr_d = c->lvl_grp_d = c->hk_pos_d = nullptr;
@@ -1331,39 +1331,17 @@ int gpl_score_stats(gpl_ctx* h, int L, const double* G, double* S) {
     return GPL_ERR_ARG;
   }
   const size_t N = c->N, J = c->J;
-  const int LB = 64;  // genotype columns per pass (two per column in the GEMM tile of 128)
-  double *dG = nullptr, *dW = nullptr, *dS = nullptr;
-  const size_t work = (size_t)2 * LB * N + (size_t)4 * LB * J;
-  if (cudaMalloc((void**)&dG, sizeof(double) * N * LB) != cudaSuccess ||
-      cudaMalloc((void**)&dW, sizeof(double) * work) != cudaSuccess ||
-      cudaMalloc((void**)&dS, sizeof(double) * J * LB) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(dG);
-    cudaFree(dW);
-    cudaFree(dS);
-    c->err = "device allocation failed: score statistics";
-    return GPL_ERR_ALLOC;
-  }
-  int rc = GPL_OK;
-  for (int l0 = 0; l0 < L && rc == GPL_OK; l0 += LB) {
+  const int LB = score_columns(c, L);
+  GPL_RUN(ensure_work(c, (N + J) * LB + score_work(c, LB)));
+  double *dG = c->work, *dS = dG + N * LB, *dW = dS + J * LB;
+  for (int l0 = 0; l0 < L; l0 += LB) {
     const int nl = std::min(LB, L - l0);
-    if (cudaMemcpyAsync(dG, G + (size_t)l0 * N, sizeof(double) * N * nl, cudaMemcpyHostToDevice, c->stream) !=
-        cudaSuccess) {
-      rc = GPL_ERR_CUDA;
-      break;
-    }
-    rc = launch_score_stats(c, nl, dG, dS, dW);
-    if (rc == GPL_OK &&
-        cudaMemcpyAsync(S + (size_t)l0 * J, dS, sizeof(double) * J * nl, cudaMemcpyDeviceToHost, c->stream) !=
-            cudaSuccess)
-      rc = GPL_ERR_CUDA;
-    if (rc == GPL_OK && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = GPL_ERR_CUDA;
+    GPL_TRY(c, cudaMemcpyAsync(dG, G + (size_t)l0 * N, sizeof(double) * N * nl, cudaMemcpyHostToDevice, c->stream));
+    GPL_RUN(launch_score_stats(c, nl, dG, dS, dW));
+    GPL_TRY(c, cudaMemcpyAsync(S + (size_t)l0 * J, dS, sizeof(double) * J * nl, cudaMemcpyDeviceToHost, c->stream));
+    GPL_TRY(c, cudaStreamSynchronize(c->stream));
   }
-  if (rc == GPL_ERR_CUDA && c->err.empty()) c->err = cudaGetErrorString(cudaGetLastError());
-  cudaFree(dG);
-  cudaFree(dW);
-  cudaFree(dS);
-  return rc;
+  return GPL_OK;
 }
 
 int gpl_de_model(gpl_ctx* h, int model) {

@@ -198,6 +198,8 @@ struct Ctx {
   int n_hk_tiles128 = 0;
   double* part = nullptr;           // split-K partial sums
   size_t part_n = 0;
+  double* work = nullptr;           // one call's scratch (placement, genotype statistics)
+  size_t work_n = 0;
   double *Dm = nullptr, *gsum = nullptr, *gT = nullptr, *HK = nullptr;
 
   // device buffers
@@ -288,7 +290,7 @@ inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // ---- launchers (one per kernel family; each returns GPL_OK or an error code) ----------
 // k_kmats.cu
 int launch_kernel_mats(Ctx* c);          // Knm into Z, Kmm, Kinv copy, chol(Kinv), KinvKmn, titsias
-int launch_kernel_mats_lv(Ctx* c, int lv);  // the same over latent dimension lv alone, all (kLvAll), none (kLvNone)
+int launch_kernel_cells(Ctx* c);         // Knm, KinvKmn and titsias at a new X, Kmm's factor unchanged
 int launch_expand_delta(Ctx* c);         // DeltaInv (upper + diag)
 int launch_chol_single(Ctx* c, double* A, int n);  // choldc on one n x n matrix
 // k_groups.cu
@@ -339,12 +341,18 @@ int pair_prepare(Ctx* c);                 // column-pair list, 1/Omega, gathered
 int recip_omega(Ctx* c, const double** rOm);  // 1/Omega (0 past N), refreshed on every call
 int dgen_zt_u(Ctx* c, int mode, const double* u, double* out);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);
 int dgen_c1_tn(Ctx* c);
+int dgen_resid_gp(Ctx* c, const double* R, const double* B, double* G);  // cells x genes against the GP coefficients
 int dgen_c2(Ctx* c);                      // C2 (M x M adjoint of Kmm) up to its final combination
 int dgen_group_sums(Ctx* c, int mode);
+int dgen_group_sums_of(Ctx* c, const double* Gg, int m);  // gsum[j][g][a] of m <= n_d columns in group order
 int dgen_unweighted_gram(Ctx* c);         // the dense block of Psi_0 with every weight 1 (GLM initialisation)
 int dgen_hk(Ctx* c);
 int dgen_weighted_colsums(Ctx* c, const double* G2, int n2, double* out);  // out[j + c*J] = sum_i W_ij G2[c][i]
 int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch);  // device G (N x L) -> S (J x L)
+int score_columns(const Ctx* c, int L);   // genotype columns per pass of L
+size_t score_work(const Ctx* c, int L);   // values of scratch of a pass of L columns
+// q[j + v*J] = t_jv^T Psi_j^{-1} t_jv with the factors of Psi, t_jv at T + j sj + v sv
+int launch_quad(Ctx* c, int J, int V, const double* Psi, const double* T, size_t sj, size_t sv, double* q);
 int dgen_unwhiten(Ctx* c, const double* Gt, double* Tt, const double* Lw);  // Psi_DD = L G L^T + DeltaInv
 int dgen_whiten_inverse(Ctx* c, const double* Lw, double* Tt, double* St);  // S~ = L^T S_DD L per gene
 int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D);  // U from the V rows of cells [c0, c1)
@@ -374,6 +382,8 @@ int launch_oinvt(Ctx* c);
 int launch_tn_sum(Ctx* c, const double* E, double* out);  // per cell: the gradient's sum over genes
 size_t cell_sums_part(const Ctx* c);      // values of c->part that the sums per cell take
 int launch_state_sums(Ctx* c);            // state_sums at the current Omega, Oinvt and titsias
+int ensure_work(Ctx* c, size_t n);        // one call's scratch (c->work), at least n values
+int cell_sum_ranges(const Ctx* c);        // gene ranges of the sums per cell
 int ensure_part(Ctx* c, size_t n);        // the split sums' buffer (c->part), at least n values (k_dgen.cu)
 // k_lkhd.cu
 int launch_beta_phi(Ctx* c, int jtr);

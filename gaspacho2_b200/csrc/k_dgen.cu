@@ -197,6 +197,12 @@ struct LdTn {  // A(r = cell, k = gene) = (O nu - O E) / phi, O = W / Omega (1/p
     return (o * v.u - o * v.e) * v.f;
   }
 };
+struct LdGeneCell {  // A(r = cell, k = gene) = R[k*ldN + r]
+  static constexpr bool kFastK = false;
+  const double* R;
+  int ldN;
+  __device__ double operator()(int r, int k, int) const { return R[(size_t)k * ldN + r]; }
+};
 struct LdTBetaGP {  // B(k = gene, c = a) = tBeta[g0 + c + k*P]
   static constexpr bool kFastK = false;
   const double* tB;
@@ -368,6 +374,21 @@ int ensure_part(Ctx* c, size_t n) {
     return GPL_ERR_ALLOC;
   }
   c->part_n = n;
+  return GPL_OK;
+}
+
+// Scratch of one call (placement, genotype statistics): kept by the context, grown when a call asks for more.
+int ensure_work(Ctx* c, size_t n) {
+  if (c->work_n >= n) return GPL_OK;
+  if (c->work) cudaFree(c->work);
+  c->work = nullptr;
+  c->work_n = 0;
+  if (cudaMalloc((void**)&c->work, sizeof(double) * n) != cudaSuccess) {
+    cudaGetLastError();
+    c->err = "device allocation failed: work buffer (" + std::to_string(sizeof(double) * n) + " bytes)";
+    return GPL_ERR_ALLOC;
+  }
+  c->work_n = n;
   return GPL_OK;
 }
 
@@ -569,28 +590,38 @@ static int c1_splits(const Ctx* c) {
   return S;
 }
 
-int dgen_c1_tn(Ctx* c) {
+// out[i, a] = sum_j A(i, j) B[g0 + a, j] over c1_splits gene ranges
+template <class LA>
+static int cells_by_gp(Ctx* c, LA A, const double* coef, double* out, const char* name) {
   using T = TileSq;
-  const double* rOm = nullptr;
-  int rc = recip_omega(c, &rOm);
-  if (rc) return rc;
-  const int g0 = c->nh[c->p - 1];
   const int S = c1_splits(c);
-  LdTn A{c->W, c->Nu, c->scratch, rOm, c->rphi, c->ldN};
-  LdTBetaGP B{c->tBeta, c->P, g0};
+  LdTBetaGP B{coef, c->P, c->nh[c->p - 1]};
+  int rc;
   if (S == 1) {
     dim3 g(div_up(c->N, T::BM), div_up(c->M, T::BN), 1);
-    return launch_dgen<T>(c, g, c->N, c->M, A, B, KAll{c->J}, EpColMajor{c->C1, (int64_t)c->ldN}, "k_dgen(c1_tn)");
+    return launch_dgen<T>(c, g, c->N, c->M, A, B, KAll{c->J}, EpColMajor{out, (int64_t)c->ldN}, name);
   }
   if ((rc = ensure_part(c, (size_t)S * c->N * c->M))) return rc;
   dim3 g(div_up(c->N, T::BM), div_up(c->M, T::BN), S);
-  rc = launch_dgen<T>(c, g, c->N, c->M, A, B, KSplit{c->J, (c->J + S - 1) / S}, EpPart{c->part, c->N, c->M},
-                      "k_dgen(c1_tn)");
+  rc = launch_dgen<T>(c, g, c->N, c->M, A, B, KSplit{c->J, (c->J + S - 1) / S}, EpPart{c->part, c->N, c->M}, name);
   if (rc) return rc;
   dim3 g2(div_up(c->N, 256), c->M);
-  k_reduce_parts_ld<<<g2, 256, 0, c->stream>>>(c->N, c->M, S, c->part, c->C1, (int64_t)c->ldN);
+  k_reduce_parts_ld<<<g2, 256, 0, c->stream>>>(c->N, c->M, S, c->part, out, (int64_t)c->ldN);
   GPL_LAUNCHED(c, "k_reduce_parts_ld");
   return GPL_OK;
+}
+
+int dgen_c1_tn(Ctx* c) {
+  const double* rOm = nullptr;
+  int rc = recip_omega(c, &rOm);
+  if (rc) return rc;
+  return cells_by_gp(c, LdTn{c->W, c->Nu, c->scratch, rOm, c->rphi, c->ldN}, c->tBeta, c->C1, "k_dgen(c1_tn)");
+}
+
+// G[i, a] = sum_j R_ij B[g0 + a, j]: a cell x gene matrix R (cell fastest, ld ldN) against the GP
+// block of coefficients (P x J), into G (cell fastest, ld ldN).
+int dgen_resid_gp(Ctx* c, const double* R, const double* B, double* G) {
+  return cells_by_gp(c, LdGeneCell{R, c->ldN}, B, G, "k_dgen(resid_gp)");
 }
 
 // S[j][g][a] = sum over group g's cells of w_ij D_ia (w = W/Omega, MODE 0; 1, MODE 1): grid
@@ -710,40 +741,54 @@ __global__ void k_reduce_groups(int m, int n, int n_grp, int ns, const double* _
   S[((size_t)j * n_grp + grp) * (m + 1) + a] = s;
 }
 
-static int group_runs(const Ctx* c, int J, int rows) {
-  const int tiles = div_up(J, kZtBN) * div_up(c->n_d, rows) * c->n_grp;
+static int group_runs(const Ctx* c, int J, int m, int rows) {
+  const int tiles = div_up(J, kZtBN) * div_up(m, rows) * c->n_grp;
   // runs of at least 128 cells on average, up to four blocks per SM
   return std::max(1, std::min(4 * c->sm_count / tiles, c->N / (c->n_grp * 128)));
 }
 
-int dgen_group_sums(Ctx* c, int mode) {
-  int rc;
-  if (mode == 0) {
-    const double* rOm = nullptr;
-    if ((rc = recip_omega(c, &rOm))) return rc;
-    if ((rc = launch_group_order(c, rOm, 1, c->rOmg))) return rc;
-  }
-  if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
+// c->gsum[j][g][a] = sum over group g of w_ij Dg_a (m columns in group order, ld ldN); w = W/Omega with
+// c->rOmg current (mode 0) or 1 for one gene (mode 1)
+static int group_sums(Ctx* c, int mode, const double* Dg, int m) {
   const int J = mode == 1 ? 1 : c->J;
-  return with_row_tiles(c->n_d, [&](auto mt) -> int {
+  return with_row_tiles(m, [&](auto mt) -> int {
     constexpr int MT = decltype(mt)::value;
-    const int ns = group_runs(c, J, MT * 16);
+    const int ns = group_runs(c, J, m, MT * 16);
     if (ns > 1) {
-      const int rp = ensure_part(c, (size_t)c->n_grp * ns * J * c->n_d);
+      const int rp = ensure_part(c, (size_t)c->n_grp * ns * J * m);
       if (rp) return rp;
     }
     auto* fn = mode == 0 ? k_group_sums_dmma<0, MT> : k_group_sums_dmma<1, MT>;
     GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
-    fn<<<dim3(div_up(c->n_d, MT * 16), div_up(J, kZtBN), c->n_grp * ns), 256, zt_smem(MT), c->stream>>>(
-        c->n_d, J, c->n_grp, ns, c->ldN, c->gstart_d, c->Dg, c->Wg, c->rOmg, c->gsum, c->part);
+    fn<<<dim3(div_up(m, MT * 16), div_up(J, kZtBN), c->n_grp * ns), 256, zt_smem(MT), c->stream>>>(
+        m, J, c->n_grp, ns, c->ldN, c->gstart_d, Dg, c->Wg, c->rOmg, c->gsum, c->part);
     GPL_LAUNCHED(c, "k_group_sums_dmma");
     if (ns > 1) {
-      k_reduce_groups<<<dim3(div_up((int64_t)J * c->n_d, 256), c->n_grp), 256, 0, c->stream>>>(c->n_d, J, c->n_grp, ns,
-                                                                                             c->part, c->gsum);
+      k_reduce_groups<<<dim3(div_up((int64_t)J * m, 256), c->n_grp), 256, 0, c->stream>>>(m, J, c->n_grp, ns, c->part,
+                                                                                         c->gsum);
       GPL_LAUNCHED(c, "k_reduce_groups");
     }
     return GPL_OK;
   });
+}
+
+static int order_romega(Ctx* c) {
+  const double* rOm = nullptr;
+  const int rc = recip_omega(c, &rOm);
+  return rc ? rc : launch_group_order(c, rOm, 1, c->rOmg);
+}
+
+int dgen_group_sums(Ctx* c, int mode) {
+  int rc;
+  if (mode == 0 && (rc = order_romega(c))) return rc;
+  if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
+  return group_sums(c, mode, c->Dg, c->n_d);
+}
+
+int dgen_group_sums_of(Ctx* c, const double* Gg, int m) {
+  if (m > c->n_d) return GPL_ERR_ARG;  // the sums' buffer
+  const int rc = order_romega(c);
+  return rc ? rc : group_sums(c, 0, Gg, m);
 }
 
 // HK[i, a] = sum_j O_ij tab[j][g(i)][a] for the 128 cell slots of each group tile (grid z =
@@ -1132,7 +1177,7 @@ static size_t part_bound(const Ctx* c) {
   size_t n = std::max(MM * (n1 + n2 + n3), (size_t)gram_splits(c) * n_d * n_d);
   with_row_tiles(c->n_d, [&](auto mt) -> int {
     n = std::max(n, (size_t)zt_splits(c, 16 * decltype(mt)::value) * n_d * J);
-    if (c->n_grp) n = std::max(n, (size_t)c->n_grp * group_runs(c, c->J, 16 * decltype(mt)::value) * J * n_d);
+    if (c->n_grp) n = std::max(n, (size_t)c->n_grp * group_runs(c, c->J, c->n_d, 16 * decltype(mt)::value) * J * n_d);
     return GPL_OK;
   });
   with_row_tiles(c->n_d + 1, [&](auto mt) -> int {

@@ -50,18 +50,6 @@ struct LoadCellGene {  // B(k = cell, c = gene) = S[c*ldN + k]
   int ldN, N, J;
   __device__ double operator()(int k, int c) const { return (k < N && c < J) ? S[(size_t)c * ldN + k] : 0.0; }
 };
-struct LoadCellGeneA {  // A(r = cell, k = gene) = S[k*ldN + r]
-  static constexpr bool kFastK = false;
-  const double* S;
-  int ldN, N, J;
-  __device__ double operator()(int r, int k) const { return (r < N && k < J) ? S[(size_t)k * ldN + r] : 0.0; }
-};
-struct LoadTBetaGP {  // B(k = gene, c = a) = tBeta[g0 + a + k*P]
-  static constexpr bool kFastK = false;
-  const double* tB;
-  int P, g0, M, J;
-  __device__ double operator()(int k, int c) const { return (k < J && c < M) ? tB[g0 + c + (size_t)k * P] : 0.0; }
-};
 
 template <class LA, class LB>
 __device__ __forceinline__ void gemm_tile(int m0, int n0, int K, const LA& A, const LB& B, double (&acc)[4][4],
@@ -390,18 +378,6 @@ int launch_gemm_cm(Ctx* c, int m, int n, int K, const double* A, int lda, bool a
     k_gemm_store<<<g, 256, 0, c->stream>>>(m, n, K, LoadD{A, lda, m, K}, LoadCellGene{B, ldb, K, n}, C,
                                            (int64_t)ldc, (const int*)nullptr);
   GPL_LAUNCHED(c, "k_gemm_store(cm)");
-  return GPL_OK;
-}
-
-// G[i, a] = sum_j R_ij B[g0 + a, j]: a cell x gene matrix R (cell fastest, ld ldN) against the GP
-// block of coefficients (P x J), into G (cell fastest, ld ldN). FFMA tile GEMM.
-int launch_resid_gp(Ctx* c, const double* R, const double* B, double* G) {
-  const int g0 = c->nh[c->p - 1];
-  dim3 g(div_up(c->N, TM), div_up(c->M, TN));
-  k_gemm_store<<<g, 256, 0, c->stream>>>(c->N, c->M, c->J, LoadCellGeneA{R, c->ldN, c->N, c->J},
-                                         LoadTBetaGP{B, c->P, g0, c->M, c->J}, G, (int64_t)c->ldN,
-                                         (const int*)nullptr);
-  GPL_LAUNCHED(c, "k_gemm_store(resid_gp)");
   return GPL_OK;
 }
 

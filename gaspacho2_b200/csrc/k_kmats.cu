@@ -232,9 +232,9 @@ __global__ void k_expand(int P, int p, int g0, int M, const int* __restrict__ mk
   D[r + (size_t)col * P] = v;
 }
 
-int launch_kernel_mats(Ctx* c) { return launch_kernel_mats_lv(c, c->kernel_lv); }
-
-int launch_kernel_mats_lv(Ctx* c, int lv) {
+// Knm, Kmm and its factor, Kmm^{-1} k_n and titsias over the latent dimensions of c->kernel_lv.
+int launch_kernel_mats(Ctx* c) {
+  const int lv = c->kernel_lv;
   double* Knm = c->Dm + (size_t)c->dg0 * c->ldN;
   if (lv == kLvNone) {
     ProfScope ps(c, "kernel_mats");
@@ -246,15 +246,22 @@ int launch_kernel_mats_lv(Ctx* c, int lv) {
   }
   {
     ProfScope ps(c, "kernel_mats");
-    dim3 g(div_up(c->N, 128), c->M);
-    k_knm<<<g, 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Q, lv, c->X, c->T, c->rho, Knm);
-    GPL_LAUNCHED(c, "k_knm");
     dim3 g2(div_up(c->M, 64), c->M);
     k_kmm<<<g2, 64, 0, c->stream>>>(c->M, c->Q, lv, c->T, c->rho, c->Kmm, c->Kinv);
     GPL_LAUNCHED(c, "k_kmm");
   }
-  int rc = launch_chol_single(c, c->Kinv, c->M);
-  if (rc) return rc;
+  const int rc = launch_chol_single(c, c->Kinv, c->M);
+  return rc ? rc : launch_kernel_cells(c);
+}
+
+int launch_kernel_cells(Ctx* c) {
+  double* Knm = c->Dm + (size_t)c->dg0 * c->ldN;
+  {
+    ProfScope ps(c, "kernel_mats");
+    dim3 g(div_up(c->N, 128), c->M);
+    k_knm<<<g, 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Q, c->kernel_lv, c->X, c->T, c->rho, Knm);
+    GPL_LAUNCHED(c, "k_knm");
+  }
   ProfScope ps(c, "kinvkmn");
   auto fn = c->M <= 32 ? k_kmm_solve<false, true> : k_kmm_solve<false, false>;
   fn<<<div_up(c->N, kSolveCells), kSolveCells, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,

@@ -21,7 +21,7 @@
 //
 //   k_place_counts  the dense counts Y (cell x gene, cell fastest) from the CSR's matched prefix
 //   k_place_resid   per cell over all genes: R = y - W (for the gradient GEMM), l_i and sum_j W
-//   k_place_grad    per cell: d l / d x from G = R beta_GP^T (FFMA GEMM) and the kernel rows
+//   k_place_grad    per cell: d l / d x from G = R beta_GP^T (FP64 tensor cores) and the kernel rows
 //   k_place_dir     per cell: the L-BFGS step (on f = -l) and the trial point
 //   k_place_accept  per cell: the line-search decision
 #include <math.h>
@@ -32,8 +32,6 @@
 #include "gpl_internal.cuh"
 
 namespace gpl {
-
-int launch_resid_gp(Ctx* c, const double* R, const double* B, double* G);  // k_gemm.cu
 
 #define PLACE_RUN(expr)            \
   do {                             \
@@ -52,23 +50,73 @@ __global__ void k_place_counts(int ldN, const int32_t* __restrict__ cell, const 
   for (int64_t l = b + threadIdx.x; l < e; l += blockDim.x) Y[(size_t)j * ldN + cell[l]] = cnt[l];
 }
 
-__global__ void k_place_resid(int N, int ldN, int J, int Q, int pvars, const double* __restrict__ E,
-                              const double* __restrict__ Y, const double* __restrict__ ls,
-                              const double* __restrict__ delta, const double* __restrict__ titsias,
-                              const double* __restrict__ X, double* __restrict__ R, double* __restrict__ obj,
-                              double* __restrict__ wsum) {
+// Residuals and per-cell sums over the genes: a block takes 64 cells (two per lane, 16-byte accesses)
+// and its eight warps every eighth gene of the range of grid y, log(y!) of small counts from a table.
+// Parts per range: part[range][cell] of l_i and of sum_j W (ldN apart), added up by k_place_sums. Bound:
+// eta and the counts read, R written, one exp() per entry (a thread per cell over all genes, with an
+// lgamma() per count, took 1.77 ms at 20,003 cells x 2,000 genes; 0.25 ms so).
+constexpr int kFactorials = 256;
+__global__ void __launch_bounds__(256) k_place_resid(int N, int ldN, int J, int jper, int pvars,
+                                                     const double* __restrict__ E, const double* __restrict__ Y,
+                                                     const double* __restrict__ ls, const double* __restrict__ delta,
+                                                     const double* __restrict__ titsias, double* __restrict__ R,
+                                                     double* __restrict__ part) {
+  __shared__ double lf[kFactorials];
+  __shared__ double sh[2][8][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  lf[threadIdx.x] = lgamma((double)threadIdx.x + 1.0);
+  __syncthreads();
+  const int i = blockIdx.x * 64 + 2 * lane;  // even; ldN is a multiple of 32
+  const int j1 = min(J, (int)(blockIdx.y + 1) * jper);
+  double2 l = make_double2(0.0, 0.0), ws = l;
+  if (i < N) {
+    const bool two = i + 1 < N;
+    const double dgp = delta[pvars - 1] * kWt;
+    const double s0 = ls[i], s1 = two ? ls[i + 1] : 1.0;
+    const double f0 = s0 * exp(dgp * titsias[i]), f1 = two ? s1 * exp(dgp * titsias[i + 1]) : 0.0;
+    const double g0 = log(s0), g1 = log(s1);
+    auto logfact = [&](double y) {  // log(y!) of a count
+      const int k = (int)y;
+      return k < kFactorials && (double)k == y ? lf[k] : lgamma(y + 1.0);
+    };
+#pragma unroll 2
+    for (int j = blockIdx.y * jper + warp; j < j1; j += 8) {
+      const size_t e = (size_t)j * ldN + i;
+      const double2 eta = *reinterpret_cast<const double2*>(E + e), y = *reinterpret_cast<const double2*>(Y + e);
+      const double w0 = exp(eta.x) * f0, w1 = exp(eta.y) * f1;
+      if (R) *reinterpret_cast<double2*>(R + e) = make_double2(y.x - w0, y.y - w1);
+      l.x += y.x * (eta.x + g0) - w0;
+      if (y.x > 0.0) l.x -= logfact(y.x);  // the full Poisson log-probability (constant in x)
+      ws.x += w0;
+      if (two) {
+        l.y += y.y * (eta.y + g1) - w1;
+        if (y.y > 0.0) l.y -= logfact(y.y);
+        ws.y += w1;
+      }
+    }
+  }
+  sh[0][warp][2 * lane] = l.x;
+  sh[0][warp][2 * lane + 1] = l.y;
+  sh[1][warp][2 * lane] = ws.x;
+  sh[1][warp][2 * lane + 1] = ws.y;
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    const int q = threadIdx.x >> 6, c = threadIdx.x & 63;
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) t += sh[q][k][c];
+    if (blockIdx.x * 64 + c < N) part[((size_t)blockIdx.y * 2 + q) * ldN + blockIdx.x * 64 + c] = t;
+  }
+}
+
+__global__ void k_place_sums(int N, int ldN, int Q, int ns, const double* __restrict__ part,
+                             const double* __restrict__ X, double* __restrict__ obj, double* __restrict__ wsum) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double lsi = ls[i], lls = log(lsi), tt = delta[pvars - 1] * titsias[i] * kWt;
   double l = 0.0, ws = 0.0;
-  for (int j = 0; j < J; j++) {
-    const size_t e = (size_t)j * ldN + i;
-    const double eta = E[e], y = Y[e];
-    const double w = exp(eta) * lsi * exp(tt);
-    if (R) R[e] = y - w;
-    l += y * (eta + lls) - w;
-    if (y > 0.0) l -= lgamma(y + 1.0);  // the full Poisson log-probability (constant in x)
-    ws += w;
+  for (int k = 0; k < ns; k++) {
+    l += part[(size_t)k * 2 * ldN + i];
+    ws += part[((size_t)k * 2 + 1) * ldN + i];
   }
   for (int q = 1; q < Q; q++) {  // N(0, 1) prior on the ARD dimensions
     const double x = X[i + (size_t)q * N];
@@ -78,25 +126,49 @@ __global__ void k_place_resid(int N, int ldN, int J, int Q, int pvars, const dou
   wsum[i] = ws;
 }
 
-// d l_i / d x_iq (stored as g[i + q N], the ascent direction of l)
-__global__ void k_place_grad(int N, int ldN, int M, int Q, int pvars, const double* __restrict__ X,
-                             const double* __restrict__ T, const double* __restrict__ rho,
-                             const double* __restrict__ Knm, const double* __restrict__ KinvKmn,
-                             const double* __restrict__ G, const double* __restrict__ wsum,
-                             const double* __restrict__ delta, double* __restrict__ g) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const double tw = kWt * delta[pvars - 1] * wsum[i];
+// d l_i / d x_iq (stored as g[i + q N], the ascent direction of l): 32 cells per block (a lane each),
+// its eight warps every eighth inducing point, their sums added in order.
+__global__ void __launch_bounds__(256) k_place_grad(int N, int ldN, int M, int Q, int pvars,
+                                                    const double* __restrict__ X, const double* __restrict__ T,
+                                                    const double* __restrict__ rho, const double* __restrict__ Knm,
+                                                    const double* __restrict__ KinvKmn, const double* __restrict__ G,
+                                                    const double* __restrict__ wsum, const double* __restrict__ delta,
+                                                    double* __restrict__ g) {
+  extern __shared__ double sums[];  // [8][Q][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   double acc[16];
-  for (int q = 0; q < Q; q++) acc[q] = 0.0;
-  for (int k = 0; k < M; k++) {
-    const double K = Knm[(size_t)k * ldN + i];
-    const double C = (G[(size_t)k * ldN + i] + tw * KinvKmn[(size_t)k * ldN + i]) * K;
-    acc[0] -= C * sin(X[i] - T[k]) / (2.0 * rho[0]);
-    for (int q = 1; q < Q; q++) acc[q] -= C * (X[i + (size_t)q * N] - T[k + (size_t)q * M]) / rho[q];
+#pragma unroll
+  for (int q = 0; q < 16; q++) acc[q] = 0.0;
+  if (i < N) {
+    const double tw = kWt * delta[pvars - 1] * wsum[i];
+    double x[16], ir[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      x[q] = q < Q ? X[i + (size_t)q * N] : 0.0;
+      ir[q] = q < Q ? 1.0 / rho[q] : 0.0;
+    }
+    for (int k = warp; k < M; k += 8) {
+      const double K = Knm[(size_t)k * ldN + i];
+      const double C = (G[(size_t)k * ldN + i] + tw * KinvKmn[(size_t)k * ldN + i]) * K;
+      acc[0] -= C * sin(x[0] - T[k]) * (0.5 * ir[0]);
+#pragma unroll
+      for (int q = 1; q < 16; q++)
+        if (q < Q) acc[q] -= C * (x[q] - T[k + (size_t)q * M]) * ir[q];
+    }
   }
-  for (int q = 1; q < Q; q++) acc[q] -= X[i + (size_t)q * N];  // the prior's gradient
-  for (int q = 0; q < Q; q++) g[i + (size_t)q * N] = acc[q];
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+    if (q < Q) sums[(warp * Q + q) * 32 + lane] = acc[q];
+  __syncthreads();
+  for (int q = warp; q < Q; q += 8) {
+    if (i >= N) continue;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) s += sums[(k * Q + q) * 32 + lane];
+    if (q > 0) s -= X[i + (size_t)q * N];  // the prior's gradient
+    g[i + (size_t)q * N] = s;
+  }
 }
 
 // The step of cell i on f = -l (gradient gf = -g): the first iteration -gf/1e5, then the two-loop
@@ -201,33 +273,50 @@ __global__ void k_fill_int(int n, int v, int* __restrict__ a) {
   if (i < n) a[i] = v;
 }
 
+// The placement's buffers, in the context's work buffer
 struct PlaceBufs {
-  double *X0 = nullptr, *d = nullptr, *g = nullptr, *g_old = nullptr, *S = nullptr, *Yh = nullptr;
-  double *f = nullptr, *f_old = nullptr, *sr = nullptr, *wsum = nullptr;
-  int *searching = nullptr, *n_open = nullptr;
-  void release() {
-    void* b[] = {X0, d, g, g_old, S, Yh, f, f_old, sr, wsum, searching, n_open};
-    for (void* p : b)
-      if (p) cudaFree(p);
-  }
+  double *X0, *d, *g, *g_old, *S, *Yh, *f, *f_old, *sr, *wsum;
+  int *searching, *n_open;
 };
+
+int place_bufs(Ctx* c, PlaceBufs* pb) {
+  const size_t nq = (size_t)c->N * c->Q, n = c->N;
+  const int rc = ensure_work(c, (4 + 2 * kMem) * nq + 5 * n + 1);
+  if (rc) return rc;
+  double* w = c->work;
+  auto take = [&](size_t k) {
+    double* p = w;
+    w += k;
+    return p;
+  };
+  *pb = PlaceBufs{take(nq), take(nq), take(nq), take(nq), take(nq * kMem), take(nq * kMem),
+                  take(n),  take(n),  take(n),  take(n),  nullptr,         nullptr};
+  pb->searching = reinterpret_cast<int*>(take(n));
+  pb->n_open = reinterpret_cast<int*>(take(1));
+  return GPL_OK;
+}
 
 }  // namespace
 
-// The objective of every cell at the X on the device (and, with `grad`, its gradient into pb.g).
-static int place_eval(Ctx* c, PlaceBufs& pb, double* f, bool grad) {
-  int rc = launch_kernel_mats(c);
+// The objective of every cell at the X on the device (and, with `grad`, its gradient into pb.g). The
+// inducing points and length-scales stay as they are during a call, so Kmm and its factor are formed
+// by the first evaluation only (first).
+static int place_eval(Ctx* c, PlaceBufs& pb, double* f, bool grad, bool first) {
+  int rc = first ? launch_kernel_mats(c) : launch_kernel_cells(c);
   if (rc) return rc;
   if ((rc = launch_zbeta(c, c->Beta, c->scratch))) return rc;  // eta
-  k_place_resid<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->J, c->Q, c->p, c->scratch, c->Nu, c->ls,
-                                                          c->delta, c->titsias, c->X, grad ? c->W : nullptr, f,
-                                                          pb.wsum);
+  const int bx = div_up(c->N, 64), ns = cell_sum_ranges(c);
+  if ((rc = ensure_part(c, (size_t)2 * ns * c->ldN))) return rc;
+  k_place_resid<<<dim3(bx, ns), 256, 0, c->stream>>>(c->N, c->ldN, c->J, div_up(c->J, ns), c->p, c->scratch, c->Nu,
+                                                     c->ls, c->delta, c->titsias, grad ? c->W : nullptr, c->part);
   GPL_LAUNCHED(c, "k_place_resid");
+  k_place_sums<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->Q, ns, c->part, c->X, f, pb.wsum);
+  GPL_LAUNCHED(c, "k_place_sums");
   if (!grad) return GPL_OK;
-  if ((rc = launch_resid_gp(c, c->W, c->Beta, c->C1))) return rc;
+  if ((rc = dgen_resid_gp(c, c->W, c->Beta, c->C1))) return rc;
   const double* Knm = c->Dm + (size_t)c->dg0 * c->ldN;
-  k_place_grad<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Q, c->p, c->X, c->T, c->rho, Knm,
-                                                         c->KinvKmn, c->C1, pb.wsum, c->delta, pb.g);
+  k_place_grad<<<div_up(c->N, 32), 256, sizeof(double) * 8 * 32 * c->Q, c->stream>>>(
+      c->N, c->ldN, c->M, c->Q, c->p, c->X, c->T, c->rho, Knm, c->KinvKmn, c->C1, pb.wsum, c->delta, pb.g);
   GPL_LAUNCHED(c, "k_place_grad");
   return GPL_OK;
 }
@@ -240,18 +329,8 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
   }
   PlaceBufs pb;
   const size_t nq = (size_t)N * Q;
-  auto al = [&](auto** p, size_t n) {
-    return cudaMalloc((void**)p, sizeof(**p) * (n ? n : 1)) == cudaSuccess;
-  };
-  if (!al(&pb.X0, nq) || !al(&pb.d, nq) || !al(&pb.g, nq) || !al(&pb.g_old, nq) || !al(&pb.S, nq * kMem) ||
-      !al(&pb.Yh, nq * kMem) || !al(&pb.f, N) || !al(&pb.f_old, N) || !al(&pb.sr, N) || !al(&pb.wsum, N) ||
-      !al(&pb.searching, N) || !al(&pb.n_open, 1)) {
-    cudaGetLastError();
-    pb.release();
-    c->err = "device allocation failed: placement buffers";
-    return GPL_ERR_ALLOC;
-  }
-  int rc = GPL_OK;
+  int rc = place_bufs(c, &pb);
+  if (rc) return rc;
   int evals = 0, tries = 0;
   auto run = [&]() -> int {
     GPL_TRY(c, cudaMemcpyAsync(c->X, X_host, sizeof(double) * nq, cudaMemcpyHostToDevice, c->stream));
@@ -259,7 +338,7 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
     GPL_TRY(c, cudaMemsetAsync(c->Nu, 0, sizeof(double) * (size_t)c->ldN * c->J, c->stream));
     k_place_counts<<<c->J, 256, 0, c->stream>>>(c->ldN, c->cell, c->gptr, c->gvalid, c->cnt, c->Nu);
     GPL_LAUNCHED(c, "k_place_counts");
-    PLACE_RUN(place_eval(c, pb, pb.f_old, true));
+    PLACE_RUN(place_eval(c, pb, pb.f_old, true, true));
     evals++;
     const int nb = div_up(N, 128);
     for (int it = 0; it < iters; it++) {
@@ -268,7 +347,7 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
       k_fill_int<<<nb, 128, 0, c->stream>>>(N, 1, pb.searching);
       GPL_LAUNCHED(c, "k_fill_int");
       for (int ktr = 1; ktr < 8; ktr++) {
-        PLACE_RUN(place_eval(c, pb, pb.f, false));
+        PLACE_RUN(place_eval(c, pb, pb.f, false, false));
         evals++;
         tries++;
         GPL_TRY(c, cudaMemsetAsync(pb.n_open, 0, sizeof(int), c->stream));
@@ -281,7 +360,7 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
         if (open == 0) break;
       }
       GPL_TRY(c, cudaMemcpyAsync(pb.g_old, pb.g, sizeof(double) * nq, cudaMemcpyDeviceToDevice, c->stream));
-      PLACE_RUN(place_eval(c, pb, pb.f_old, true));
+      PLACE_RUN(place_eval(c, pb, pb.f_old, true, false));
       evals++;
       k_place_hist<<<nb, 128, 0, c->stream>>>(N, Q, it, c->X, pb.X0, pb.g, pb.g_old, pb.S, pb.Yh);
       GPL_LAUNCHED(c, "k_place_hist");
@@ -292,7 +371,6 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
     return GPL_OK;
   };
   rc = run();
-  pb.release();
   if (stats) {
     stats[0] = iters;
     stats[1] = evals;
@@ -309,27 +387,20 @@ int cell_objective(Ctx* c, const double* X_host, double* obj_host, double* grad_
     return GPL_ERR_ARG;
   }
   PlaceBufs pb;
-  if (cudaMalloc((void**)&pb.f, sizeof(double) * N) != cudaSuccess ||
-      cudaMalloc((void**)&pb.wsum, sizeof(double) * N) != cudaSuccess ||
-      (grad_host && cudaMalloc((void**)&pb.g, sizeof(double) * nq) != cudaSuccess)) {
-    cudaGetLastError();
-    pb.release();
-    c->err = "device allocation failed: placement buffers";
-    return GPL_ERR_ALLOC;
-  }
+  int rc = place_bufs(c, &pb);
+  if (rc) return rc;
   auto run = [&]() -> int {
     GPL_TRY(c, cudaMemcpyAsync(c->X, X_host, sizeof(double) * nq, cudaMemcpyHostToDevice, c->stream));
     GPL_TRY(c, cudaMemsetAsync(c->Nu, 0, sizeof(double) * (size_t)c->ldN * c->J, c->stream));
     k_place_counts<<<c->J, 256, 0, c->stream>>>(c->ldN, c->cell, c->gptr, c->gvalid, c->cnt, c->Nu);
     GPL_LAUNCHED(c, "k_place_counts");
-    PLACE_RUN(place_eval(c, pb, pb.f, grad_host != nullptr));
+    PLACE_RUN(place_eval(c, pb, pb.f, grad_host != nullptr, true));
     GPL_TRY(c, cudaMemcpyAsync(obj_host, pb.f, sizeof(double) * N, cudaMemcpyDeviceToHost, c->stream));
     if (grad_host) GPL_TRY(c, cudaMemcpyAsync(grad_host, pb.g, sizeof(double) * nq, cudaMemcpyDeviceToHost, c->stream));
     GPL_TRY(c, cudaStreamSynchronize(c->stream));
     return GPL_OK;
   };
-  const int rc = run();
-  pb.release();
+  rc = run();
   return rc;
 }
 

@@ -14,6 +14,11 @@
 
 namespace gpl {
 
+// Gene ranges of a sum per cell over all genes in blocks of 64 cells: about six blocks per SM, 32 genes at least.
+int cell_sum_ranges(const Ctx* c) {
+  return std::max(1, std::min(6 * c->sm_count / div_up(c->N, 64), c->J / 32));
+}
+
 namespace {
 constexpr int kOinvt = 0, kTn = 1;
 
@@ -72,10 +77,6 @@ __global__ void k_cell_sums_add(int N, int ldN, int ns, const double* __restrict
   out[i] = cell_sum_out<MODE>(s, Omega[i]);
 }
 
-int cell_sum_ranges(const Ctx* c) {
-  return std::max(1, std::min(6 * c->sm_count / div_up(c->N, 64), c->J / 32));
-}
-
 template <int MODE>
 int launch_cell_sums(Ctx* c, const double* E, double* out) {
   const int bx = div_up(c->N, 64), ns = cell_sum_ranges(c);
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(256) k_state_sums(int N, const double* __restr
 }
 }  // namespace
 
-size_t cell_sums_part(const Ctx* c) { return (size_t)cell_sum_ranges(c) * c->ldN; }
+size_t cell_sums_part(const Ctx* c) { return (size_t)2 * cell_sum_ranges(c) * c->ldN; }  // two sums: the placement's
 
 int launch_oinvt(Ctx* c) {
   ProfScope ps(c, "oinvt");
