@@ -7,8 +7,9 @@
 // FP32 accumulation in TMEM), operands staged by TMA in 128-byte-swizzled K-major tiles.
 //
 //   k_mlp_gemm     C[m, n] = sum_k A[m, k] B[n, k], A and B BF16 K-major (row = output index,
-//                  K contiguous), one 128 x 128 output tile per CTA, K in 64-wide chunks through
-//                  a 4-stage TMA pipeline; warp 0 issues the TMA loads, warp 1 the MMAs (one
+//                  K contiguous), one 128 x 32 (training, the output layer) or 128 x 128 (the hidden
+//                  layers of a prediction) output tile per CTA, K in 64-wide chunks through a 4-stage
+//                  TMA pipeline; warp 0 issues the TMA loads, warp 1 the MMAs (one
 //                  thread), warps 2-5 read the accumulator and run the epilogue:
 //                    kFwdGelu  v = acc + b[n]; pre = v (FP32); act = bf16(gelu(v)) in both the
 //                              K-major layout (next layer's A) and transposed (the weight
@@ -17,16 +18,18 @@
 //                    kBwdGelu  d = acc * gelu'(pre); dpre = d (FP32, bias gradient); bf16(d) in
 //                              both layouts
 //                    kStore    out = acc (FP32: weight gradients)
+//                    kPredGelu act = bf16(gelu(acc + b[n])), K-major only (nothing is differentiated)
+//                  A lane holds 32 neighbouring columns of a row, stored as 16-byte pieces.
 //                  Every mbarrier wait is bounded; a wait that runs out records an error code,
 //                  the MMA thread waits (bounded) for its MMAs before TMEM is freed.
 //   k_enc_features log1p(y / s) of the selected genes' counts, written as BF16 into the
 //                  cell-major feature matrix F and its transpose FT (rows = features).
 //   k_enc_loss     the Gaussian negative log-likelihood of the targets per cell and the
 //                  output gradient, FP32 and BF16 (both layouts).
-//   k_colsum       bias gradients: column sums over the batch, one thread per column, rows in
-//                  order (deterministic).
+//   k_enc_sums     bias gradients and the batch loss: sums over the batch in a fixed order.
 //   k_adam         Adam on the FP32 masters, then the BF16 copies the GEMMs read (and the
-//                  transposed copies of W2 and W3 for the backward products).
+//                  transposed copies of W2 and W3 for the backward products), all blocks at once.
+//   k_enc_scatter  predicted rows to the cells' places.
 //
 // Layout (device, all row-major): F [Npad][Kin] and FT [Kin][Npad] (Kin = n_in rounded up to 128,
 // Npad = cells rounded up to the batch), per-batch activations [B][H] and transposes [H][B],
@@ -51,9 +54,8 @@ namespace {
 constexpr int kThreads = 192;
 constexpr int kStages = 4;
 constexpr int kTile = 128 * 128;  // bytes of a 128-row x 64-column BF16 tile
-constexpr uint32_t kIdesc = idesc_bf16_f32(128, 128);
 
-enum Epi { kFwdGelu = 0, kFwdOut = 1, kBwdGelu = 2, kStore = 3 };
+enum Epi { kFwdGelu = 0, kFwdOut = 1, kBwdGelu = 2, kStore = 3, kPredGelu = 4 };
 
 struct EpiArgs {
   int mode, m_valid, n_valid;
@@ -61,7 +63,7 @@ struct EpiArgs {
   const float* pre_in;     // kBwdGelu: the forward pre-activations [m][ld32]
   float* out32;            // pre (kFwdGelu), out (kFwdOut, kStore), dpre (kBwdGelu): [m][ld32]
   int ld32;
-  __nv_bfloat16* act;      // [m][ldb] (kFwdGelu, kBwdGelu)
+  __nv_bfloat16* act;      // [m][ldb] (kFwdGelu, kBwdGelu, kPredGelu)
   int ldb;
   __nv_bfloat16* actT;     // [n][ldt] (kFwdGelu, kBwdGelu)
   int ldt;
@@ -86,16 +88,19 @@ __device__ __forceinline__ void mlp_fail(int* err, MlpShared* sh, int code) {
   atomicCAS(err, 0, code);
 }
 
+template <int NT>
 __global__ void __launch_bounds__(kThreads, 1)
     k_mlp_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int nch,
                int a_x0, int a_y0, int b_x0, int b_y0, EpiArgs ep, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* As = base;
+  constexpr int kTileN = NT * 128;  // NT rows x 64 BF16
+  constexpr uint32_t kIdesc = idesc_bf16_f32(128, NT);
   unsigned char* Bs = As + kStages * kTile;
-  MlpShared* sh = (MlpShared*)(Bs + kStages * kTile);
+  MlpShared* sh = (MlpShared*)(Bs + kStages * kTileN);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * 128;
+  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * NT;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -110,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (sh->abort) return;
   if (warp == 0) {
-    tmem_alloc(&sh->tmem, 128);
+    tmem_alloc(&sh->tmem, NT);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -128,9 +133,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         if (*(volatile int*)&sh->abort) break;
-        mbar_arrive_expect_tx(&sh->full[s], 2u * kTile);
+        mbar_arrive_expect_tx(&sh->full[s], kTile + kTileN);
         tma_load_2d(As + s * kTile, &map_a, &sh->full[s], a_x0 + it * 64, a_y0 + m0);
-        tma_load_2d(Bs + s * kTile, &map_b, &sh->full[s], b_x0 + it * 64, b_y0 + n0);
+        tma_load_2d(Bs + s * kTileN, &map_b, &sh->full[s], b_x0 + it * 64, b_y0 + n0);
         issued = it + 1;
       }
       // copies still in flight land before the CTA may exit
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (*(volatile int*)&sh->abort) break;
         tc_fence_after();
-        const uint32_t a = smem_u32(As + s * kTile), b = smem_u32(Bs + s * kTile);
+        const uint32_t a = smem_u32(As + s * kTile), b = smem_u32(Bs + s * kTileN);
 #pragma unroll
         for (int k = 0; k < 4; k++)
           mma_bf16(tmem, umma_desc_sw128(a + k * 32), umma_desc_sw128(b + k * 32), kIdesc, (it | k) ? 1u : 0u);
@@ -169,32 +174,61 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (!__any_sync(0xffffffffu, *(volatile int*)&sh->abort != 0)) {
       tc_fence_after();
       const bool live_m = m < ep.m_valid;
-      for (int cb = 0; cb < 128; cb += 32) {
+      for (int cb = 0; cb < NT; cb += 32) {
         float v[32];
         tmem_ld32(lane_addr + cb, v);  // warp-wide: every lane loads
         if (!live_m) continue;
-#pragma unroll 4
-        for (int k = 0; k < 32; k++) {
-          const int n = n0 + cb + k;
-          if (n >= ep.n_valid) break;
-          const float a = v[k];
-          if (ep.mode == kStore) {
-            ep.out32[(size_t)m * ep.ld32 + n] = a;
-          } else if (ep.mode == kFwdOut) {
-            ep.out32[(size_t)m * ep.ld32 + n] = a + ep.bias[n];
-          } else if (ep.mode == kFwdGelu) {
-            const float pre = a + ep.bias[n];
-            ep.out32[(size_t)m * ep.ld32 + n] = pre;
-            const __nv_bfloat16 h = __float2bfloat16_rn(gelu_f(pre));
-            ep.act[(size_t)m * ep.ldb + n] = h;
-            ep.actT[(size_t)n * ep.ldt + m] = h;
-          } else {  // kBwdGelu
-            const float d = a * gelu_grad_f(ep.pre_in[(size_t)m * ep.ld32 + n]);
-            ep.out32[(size_t)m * ep.ld32 + n] = d;
-            const __nv_bfloat16 h = __float2bfloat16_rn(d);
-            ep.act[(size_t)m * ep.ldb + n] = h;
-            ep.actT[(size_t)n * ep.ldt + m] = h;
+        const int nb = n0 + cb, nv = ep.n_valid - nb;  // columns of this piece that exist
+        if (nv <= 0) continue;
+        float* o = ep.out32 + (size_t)m * ep.ld32 + nb;
+        if (ep.mode == kFwdGelu || ep.mode == kBwdGelu || ep.mode == kPredGelu) {
+          // hidden layers: n_valid is a multiple of 128, so the piece is whole
+          float x[32];
+#pragma unroll
+          for (int k = 0; k < 32; k += 4) {
+            const float4 y = ep.mode == kBwdGelu
+                                 ? *reinterpret_cast<const float4*>(ep.pre_in + (size_t)m * ep.ld32 + nb + k)
+                                 : *reinterpret_cast<const float4*>(ep.bias + nb + k);
+            x[k] = y.x;
+            x[k + 1] = y.y;
+            x[k + 2] = y.z;
+            x[k + 3] = y.w;
           }
+          uint32_t h[16];
+#pragma unroll
+          for (int k = 0; k < 32; k += 2) {
+            __nv_bfloat162 p;
+            if (ep.mode == kBwdGelu) {
+              v[k] = v[k] * gelu_grad_f(x[k]);
+              v[k + 1] = v[k + 1] * gelu_grad_f(x[k + 1]);
+              p = __floats2bfloat162_rn(v[k], v[k + 1]);
+            } else {
+              v[k] = v[k] + x[k];
+              v[k + 1] = v[k + 1] + x[k + 1];
+              p = __floats2bfloat162_rn(gelu_f(v[k]), gelu_f(v[k + 1]));
+            }
+            h[k / 2] = *reinterpret_cast<uint32_t*>(&p);
+          }
+          uint4* act = reinterpret_cast<uint4*>(ep.act + (size_t)m * ep.ldb + nb);
+#pragma unroll
+          for (int k = 0; k < 4; k++) act[k] = make_uint4(h[4 * k], h[4 * k + 1], h[4 * k + 2], h[4 * k + 3]);
+          if (ep.mode == kPredGelu) continue;
+#pragma unroll
+          for (int k = 0; k < 32; k += 4)
+            *reinterpret_cast<float4*>(o + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+#pragma unroll
+          for (int k = 0; k < 32; k++) {
+            const uint16_t bits = (uint16_t)(h[k / 2] >> (16 * (k & 1)));
+            ep.actT[(size_t)(nb + k) * ep.ldt + m] = *reinterpret_cast<const __nv_bfloat16*>(&bits);
+          }
+        } else if (ep.mode == kStore && nv >= 32) {
+#pragma unroll
+          for (int k = 0; k < 32; k += 4)
+            *reinterpret_cast<float4*>(o + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 32; k++)
+            if (k < nv) o[k] = ep.mode == kFwdOut ? v[k] + ep.bias[nb + k] : v[k];
         }
       }
     }
@@ -202,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_dealloc(tmem, 128);
+  if (warp == 0) tmem_dealloc(tmem, NT);
 }
 
 // log1p(y / s) of feature f's gene for the cells of its matched counts; rows in `row_of` order.
@@ -249,31 +283,68 @@ __global__ void k_enc_loss(int rows, int Q, const float* __restrict__ out, int l
   loss_rows[r] = 0.5f * l;
 }
 
-// out[n] = sum_{r < rows} d[r][n] for n < cols (rows in order)
-__global__ void k_colsum(int rows, int cols, const float* __restrict__ d, int ld, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; r++) s += d[(size_t)r * ld + n];
-  out[n] = s;
+// The batch's sums over its rows: the bias gradients out[n] = sum_r d[r][n] of the three layers in row
+// order, 32 columns per block (its threads stage 64 rows at a time, two buffers, while a lane per column
+// adds), and in the last block the batch loss in double. Bound by the chain of additions: 1,024 rows
+// take 21 us for all four, where a thread per column that waited on its loads took 58 us for each layer
+// and one thread 25 us for the loss.
+struct EncSums {
+  const float* d[3];
+  float* out[3];
+  int cols[3], ld[3];
+  const float* loss_rows;
+  double* loss;
+};
+__global__ void __launch_bounds__(256) k_enc_sums(int rows, EncSums a) {
+  __shared__ float buf[2][64][32];
+  __shared__ double part[256];
+  int block = blockIdx.x, layer = 0;
+  while (layer < 3 && block >= (a.cols[layer] + 31) / 32) block -= (a.cols[layer++] + 31) / 32;
+  const int tid = threadIdx.x, w = tid >> 5, c = tid & 31;
+  if (layer == 3) {
+    double t = 0.0;
+    for (int r = tid; r < rows; r += 256) t += a.loss_rows[r];
+    part[tid] = t;
+    __syncthreads();
+    for (int k = 128; k > 0; k >>= 1) {
+      if (tid < k) part[tid] += part[tid + k];
+      __syncthreads();
+    }
+    if (tid == 0) *a.loss = part[0];
+    return;
+  }
+  const int ld = a.ld[layer];
+  const bool in = block * 32 + c < a.cols[layer];
+  const float* src = a.d[layer] + block * 32 + c;
+  float v[8], s = 0.f;
+  auto load = [&](int r0) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = in && r0 + q * 8 + w < rows ? src[(size_t)(r0 + q * 8 + w) * ld] : 0.f;
+  };
+  load(0);
+  for (int r0 = 0, b = 0; r0 < rows; r0 += 64, b ^= 1) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) buf[b][q * 8 + w][c] = v[q];
+    __syncthreads();
+    // the buffer written next is the one warp 0 read before this barrier
+    if (r0 + 64 < rows) load(r0 + 64);
+    if (w == 0) {
+#pragma unroll
+      for (int r = 0; r < 64; r++) s += buf[b][r][c];  // a batch is a multiple of 128 rows
+    }
+  }
+  if (w == 0 && in) a.out[layer][block * 32 + c] = s;
 }
 
-// sum of a small array in order (one thread): the batch loss
-__global__ void k_sum_ordered(int n, const float* __restrict__ a, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < n; i++) s += a[i];
-  *out = s;
-}
-
-// Adam on one parameter block of rows x cols (FP32 master w, gradient g, moments m, v), then
-// the BF16 copy wb[r][c] (row-major ld ldw) and, if given, the transposed copy wt[c][r] (ld ldwt).
-__global__ void k_adam(int rows, int cols, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* __restrict__ wb, int ldw, __nv_bfloat16* __restrict__ wt, int ldwt) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= rows * cols) return;
-  const int r = e / cols, c = e - r * cols;
+// Adam on the flat parameters W1 [H][Kin] b1 [H] W2 [H][H] b2 [H] W3 [2Q][H] b3 [2Q] (FP32 master w,
+// gradient g, moments m, v), with the weights' BF16 copies and their transposes (W2T [H][H], W3T [H][64]).
+__global__ void k_adam(int H, int Kin, int Q2, size_t n, float* __restrict__ w, const float* __restrict__ g,
+                       float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps, float c1,
+                       float c2, __nv_bfloat16* __restrict__ W1b, __nv_bfloat16* __restrict__ W2b,
+                       __nv_bfloat16* __restrict__ W2T, __nv_bfloat16* __restrict__ W3b,
+                       __nv_bfloat16* __restrict__ W3T) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
   const float gr = g[e];
   const float mm = b1 * m[e] + (1.f - b1) * gr;
   const float vv = b2 * v[e] + (1.f - b2) * gr * gr;
@@ -281,8 +352,32 @@ __global__ void k_adam(int rows, int cols, float* __restrict__ w, const float* _
   v[e] = vv;
   const float nw = w[e] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
   w[e] = nw;
-  if (wb) wb[(size_t)r * ldw + c] = __float2bfloat16_rn(nw);
-  if (wt) wt[(size_t)c * ldwt + r] = __float2bfloat16_rn(nw);
+  const __nv_bfloat16 h = __float2bfloat16_rn(nw);
+  const size_t o2 = (size_t)H * Kin + H, o3 = o2 + (size_t)H * H + H;
+  if (e < (size_t)H * Kin) {
+    W1b[e] = h;
+  } else if (e >= o2 && e < o2 + (size_t)H * H) {
+    const int k = (int)(e - o2), r = k / H, c = k - r * H;
+    W2b[k] = h;
+    W2T[(size_t)c * H + r] = h;
+  } else if (e >= o3 && e < o3 + (size_t)Q2 * H) {
+    const int k = (int)(e - o3), r = k / H, c = k - r * H;
+    W3b[k] = h;
+    W3T[(size_t)c * 64 + r] = h;
+  }
+}
+
+// Predicted rows [r0, r0 + rows) to the cells' places: mean[i + q N], logvar[i + q N]
+__global__ void k_enc_scatter(int rows, int r0, int N, int Q, const float* __restrict__ out, int ldo,
+                              const int32_t* __restrict__ cell_of_row, double* __restrict__ mean,
+                              double* __restrict__ logvar) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= rows) return;
+  const int i = cell_of_row[r0 + r];
+  for (int q = 0; q < Q; q++) {
+    mean[i + (size_t)q * N] = out[(size_t)r * ldo + q];
+    logvar[i + (size_t)q * N] = out[(size_t)r * ldo + Q + q];
+  }
 }
 
 // BF16 copies of an FP32 block (after the weights are set from the host)
@@ -319,13 +414,13 @@ EncodeTiledFn2 encode_fn2() {
   return fn;
 }
 
-// BF16 row-major [rows][cols] (cols a multiple of 64, rows a multiple of 128), box 64 x 128
-bool bf16_map(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows) {
+// BF16 row-major [rows][cols] (cols a multiple of 64, rows a multiple of the box's), box 64 x box_rows
+bool bf16_map(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows, uint32_t box_rows = 128) {
   EncodeTiledFn2 fn = encode_fn2();
   if (!fn) return false;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * 2};
-  const cuuint32_t box[2] = {64, 128};
+  const cuuint32_t box[2] = {64, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -362,10 +457,19 @@ struct gpl_enc {
     int N = 0, Npad = 0;
     __nv_bfloat16 *F = nullptr, *FT = nullptr;
     float* X = nullptr;  // targets [Npad][Q] in row order (training set)
+    int32_t* rows_d = nullptr;  // cell_of_row on the device
     std::vector<int32_t> cell_of_row;
     CUtensorMap mapF, mapFT;
   } set[2];
-  CUtensorMap mW1, mW2, mW2T, mW3, mW3T, mH1, mH1T, mH2, mH2T, mdq, mdqT, mdP2, mdP2T, mdP1T;
+  size_t n_loss = 1;  // batch losses held by loss_sum
+  // a prediction's rows at a time, its hidden layers and results (kept, grown to the largest set)
+  int pred_rows = 0, pred_cells = 0;
+  __nv_bfloat16 *pH1 = nullptr, *pH2 = nullptr;
+  float* pout = nullptr;
+  double* pres = nullptr;  // mean then logvar
+  // operands in 128-row boxes (A, and B of wide launches) and in 32-row boxes (B of narrow ones)
+  CUtensorMap mW1, mW2, mW3, mH1, mH2, mdq, mdqT, mdP2, mdP2T, mdP1T, mpH1, mpH2;
+  CUtensorMap nW1, nW2, nW2T, nW3, nW3T, nH1T, nH2T;
 };
 
 #define ENC_TRY(e, expr)                                                 \
@@ -398,17 +502,22 @@ int ealloc(gpl_enc* e, T** p, size_t n) {
   return cudaMemsetAsync(*p, 0, sizeof(T) * (n ? n : 1), e->stream) == cudaSuccess ? GPL_OK : GPL_ERR_CUDA;
 }
 
-constexpr int kSmem = 1024 + kStages * 2 * kTile + (int)sizeof(MlpShared);
+template <int NT>
+constexpr int mlp_smem() {
+  return 1024 + kStages * (kTile + NT * 128) + (int)sizeof(MlpShared);
+}
 
-int gemm(gpl_enc* e, const CUtensorMap& A, const CUtensorMap& Bm, int M, int N, int K, int a_x0, int a_y0, int b_x0,
+// C = A B^T over 128-row tiles of A and `cols` columns. A batch's products are a few tiles and bound by
+// their latency and epilogue: 32 columns per CTA put 1,024 x 256 outputs on 64 SMs instead of 16, and the
+// 275 launches of 16 batches of 1,024 (2,000 features) and 50,001 predicted rows went from 34 us to 11 us
+// each, with 16-byte stores. A prediction's hidden layers have tiles enough for 128 columns (51 us for
+// 32,768 rows), each row's features read by two CTAs. Bm: 32-row boxes for NT = 32, else 128.
+template <int NT>
+int gemm(gpl_enc* e, const CUtensorMap& A, const CUtensorMap& Bm, int M, int cols, int K, int a_x0, int a_y0, int b_x0,
          int b_y0, const EpiArgs& ep) {
-  static bool attr = false;
-  if (!attr) {
-    ENC_TRY(e, cudaFuncSetAttribute(k_mlp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    attr = true;
-  }
-  dim3 g(M / 128, N / 128);
-  k_mlp_gemm<<<g, kThreads, kSmem, e->stream>>>(A, Bm, K / 64, a_x0, a_y0, b_x0, b_y0, ep, e->err_d);
+  ENC_TRY(e, cudaFuncSetAttribute(k_mlp_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp_smem<NT>()));
+  dim3 g(M / 128, (cols + NT - 1) / NT);
+  k_mlp_gemm<NT><<<g, kThreads, mlp_smem<NT>(), e->stream>>>(A, Bm, K / 64, a_x0, a_y0, b_x0, b_y0, ep, e->err_d);
   ENC_LAUNCHED(e, "k_mlp_gemm");
   return GPL_OK;
 }
@@ -424,13 +533,12 @@ int check_err(gpl_enc* e) {
   return GPL_OK;
 }
 
-// Forward of rows [r0, r0 + B) of a cell set into the batch buffers (pre1/H1/H1T, pre2/H2/H2T,
-// out). m_valid limits the rows written (the last, partial batch of a prediction).
-int forward(gpl_enc* e, int s, int r0, int m_valid) {
+// Forward of training rows [r0, r0 + B) into the batch buffers (pre1/H1/H1T, pre2/H2/H2T, out).
+int forward(gpl_enc* e, int r0) {
   const int H = e->H, B = e->B;
   EpiArgs ep{};
   ep.mode = kFwdGelu;
-  ep.m_valid = m_valid;
+  ep.m_valid = B;
   ep.n_valid = H;
   ep.bias = e->b1;
   ep.out32 = e->pre1;
@@ -439,25 +547,51 @@ int forward(gpl_enc* e, int s, int r0, int m_valid) {
   ep.ldb = H;
   ep.actT = e->H1T;
   ep.ldt = B;
-  int rc = gemm(e, e->set[s].mapF, e->mW1, B, H, e->Kin, 0, r0, 0, 0, ep);
+  int rc = gemm<32>(e, e->set[0].mapF, e->nW1, B, H, e->Kin, 0, r0, 0, 0, ep);
   if (rc) return rc;
   ep.bias = e->b2;
   ep.out32 = e->pre2;
   ep.act = e->H2;
   ep.actT = e->H2T;
-  if ((rc = gemm(e, e->mH1, e->mW2, B, H, H, 0, 0, 0, 0, ep))) return rc;
+  if ((rc = gemm<32>(e, e->mH1, e->nW2, B, H, H, 0, 0, 0, 0, ep))) return rc;
   EpiArgs eo{};
   eo.mode = kFwdOut;
-  eo.m_valid = m_valid;
+  eo.m_valid = B;
   eo.n_valid = 2 * e->Q;
   eo.bias = e->b3;
   eo.out32 = e->out;
   eo.ld32 = 128;
-  return gemm(e, e->mH2, e->mW3, B, 128, H, 0, 0, 0, 0, eo);
+  return gemm<32>(e, e->mH2, e->nW3, B, 2 * e->Q, H, 0, 0, 0, 0, eo);
+}
+
+// The same layers without what only the gradient needs, for rows [r0, r0 + rows) of a cell set: the
+// per-row results do not depend on how many rows a launch takes.
+int predict_rows(gpl_enc* e, int s, int r0, int rows) {
+  const int H = e->H, M = rup(rows, 128);
+  EpiArgs ep{};
+  ep.mode = kPredGelu;
+  ep.m_valid = rows;
+  ep.n_valid = H;
+  ep.bias = e->b1;
+  ep.act = e->pH1;
+  ep.ldb = H;
+  int rc = gemm<128>(e, e->set[s].mapF, e->mW1, M, H, e->Kin, 0, r0, 0, 0, ep);
+  if (rc) return rc;
+  ep.bias = e->b2;
+  ep.act = e->pH2;
+  if ((rc = gemm<128>(e, e->mpH1, e->mW2, M, H, H, 0, 0, 0, 0, ep))) return rc;
+  EpiArgs eo{};
+  eo.mode = kFwdOut;
+  eo.m_valid = rows;
+  eo.n_valid = 2 * e->Q;
+  eo.bias = e->b3;
+  eo.out32 = e->pout;
+  eo.ld32 = 64;
+  return gemm<32>(e, e->mpH2, e->nW3, M, 2 * e->Q, H, 0, 0, 0, 0, eo);
 }
 
 // Loss and every gradient of one training batch (rows [r0, r0 + B) of set 0) into gW*, gb*.
-int backward(gpl_enc* e, int r0) {
+int backward(gpl_enc* e, int r0, double* loss) {
   const int H = e->H, B = e->B, Q = e->Q;
   gpl_enc::Set& S = e->set[0];
   k_enc_loss<<<(B + 127) / 128, 128, 0, e->stream>>>(B, Q, e->out, 128, S.X + (size_t)r0 * Q, e->loss_rows, e->d32,
@@ -469,7 +603,7 @@ int backward(gpl_enc* e, int r0) {
   st.n_valid = H;
   st.out32 = e->gW3;
   st.ld32 = H;
-  int rc = gemm(e, e->mdqT, e->mH2T, 128, H, B, 0, 0, 0, 0, st);  // dW3 = dO^T H2
+  int rc = gemm<32>(e, e->mdqT, e->nH2T, 128, H, B, 0, 0, 0, 0, st);  // dW3 = dO^T H2
   if (rc) return rc;
   EpiArgs bg{};
   bg.mode = kBwdGelu;
@@ -482,32 +616,38 @@ int backward(gpl_enc* e, int r0) {
   bg.ldb = H;
   bg.actT = e->dP2T;
   bg.ldt = B;
-  if ((rc = gemm(e, e->mdq, e->mW3T, B, H, 64, 0, 0, 0, 0, bg))) return rc;  // dA2 = (dO W3) * gelu'(a2)
+  if ((rc = gemm<32>(e, e->mdq, e->nW3T, B, H, 64, 0, 0, 0, 0, bg))) return rc;  // dA2 = (dO W3) * gelu'(a2)
   st.m_valid = H;
   st.out32 = e->gW2;
-  if ((rc = gemm(e, e->mdP2T, e->mH1T, H, H, B, 0, 0, 0, 0, st))) return rc;  // dW2 = dA2^T H1
+  if ((rc = gemm<32>(e, e->mdP2T, e->nH1T, H, H, B, 0, 0, 0, 0, st))) return rc;  // dW2 = dA2^T H1
   bg.pre_in = e->pre1;
   bg.out32 = e->dpre1;
   bg.act = e->dP1;
   bg.actT = e->dP1T;
-  if ((rc = gemm(e, e->mdP2, e->mW2T, B, H, H, 0, 0, 0, 0, bg))) return rc;  // dA1 = (dA2 W2) * gelu'(a1)
+  if ((rc = gemm<32>(e, e->mdP2, e->nW2T, B, H, H, 0, 0, 0, 0, bg))) return rc;  // dA1 = (dA2 W2) * gelu'(a1)
   st.out32 = e->gW1;
   st.ld32 = e->Kin;
   st.n_valid = e->n_in;
-  if ((rc = gemm(e, e->mdP1T, S.mapFT, H, e->Kin, B, 0, 0, r0, 0, st))) return rc;  // dW1 = dA1^T F
-  k_colsum<<<(H + 127) / 128, 128, 0, e->stream>>>(B, H, e->dpre1, H, e->gb1);
-  ENC_LAUNCHED(e, "k_colsum");
-  k_colsum<<<(H + 127) / 128, 128, 0, e->stream>>>(B, H, e->dpre2, H, e->gb2);
-  ENC_LAUNCHED(e, "k_colsum");
-  k_colsum<<<1, 128, 0, e->stream>>>(B, 2 * Q, e->d32, 128, e->gb3);
-  ENC_LAUNCHED(e, "k_colsum");
-  k_sum_ordered<<<1, 32, 0, e->stream>>>(B, e->loss_rows, e->loss_sum);
-  ENC_LAUNCHED(e, "k_sum_ordered");
+  if ((rc = gemm<32>(e, e->mdP1T, S.mapFT, H, e->n_in, B, 0, 0, r0, 0, st))) return rc;  // dW1 = dA1^T F
+  const EncSums sums{{e->dpre1, e->dpre2, e->d32}, {e->gb1, e->gb2, e->gb3}, {H, H, 2 * Q}, {H, H, 128}, e->loss_rows, loss};
+  k_enc_sums<<<2 * (H / 32) + (2 * Q + 31) / 32 + 1, 256, 0, e->stream>>>(B, sums);
+  ENC_LAUNCHED(e, "k_enc_sums");
+  return GPL_OK;
+}
+
+int adam_step(gpl_enc* e, float lr) {
+  e->step++;
+  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const float c1 = 1.f - powf(b1, (float)e->step), c2 = 1.f - powf(b2, (float)e->step);
+  k_adam<<<(unsigned)((e->n_par + 255) / 256), 256, 0, e->stream>>>(e->H, e->Kin, 2 * e->Q, e->n_par, e->W1, e->gW1,
+                                                                    e->adam, e->adam + e->n_par, lr, b1, b2, eps, c1,
+                                                                    c2, e->W1b, e->W2b, e->W2T, e->W3b, e->W3T);
+  ENC_LAUNCHED(e, "k_adam");
   return GPL_OK;
 }
 
 struct Block {
-  float *w, *g;
+  const float* w;
   int rows, cols;
   __nv_bfloat16* wb;
   int ldw;
@@ -517,34 +657,13 @@ struct Block {
 
 std::vector<Block> blocks(gpl_enc* e) {
   const int H = e->H, Q = e->Q;
-  return {{e->W1, e->gW1, H, e->Kin, e->W1b, e->Kin, nullptr, 0},
-          {e->b1, e->gb1, 1, H, nullptr, 0, nullptr, 0},
-          {e->W2, e->gW2, H, H, e->W2b, H, e->W2T, H},
-          {e->b2, e->gb2, 1, H, nullptr, 0, nullptr, 0},
-          {e->W3, e->gW3, 2 * Q, H, e->W3b, H, e->W3T, 64},
-          {e->b3, e->gb3, 1, 2 * Q, nullptr, 0, nullptr, 0}};
-}
-
-int adam_step(gpl_enc* e, float lr) {
-  e->step++;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float c1 = 1.f - powf(b1, (float)e->step), c2 = 1.f - powf(b2, (float)e->step);
-  size_t off = 0;
-  for (const Block& b : blocks(e)) {
-    const int n = b.rows * b.cols;
-    float* m = e->adam + off;
-    float* v = e->adam + e->n_par + off;
-    k_adam<<<(n + 255) / 256, 256, 0, e->stream>>>(b.rows, b.cols, b.w, b.g, m, v, lr, b1, b2, eps, c1, c2, b.wb,
-                                                   b.ldw, b.wt, b.ldwt);
-    ENC_LAUNCHED(e, "k_adam");
-    off += (size_t)n;
-  }
-  return GPL_OK;
+  return {{e->W1, H, e->Kin, e->W1b, e->Kin, nullptr, 0},
+          {e->W2, H, H, e->W2b, H, e->W2T, H},
+          {e->W3, 2 * Q, H, e->W3b, H, e->W3T, 64}};
 }
 
 int refresh_bf16(gpl_enc* e) {
   for (const Block& b : blocks(e)) {
-    if (!b.wb && !b.wt) continue;
     const int n = b.rows * b.cols;
     k_to_bf16<<<(n + 255) / 256, 256, 0, e->stream>>>(b.rows, b.cols, b.w, b.wb, b.ldw, b.wt, b.ldwt);
     ENC_LAUNCHED(e, "k_to_bf16");
@@ -610,11 +729,14 @@ int gpl_enc_create(gpl_enc** out, int device, void* stream, int n_in, int hidden
     *gp[k] = G + off;
     off += sz[k];
   }
-  if (!bf16_map(&e->mW1, e->W1b, Kin, H) || !bf16_map(&e->mW2, e->W2b, H, H) || !bf16_map(&e->mW2T, e->W2T, H, H) ||
-      !bf16_map(&e->mW3, e->W3b, H, 128) || !bf16_map(&e->mW3T, e->W3T, 64, H) || !bf16_map(&e->mH1, e->H1, H, B) ||
-      !bf16_map(&e->mH1T, e->H1T, B, H) || !bf16_map(&e->mH2, e->H2, H, B) || !bf16_map(&e->mH2T, e->H2T, B, H) ||
-      !bf16_map(&e->mdq, e->dq, 64, B) || !bf16_map(&e->mdqT, e->dqT, B, 128) || !bf16_map(&e->mdP2, e->dP2, H, B) ||
-      !bf16_map(&e->mdP2T, e->dP2T, B, H) || !bf16_map(&e->mdP1T, e->dP1T, B, H)) {
+  if (!bf16_map(&e->mW1, e->W1b, Kin, H) || !bf16_map(&e->mW2, e->W2b, H, H) || !bf16_map(&e->mW3, e->W3b, H, 128) ||
+      !bf16_map(&e->mH1, e->H1, H, B) || !bf16_map(&e->mH2, e->H2, H, B) || !bf16_map(&e->mdq, e->dq, 64, B) ||
+      !bf16_map(&e->mdqT, e->dqT, B, 128) || !bf16_map(&e->mdP2, e->dP2, H, B) ||
+      !bf16_map(&e->mdP2T, e->dP2T, B, H) || !bf16_map(&e->mdP1T, e->dP1T, B, H) ||
+      !bf16_map(&e->nW1, e->W1b, Kin, H, 32) || !bf16_map(&e->nW2, e->W2b, H, H, 32) ||
+      !bf16_map(&e->nW2T, e->W2T, H, H, 32) || !bf16_map(&e->nW3, e->W3b, H, 128, 32) ||
+      !bf16_map(&e->nW3T, e->W3T, 64, H, 32) || !bf16_map(&e->nH1T, e->H1T, B, H, 32) ||
+      !bf16_map(&e->nH2T, e->H2T, B, H, 32)) {
     e->err = "cuTensorMapEncodeTiled failed";
     gpl_enc_destroy(e);
     return GPL_ERR_CUDA;
@@ -643,13 +765,14 @@ int gpl_enc_destroy(gpl_enc* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   void* bufs[] = {e->W1,  e->gW1, e->adam, e->W1b, e->W2b,   e->W2T,  e->W3b, e->W3T,  e->pre1, e->pre2,
                   e->out, e->d32, e->dpre1, e->dpre2, e->loss_rows, e->loss_sum, e->H1, e->H1T, e->H2, e->H2T,
-                  e->dq,  e->dqT, e->dP2,  e->dP2T, e->dP1,  e->dP1T, e->err_d};
+                  e->dq,  e->dqT, e->dP2,  e->dP2T, e->dP1,  e->dP1T, e->err_d, e->pH1, e->pH2, e->pout, e->pres};
   for (void* p : bufs)
     if (p) cudaFree(p);
   for (auto& s : e->set) {
     if (s.F) cudaFree(s.F);
     if (s.FT) cudaFree(s.FT);
     if (s.X) cudaFree(s.X);
+    if (s.rows_d) cudaFree(s.rows_d);
   }
   if (e->own_stream && e->stream) cudaStreamDestroy(e->stream);
   delete e;
@@ -674,6 +797,7 @@ int gpl_enc_set_cells(gpl_enc* e, int which, int N, int J, int64_t nnz, const in
   if (S.F) cudaFree(S.F);
   if (S.FT) cudaFree(S.FT);
   if (S.X) cudaFree(S.X);
+  if (S.rows_d) cudaFree(S.rows_d);
   S = gpl_enc::Set();
   S.N = N;
   S.Npad = rup(N, e->B);
@@ -711,7 +835,7 @@ int gpl_enc_set_cells(gpl_enc* e, int which, int N, int J, int64_t nnz, const in
   int64_t* gp_d = nullptr;
   double *cnt_d = nullptr, *ls_d = nullptr;
   if ((rc = ealloc(e, &S.F, (size_t)S.Npad * e->Kin)) || (rc = ealloc(e, &S.FT, (size_t)e->Kin * S.Npad)) ||
-      (rc = ealloc(e, &S.X, (size_t)S.Npad * e->Q)) || (rc = ealloc(e, &cell_d, (size_t)nnz)) ||
+      (rc = ealloc(e, &S.X, (size_t)S.Npad * e->Q)) || (rc = ealloc(e, &S.rows_d, (size_t)N)) || (rc = ealloc(e, &cell_d, (size_t)nnz)) ||
       (rc = ealloc(e, &gv_d, (size_t)J)) || (rc = ealloc(e, &genes_d, (size_t)e->n_in)) ||
       (rc = ealloc(e, &row_d, (size_t)N)) || (rc = ealloc(e, &gp_d, (size_t)J + 1)) ||
       (rc = ealloc(e, &cnt_d, (size_t)nnz)) || (rc = ealloc(e, &ls_d, (size_t)N)))
@@ -723,6 +847,7 @@ int gpl_enc_set_cells(gpl_enc* e, int which, int N, int J, int64_t nnz, const in
   ENC_TRY(e, cudaMemcpyAsync(genes_d, genes, sizeof(int32_t) * e->n_in, cudaMemcpyHostToDevice, e->stream));
   ENC_TRY(e, cudaMemcpyAsync(row_d, row_of.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, e->stream));
   ENC_TRY(e, cudaMemcpyAsync(ls_d, ls, sizeof(double) * N, cudaMemcpyHostToDevice, e->stream));
+  ENC_TRY(e, cudaMemcpyAsync(S.rows_d, S.cell_of_row.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, e->stream));
   dim3 g(8, e->n_in);
   k_enc_features<<<g, 256, 0, e->stream>>>(e->n_in, genes_d, gp_d, gv_d, cell_d, cnt_d, ls_d, row_d, S.F, e->Kin,
                                            S.FT, S.Npad);
@@ -730,7 +855,7 @@ int gpl_enc_set_cells(gpl_enc* e, int which, int N, int J, int64_t nnz, const in
   ENC_TRY(e, cudaStreamSynchronize(e->stream));
   void* tmp[] = {cell_d, gv_d, genes_d, row_d, gp_d, cnt_d, ls_d};
   for (void* p : tmp) cudaFree(p);
-  if (!bf16_map(&S.mapF, S.F, e->Kin, S.Npad) || !bf16_map(&S.mapFT, S.FT, S.Npad, e->Kin)) {
+  if (!bf16_map(&S.mapF, S.F, e->Kin, S.Npad) || !bf16_map(&S.mapFT, S.FT, S.Npad, e->Kin, 32)) {
     e->err = "cuTensorMapEncodeTiled failed";
     return GPL_ERR_CUDA;
   }
@@ -792,7 +917,7 @@ int gpl_enc_grads(gpl_enc* e, int batch_index, double* loss, float* grads) {
   const int r0 = batch_index * e->B;
   if (batch_index < 0 || r0 + e->B > e->set[0].Npad) return GPL_ERR_ARG;
   int rc;
-  if ((rc = forward(e, 0, r0, e->B)) || (rc = backward(e, r0))) return rc;
+  if ((rc = forward(e, r0)) || (rc = backward(e, r0, e->loss_sum))) return rc;
   double s = 0.0;
   ENC_TRY(e, cudaMemcpyAsync(&s, e->loss_sum, sizeof(double), cudaMemcpyDeviceToHost, e->stream));
   if ((rc = check_err(e))) return rc;
@@ -807,19 +932,26 @@ int gpl_enc_train(gpl_enc* e, int epochs, double lr, uint64_t seed, double* loss
   std::mt19937_64 rng(seed);
   std::vector<int> order(nb);
   std::vector<double> bl(nb);
+  int rc;
+  if ((size_t)nb > e->n_loss) {  // a loss per batch, read once per epoch
+    ENC_TRY(e, cudaStreamSynchronize(e->stream));
+    double* p = nullptr;
+    if ((rc = ealloc(e, &p, nb))) return rc;
+    cudaFree(e->loss_sum);
+    e->loss_sum = p;
+    e->n_loss = nb;
+  }
   for (int ep = 0; ep < epochs; ep++) {
     for (int b = 0; b < nb; b++) order[b] = b;
     std::shuffle(order.begin(), order.end(), rng);
-    double tot = 0.0;
     for (int k = 0; k < nb; k++) {
       const int r0 = order[k] * e->B;
-      int rc;
-      if ((rc = forward(e, 0, r0, e->B)) || (rc = backward(e, r0)) || (rc = adam_step(e, (float)lr))) return rc;
-      double s = 0.0;
-      ENC_TRY(e, cudaMemcpyAsync(&s, e->loss_sum, sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-      ENC_TRY(e, cudaStreamSynchronize(e->stream));
-      tot += s;
+      if ((rc = forward(e, r0)) || (rc = backward(e, r0, e->loss_sum + k)) || (rc = adam_step(e, (float)lr))) return rc;
     }
+    ENC_TRY(e, cudaMemcpyAsync(bl.data(), e->loss_sum, sizeof(double) * nb, cudaMemcpyDeviceToHost, e->stream));
+    ENC_TRY(e, cudaStreamSynchronize(e->stream));
+    double tot = 0.0;
+    for (int k = 0; k < nb; k++) tot += bl[k];
     if (loss_per_epoch) loss_per_epoch[ep] = tot / ((double)nb * e->B);
   }
   return check_err(e);
@@ -829,22 +961,43 @@ int gpl_enc_predict(gpl_enc* e, int which, double* mean, double* logvar) {
   if (!e || which < 0 || which > 1 || e->set[which].N == 0 || (!mean && !logvar)) return GPL_ERR_ARG;
   cudaSetDevice(e->device);
   gpl_enc::Set& S = e->set[which];
-  const int N = S.N, Q = e->Q, B = e->B;
-  std::vector<float> o((size_t)B * 128);
-  for (int r0 = 0; r0 < N; r0 += B) {
-    const int rows = std::min(B, N - r0);
-    int rc = forward(e, which, r0, rows);
-    if (rc) return rc;
-    ENC_TRY(e, cudaMemcpyAsync(o.data(), e->out, sizeof(float) * (size_t)B * 128, cudaMemcpyDeviceToHost, e->stream));
+  const int N = S.N, Q = e->Q, H = e->H, most = std::min(rup(N, 128), 32768);
+  const size_t nq = (size_t)N * Q;
+  int rc;
+  if (most > e->pred_rows) {
     ENC_TRY(e, cudaStreamSynchronize(e->stream));
-    for (int r = 0; r < rows; r++) {
-      const int i = S.cell_of_row[r0 + r];
-      for (int q = 0; q < Q; q++) {
-        if (mean) mean[i + (size_t)q * N] = o[(size_t)r * 128 + q];
-        if (logvar) logvar[i + (size_t)q * N] = o[(size_t)r * 128 + Q + q];
-      }
+    void* old[] = {e->pH1, e->pH2, e->pout};
+    for (void* p : old)
+      if (p) cudaFree(p);
+    e->pH1 = e->pH2 = nullptr;
+    e->pout = nullptr;
+    e->pred_rows = 0;
+    if ((rc = ealloc(e, &e->pH1, (size_t)most * H)) || (rc = ealloc(e, &e->pH2, (size_t)most * H)) ||
+        (rc = ealloc(e, &e->pout, (size_t)most * 64)))
+      return rc;
+    if (!bf16_map(&e->mpH1, e->pH1, H, most) || !bf16_map(&e->mpH2, e->pH2, H, most)) {
+      e->err = "cuTensorMapEncodeTiled failed";
+      return GPL_ERR_CUDA;
     }
+    e->pred_rows = most;
   }
+  if (N > e->pred_cells) {
+    ENC_TRY(e, cudaStreamSynchronize(e->stream));
+    if (e->pres) cudaFree(e->pres);
+    e->pres = nullptr;
+    e->pred_cells = 0;
+    if ((rc = ealloc(e, &e->pres, 2 * nq))) return rc;
+    e->pred_cells = N;
+  }
+  for (int r0 = 0; r0 < N; r0 += e->pred_rows) {
+    const int rows = std::min(e->pred_rows, N - r0);
+    if ((rc = predict_rows(e, which, r0, rows))) return rc;
+    k_enc_scatter<<<(rows + 255) / 256, 256, 0, e->stream>>>(rows, r0, N, Q, e->pout, 64, S.rows_d, e->pres,
+                                                             e->pres + nq);
+    ENC_LAUNCHED(e, "k_enc_scatter");
+  }
+  if (mean) ENC_TRY(e, cudaMemcpyAsync(mean, e->pres, sizeof(double) * nq, cudaMemcpyDeviceToHost, e->stream));
+  if (logvar) ENC_TRY(e, cudaMemcpyAsync(logvar, e->pres + nq, sizeof(double) * nq, cudaMemcpyDeviceToHost, e->stream));
   return check_err(e);
 }
 
