@@ -103,7 +103,8 @@ GPL_API int gpl_set_precision(gpl_ctx* ctx, int precision);
  *   "fused_tail"        1: each IRLS sweep's per-gene tail (cholPsi, the solve and coefficient
  *                       update of getBetaPhi, getLkhdPois: ggplvm.cu:683-692, 418-464, 703-724)
  *                       runs as one persistent launch whose CTAs take genes from a queue ordered
- *                       by decreasing count (FP64 path, P <= 288; else the separate kernels).
+ *                       by decreasing count (FP64 path, P <= 288 and no more genes than CTAs fit,
+ *                       two per SM; else the separate kernels, which are faster there).
  *                       Same results bit for bit. Default 0.
  *   "tail_ctas_per_sm"  CTAs per SM of that launch (1 or 2, default 2)
  *   "autotune"          1: the tile orders of the FP64 pair GEMMs and of the tensor-core

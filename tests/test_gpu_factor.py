@@ -78,3 +78,46 @@ def test_prior_factor(M):
     assert np.count_nonzero(np.tril(L, -1)[:, :g0]) == 0
     d = np.sqrt(np.diag(A))
     assert np.all(np.abs(L @ L.T - A) <= 2 * (P + 1) * U * np.outer(d, d))
+
+
+# P = M + 4 at the edges of the 32-column panels, of the half-size kernel (160) and of the panel kernel
+# (288), odd (8-byte copies) and even
+@pytest.mark.parametrize("M", [1, 27, 28, 29, 60, 61, 92, 125, 156, 157, 188, 253, 284, 317])
+def test_factor_and_inverse(M):
+    ds = _dataset(700, 4, M)
+    with GPLVM.from_dataset(ds) as m:
+        m.set_params(ds.init)
+        P, J = m.P, m.J
+        assert P == M + 4
+        m.kernel_mats()
+        m.glm_init()
+        m.irls_sweep(0, 0)
+        m.objective(0, 1)
+        L = np.tril(m.get("Psi").reshape(J, P, P).transpose(0, 2, 1))
+        m.gradient()
+        X = m.get("PsiInv").reshape(J, P, P)
+    for j in range(J):
+        # with V = L^-1 (1 + E), |E| <= 2 (P + 2) u |L||V| (its diagonal blocks' inverses included) and
+        # X = fl(V^T V): L L^T X - 1 is at most, to first order, 8 (P + 2) u |L||L^T||V^T||L^T||V^T||V|
+        V = np.linalg.inv(L[j])
+        aL, aV = np.abs(L[j]), np.abs(V)
+        bound = aL @ (aL.T @ aV.T @ aL.T @ aV.T) @ aV
+        assert np.array_equal(X[j], X[j].T)
+        assert np.all(np.abs(L[j] @ (L[j].T @ X[j]) - np.eye(P)) <= 8 * (P + 2) * U * bound)
+
+
+# the last gene count of the fused tail (one gene per resident CTA) and the first of the separate kernels
+@pytest.mark.parametrize("J", [296, 297])
+def test_tail_rule_same_bits(J):
+    out = []
+    for fused in (0, 1):
+        ds = _dataset(400, J, 9, 5)
+        with GPLVM.from_dataset(ds) as m:
+            m.set_option("fused_tail", fused)
+            m.set_params(ds.init)
+            m.kernel_mats()
+            m.glm_init()
+            m.irls_sweep(0, 0)
+            out.append({k: m.get(k) for k in ("Beta", "phi", "Psi", "lkhds")})
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k], equal_nan=True), k
