@@ -69,9 +69,9 @@ struct CrtState {
 };
 
 struct PairState {
-  bool ready = false, wide = false;  // wide: a cell's V row exceeds k_v_to_u's shared memory
+  bool ready = false;
   int n_pairs = 0, pairs_pad = 0, cpad = 0, v_cells = 0;
-  int smem_gram = 0, smem_v = 0, smem_vu = 0;
+  int smem_gram = 0, smem_v = 0;
   int2* pairs = nullptr;
   double *rOm = nullptr, *Sp = nullptr, *V = nullptr;
   double* Gacc = nullptr;  // pairs x genes Gram accumulator when the cells need several ranges

@@ -31,6 +31,7 @@
 #include <cmath>
 
 #include "gpl_internal.cuh"
+#include "pair_rows.cuh"
 #include "tc_common.cuh"
 
 namespace gpl {
@@ -628,78 +629,30 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
   }
 }
 
-// U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], one CTA per cell: the
-// cell's row of V from its residues into shared memory, whole rows a of the pair triangle at a time,
-// then every entry used once for both of its columns (a warp per row a: the row's sum over the
-// lanes, the other column's sums in the lanes' registers). S: 32-column slots, n_d <= 32 S.
-constexpr int kUPairs = 4096;  // entries of V in shared memory at a time
-template <int S>
-__global__ void __launch_bounds__(256) k_crt_u(int ldN, int n_d, int n_pairs, int c0, int64_t ldo, size_t plane,
+// U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], W warps per cell: the
+// cell's row of V from its residues into shared memory (pair_rows.cuh).
+template <int S, int W>
+__global__ void __launch_bounds__(256, S == 9 ? 4 : 1) k_crt_u(int ldN, int n_d, int len, int c0, int64_t ldo, size_t plane,
                                                const uint8_t* __restrict__ in, const double* __restrict__ inv_i,
                                                const double* __restrict__ inv_p, const double* __restrict__ rOm,
                                                const double* __restrict__ D, double* __restrict__ U,
                                                const int* __restrict__ flag) {
-  extern __shared__ __align__(16) double vs[];  // [kUPairs + 4] V, [n_d] D row, [n_d] row sums
+  extern __shared__ __align__(16) double vs[];
   if (*flag) return;
-  double *ds = vs + kUPairs + 4, *rs = ds + n_d;
-  const int r = blockIdx.x, i = c0 + r;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int a = threadIdx.x; a < n_d; a += 256) ds[a] = D[(size_t)a * ldN + i];
+  const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g, i = c0 + r;
+  if (r >= len) return;  // W = 1: a whole warp, no barrier of the block follows
+  double* vc = vs + g * u_space<W>(n_d);
   const double s = inv_i[r] * rOm[i] * kUnit;
   const uint8_t* row_in = in + (size_t)r * ldo;
-  __syncthreads();
-  double col[S], db[S];
-#pragma unroll
-  for (int t = 0; t < S; t++) {
-    col[t] = 0.0;
-    db[t] = 32 * t + lane < n_d ? ds[32 * t + lane] : 0.0;
-  }
-  for (int a0 = 0, p0 = 0; a0 < n_d;) {
-    // rows [a0, a1): pairs [p0, p1), from the multiple of four at or below p0
-    int a1 = a0, p1 = p0;
-    const int from = p0 & ~3;
-    while (a1 < n_d && p1 + (n_d - a1) - from <= kUPairs) p1 += n_d - a1++;
-    for (int p = from + 4 * threadIdx.x; p < p1; p += 1024) {
+  pair_rows_to_u<S, W>(i, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
+    for (int p = from + 4 * tid; p < p1; p += 4 * nt) {
       double v[4];
       crt_values(row_in + p, plane, v);
       const double2 x = *reinterpret_cast<const double2*>(inv_p + p), y = *reinterpret_cast<const double2*>(inv_p + p + 2);
-      *reinterpret_cast<double2*>(vs + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
-      *reinterpret_cast<double2*>(vs + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
+      *reinterpret_cast<double2*>(vc + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
+      *reinterpret_cast<double2*>(vc + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
     }
-    __syncthreads();
-    for (int a = a0 + warp; a < a1; a += 8) {
-      const double* row = vs + (a * n_d - a * (a - 1) / 2 - a - from);  // V[pair(a, b)] at row[b], b >= a
-      const double da = ds[a];
-      double sum = 0.0;
-#pragma unroll
-      for (int t = 0; t < S; t++) {
-        const int b = 32 * t + lane;
-        if (32 * t < n_d && 32 * t + 31 >= a) {
-          if (b >= a && b < n_d) {
-            const double v = row[b];
-            sum = fma(db[t], v, sum);
-            if (b > a) col[t] = fma(da, v, col[t]);
-          }
-        }
-      }
-      sum = warp_sum(sum);
-      if (lane == 0) rs[a] = sum;
-    }
-    a0 = a1;
-    p0 = p1;
-    __syncthreads();
-  }
-  double* cs = vs;  // [8][n_d] the warps' column sums
-#pragma unroll
-  for (int t = 0; t < S; t++)
-    if (32 * t + lane < n_d) cs[warp * n_d + 32 * t + lane] = col[t];
-  __syncthreads();
-  for (int a = threadIdx.x; a < n_d; a += 256) {
-    double u = rs[a];
-#pragma unroll
-    for (int w = 0; w < 8; w++) u += cs[w * n_d + a];
-    U[i + (size_t)a * ldN] = u;
-  }
+  });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -711,23 +664,25 @@ constexpr int kSmemTurn = kMod * 32 * kTurnWords * (int)sizeof(uint32_t);
 constexpr int kGroupI8 = 8;
 
 int up(int64_t v, int m) { return (int)((v + m - 1) / m * m); }
-
-constexpr int kMaxDense = 512;  // dense columns k_crt_u's slots cover
-
-int smem_u(const Ctx* c) { return (int)sizeof(double) * (kUPairs + 4 + 2 * c->n_d); }
 }  // namespace
 
-// Where the integer form is taken (measured against the DMMA form on B200, both products at 1,000 to
-// 100,000 cells, 100 to 3,000 genes, 36 to 260 dense columns). The Gram: from 4e8 entry products on
-// (0.18 -> 0.10 ms at 7e8, 3.0 -> 0.25 ms at 20,000 cells x 100 genes x 666 pairs, where the DMMA
-// tiles leave most SMs idle), except for a few genes, whose 256-row tile is mostly padding. The
-// gradient pairs: their conversions and the way back to FP64 grow with cells x pairs whatever the
-// genes, so they need about 200 genes (0.6-0.9x at 100, 1.2-1.7x at 300, 3.5x at 1,000).
-constexpr double kMinWork = 4e8;
-constexpr int kMinGenesGram = 64, kMinGenesGrad = 200;
-
-// Sizes of the integer form for a context whose pair buffer may hold `cap` bytes: the cells per range
-// of both products. Leaves s.crt.on false where the DMMA form is the better one (or the only one).
+// Where the integer form is taken. The Gram: from 512 cells on. The DMMA form has one CTA per 128
+// pairs x 128 genes and takes 0.15 us for every cell in it (K in slices of 16), however few the tiles;
+// measured from 1,000 x 20 x 21 (cells, genes, pairs: 0.163 -> 0.071 ms) over 20,000 x 1,001 x 15 (2.98
+// -> 0.32) to 10,000 x 1,000 x 4,851 (4.64 -> 0.98) the integer form was 1.3 to 25 times as fast. A few
+// genes keep the DMMA form, whose tile order the autotuner can choose (2,000 cells: 0.2 ms lost).
+// The gradient pairs: the two forms' times as estimated by the costs measured over 1,000 to 30,000
+// cells, 20 to 1,000 genes and 21 to 4,851 pairs (us). DMMA: 0.165 per gene and wave of 148 tiles, and
+// the pair rows. Integer: the conversions of both operands, the way back to FP64, padded tiles and
+// chunks, and the products. E.g. 1,000 x 1,000 x 105: 169 / 65; 3,000 x 300 x 595: 74 / 107;
+// 30,000 x 300 x 105: 167 / 391; 30,000 x 300 x 4,851: 3,707 / 2,495.
+constexpr int kMinCells = 512, kMinGenes = 32;
+static bool crt_grad_faster(double N, double J, double pairs, double Jk, double Pp) {
+  const double waves = std::ceil(std::ceil(N / 128) * std::ceil(pairs / 128) / 148);
+  const double dmma = 10 + 0.165 * J * waves + 5e-6 * N * pairs;
+  const double integer = 50 + N * (15e-6 * Pp + 10e-6 * Jk) + N * Jk * Pp * 2 * kMod / 2.9e9;
+  return integer < dmma;
+}
 void crt_plan(Ctx* c, size_t cap) {
   PairState& s = c->pr;
   CrtState& t = s.crt;
@@ -736,9 +691,7 @@ void crt_plan(Ctx* c, size_t cap) {
   t.Jp = up(J, kTile);
   t.Pp = up(s.n_pairs, kTile);
   t.Jk = up(J, kChunk);
-  if (J > kMaxK || J < kMinGenesGram || c->n_d > kMaxDense ||
-      (double)N * (double)J * (double)s.n_pairs < kMinWork)
-    return;
+  if (N < kMinCells || J < kMinGenes || J > kMaxK || c->n_d > kUMaxDense) return;
   int64_t most = std::min<int64_t>(up(N, kTile), kMaxK / kTile * kTile);
   if (c->pair_range_cells > 0) {  // ranges below a tile: the DMMA form
     if (c->pair_range_cells < kTile) return;
@@ -761,7 +714,7 @@ void crt_plan(Ctx* c, size_t cap) {
     return std::min<int64_t>(n, up((N + ranges - 1) / ranges, kTile));
   };
   t.gram_cells = (int)cells(gram);
-  t.grad_cells = J >= kMinGenesGrad ? (int)cells(grad) : 0;
+  t.grad_cells = crt_grad_faster(N, J, s.n_pairs, t.Jk, t.Pp) ? (int)cells(grad) : 0;
   t.bytes = (size_t)std::max(t.gram_cells ? gram(t.gram_cells) : 0, t.grad_cells ? grad(t.grad_cells) : 0);
   t.on = t.gram_cells > 0 || t.grad_cells > 0;
 }
@@ -910,9 +863,12 @@ int launch_crt_uq(Ctx* c) {
         return rc;
     }
     ProfScope ps(c, "v_to_u");
-    auto ku = c->n_d <= 160 ? k_crt_u<5> : c->n_d <= 288 ? k_crt_u<9> : k_crt_u<16>;
-    ku<<<len, 256, smem_u(c), c->stream>>>(c->ldN, c->n_d, s.n_pairs, c0, t.Pp, plane_o, t.v_out, inv_i, inv_p, s.rOm,
-                                           c->Dm, c->U, t.flag);
+    pair_rows_form(c->n_d, len, 96, [&](auto S, auto W) {
+      constexpr int per = 8 / W;
+      const int smem = (int)sizeof(double) * u_space<W>(c->n_d) * per;
+      k_crt_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, len, c0, t.Pp, plane_o, t.v_out, inv_i,
+                                                               inv_p, s.rOm, c->Dm, c->U, t.flag);
+    });
     GPL_LAUNCHED(c, "k_crt_u");
   }
   return GPL_OK;

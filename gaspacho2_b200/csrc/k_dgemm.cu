@@ -28,6 +28,7 @@
 
 #include "dmma_common.cuh"
 #include "gpl_internal.cuh"
+#include "pair_rows.cuh"
 
 namespace gpl {
 
@@ -333,36 +334,27 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-// U[i, a] = sum_b D_ib V[i, pair(min(a,b), max(a,b))], one CTA per cell, the V row staged in
-// shared memory; pair(a, b) = a*n_d - a*(a-1)/2 + (b - a) (row-major upper triangle).
-__global__ void __launch_bounds__(256) k_v_to_u(int N, int ldN, int n_d, int n_pairs, int pairs_pad, int c0,
-                                                int c1, const double* __restrict__ D,
-                                                const double* __restrict__ V, double* __restrict__ U,
-                                                const int* __restrict__ gate) {
+// U[i, a] = sum_b D_ib V[i, pair(min(a,b), max(a,b))], W warps per cell (pair_rows.cuh), the cell's V row
+// by asynchronous copies.
+template <int S, int W>
+__global__ void __launch_bounds__(256, S > 9 ? 2 : 4) k_v_to_u(int ldN, int n_d, int pairs_pad, int c0, int c1,
+                                                   const double* __restrict__ D, const double* __restrict__ V,
+                                                   double* __restrict__ U, const int* __restrict__ gate) {
   extern __shared__ __align__(16) double vs[];
   if (gate && *gate == 0) return;
-  double* ds = vs + pairs_pad;  // D row of the cell
-  for (int i = c0 + blockIdx.x; i < c1 && i < N; i += gridDim.x) {
-    const double* vr = V + (size_t)(i - c0) * pairs_pad;
-    for (int e = threadIdx.x; e < n_pairs; e += blockDim.x) vs[e] = vr[e];
-    for (int e = threadIdx.x; e < n_d; e += blockDim.x) ds[e] = D[(size_t)e * ldN + i];
-    __syncthreads();
-    for (int a = threadIdx.x; a < n_d; a += blockDim.x) {
-      double s = 0.0;
-      // b < a: pair(b, a)
-      for (int b = 0; b < a; b++) s = fma(ds[b], vs[b * n_d - b * (b - 1) / 2 + (a - b)], s);
-      // b >= a: pair(a, b), contiguous
-      const double* row = vs + a * n_d - a * (a - 1) / 2 - a;
-      for (int b = a; b < n_d; b++) s = fma(ds[b], row[b], s);
-      U[i + (size_t)a * ldN] = s;
-    }
-    __syncthreads();
-  }
+  const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g;
+  if (c0 + r >= c1) return;  // W = 1: a whole warp, no barrier of the block follows
+  double* vc = vs + g * u_space<W>(n_d);
+  const double* vr = V + (size_t)r * pairs_pad;
+  pair_rows_to_u<S, W>(c0 + r, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
+    for (int p = from + 2 * tid; p < p1; p += 2 * nt) cp_async16(vc + p - from, vr + p, 16);
+    cp_async_commit();
+    cp_async_wait<0>();
+  });
 }
 
-// The same sums when a cell's V row exceeds the shared-memory budget (more than about 220 dense
-// columns): the row is read from global memory (L1 / L2) instead of staged, the dense row of
-// the cell is staged; identical operations in identical order.
+// The same for more dense columns than that takes (512): the row is read from global memory (L1 / L2)
+// instead of staged, the dense row of the cell is staged.
 __global__ void __launch_bounds__(256) k_v_to_u_wide(int N, int ldN, int n_d, int pairs_pad, int c0, int c1,
                                                      const double* __restrict__ D, const double* __restrict__ V,
                                                      double* __restrict__ U, const int* __restrict__ gate) {
@@ -405,10 +397,6 @@ int pair_prepare(Ctx* c) {
   s.v_cells = (int)std::min<size_t>((size_t)s.cpad, cap);
   s.smem_gram = (int)sizeof(double) * 3 * (BK * SA + BN * SBT);
   s.smem_v = (int)sizeof(double) * 3 * (BK * SA + BK * SBN);
-  s.smem_vu = (int)sizeof(double) * (s.pairs_pad + n_d);
-  // more dense columns than k_v_to_u stages per cell: k_v_to_u_wide reads the V rows from
-  // global memory instead
-  s.wide = s.smem_vu > 200 * 1024;
   // the integer form (k_crt.cu) keeps its operands in the same buffer, of 1 GiB at least: with 14 bytes
   // per operand entry it takes the cells in a few ranges where the DMMA form takes one, which costs it
   // less than a larger buffer costs a new context (about 10 ms per GiB)
@@ -434,7 +422,6 @@ int pair_prepare(Ctx* c) {
   }
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_gram));
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_v, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_v));
-  if (!s.wide) GPL_TRY(c, cudaFuncSetAttribute(k_v_to_u, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_vu));
   const int rc = crt_prepare(c);
   if (rc) {
     pair_release(c);
@@ -544,15 +531,22 @@ int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D) {
 int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* gate) {
   PairState& s = c->pr;
   ProfScope ps(c, "v_to_u");
-  const int grid = std::min(c1 - c0, 148 * 8);
-  if (s.wide) {
+  if (c->n_d > kUMaxDense) {
+    const int grid = std::min(c1 - c0, 148 * 8);
     k_v_to_u_wide<<<grid, 256, sizeof(double) * c->n_d, c->stream>>>(c->N, c->ldN, c->n_d, s.pairs_pad, c0, c1, D,
                                                                     V, c->U, gate);
     GPL_LAUNCHED(c, "k_v_to_u_wide");
     return GPL_OK;
   }
-  k_v_to_u<<<grid, 256, s.smem_vu, c->stream>>>(c->N, c->ldN, c->n_d, s.n_pairs, s.pairs_pad, c0, c1, D, V, c->U,
-                                                gate);
+  const int len = std::min(c1, c->N) - c0;
+  pair_rows_form(c->n_d, len, 160, [&](auto S, auto W) {
+    constexpr int per = 8 / W;
+    const int smem = (int)sizeof(double) * u_space<W>(c->n_d) * per;
+    if (smem > 48 * 1024)  // 97 or more columns, a warp per cell
+      cudaFuncSetAttribute(k_v_to_u<S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_v_to_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, s.pairs_pad, c0, c0 + len, D, V, c->U,
+                                                              gate);
+  });
   GPL_LAUNCHED(c, "k_v_to_u");
   return GPL_OK;
 }

@@ -94,3 +94,21 @@ def test_non_finite_operands_take_the_dmma_form(bad):
     assert not np.all(np.isfinite(a))
     f = np.isfinite(a)
     assert np.allclose(a[f], b[f], rtol=1e-12, atol=1e-12 * np.abs(b[f]).max())
+
+
+# The sums over a cell's pair row, a warp or a block per cell (2,368 cells, 96 and 160 columns), V from
+# memory (few genes) and from residues, against ranges of 128 cells, which take the DMMA form and a block
+# per cell; and the rules' edges in cells and genes. Tolerances as above.
+@pytest.mark.parametrize("N,G,M", [(2368, 40, 94), (2368, 40, 95), (2367, 40, 94), (2368, 40, 158), (2369, 40, 159),
+                                   (2368, 600, 94), (2369, 600, 95), (2368, 600, 20), (511, 40, 20), (512, 32, 20),
+                                   (513, 31, 21), (520, 1000, 3)])
+def test_pair_rows_forms(N, G, M):
+    ds = _dataset(N, G, M, 10, 1)
+    out = []
+    for cells in (0, 128):
+        with _context(ds, cells) as m:
+            x = m.params_vector()
+            v, g = m.evaluate(x)
+            out.append((v, g.copy()))
+    assert abs(out[0][0] - out[1][0]) <= 1e-12 * abs(out[1][0])
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 1e-10 * np.linalg.norm(out[1][1])
