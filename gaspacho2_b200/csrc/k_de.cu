@@ -17,6 +17,7 @@
 // All are per-gene (or per-coefficient) reductions over HBM-resident W, nu: bandwidth-bound
 // and small next to the Gram of each sweep.
 #include "gpl_internal.cuh"
+#include "in_order.cuh"
 
 namespace gpl {
 
@@ -98,14 +99,18 @@ __global__ void __launch_bounds__(256) k_de_lkhd(int N, int ldN, int P, int p_ef
   const int j = blockIdx.x;
   const double* Wj = W + (size_t)j * ldN;
   double part = 0.0;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) part -= Wj[i] / Omega[i];
+  in_order<8>(
+      (int)threadIdx.x, N, 256, [&](int i) { return make_double2(Wj[i], Omega[i]); },
+      [&](const double2& v) { part -= v.x / v.y; });
   const double dgp = delta[pvars - 1];
   const int64_t b = gptr[j], e = gptr[j] + gvalid[j];
-  for (int64_t l = b + threadIdx.x; l < e; l += blockDim.x) {
-    const int i = cell[l];
-    const double w = Wj[i], om = Omega[i];
-    part += ((log(w) - dgp * titsias[i]) * cnt[l] - w) / om + w / om;
-  }
+  in_order<4>(
+      b + threadIdx.x, e, 256, [&](int64_t l) { return CountAt{cell[l], cnt[l]}; },
+      [&](const CountAt& x) { return make_double3(Wj[x.cell], Omega[x.cell], titsias[x.cell]); },
+      [&](const CountAt& x, const double3& v) {
+        const double w = v.x, om = v.y;
+        part += ((log(w) - dgp * v.z) * x.y - w) / om + w / om;
+      });
   const double* Lj = Psi + (size_t)j * P * P;
   double ld = 0.0;
   for (int k = threadIdx.x; k < p_eff; k += blockDim.x) ld += log(Lj[k + (size_t)k * P]);

@@ -26,6 +26,7 @@
 
 #include "dmma_common.cuh"
 #include "gpl_internal.cuh"
+#include "in_order.cuh"
 
 namespace gpl {
 
@@ -787,49 +788,18 @@ __global__ void __launch_bounds__(256, 2)
     const double* Wj = W + (size_t)j * ldN;
     const double* nj = Nu + (size_t)j * ldN;
     double qpart = 0.0, lpart = 0.0;
-    // a batch's loads are issued before its first use: a load at a time made this pass 0.13 ms a gene
-    int i0 = tid;
-    for (; i0 + 7 * 256 < N; i0 += 8 * 256) {
-      double n8[8], w8[8], o8[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        n8[k] = nj[i0 + 256 * k];
-        w8[k] = Wj[i0 + 256 * k];
-        o8[k] = Omega[i0 + 256 * k];
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        qpart += n8[k] * n8[k] * w8[k] / o8[k];
-        lpart -= w8[k];
-      }
-    }
-    for (; i0 < N; i0 += 256) {
-      qpart += nj[i0] * nj[i0] * Wj[i0] / Omega[i0];
-      lpart -= Wj[i0];
-    }
+    in_order<8>(
+        tid, N, 256, [&](int i) { return make_double3(nj[i], Wj[i], Omega[i]); },
+        [&](const double3& v) {
+          qpart += v.x * v.x * v.y / v.z;
+          lpart -= v.y;
+        });
     const int64_t b0 = gptr[j], b1 = gptr[j] + gvalid[j];
     const double dgp = delta[pvars - 1];
-    int64_t l0 = b0 + tid;
-    for (; l0 + 3 * 256 < b1; l0 += 4 * 256) {
-      int c4[4];
-      double y4[4], w4[4], t4[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        c4[k] = cell[l0 + 256 * k];
-        y4[k] = cnt[l0 + 256 * k];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        w4[k] = Wj[c4[k]];
-        t4[k] = titsias[c4[k]];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) lpart += (log(w4[k]) - dgp * t4[k] * wt) * y4[k];
-    }
-    for (; l0 < b1; l0 += 256) {
-      const int i = cell[l0];
-      lpart += (log(Wj[i]) - dgp * titsias[i] * wt) * cnt[l0];
-    }
+    in_order<4>(
+        b0 + tid, b1, 256, [&](int64_t l) { return CountAt{cell[l], cnt[l]}; },
+        [&](const CountAt& x) { return make_double2(Wj[x.cell], titsias[x.cell]); },
+        [&](const CountAt& x, const double2& v) { lpart += (log(v.x) - dgp * v.y * wt) * x.y; });
     const double quad = block_sum(qpart, sh);  // syncs: the solution y is complete
     double* bj = Beta + (size_t)j * P;
     for (int k = tid; k < P; k += blockDim.x) {

@@ -10,6 +10,7 @@
 //   k_collect     sum_j l_j - wt delta_GP sum_i Oinvt_i titsias_i - inverse-gamma prior on Omega
 //                 (and the variance-component driver's N(0, 1) priors on X and T)
 #include "gpl_internal.cuh"
+#include "in_order.cuh"
 
 namespace gpl {
 
@@ -180,13 +181,13 @@ __global__ void __launch_bounds__(256) k_lkhd_pois(int N, int ldN, int pvars, do
   const int j = blockIdx.x;
   const double* Wj = W + (size_t)j * ldN;
   double part = 0.0;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) part -= Wj[i];
+  in_order<8>((int)threadIdx.x, N, 256, [&](int i) { return Wj[i]; }, [&](double w) { part -= w; });
   const int64_t b = gptr[j], e = gptr[j] + gvalid[j];
   const double dgp = delta[pvars - 1];
-  for (int64_t l = b + threadIdx.x; l < e; l += blockDim.x) {
-    const int i = cell[l];
-    part += (log(Wj[i]) - dgp * titsias[i] * wt) * cnt[l];
-  }
+  in_order<4>(
+      b + threadIdx.x, e, 256, [&](int64_t l) { return CountAt{cell[l], cnt[l]}; },
+      [&](const CountAt& x) { return make_double2(Wj[x.cell], titsias[x.cell]); },
+      [&](const CountAt& x, const double2& v) { part += (log(v.x) - dgp * v.y * wt) * x.y; });
   const double s = block_sum(part, sh);
   if (threadIdx.x == 0) lkhds[j] = s;
 }
