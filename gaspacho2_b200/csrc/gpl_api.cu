@@ -1332,12 +1332,16 @@ int gpl_score_stats(gpl_ctx* h, int L, const double* G, double* S) {
   }
   const size_t N = c->N, J = c->J;
   const int LB = score_columns(c, L);
-  GPL_RUN(ensure_work(c, (N + J) * LB + score_work(c, LB)));
+  // the integer form's scratch where it can be had
+  const size_t need = (N + J) * LB + score_work(c, LB);
+  bool crt = crt_columns_faster(c, LB);
+  if (crt && ensure_work(c, need + crt_columns_work(c, LB)) != GPL_OK) crt = false;
+  GPL_RUN(ensure_work(c, need));
   double *dG = c->work, *dS = dG + N * LB, *dW = dS + J * LB;
   for (int l0 = 0; l0 < L; l0 += LB) {
     const int nl = std::min(LB, L - l0);
     GPL_TRY(c, cudaMemcpyAsync(dG, G + (size_t)l0 * N, sizeof(double) * N * nl, cudaMemcpyHostToDevice, c->stream));
-    GPL_RUN(launch_score_stats(c, nl, dG, dS, dW));
+    GPL_RUN(launch_score_stats(c, nl, dG, dS, dW, crt && crt_columns_faster(c, nl)));
     GPL_TRY(c, cudaMemcpyAsync(S + (size_t)l0 * J, dS, sizeof(double) * J * nl, cudaMemcpyDeviceToHost, c->stream));
     GPL_TRY(c, cudaStreamSynchronize(c->stream));
   }

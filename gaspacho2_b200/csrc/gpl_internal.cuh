@@ -348,7 +348,7 @@ int dgen_group_sums_of(Ctx* c, const double* Gg, int m);  // gsum[j][g][a] of m 
 int dgen_unweighted_gram(Ctx* c);         // the dense block of Psi_0 with every weight 1 (GLM initialisation)
 int dgen_hk(Ctx* c);
 int dgen_weighted_colsums(Ctx* c, const double* G2, int n2, double* out);  // out[j + c*J] = sum_i W_ij G2[c][i]
-int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch);  // device G (N x L) -> S (J x L)
+int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch, bool crt);  // device G (N x L) -> S (J x L)
 int score_columns(const Ctx* c, int L);   // genotype columns per pass of L
 size_t score_work(const Ctx* c, int L);   // values of scratch of a pass of L columns
 // q[j + v*J] = t_jv^T Psi_j^{-1} t_jv with the factors of Psi, t_jv at T + j sj + v sv
@@ -364,6 +364,9 @@ void crt_release(Ctx* c);
 int launch_crt_gram(Ctx* c);
 int launch_crt_uq(Ctx* c);
 int crt_error_flag(Ctx* c);
+bool crt_columns_faster(const Ctx* c, int L);    // Z^T diag(W/Omega) g of L per-cell columns there
+size_t crt_columns_work(const Ctx* c, int L);    // doubles of scratch that takes
+int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, bool* done);
 bool tc_map_u8(CUtensorMap* m, void* ptr, uint64_t cols, uint64_t rows);  // 128 x 128 byte boxes, swizzled
 int launch_tc_gram(Ctx* c);               // dense block of every Psi_j on tensor cores
 int launch_tc_grad(Ctx* c);               // U = sum_j O_ij S_j[DD] d_i on tensor cores

@@ -661,6 +661,7 @@ __global__ void __launch_bounds__(256, S == 9 ? 4 : 1) k_crt_u(int ldN, int n_d,
 namespace {
 constexpr int kSmemI8 = 1024 + kStagesI8 * 2 * kOperand + (int)sizeof(I8Shared);
 constexpr int kSmemTurn = kMod * 32 * kTurnWords * (int)sizeof(uint32_t);
+constexpr int kNormSmem = (int)sizeof(double) * 32 * (kUMaxDense + 1);
 constexpr int kGroupI8 = 8;
 
 int up(int64_t v, int m) { return (int)((v + m - 1) / m * m); }
@@ -752,8 +753,7 @@ int crt_prepare(Ctx* c) {
   GPL_TRY(c, cudaFuncSetAttribute(k_crt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemI8));
   GPL_TRY(c, cudaFuncSetAttribute(k_crt_conv_cols<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTurn));
   GPL_TRY(c, cudaFuncSetAttribute(k_crt_conv_cols<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTurn));
-  const int smem_n = (int)sizeof(double) * 32 * (c->n_d + 1);
-  GPL_TRY(c, cudaFuncSetAttribute(k_crt_norm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_n));
+  GPL_TRY(c, cudaFuncSetAttribute(k_crt_norm_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, kNormSmem));
   return GPL_OK;
 }
 
@@ -871,6 +871,109 @@ int launch_crt_uq(Ctx* c) {
     });
     GPL_LAUNCHED(c, "k_crt_u");
   }
+  return GPL_OK;
+}
+
+// T[l][j][dcol a] = sum_i D_ia g_il W_ij / Omega_i: the Gram's operands and kernels with the products of the
+// dense columns and the L per-cell columns in place of the dense pairs, as many columns at a time as
+// the pairs' space holds.
+__global__ void k_crt_column_pairs(int n_d, int rows, int2* __restrict__ pairs) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < rows) pairs[r] = make_int2(r % n_d, n_d + r / n_d);
+}
+__global__ void __launch_bounds__(256) k_crt_t(int J, int P, int n_d, int rows, int64_t ldo, size_t plane,
+                                               const uint8_t* __restrict__ in, const double* __restrict__ inv_j,
+                                               const double* __restrict__ inv_p, const int* __restrict__ dcol,
+                                               int first, double* __restrict__ T, const int* __restrict__ flag) {
+  if (*flag) return;
+  const int j = blockIdx.y, r0 = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (r0 >= rows) return;
+  double v[4];
+  crt_values(in + (size_t)j * ldo + r0, plane, v);
+  const double sj = inv_j[j] * kUnit;
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const int r = r0 + e;
+    if (r >= rows) break;
+    double* t = T + ((size_t)(r / n_d) * J + j) * P + dcol[r % n_d];
+    const double x = v[e] * inv_p[r] * sj;
+    *t = first ? x : *t + x;
+  }
+}
+
+// The two forms' times (us), by the rates measured at 30,000 x 1,000 with 132 dense columns: 330 per
+// column for the DMMA form (24 TFLOP/s, at least 15), and for this one the conversions, the products
+// (at 2.7e9 per us) and some nine launches. 20 columns there: 6.5 ms and 1.1 ms.
+static int crt_column_group(const Ctx* c, int L) { return std::min(L, c->pr.n_pairs / c->n_d); }
+bool crt_columns_faster(const Ctx* c, int L) {
+  const PairState& s = c->pr;
+  if (!s.ready || !s.crt.on || !s.crt.gram_cells || c->n_d > 144) return false;
+  const double N = c->N, J = c->J, per = crt_column_group(c, L), rows = per * c->n_d;
+  const double dmma = L * std::max(15.0, 2.0 * N * J * c->n_d / 24e6);
+  const double one = 60 + N * (2.2e-6 * J + 2.3e-6 * rows) + 2.0 * kMod * N * s.crt.Jp * up(rows, kTile) / 2.7e9;
+  return std::ceil(L / per) * one < dmma;
+}
+size_t crt_columns_work(const Ctx* c, int L) {
+  const int per = crt_column_group(c, L);
+  return (size_t)(c->n_d + per) * c->ldN + (size_t)per * c->n_d + 2;
+}
+
+// *done is false where an operand is not finite (nothing of T is to be used then).
+int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, bool* done) {
+  PairState& s = c->pr;
+  CrtState& t = s.crt;
+  const int per = crt_column_group(c, L);
+  const double* rOm = nullptr;
+  int rc = recip_omega(c, &rOm);
+  if (rc) return rc;
+  ProfScope ps(c, "zt_u");
+  double* D = work + (reinterpret_cast<uintptr_t>(work) / sizeof(double) & 1);  // 16-byte aligned columns
+  int2* pairs = reinterpret_cast<int2*>(D + (size_t)(c->n_d + per) * c->ldN);
+  const double R = crt_norm_limit();
+  double *sc_j = t.scales, *inv_j = sc_j + t.Jp, *sc_p = inv_j + t.Jp, *inv_p = sc_p + t.Pp;
+  double* part = reinterpret_cast<double*>(t.g_out);
+  const size_t plane_a = (size_t)t.Jp * t.gram_cells, plane_b = (size_t)t.Pp * t.gram_cells;
+  const size_t plane_o = (size_t)t.Jp * t.Pp, col = sizeof(double) * c->ldN;
+  const int smem_n = (int)sizeof(double) * 32 * (c->n_d + per + 1);
+  GPL_TRY(c, cudaMemsetAsync(t.flag, 0, sizeof(int), c->stream));
+  GPL_TRY(c, cudaMemcpyAsync(D, c->Dm, col * c->n_d, cudaMemcpyDeviceToDevice, c->stream));
+  GPL_TRY(c, cudaMemsetAsync(D + (size_t)c->n_d * c->ldN, 0, col * per, c->stream));
+  k_crt_column_pairs<<<div_up(per * c->n_d, 256), 256, 0, c->stream>>>(c->n_d, per * c->n_d, pairs);
+  GPL_LAUNCHED(c, "k_crt_column_pairs");
+  for (int l0 = 0; l0 < L; l0 += per) {
+    const int nl = std::min(per, L - l0), rows = nl * c->n_d, cols = c->n_d + nl;
+    GPL_TRY(c, cudaMemcpy2DAsync(D + (size_t)c->n_d * c->ldN, col, G + (size_t)l0 * c->N, sizeof(double) * c->N,
+                                 sizeof(double) * c->N, nl, cudaMemcpyDeviceToDevice, c->stream));
+    for (int c0 = 0; c0 < c->N; c0 += t.gram_cells) {
+      const int len = std::min(t.gram_cells, c->N - c0), kpad = up(len, kChunk);
+      k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, t.flag);
+      GPL_LAUNCHED(c, "k_crt_norm_rows");
+      const int gx = div_up(rows, 256 * kNormPairs);
+      const int gy = std::max(1, std::min({div_up(len, 64), 592 / gx, 256}));
+      const int cper = up(div_up(len, gy), 32);
+      const int ny = div_up(len, cper);
+      k_crt_norm_pairs<<<dim3(gx, ny), 256, smem_n, c->stream>>>(c->ldN, cols, c0, c0 + len, cper, rows, pairs, D, rOm,
+                                                                part);
+      GPL_LAUNCHED(c, "k_crt_norm_pairs");
+      k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.flag);
+      GPL_LAUNCHED(c, "k_crt_scales");
+      k_crt_conv_rows<<<dim3(div_up(kpad, 2048), c->J), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad,
+                                                                            t.gram_cells, plane_a, sc_j, t.g_a, t.flag);
+      GPL_LAUNCHED(c, "k_crt_conv_rows");
+      k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(rows, kConvPairs)), 256, 0, c->stream>>>(
+          c->ldN, c0, len, kpad, t.gram_cells, plane_b, rows, pairs, D, rOm, sc_p, t.g_b, t.flag);
+      GPL_LAUNCHED(c, "k_crt_conv_pairs");
+      if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp))) return rc;
+      k_crt_t<<<dim3(div_up(rows, 1024), c->J), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
+                                                                    inv_j, inv_p, c->dcol_d, c0 == 0,
+                                                                    T + (size_t)l0 * c->J * c->P, t.flag);
+      GPL_LAUNCHED(c, "k_crt_t");
+    }
+  }
+  int flag = 0;
+  GPL_TRY(c, cudaMemcpyAsync(&flag, t.flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if ((rc = crt_error_flag(c))) return rc;  // waits for the stream
+  *done = flag == 0;
   return GPL_OK;
 }
 

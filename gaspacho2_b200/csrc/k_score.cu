@@ -208,7 +208,8 @@ size_t score_work(const Ctx* c, int L) {
   return (size_t)L * ((size_t)3 * c->N + c->ldN + (size_t)4 * c->J + (size_t)c->J * c->P) + 1;
 }
 
-int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch) {
+// crt: scratch goes on with crt_columns_work values for the integer form
+int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratch, bool crt) {
   const size_t N = c->N, J = c->J, P = c->P;
   // scratch: G2 (2L x N), Gt (N x L), C (J x 2L), td (J x L), sp (J x L), G in group order, t (L x J x P)
   double* G2 = scratch;
@@ -220,7 +221,9 @@ int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratc
   double* T = Gg + (size_t)L * c->ldN;
   T += (T - scratch) & 1;
   int rc;
-  for (int l = 0; l < L; l++)
+  bool done = false;
+  if (crt && (rc = launch_crt_columns(c, L, G, T, scratch + score_work(c, L), &done))) return rc;
+  for (int l = 0; l < L && !done; l++)
     if ((rc = dgen_zt_u(c, 2, G + (size_t)l * N, T + (size_t)l * J * P))) {
       if (rc == GPL_ERR_ARG) c->err = "per-cell Z^T u takes at most 144 dense columns";
       return rc;

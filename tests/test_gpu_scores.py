@@ -57,3 +57,26 @@ def test_scores_against_numpy(config, N, G, M, L, V, donors):
             s, kept = ref(dos[np.asarray(z.columns[-1]), j, :].astype(float))
             assert np.all(np.abs(cis[j] - s) <= 1e-10 * (1.0 + np.abs(s)) / np.minimum(kept, 1.0))
             assert np.array_equal(lr[j], cis[j] ** 2)
+
+
+@pytest.mark.parametrize("N,G,M,L", [(513, 32, 20, 2), (1000, 40, 33, 40), (2400, 257, 8, 33), (3001, 300, 128, 64)])
+def test_columns_in_integer_arithmetic(N, G, M, L):
+    """Z^T diag(W/Omega) g of the columns by the integer form (one group of columns and several, one range of
+    cells) against the DMMA form, which a single column and a column that is not finite take. Both are exact
+    to some 2^-50 of the norms; a score's variance is what is left of g^T diag(w) g, here at least 1e-3."""
+    ds = synth.make(2, 4, N=N, G=G, M=M, Q=5, init=False)
+    ds.init.rho[:] = 2.0
+    geno = np.random.default_rng(7).normal(1.0, 0.7, (N, L))
+    with GPLVM.from_dataset(ds) as m:
+        m.set_params(ds.init)
+        m.kernel_mats()
+        m.glm_init()
+        m.irls_sweep(0, 30)
+        S = m.score_stats(geno)
+        one = np.concatenate([m.score_stats(geno[:, k:k + 1]) for k in range(L)], 1)
+        geno[5, L - 1] = np.nan
+        T = m.score_stats(geno)
+    assert np.all(np.isfinite(S))
+    assert np.all(np.abs(S - one) <= 1e-9 * (1.0 + np.abs(one)))
+    assert np.all(np.isnan(T[:, L - 1]))
+    assert np.all(np.abs(T[:, :L - 1] - one[:, :L - 1]) <= 1e-9 * (1.0 + np.abs(one[:, :L - 1])))
