@@ -410,12 +410,11 @@ def de_leg(args, ds, stream, device):
     return res
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one Gram (the pair products
-# written once, then the GEMM), from a single-pass ncu capture of this bench's own command at
-# config 2 (the metric is not available inside the timed run): k_pair_products read 0.11 GB and
-# wrote 7.00 GB, k_pair_gram read 174.40 GB and wrote 1.73 GB, against 16.6 GB of algorithmic
-# bytes (products 7.1 GB written and read once, W 8.0 GB read, Psi dense blocks 1.4 GB written):
-# the grouped tile order leaves each operand tile read from DRAM about 11 times, at 0.3 TB/s.
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one Gram in its FP64 multiply-add form
+# (the pair products written once, then the GEMM), from a single-pass ncu capture of this bench's own
+# command at config 2 (the metric is not available inside the timed run): k_pair_products read 0.11 GB
+# and wrote 7.00 GB, k_pair_gram read 174.40 GB and wrote 1.73 GB. The integer form is not captured.
+MODULI = 14  # of the integer form of the FP64 pair products
 TRAFFIC_BYTES = {("gram", 2, 100000, 10000, 128, 10): 0.11e9 + 7.00e9 + 174.40e9 + 1.73e9}
 
 
@@ -705,6 +704,20 @@ def run_ours(args):
                                     if peaks.get("bf16_tflops_sustained") else "of fallback: 1.4 PFLOP/s sustained"),
                     "flops_per_launch": tflops, "flops_note": "useful flops of the contraction, padding "
                     "excluded; the tensor pipe executes 3x this (hi*hi + hi*lo + lo*hi BF16 products)",
+                    "avg_launch_ms": avg_s * 1e3, "share_of_step": prof[dom][0] / max(total_prof, 1e-30)}
+        elif dom in ft and m.get_option("pair_form") & {"gram": 1, "uq": 2}.get(dom, 0):
+            # FP64 sums by residues: fourteen INT8 products of the same size on tcgen05
+            ops = MODULI * ft[dom]
+            pk = 2.0 * (peaks.get("bf16_tflops_sustained") or FALLBACK_BF16_SUSTAINED)
+            avg_s = prof[dom][0] / args.profile_steps / 1e3
+            achieved = ops / avg_s / 1e12
+            roof = {"kernel": dom, "bound": "tensor", "pipe": "INT8 (tcgen05.mma kind::i8), fourteen moduli",
+                    "achieved": achieved, "peak": pk, "unit": "TOP/s", "frac": achieved / pk, "traffic": None,
+                    "peak_source": "twice the measured bf16_tflops_sustained (INT8 has twice the BF16 peak; "
+                                   "MEASURED_PEAKS.json has no INT8 entry)",
+                    "flops_per_launch": ops, "flops_note": f"{MODULI} products of the unique column pairs, padding "
+                    "excluded; the time includes the operands' conversions and the way back to FP64",
+                    "fp64_equivalent_tflops": ft[dom] / avg_s / 1e12,
                     "avg_launch_ms": avg_s * 1e3, "share_of_step": prof[dom][0] / max(total_prof, 1e-30)}
         elif dom in ft:
             f64 = fp64_peak_tflops(torch)

@@ -84,7 +84,7 @@ static void free_state(Ctx* c) {
   tc_release(c);
   pair_release(c);
   void* extra[] = {c->cellfac, c->lvt, c->Dm, c->gsum, c->gT, c->HK, c->dcol_d, c->cv_nh_d, c->cv_nlev_d, c->gid_d, c->glev_d,
-                   c->gcells_d, c->gstart_d, c->codes_d, c->hk_tiles_d, c->hk_tiles128_d, c->part, c->work, c->hk_cells_d,
+                   c->gcells_d, c->gstart_d, c->codes_d, c->hk_tiles128_d, c->part, c->work, c->hk_cells_d,
                    c->lvl_cc_d, c->lvl_v_d, c->lvl_ptr_d, c->lvl_grp_d, c->hk_pos_d, c->Wg, c->Dg, c->rOmg,
                    c->gpos_d};
   for (void* q : extra)
@@ -100,7 +100,6 @@ static void free_state(Ctx* c) {
   c->Wg = c->Dg = c->rOmg = nullptr;
   c->gpos_d = nullptr;
   c->n_lvl = 0;
-  c->hk_tiles_d = nullptr;
   c->n_grp = c->n_cv = 0;
   void* bufs[] = {c->Z,      c->W,      c->Nu,      c->Psi,     c->PsiInv, c->Beta,   c->tBeta,  c->scratch,
                   c->U,      c->Kmm,    c->Kinv,    c->KinvKmn, c->titsias, c->DeltaInv, c->Omega, c->delta,
@@ -753,6 +752,7 @@ int gpl_get_option(const gpl_ctx* h, const char* name, int64_t* value) {
   else if (s == "autotune") *value = c->autotune ? 1 : 0;
   else if (s == "tail_ctas_per_sm") *value = c->tail_ctas_per_sm;
   else if (s == "graph_replays") *value = c->graph_replays;
+  else if (s == "pair_form") *value = (c->pr.crt.gram_cells > 0 ? 1 : 0) | (c->pr.crt.grad_cells > 0 ? 2 : 0);
   else return GPL_ERR_ARG;
   return GPL_OK;
 }
@@ -953,11 +953,6 @@ int gpl_load_design(gpl_ctx* h, int N, int n_var, const int32_t* cv, const int32
       c->cv_nh.push_back(nh[catv[v]]);
       c->cv_nlev.push_back(vc[catv[v]] * vvv[catv[v]]);
     }
-  std::vector<int2> tiles;
-  if (grouped)
-    for (int g = 0; g < n_grp; g++)
-      for (int r0 = 0; r0 < gstart[g + 1] - gstart[g]; r0 += 64) tiles.push_back(make_int2(g, r0));
-  c->n_hk_tiles = (int)tiles.size();
   std::vector<int2> tiles128;
   std::vector<int32_t> tile_cells;  // the cell of each of the 128 slots of every tile, -1 past the group
   std::vector<int32_t> tile_pos;    // the same slots as positions in group order
@@ -1035,7 +1030,6 @@ int gpl_load_design(gpl_ctx* h, int N, int n_var, const int32_t* cv, const int32
     GPL_RUN(dalloc(c, &c->gid_d, (size_t)N, "cell groups"));
     GPL_RUN(dalloc(c, &c->lvt, (size_t)lvt_ld(J) * n_grp, "level sums per group"));
     GPL_RUN(dalloc(c, &c->gstart_d, gstart.size(), "group offsets"));
-    GPL_RUN(dalloc(c, &c->hk_tiles_d, tiles.size(), "group tiles"));
     GPL_RUN(dalloc(c, &c->hk_tiles128_d, tiles128.size(), "group tiles"));
     GPL_RUN(dalloc(c, &c->hk_cells_d, tile_cells.size(), "group tile cells"));
     GPL_RUN(dalloc(c, &c->hk_pos_d, tile_pos.size(), "group tile positions"));
@@ -1080,7 +1074,6 @@ int gpl_load_design(gpl_ctx* h, int N, int n_var, const int32_t* cv, const int32
     GPL_TRY(c, cudaMemcpy(c->lvl_ptr_d, lvl_ptr.data(), sizeof(int32_t) * lvl_ptr.size(), cudaMemcpyHostToDevice));
     if (!lvl_grp.empty())
       GPL_TRY(c, cudaMemcpy(c->lvl_grp_d, lvl_grp.data(), sizeof(int32_t) * lvl_grp.size(), cudaMemcpyHostToDevice));
-    GPL_TRY(c, cudaMemcpy(c->hk_tiles_d, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice));
     GPL_TRY(c, cudaMemcpy(c->hk_tiles128_d, tiles128.data(), sizeof(int2) * tiles128.size(), cudaMemcpyHostToDevice));
     GPL_TRY(c, cudaMemcpy(c->hk_pos_d, tile_pos.data(), sizeof(int32_t) * tile_pos.size(), cudaMemcpyHostToDevice));
     GPL_TRY(c, cudaMemcpy(c->hk_cells_d, tile_cells.data(), sizeof(int32_t) * tile_cells.size(),

@@ -187,9 +187,7 @@ struct Ctx {
   // (ascending) as offsets into a list
   int n_lvl = 0;
   int *lvl_cc_d = nullptr, *lvl_v_d = nullptr, *lvl_ptr_d = nullptr, *lvl_grp_d = nullptr;
-  int2* hk_tiles_d = nullptr;       // (group, first row) of every 64-cell tile of the group lists
-  int n_hk_tiles = 0;
-  int2* hk_tiles128_d = nullptr;    // the same for 128-cell tiles
+  int2* hk_tiles128_d = nullptr;    // (group, first row) of every 128-cell tile of the group lists
   int* hk_cells_d = nullptr;        // the cell of each slot of those tiles (-1 past the group)
   int* hk_pos_d = nullptr;          // the same slots as positions in group order (-1 past the group)
   // cells in group order (the cells of each group contiguous): W (refreshed with W), the dense

@@ -100,6 +100,9 @@ GPL_API int gpl_set_precision(gpl_ctx* ctx, int precision);
  *                       Not while profiling or tc_check is on. Reads back as 0 if the capture
  *                       was refused; the context then runs eagerly. Default 0.
  *   "graph_replays"     (read only) graph launches so far
+ *   "pair_form"         (read only) the FP64 column-pair products that run in integer arithmetic
+ *                       modulo fourteen moduli: 1 the Gram, 2 the gradient's, added (0 before
+ *                       the first of them)
  *   "fused_tail"        1: each IRLS sweep's per-gene tail (cholPsi, the solve and coefficient
  *                       update of getBetaPhi, getLkhdPois: ggplvm.cu:683-692, 418-464, 703-724)
  *                       runs as one persistent launch whose CTAs take genes from a queue ordered
