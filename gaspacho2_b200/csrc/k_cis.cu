@@ -62,7 +62,7 @@ __global__ void k_group_resid(int N, int ldN, int J, int n_grp, int pvars, const
 // its level's groups, a warp per variant the sums over all groups. T[(j - j0) V + v][P];
 // num[j + v J] = s, gw[j + v J] = g^T diag(w) g. A block per gene that walked the groups once per variant
 // and column, and the levels in one thread, took 10.7 ms for 1,000 genes x 20 variants with the
-// substitution (400 groups, P = 236); the two kernels take 0.6 ms.
+// substitution (400 groups, P = 236); this kernel and k_fwd_quad take 0.54 + 0.5 ms.
 constexpr int kCisV = 16, kCisGroups = 128;
 __global__ void __launch_bounds__(1024) k_cis_t(int j0, int J, int P, int n_d, int n_dp, int n_grp, int n_lvl, int V,
                                                 const int* __restrict__ dcol, const int* __restrict__ lvl_cc,

@@ -58,7 +58,7 @@ struct CrtConst {
   float ca[kMod][4], cb[kMod][4];  // 2^(16 l) y mod p and 2^(16 l) mod p, symmetric
   float p[kMod], ip[kMod];
   uint32_t pu[kMod], off[kMod], magic[kMod];  // INT32 -> byte: (x + off) mod p by a multiply-high
-  uint32_t f2[kMod], f1[kMod], f0[kMod];      // 1 / p_l: 32 + 32 + 16 fractional bits
+  uint32_t fr[5][kMod / 2];  // 1 / p_l to 80 bits in 16-bit digits (lowest first), two moduli per word
 };
 
 constexpr u128 product() {
@@ -91,9 +91,7 @@ constexpr CrtConst make_const() {
     c.off[l] = (uint32_t)(((2147483648ull + p - 1) / p) * p);
     c.magic[l] = (uint32_t)((1ull << 39) / (unsigned long long)p);
     const u128 f = (((u128)1 << 80) + p / 2) / (u128)p;
-    c.f2[l] = (uint32_t)(f >> 48);
-    c.f1[l] = (uint32_t)(f >> 16);
-    c.f0[l] = (uint32_t)(f & 0xffff);
+    for (int k = 0; k < 5; k++) c.fr[k][l / 2] |= (uint32_t)((f >> (16 * k)) & 0xffff) << (16 * (l & 1));
   }
   return c;
 }
@@ -580,19 +578,27 @@ __device__ __forceinline__ void crt_values(const uint8_t* __restrict__ in, size_
   uint32_t w[kMod];
 #pragma unroll
   for (int l = 0; l < kMod; l++) w[l] = __ldcs(reinterpret_cast<const uint32_t*>(in + (size_t)l * plane));
+  // two entries at a time: digit sums q[k] = sum_l c_l (digit k of 1 / p_l) < 2^28, two moduli per
+  // instruction (64 a clock and SM, as a multiply-add; the 64-bit multiply-adds they replace, 20)
 #pragma unroll
-  for (int e = 0; e < 4; e++) {
-    uint64_t s1 = 0;
-    uint32_t s2 = 0, s0 = 1u << 15;
+  for (int e = 0; e < 4; e += 2) {
+    uint32_t q0[5] = {1u << 15, 0, 0, 0, 0}, q1[5] = {1u << 15, 0, 0, 0, 0};
 #pragma unroll
-    for (int l = 0; l < kMod; l++) {
-      const uint32_t c = (w[l] >> (8 * e)) & 255u;
-      s2 += c * crt.f2[l];
-      s1 += (uint64_t)c * crt.f1[l];
-      s0 += c * crt.f0[l];
+    for (int h = 0; h < kMod / 2; h++) {
+      const uint32_t c = __byte_perm(w[2 * h], w[2 * h + 1], e ? 0x7362 : 0x5140);  // bytes of both planes
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        q0[k] = __dp2a_lo(crt.fr[k][h], c, q0[k]);
+        q1[k] = __dp2a_hi(crt.fr[k][h], c, q1[k]);
+      }
     }
-    const int64_t x = (int64_t)(((uint64_t)s2 << 32) + s1 + (s0 >> 16));
-    v[e] = (double)x;
+    auto value = [](const uint32_t (&q)[5]) {
+      const uint64_t x = (uint64_t)((q[0] >> 16) + q[1]) + ((uint64_t)q[2] << 16) + ((uint64_t)q[3] << 32) +
+                         ((uint64_t)q[4] << 48);
+      return (double)(int64_t)x;
+    };
+    v[e] = value(q0);
+    v[e + 1] = value(q1);
   }
 }
 
@@ -631,8 +637,11 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
 
 // U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], W warps per cell: the
 // cell's row of V from its residues into shared memory (pair_rows.cuh).
+// Bound by the entries' arithmetic (crt_values) while 24 to 32 warps share an SM; without the limit on
+// registers the compiler keeps several entries' loads and all the digits in flight at half the warps
+// (50,000 cells x 132 columns x 1,000 genes: 6.0 against 2.9 ms).
 template <int S, int W>
-__global__ void __launch_bounds__(256, S == 9 ? 4 : 1) k_crt_u(int ldN, int n_d, int len, int c0, int64_t ldo, size_t plane,
+__global__ void __launch_bounds__(256, S > 9 ? 2 : S > 5 ? 4 : 3) k_crt_u(int ldN, int n_d, int len, int c0, int64_t ldo, size_t plane,
                                                const uint8_t* __restrict__ in, const double* __restrict__ inv_i,
                                                const double* __restrict__ inv_p, const double* __restrict__ rOm,
                                                const double* __restrict__ D, double* __restrict__ U,

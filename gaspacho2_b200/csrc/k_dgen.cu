@@ -631,7 +631,7 @@ int dgen_resid_gp(Ctx* c, const double* R, const double* B, double* G) {
 // [gene][cell] and 1/Omega [cell]; w formed at the fragment loads, the same product in the same
 // order as the register-staged form. With few groups the group's cells are split into ns runs of
 // whole slices (grid z = group x ns) whose partial sums part[z][j][a] k_reduce_groups adds in order:
-// 4 groups of 20,000 cells x 2,000 genes (68 columns) took 0.94 ms as 64 blocks, 0.17 ms split.
+// 4 groups of 20,000 cells x 2,000 genes (68 columns) took 0.94 ms as 64 blocks, 0.28 ms split.
 template <int MODE, int MT>
 __global__ void __launch_bounds__(256, 1)
     k_group_sums_dmma(int m, int n, int n_grp, int ns, int ldN, const int* __restrict__ gstart,
@@ -799,7 +799,7 @@ int dgen_group_sums_of(Ctx* c, const double* Gg, int m) {
 // the same product in the same order as the register-staged form. Table rows in tiles of MT x 16
 // (grid x); with few cell tiles, or a last wave that would be nearly empty, the genes are split into
 // ns ranges (grid y) whose partial sums part[s][r][slot] k_reduce_hk adds in order: 157 tiles on 148
-// SMs (20,000 cells, 2,000 genes, 69 rows) took 0.82 ms, 0.27 ms split.
+// SMs (20,000 cells, 2,000 genes, 69 rows) took 0.82 ms, 0.34 ms split.
 namespace {
 constexpr int kHkBK = 16, kHkSB = 132, kHkStages = 4;         // row strides 4 mod 16
 constexpr int hk_sa(int mt) { return mt * 16 + 4; }
@@ -1031,7 +1031,7 @@ __global__ void k_reduce_parts(int m, int n, int nz, const double* __restrict__ 
 // The unweighted Gram of the dense columns (initPsi, init.cu:125-181), for one matrix: Psi_0[mk, ml] =
 // Psi_0[ml, mk] = sum_i D_ia D_ib + DeltaInv. Its outputs are one to a few tiles, so the cells are split
 // over the SMs (one CTA per SM and tile, at least 64 cells each) and the partials added in order. At
-// 60,000 cells x 132 columns: 13.9 ms as 15 blocks that walked every cell, 0.16 ms so.
+// 60,000 cells x 132 columns: 13.9 ms as 15 blocks that walked every cell, 0.29 ms so.
 namespace {
 struct LdDrow {  // A(r = dense column, k = cell)
   static constexpr bool kFastK = true;

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kCholThreads) k_chol_exact(double* __restrict_
 // (L L^T) x = b for `batch` systems, one warp each; y in shared memory, the factor's next columns in
 // registers two steps ahead (NR rows per lane), so that the dependent chain does not wait on a load
 // per step. The same operations in the same order for every NR. 3,000 systems of 236: 0.70 ms with the
-// loads in the chain, 0.33 ms so.
+// loads in the chain, 0.37 ms so.
 template <int NR>
 __global__ void __launch_bounds__(128) k_solve(const double* __restrict__ L, int n, int64_t lstride,
                                                const double* __restrict__ B, int64_t bstride, double* __restrict__ X,

@@ -227,7 +227,7 @@ struct LogProduct {
 // l_j = -N/2 log phi - sum_i log(Omega/W)/2 - sum_k log L_kk + sum_k log LD_kk
 //       - sum_i nu^2 (W/Omega) / (2 phi) + b^T Psi^{-1} b / (2 phi)
 // with sum_i log Omega from the shared sums. Bound: one read of W and nu; with a log() and two
-// divisions per entry it was bound by their instructions (1.9 ms at 100,000 x 3,000 against 0.85 ms).
+// divisions per entry it was bound by their instructions (1.9 ms at 100,000 x 3,000 against 0.83 ms).
 __global__ void __launch_bounds__(256) k_lkhd_genes(int N, int ldN, int P, const double* __restrict__ W,
                                                     const double* __restrict__ Nu, const double* __restrict__ rOm,
                                                     const double* __restrict__ sums, const double* __restrict__ Psi,

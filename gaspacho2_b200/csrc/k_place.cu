@@ -54,7 +54,7 @@ __global__ void k_place_counts(int ldN, const int32_t* __restrict__ cell, const 
 // and its eight warps every eighth gene of the range of grid y, log(y!) of small counts from a table.
 // Parts per range: part[range][cell] of l_i and of sum_j W (ldN apart), added up by k_place_sums. Bound:
 // eta and the counts read, R written, one exp() per entry (a thread per cell over all genes, with an
-// lgamma() per count, took 1.77 ms at 20,003 cells x 2,000 genes; 0.25 ms so).
+// lgamma() per count, took 1.77 ms at 20,003 cells x 2,000 genes; 0.27 ms so).
 constexpr int kFactorials = 256;
 __global__ void __launch_bounds__(256) k_place_resid(int N, int ldN, int J, int jper, int pvars,
                                                      const double* __restrict__ E, const double* __restrict__ Y,

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(256) k_score_levels(int J, int P, int L, int n
 // kQuadV right-hand sides, which stay in shared memory; 16 columns of the factor at a time (their
 // diagonal block by a thread per right-hand side, the rows below by a thread per row and eight right-
 // hand sides), so that the factor is read once for all of them and the chain has P / 16 steps. 20
-// columns of 1,000 genes at P = 236 took 13 ms as one solve per column, 0.2 ms so.
+// columns of 1,000 genes at P = 236 took 13 ms as one solve per column, 0.5 ms so.
 constexpr int kQuadV = 16, kQuadRows = 128, kQuadS = kQuadV + 2;
 __global__ void __launch_bounds__(256) k_fwd_quad(int J, int P, int V, const double* __restrict__ Psi,
                                                   const double* __restrict__ T, size_t sj, size_t sv,
