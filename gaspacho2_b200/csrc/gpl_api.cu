@@ -163,6 +163,7 @@ static int read_slot(Ctx* c, int slot, double* out) {
 // not read the factor) and one persistent launch does every gene's Cholesky, solve, coefficient
 // update and Poisson likelihood; the results are the same bits as the separate kernels'.
 static int irls_sweep(Ctx* c, int jtr, double* lk) {
+  PhaseScope phase(c);
   GPL_RUN(launch_w_nu(c));
   GPL_RUN(launch_gram(c, false));
   bool fused = false;
@@ -206,6 +207,7 @@ static int irls(Ctx* c, int jtr_max, int* n_sweeps) {
 }
 
 static int objective_after_irls(Ctx* c, double* lk) {
+  PhaseScope phase(c);
   GPL_RUN(launch_oinvt(c));
   GPL_RUN(launch_chol_prior(c));
   GPL_RUN(launch_zt_u(c, 0));
@@ -215,6 +217,7 @@ static int objective_after_irls(Ctx* c, double* lk) {
 }
 
 static int objective_launch(Ctx* c, int slot) {
+  PhaseScope phase(c);
   GPL_RUN(launch_oinvt(c));
   GPL_RUN(launch_kernel_mats(c));
   GPL_RUN(launch_expand_delta(c));
@@ -232,6 +235,7 @@ static int objective_launch(Ctx* c, int slot) {
 // nu_j (ggplvm.cu:406-414) is the one getLkhd already made with the same factor and right-hand
 // side (ggplvm.cu:744-784): tilde-beta is that solution, copied instead of solved again.
 static int gradient_launch(Ctx* c, bool after_objective = false) {
+  PhaseScope phase(c);
   GPL_RUN(launch_expand_delta(c));
   if (after_objective) {
     GPL_TRY(c, cudaMemcpyAsync(c->tBeta, c->sol, sizeof(double) * (size_t)c->P * c->J, cudaMemcpyDeviceToDevice,
@@ -447,6 +451,7 @@ static int de_irls(Ctx* c, int jtr_max, double tol, int* n_sweeps, double* trace
   double prev = 0.0;
   int jtr;
   for (jtr = 0; jtr < jtr_max; jtr++) {
+    PhaseScope phase(c);
     GPL_RUN(launch_w_nu(c));
     GPL_RUN(launch_gram(c, false));
     GPL_RUN(launch_chol_batched(c, c->Psi, c->P, c->J, PP));
@@ -524,6 +529,7 @@ static int vc_fit(Ctx* c, int itr_max, int lbfgs_max, double* dg, double* obj, i
   for (itr = 0; itr < itr_max; itr++) {
     double prev = 0.0;
     for (int jtr = 0; jtr < 30; jtr++) {
+      PhaseScope phase(c);
       GPL_RUN(launch_w_nu(c));
       GPL_RUN(launch_gram(c, false));
       GPL_RUN(launch_chol_batched(c, c->Psi, c->P, c->J, PP));

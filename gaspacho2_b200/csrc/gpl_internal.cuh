@@ -188,10 +188,12 @@ struct Ctx {
   int n_lvl = 0;
   int *lvl_cc_d = nullptr, *lvl_v_d = nullptr, *lvl_ptr_d = nullptr, *lvl_grp_d = nullptr;
   int2* hk_tiles128_d = nullptr;    // (group, first row) of every 128-cell tile of the group lists
+  // within a PhaseScope: which copies that only Omega and the dense columns determine are current
+  bool in_phase = false, rOm_done = false, rOmg_done = false, Dg_done = false;
   int* hk_cells_d = nullptr;        // the cell of each slot of those tiles (-1 past the group)
   int* hk_pos_d = nullptr;          // the same slots as positions in group order (-1 past the group)
   // cells in group order (the cells of each group contiguous): W (refreshed with W), the dense
-  // columns and 1/Omega (refreshed per use), so that the group-sum GEMMs read contiguous rows
+  // columns and 1/Omega (refreshed per phase), so that the group-sum GEMMs read contiguous rows
   double *Wg = nullptr, *Dg = nullptr, *rOmg = nullptr;
   int n_hk_tiles128 = 0;
   double* part = nullptr;           // split-K partial sums
@@ -298,6 +300,21 @@ int launch_assemble_psi(Ctx* c, int J);   // categorical rows/columns of Psi fro
 int launch_assemble_b(Ctx* c, double* out);  // categorical entries of Z^T u (P x J) from the group sums
 int launch_group_tables(Ctx* c);          // per (gene, group) categorical blocks of Psi^{-1}
 int launch_hk(Ctx* c);                    // HK[i] = sum_j O_ij [h_{j,g(i)} | kappa_{j,g(i)}]
+// One phase of a call (a sweep, an objective, a gradient), during which nothing writes Omega: 1/Omega, its
+// group-ordered copy and the dense columns' (until the kernel matrices change) are made once, by their
+// first reader, in place of once per reader (4 + 3 launches of 3 us a sweep).
+struct PhaseScope {
+  Ctx* c;
+  explicit PhaseScope(Ctx* ctx) : c(ctx) { set(true); }
+  ~PhaseScope() { set(false); }
+  void set(bool on) {
+    c->in_phase = on;
+    c->rOm_done = c->rOmg_done = c->Dg_done = false;
+  }
+  PhaseScope(const PhaseScope&) = delete;
+  PhaseScope& operator=(const PhaseScope&) = delete;
+};
+int recip_omega_grouped(Ctx* c);  // c->rOmg current
 int launch_group_order(Ctx* c, const double* src, int ncols, double* dst);  // dst[col][pos] = src[col][cell(pos)]
 // k_gemm.cu
 int launch_w_nu(Ctx* c);                 // W, Nu from Beta (getWForBeta)

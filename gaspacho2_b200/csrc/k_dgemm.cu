@@ -445,24 +445,19 @@ int recip_omega(Ctx* c, const double** rOm) {
   int rc = pair_prepare(c);
   if (rc) return rc;
   PairState& s = c->pr;
-  k_recip_omega<<<div_up(s.cpad, 256), 256, 0, c->stream>>>(c->N, s.cpad, c->Omega, s.rOm);
-  GPL_LAUNCHED(c, "k_recip_omega");
   *rOm = s.rOm;
-  return GPL_OK;
-}
-
-static int launch_recip(Ctx* c) {
-  PairState& s = c->pr;
+  if (c->rOm_done) return GPL_OK;
   k_recip_omega<<<div_up(s.cpad, 256), 256, 0, c->stream>>>(c->N, s.cpad, c->Omega, s.rOm);
   GPL_LAUNCHED(c, "k_recip_omega");
+  c->rOm_done = c->in_phase;
   return GPL_OK;
 }
 
 int launch_pair_gram(Ctx* c) {
-  int rc = pair_prepare(c);
+  const double* rOm = nullptr;
+  int rc = recip_omega(c, &rOm);
   if (rc) return rc;
   PairState& s = c->pr;
-  if ((rc = launch_recip(c))) return rc;
   ProfScope ps(c, "gram");
   // the integer form, where it is planned; the kernels below then run only if it found operands out of
   // its range (gate), as they do for non-finite values
@@ -494,10 +489,10 @@ int launch_pair_gram(Ctx* c) {
 }
 
 int launch_pair_uq(Ctx* c) {
-  int rc = pair_prepare(c);
+  const double* rOm = nullptr;
+  int rc = recip_omega(c, &rOm);
   if (rc) return rc;
   PairState& s = c->pr;
-  if ((rc = launch_recip(c))) return rc;
   {
     ProfScope ps(c, "spair");
     dim3 g(div_up(s.pairs_pad, 256), std::min(c->J, 65535));

@@ -772,22 +772,28 @@ static int group_sums(Ctx* c, int mode, const double* Dg, int m) {
   });
 }
 
-static int order_romega(Ctx* c) {
+int recip_omega_grouped(Ctx* c) {
   const double* rOm = nullptr;
-  const int rc = recip_omega(c, &rOm);
-  return rc ? rc : launch_group_order(c, rOm, 1, c->rOmg);
+  int rc = recip_omega(c, &rOm);
+  if (rc || c->rOmg_done) return rc;
+  if ((rc = launch_group_order(c, rOm, 1, c->rOmg))) return rc;
+  c->rOmg_done = c->in_phase;
+  return GPL_OK;
 }
 
 int dgen_group_sums(Ctx* c, int mode) {
   int rc;
-  if (mode == 0 && (rc = order_romega(c))) return rc;
-  if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
+  if (mode == 0 && (rc = recip_omega_grouped(c))) return rc;
+  if (!c->Dg_done) {
+    if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
+    c->Dg_done = c->in_phase;
+  }
   return group_sums(c, mode, c->Dg, c->n_d);
 }
 
 int dgen_group_sums_of(Ctx* c, const double* Gg, int m) {
   if (m > c->n_d) return GPL_ERR_ARG;  // the sums' buffer
-  const int rc = order_romega(c);
+  const int rc = recip_omega_grouped(c);
   return rc ? rc : group_sums(c, 0, Gg, m);
 }
 
@@ -927,10 +933,8 @@ static int hk_ranges(const Ctx* c, int rows) {
 
 int dgen_hk(Ctx* c) {
   const int ld = c->n_d + 1;
-  const double* rOm = nullptr;
-  int rc = recip_omega(c, &rOm);
+  const int rc = recip_omega_grouped(c);
   if (rc) return rc;
-  if ((rc = launch_group_order(c, rOm, 1, c->rOmg))) return rc;
   const int nt = c->n_hk_tiles128;
   if (nt == 0) return GPL_OK;
   return with_row_tiles(ld, [&](auto mt) -> int {

@@ -64,9 +64,8 @@ int launch_group_sums(Ctx* c, int mode) {
   ProfScope pt(c, "group_t");
   dim3 g(c->n_grp, div_up(c->J, 8));
   if (mode != 2) {
-    const double* rOm = nullptr;
-    int rc = recip_omega(c, &rOm);
-    if (rc || (rc = launch_group_order(c, rOm, 1, c->rOmg))) return rc;
+    const int rc = recip_omega_grouped(c);
+    if (rc) return rc;
   }
   if (mode == 2)
     k_group_t<2><<<g, 256, 0, c->stream>>>(c->ldN, c->J, c->n_grp, c->gcells_d, c->gstart_d, c->Wg, c->rOmg,

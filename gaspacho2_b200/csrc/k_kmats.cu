@@ -235,6 +235,7 @@ __global__ void k_expand(int P, int p, int g0, int M, const int* __restrict__ mk
 // Knm, Kmm and its factor, Kmm^{-1} k_n and titsias over the latent dimensions of c->kernel_lv.
 int launch_kernel_mats(Ctx* c) {
   const int lv = c->kernel_lv;
+  c->Dg_done = false;  // the kernel columns of Dm are written
   double* Knm = c->Dm + (size_t)c->dg0 * c->ldN;
   if (lv == kLvNone) {
     ProfScope ps(c, "kernel_mats");
