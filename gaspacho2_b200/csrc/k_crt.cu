@@ -24,6 +24,7 @@
 //                  accumulators in TMEM, TMA operands), residues out as bytes. Persistent.
 //   k_crt_psi      residues -> integers -> FP64, into every gene's Psi_j.
 //   k_crt_u        residues of a cell's pair row -> V in shared memory -> U_i = sum_b D_ib V[i, ab].
+//   k_crt_t        residues -> Z^T diag(W/Omega) g of the genotype columns.
 //
 // The operands of all moduli take 14 bytes per entry in place of 8, so the cells are taken in
 // ranges that fit the buffer the DMMA form uses for its pair products (at most 8 GiB).
