@@ -246,34 +246,16 @@ __global__ void __launch_bounds__(256, 2)
   }
 }
 
-// 1 / sqrt(x) and l = sqrt(x). kNormal: from the hardware's estimate r (2^-20 or better), with
-// e = 1 - x r^2, the third-order step r (1 + e/2 + 3 e^2/8), which leaves 5 e^3 / 16 < 2^-60, and one more
-// Newton step for l outside the chain from pivot to pivot; x must be a normal number far from the limits.
-// It has no branch: a library root and a division each have one for their rare cases, and nothing is
-// scheduled across them.
-template <bool kNormal>
-__device__ __forceinline__ double inv_sqrt(double x, double& l) {
-  if (!kNormal) {
-    l = sqrt(x);
-    return 1.0 / l;
-  }
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x * r, r, 1.0);
-  r = fma(fma(0.375, e, 0.5), r * e, r);
-  const double y = x * r;
-  l = fma(0.5 * r, fma(-y, y, x), y);
-  return r;
-}
-
 // A 32 x 32 diagonal block in columns at Ap (column stride SP), the first ncol of its rows and columns
 // in use, factored in place by one warp, right-looking with row `lane` in registers; Rd gets the
 // diagonal's reciprocals. Entry (r, q) takes its products l_rk l_qk in increasing k and is scaled by
 // 1/l_qq last, as choldc's sums. The chain from pivot to pivot (lane cc + 1 needs only its own entries)
 // is kept apart from the update of the other columns, which fills its gaps; a finished column is
-// read back from shared memory (4,500 cycles for a block; with the columns passed by shuffles and a
-// library root and division, 9,000). Returns true for a pivot <= 0; a NaN pivot passes, as in choldc.
-template <bool kNormal, bool kFull>
+// read back from shared memory. The root and its reciprocal are the library's, rounded correctly over the
+// whole range of a pivot. (A hand-made root without their rare branches took half the cycles of a block,
+// but a pivot that cancels to a subnormal number has no estimate there.) Returns true for a pivot <= 0; a
+// NaN pivot passes, as in choldc.
+template <bool kFull>
 __device__ __noinline__ bool factor_block(double* Ap, int SP, int ncol, double* Rd) {
   const int lane = threadIdx.x & 31;
   double a[IB];
@@ -284,8 +266,7 @@ __device__ __noinline__ bool factor_block(double* Ap, int SP, int ncol, double* 
 #pragma unroll
   for (int cc = 0; cc < IB; cc++) {
     if (kFull || cc < ncol) {
-      double l;
-      const double rd = inv_sqrt<kNormal>(piv, l);
+      const double l = sqrt(piv), rd = 1.0 / l;
       bad |= piv <= 0.0;
       if (lane == 0) Rd[cc] = rd;
       const double x = a[cc] * rd;
@@ -300,13 +281,8 @@ __device__ __noinline__ bool factor_block(double* Ap, int SP, int ncol, double* 
   }
   return bad;
 }
-// With every diagonal entry in [1e-250, 1e290] no pivot leaves the normal range: pivots only fall,
-// and a fused a - x x that is not zero is at least 2^-106 a.
 __device__ __forceinline__ bool factor_diagonal(double* Ap, int SP, int ncol, double* Rd) {
-  const int lane = threadIdx.x & 31;
-  const double d = lane < ncol ? Ap[lane * SP + lane] : 1.0;
-  if (!__all_sync(0xffffffffu, d >= 1e-250 && d <= 1e290)) return factor_block<false, false>(Ap, SP, ncol, Rd);
-  return ncol == IB ? factor_block<true, true>(Ap, SP, ncol, Rd) : factor_block<true, false>(Ap, SP, ncol, Rd);
+  return ncol == IB ? factor_block<true>(Ap, SP, ncol, Rd) : factor_block<false>(Ap, SP, ncol, Rd);
 }
 
 // Batched Cholesky (cholPsi, ggplvm.cu:683-692), one CTA per gene, 32-column panels left to
@@ -325,8 +301,8 @@ __device__ __forceinline__ bool factor_diagonal(double* Ap, int SP, int ncol, do
 // 146,000 on the diagonal blocks. Here the panel lies in columns, everything arrives by asynchronous
 // copies (16 bytes where P is even), a chunk is as many columns as the space holds at the panel's
 // height with one or two more in flight, and the next panel's first chunks arrive during the
-// diagonal block. 3,000 matrices of P = 232: 3.1 -> 1.66 ms; 2,000 of 69: 0.28 -> 0.16 ms; 1,000 of
-// 285: 2.4 -> 0.89 ms. Each entry's operations and their order are the same but for the roots.
+// diagonal block. 3,000 matrices of P = 232: 3.1 -> 1.93 ms; 2,000 of 69: 0.28 -> 0.19 ms; 1,000 of
+// 285: 2.4 -> 1.01 ms. Each entry's operations and their order are the same.
 template <int T>
 __device__ __forceinline__ void potrf_panel_one(double* A, int P, int ns, double* sm, int& fail) {
   const int rows_pad = max(IB, (P + 15) / 16 * 16);
@@ -479,7 +455,7 @@ int potrf_buffers(int P, int extra) { return 2 * (potrf_panel_smem(P, 3) + extra
 // panel's 32 diagonal rows, 16 columns per chunk through two buffers), the first one then factoring
 // the diagonal block, all solving against it. 85 KB of shared memory whatever n is, two CTAs per
 // SM. At n = 564 (501 matrices) a column-at-a-time kernel that read the finished columns from
-// global memory for every entry took 57.6 ms, this one 2.6 ms.
+// global memory for every entry took 57.6 ms, this one 2.8 ms.
 namespace {
 constexpr int RB = 128, RC = 16;           // rows per block, finished columns per chunk
 constexpr int RSA = RB + 4, RSB = IB + 4;  // strides 4 mod 16

@@ -121,3 +121,22 @@ def test_tail_rule_same_bits(J):
             out.append({k: m.get(k) for k in ("Beta", "phi", "Psi", "lkhds")})
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k], equal_nan=True), k
+
+
+# the first column of a panel is the root of its pivot and the entries times the root's reciprocal, both
+# rounded correctly: P = M + 4 in the half-size panel kernel, the panel kernel and the row-block kernel
+@pytest.mark.parametrize("M,J", [(9, 2000), (170, 300), (300, 100)])
+def test_first_column_rounded_correctly(M, J):
+    ds = _dataset(400, J, M)
+    with GPLVM.from_dataset(ds) as m:
+        m.set_params(ds.init)
+        P = m.P
+        m.kernel_mats()
+        m.glm_init()
+        m.irls_sweep(0, 0)
+        L = m.get("Psi").reshape(J, P, P).transpose(0, 2, 1)[:, :, 0].copy()
+        m.gram()
+        psi = m.get("Psi").reshape(J, P, P).transpose(0, 2, 1)[:, :, 0]
+    root = np.sqrt(psi[:, 0])
+    assert np.array_equal(L[:, 0], root)
+    assert np.array_equal(L[:, 1:], psi[:, 1:] * (1.0 / root)[:, None])
