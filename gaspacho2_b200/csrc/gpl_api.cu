@@ -445,6 +445,7 @@ static int glm_init(Ctx* c) {
 // others): GLM initialisation, zeta, then IRLS sweeps in the DE forms with its stopping rule.
 // The summed likelihood is read back after every sweep, as the reference does.
 static int de_irls(Ctx* c, int jtr_max, double tol, int* n_sweeps, double* trace, int trace_cap) {
+  OrderScope order(c);
   GPL_RUN(glm_init(c));
   GPL_RUN(launch_de_zeta(c));
   const int64_t PP = (int64_t)c->P * c->P;
@@ -518,9 +519,12 @@ static int set_delta_dg(Ctx* c, double v) {
 static int vc_fit(Ctx* c, int itr_max, int lbfgs_max, double* dg, double* obj, int cap, int* n_itr) {
   const int p = c->p, N = c->N;
   const int64_t PP = (int64_t)c->P * c->P;
-  GPL_RUN(launch_kernel_mats(c));
-  GPL_RUN(glm_init(c));
-  GPL_RUN(launch_de_zeta(c));
+  {
+    OrderScope order(c);
+    GPL_RUN(launch_kernel_mats(c));
+    GPL_RUN(glm_init(c));
+    GPL_RUN(launch_de_zeta(c));
+  }
   VcLbfgs h;
   double dgv = 0.0;
   GPL_TRY(c, cudaMemcpy(&dgv, c->delta + (p - 2), sizeof(double), cudaMemcpyDeviceToHost));
@@ -529,6 +533,7 @@ static int vc_fit(Ctx* c, int itr_max, int lbfgs_max, double* dg, double* obj, i
   for (itr = 0; itr < itr_max; itr++) {
     double prev = 0.0;
     for (int jtr = 0; jtr < 30; jtr++) {
+      OrderScope order(c);
       PhaseScope phase(c);
       GPL_RUN(launch_w_nu(c));
       GPL_RUN(launch_gram(c, false));
@@ -1358,7 +1363,10 @@ int gpl_de_model(gpl_ctx* h, int model) {
   GPL_RUN(de_loader_value(c, model == GPL_DE_NULL));
   c->de = true;
   c->kernel_lv = model == GPL_DE_NULL ? kLvNone : (model == GPL_DE_FULL ? kLvAll : model);
-  GPL_RUN(launch_kernel_mats(c));
+  {
+    OrderScope order(c);
+    GPL_RUN(launch_kernel_mats(c));
+  }
   GPL_TRY(c, cudaStreamSynchronize(c->stream));
   return GPL_OK;
 }

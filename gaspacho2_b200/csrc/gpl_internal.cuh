@@ -71,7 +71,7 @@ struct CrtState {
 struct PairState {
   bool ready = false;
   int n_pairs = 0, pairs_pad = 0, cpad = 0, v_cells = 0;
-  int smem_gram = 0, smem_v = 0;
+  int smem_v = 0;
   int2* pairs = nullptr;
   double *rOm = nullptr, *Sp = nullptr, *V = nullptr;
   double* Gacc = nullptr;  // pairs x genes Gram accumulator when the cells need several ranges
@@ -190,6 +190,7 @@ struct Ctx {
   int2* hk_tiles128_d = nullptr;    // (group, first row) of every 128-cell tile of the group lists
   // within a PhaseScope: which copies that only Omega and the dense columns determine are current
   bool in_phase = false, rOm_done = false, rOmg_done = false, Dg_done = false;
+  bool one_order = false;           // within an OrderScope
   int* hk_cells_d = nullptr;        // the cell of each slot of those tiles (-1 past the group)
   int* hk_pos_d = nullptr;          // the same slots as positions in group order (-1 past the group)
   // cells in group order (the cells of each group contiguous): W (refreshed with W), the dense
@@ -314,6 +315,22 @@ struct PhaseScope {
   PhaseScope(const PhaseScope&) = delete;
   PhaseScope& operator=(const PhaseScope&) = delete;
 };
+// Within one, every sum of a sweep is taken in one order that no split, tile or form of a product changes:
+// the undamped IRLS of the model comparison and of the variance-component driver. A gene whose coefficients
+// overshoot there reaches weights of 1e20 times the median, its system is singular to working precision,
+// and its entries lead the table: 2,227 cells x 1,553 genes, Q = 5, three sweeps, gave a table that
+// differed by 13 times its norm between two orders of the same sums, and other entries that were not
+// finite. So the sums keep the order that they had: the Gram, the group sums and the per-gene products
+// as chains over the cells (a DMMA adds its four products in ascending order, as four multiply-adds), the
+// kernel solve and the wide Cholesky entry by entry.
+struct OrderScope {
+  Ctx* c;
+  bool before;
+  explicit OrderScope(Ctx* ctx) : c(ctx), before(ctx->one_order) { c->one_order = true; }
+  ~OrderScope() { c->one_order = before; }
+  OrderScope(const OrderScope&) = delete;
+  OrderScope& operator=(const OrderScope&) = delete;
+};
 int recip_omega_grouped(Ctx* c);  // c->rOmg current
 int launch_group_order(Ctx* c, const double* src, int ncols, double* dst);  // dst[col][pos] = src[col][cell(pos)]
 // k_gemm.cu
@@ -338,6 +355,7 @@ int launch_solve_batched(Ctx* c, const double* L, int n, int64_t lstride, const 
                          double* X, int64_t xstride, int batch);
 int launch_inverse_batched(Ctx* c);      // PsiInv from Psi's factor
 int launch_potrf_panels(Ctx* c, double* A, int n, int batch, int64_t stride);  // 32-column panels, DMMA
+constexpr int kPotrfMaxP = 288;           // widest matrix of the panel Cholesky
 int launch_inverse_panels(Ctx* c);       // the same in 32-column panels with DMMA block products
 int launch_irls_tail(Ctx* c, int jtr, int ctas_per_sm);  // persistent per-gene IRLS tail; GPL_ERR_ARG:
                                                           // P beyond the panel Cholesky's range

@@ -55,8 +55,7 @@ __device__ __forceinline__ int2 grouped_tile(int id, int tm, int tn, int group_m
   return make_int2(first + r % gm, r / gm);
 }
 
-// One 16-deep K slice of the warp tile. kNT: B stored [n][k] (true) or [k][n] (false).
-template <bool kNT>
+// One 16-deep K slice of the 64 x 32 warp tile, both operands stored [k][..].
 __device__ __forceinline__ void warp_slice(const double* __restrict__ As, const double* __restrict__ Bs, int wm,
                                            int wn, int g, int t, double (&acc)[4][4][4]) {
 #pragma unroll
@@ -71,7 +70,7 @@ __device__ __forceinline__ void warp_slice(const double* __restrict__ As, const 
 #pragma unroll
     for (int nt = 0; nt < 4; nt++) {
       const int n = wn * 32 + nt * 8 + g;
-      b[nt] = kNT ? Bs[n * SBT + kk * 4 + t] : Bs[(kk * 4 + t) * SBN + n];
+      b[nt] = Bs[(kk * 4 + t) * SBN + n];
     }
 #pragma unroll
     for (int mt = 0; mt < 4; mt++)
@@ -124,19 +123,33 @@ constexpr int kGramPsi = 0;  // one range: Psi_j[mk, ml] = Psi_j[ml, mk] = G + D
 constexpr int kGramSet = 1;  // first of several ranges: Gacc[p * J + j] = G
 constexpr int kGramAdd = 2;  // later ranges: Gacc[p * J + j] += G
 
-__global__ void __launch_bounds__(kThreads, 1)
+// Output tiles of TM pairs x TN genes, WM x WN warps. An entry is one chain of DMMAs over the cells whatever
+// the tile, so the tile's size changes no bits; a CTA's time is its tile's multiply-adds for every cell,
+// so few pairs or genes, or a last wave that is nearly empty, want small tiles (launch_pair_gram).
+template <int TM, int TN>
+struct GramTile {
+  static constexpr int WM = TM / TN >= 4 ? 4 : 2, WN = 8 / WM;
+  static constexpr int MT = TM / WM / 16, NT = TN / WN / 8;
+  static constexpr int SAm = TM + 4;  // As[k][m], 4 mod 16
+  static constexpr int smem = (int)sizeof(double) * 3 * (BK * SAm + TN * SBT);
+};
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
     k_pair_gram(int N, int ldN, int J, int P, int c0, int c1, int pairs_pad, int n_pairs, int mode,
                 const double* __restrict__ A, const int2* __restrict__ pairs, const int* __restrict__ dcol,
                 const double* __restrict__ W, const double* __restrict__ Dinv, double* __restrict__ Psi,
                 double* __restrict__ Gacc, int group_m, const int* __restrict__ gate) {
+  using G = GramTile<TM, TN>;
+  constexpr int SAm = G::SAm, MT = G::MT, NT = G::NT;
   extern __shared__ __align__(16) double smem_d[];
   if (gate && *gate == 0) return;
-  double* As = smem_d;              // [3][BK][SA]   pair products (pairs contiguous)
-  double* Bs = As + 3 * BK * SA;    // [3][BN][SBT]  weights (cells contiguous)
+  double* As = smem_d;               // [3][BK][SAm]  pair products (pairs contiguous)
+  double* Bs = As + 3 * BK * SAm;    // [3][TN][SBT]  weights (cells contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3, wm = warp >> 2, wn = warp & 3;
-  const int2 tile = grouped_tile(blockIdx.x, (n_pairs + BM - 1) / BM, (J + BN - 1) / BN, group_m);
-  const int p0 = tile.x * BM, j0 = tile.y * BN;
+  const int g = lane >> 2, t = lane & 3, wm = warp / G::WN, wn = warp % G::WN;
+  const int2 tile = grouped_tile(blockIdx.x, (n_pairs + TM - 1) / TM, (J + TN - 1) / TN, group_m);
+  const int p0 = tile.x * TM, j0 = tile.y * TN;
   const int nsl = (c1 - c0 + BK - 1) / BK;
 
   // slice s: cells [c0 + 16 s, c0 + 16 s + 16) of both operands (16-byte copies; rows of A
@@ -144,30 +157,31 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto load = [&](int s, int st) {
     const int kb = s * BK;
 #pragma unroll
-    for (int r = 0; r < (BM * BK / 2) / kThreads; r++) {
+    for (int r = 0; r < (TM * BK / 2) / kThreads; r++) {
       const int ch = tid + r * kThreads;
-      const int k = ch >> 6, part = ch & 63;
+      const int k = ch / (TM / 2), part = ch % (TM / 2);
       const int row = kb + k;
       const int nb = (c0 + row < c1) ? 16 : 0;
       const double* src = A + (size_t)min(row, c1 - c0 - 1) * pairs_pad + p0 + part * 2;
-      cp_async16(As + st * BK * SA + k * SA + part * 2, src, nb);
+      cp_async16(As + st * BK * SAm + k * SAm + part * 2, src, nb);
     }
 #pragma unroll
-    for (int r = 0; r < (BN * BK / 2) / kThreads; r++) {
+    for (int r = 0; r < (TN * BK / 2 + kThreads - 1) / kThreads; r++) {
       const int ch = tid + r * kThreads;
+      if (TN * BK / 2 < kThreads && ch >= TN * BK / 2) break;
       const int n = ch >> 3, part = ch & 7;
       const int j = j0 + n, i = c0 + kb + part * 2;
       const int nb = (j < J) ? 8 * max(0, min(2, min(N, c1) - i)) : 0;
       const double* src = W + (size_t)min(j, J - 1) * ldN + min(i, ldN - 2);
-      cp_async16(Bs + st * BN * SBT + n * SBT + part * 2, src, nb);
+      cp_async16(Bs + st * TN * SBT + n * SBT + part * 2, src, nb);
     }
   };
 
-  double acc[4][4][4];
+  double acc[MT][NT][4];
 #pragma unroll
-  for (int x = 0; x < 4; x++)
+  for (int x = 0; x < MT; x++)
 #pragma unroll
-    for (int y = 0; y < 4; y++)
+    for (int y = 0; y < NT; y++)
 #pragma unroll
       for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
 
@@ -181,15 +195,32 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
     cp_async_commit();
-    warp_slice<true>(As + (s % 3) * BK * SA, Bs + (s % 3) * BN * SBT, wm, wn, g, t, acc);
+    const double* as = As + (s % 3) * BK * SAm;
+    const double* bs = Bs + (s % 3) * TN * SBT;
+#pragma unroll
+    for (int kk = 0; kk < BK / 4; kk++) {
+      double a[MT][2], b[NT];
+      const double* ar = as + (kk * 4 + t) * SAm + wm * MT * 16 + g;
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++) {
+        a[mt][0] = ar[mt * 16];
+        a[mt][1] = ar[mt * 16 + 8];
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; nt++) b[nt] = bs[(wn * NT * 8 + nt * 8 + g) * SBT + kk * 4 + t];
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
+    }
   }
   cp_async_wait<0>();
 
 #pragma unroll
-  for (int mt = 0; mt < 4; mt++)
+  for (int mt = 0; mt < MT; mt++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int p = p0 + wm * 64 + mt * 16 + g + h * 8;
+      const int p = p0 + (wm * MT + mt) * 16 + g + h * 8;
       if (p >= n_pairs) continue;
       size_t mk = 0, ml = 0;
       double dv = 0.0;
@@ -200,10 +231,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         dv = Dinv[mk + ml * P];
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; nt++)
+      for (int nt = 0; nt < NT; nt++)
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-          const int j = j0 + wn * 32 + nt * 8 + 2 * t + e;
+          const int j = j0 + (wn * NT + nt) * 8 + 2 * t + e;
           if (j >= J) continue;
           const double v = acc[mt][nt][h * 2 + e];
           if (mode == kGramPsi) {
@@ -314,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
     cp_async_commit();
-    warp_slice<false>(As + (s % 3) * BK * SA, Bs + (s % 3) * BK * SBN, wm, wn, g, t, acc);
+    warp_slice(As + (s % 3) * BK * SA, Bs + (s % 3) * BK * SBN, wm, wn, g, t, acc);
   }
   cp_async_wait<0>();
 
@@ -395,7 +426,6 @@ int pair_prepare(Ctx* c) {
   size_t cap = std::max<size_t>(BM, ((size_t)8 << 30) / row / BM * BM);
   if (c->pair_range_cells >= BM) cap = std::min<size_t>(cap, (size_t)c->pair_range_cells / BM * BM);
   s.v_cells = (int)std::min<size_t>((size_t)s.cpad, cap);
-  s.smem_gram = (int)sizeof(double) * 3 * (BK * SA + BN * SBT);
   s.smem_v = (int)sizeof(double) * 3 * (BK * SA + BK * SBN);
   // the integer form (k_crt.cu) keeps its operands in the same buffer, of 1 GiB at least: with 14 bytes
   // per operand entry it takes the cells in a few ranges where the DMMA form takes one, which costs it
@@ -420,7 +450,10 @@ int pair_prepare(Ctx* c) {
     c->err = "device allocation failed: pair Gram accumulator";
     return GPL_ERR_ALLOC;
   }
-  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_gram));
+  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  GramTile<128, 128>::smem));
+  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  GramTile<64, 64>::smem));
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_v, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_v));
   const int rc = crt_prepare(c);
   if (rc) {
@@ -453,6 +486,18 @@ int recip_omega(Ctx* c, const double** rOm) {
   return GPL_OK;
 }
 
+// The Gram's tile for n_pairs x J outputs, by its time per 16 cells: the tile's multiply-adds (64 per clock
+// and SM) times the tiles an SM takes, at least 400 clocks of copies and barriers; the smaller tiles with a
+// tenth for their operands' traffic.
+static int gram_tile(const Ctx* c, int n_pairs) {
+  const auto cost = [&](int tm, int tn) {
+    const double tiles = (double)div_up(n_pairs, tm) * div_up(c->J, tn);
+    return std::ceil(tiles / c->sm_count) * std::max(tm * tn * 16 / 64, 400) * (tm < 128 ? 1.1 : 1.0);
+  };
+  const double big = cost(128, 128), mid = cost(64, 64), small = cost(64, 16);
+  return big <= mid && big <= small ? 0 : mid <= small ? 1 : 2;
+}
+
 int launch_pair_gram(Ctx* c) {
   const double* rOm = nullptr;
   int rc = recip_omega(c, &rOm);
@@ -461,7 +506,7 @@ int launch_pair_gram(Ctx* c) {
   ProfScope ps(c, "gram");
   // the integer form, where it is planned; the kernels below then run only if it found operands out of
   // its range (gate), as they do for non-finite values
-  const int* gate = s.crt.gram_cells ? s.crt.flag : nullptr;
+  const int* gate = s.crt.gram_cells && !c->one_order ? s.crt.flag : nullptr;
   if (gate && (rc = launch_crt_gram(c))) return rc;
   const bool one = s.v_cells >= c->N;
   for (int c0 = 0; c0 < c->N; c0 += s.v_cells) {
@@ -471,13 +516,20 @@ int launch_pair_gram(Ctx* c) {
         c->ldN, c->n_d, c0, c1, s.n_pairs, s.pairs_pad, s.pairs, c->Dm, s.rOm, s.V, gate);
     GPL_LAUNCHED(c, "k_pair_products");
     const int mode = one ? kGramPsi : (c0 == 0 ? kGramSet : kGramAdd);
-    const int g = div_up(s.n_pairs, BM) * div_up(c->J, BN);
     Tunable* tu = nullptr;
     const int gm = gate ? kGroupM : tune_pick(c, "pair_gram", {8, 12, 16}, kGroupM, &tu);
     TuneScope ts(c, one ? tu : nullptr);
-    k_pair_gram<<<g, kThreads, s.smem_gram, c->stream>>>(c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs,
-                                                        mode, s.V, s.pairs, c->dcol_d, c->W, c->DeltaInv, c->Psi,
-                                                        s.Gacc, gm, gate);
+    auto run = [&](auto tm, auto tn) {
+      constexpr int TM = decltype(tm)::value, TN = decltype(tn)::value;
+      k_pair_gram<TM, TN><<<div_up(s.n_pairs, TM) * div_up(c->J, TN), kThreads, GramTile<TM, TN>::smem, c->stream>>>(
+          c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs, mode, s.V, s.pairs, c->dcol_d, c->W, c->DeltaInv,
+          c->Psi, s.Gacc, gm, gate);
+    };
+    using std::integral_constant;
+    const int form = gram_tile(c, s.n_pairs);
+    if (form == 0) run(integral_constant<int, 128>(), integral_constant<int, 128>());
+    else if (form == 1) run(integral_constant<int, 64>(), integral_constant<int, 64>());
+    else run(integral_constant<int, 64>(), integral_constant<int, 16>());
     GPL_LAUNCHED(c, "k_pair_gram");
   }
   if (!one) {

@@ -416,7 +416,8 @@ static int split_count(int tiles, int sms) {
 // form, so the sums are those of TileTall's k_dgen over the same cell ranges). Tile: all dense
 // columns (<= 144) x 128 genes, 8 warps along the genes, each 9 x 2 DMMA tiles of 16 x 8; CTA
 // (gene tile, cell range z) writes its partial sums to part[z][a][j]. MODE 0: B = W u / Omega
-// (u cells x genes); 1: B = u; 2: B = W g / Omega with g one value per cell. The cell ranges
+// (u cells x genes); 1: B = u; 2: B = W g / Omega with g one value per cell; 3: as 0, with Omega in rOm's
+// place and W / Omega by division (an OrderScope beyond 144 columns). The cell ranges
 // start at even cells, so every 16-byte copy is aligned (ldN is a multiple of 32).
 // The dense columns are taken in row tiles of MT x 16 (grid x): one tile of the least MT in {1, 3, 5, 9}
 // that holds them, 144-row tiles beyond that.
@@ -497,6 +498,7 @@ __global__ void __launch_bounds__(256, 1)
     const double* Us = Ws + kZtBN * kZtS;
     const double* Rs = Us + kZtBN * kZtS;
     const double* Vs = Rs + kZtBK;
+    const int live = kend - (kbeg + s * kZtBK);  // cells of this slice in the range
 #pragma unroll
     for (int k4 = 0; k4 < kZtBK / 4; k4++) {
       const int kk = k4 * 4 + t;
@@ -509,7 +511,8 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
       for (int y = 0; y < 2; y++) {
         const int e = (wn * 16 + y * 8 + g) * kZtS + kk;
-        b[y] = MODE == 1 ? Us[e] : MODE == 0 ? Ws[e] * Rs[kk] * Us[e] : Ws[e] * Rs[kk] * Vs[kk];
+        if (MODE == 3) b[y] = kk < live ? Ws[e] / Rs[kk] * Us[e] : 0.0;
+        else b[y] = MODE == 1 ? Us[e] : MODE == 0 ? Ws[e] * Rs[kk] * Us[e] : Ws[e] * Rs[kk] * Vs[kk];
       }
 #pragma unroll
       for (int x = 0; x < MT; x++)
@@ -545,15 +548,18 @@ int dgen_zt_u(Ctx* c, int mode, const double* u, double* out) {
     int rc = recip_omega(c, &rOm);
     if (rc) return rc;
   }
-  return with_row_tiles(c->n_d, [&](auto mt) -> int {
+  // an OrderScope beyond 144 columns: one range of cells, in row tiles that fill the SMs better
+  const bool chain = c->one_order && c->n_d > 144;
+  if (chain && mode == 0) rOm = c->Omega;
+  return with_row_tiles(chain ? 48 : c->n_d, [&](auto mt) -> int {
     constexpr int MT = decltype(mt)::value;
     const int tiles = div_up(c->J, kZtBN), mtiles = div_up(c->n_d, MT * 16);
-    const int S = zt_splits(c, MT * 16);
+    const int S = chain ? 1 : zt_splits(c, MT * 16);
     int rc = ensure_part(c, (size_t)S * c->n_d * c->J);
     if (rc) return rc;
     int per = (c->N + S - 1) / S;
     per += per & 1;  // even range starts: aligned 16-byte copies
-    auto* fn = mode == 0 ? k_zt_u<0, MT> : mode == 1 ? k_zt_u<1, MT> : k_zt_u<2, MT>;
+    auto* fn = mode == 0 ? chain ? k_zt_u<3, MT> : k_zt_u<0, MT> : mode == 1 ? k_zt_u<1, MT> : k_zt_u<2, MT>;
     GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
     fn<<<dim3(mtiles, tiles, S), 256, zt_smem(MT), c->stream>>>(c->n_d, c->J, c->N, c->ldN, per, c->Dm, c->W, u, rOm,
                                                                c->part);
@@ -631,7 +637,8 @@ int dgen_resid_gp(Ctx* c, const double* R, const double* B, double* G) {
 // [gene][cell] and 1/Omega [cell]; w formed at the fragment loads, the same product in the same
 // order as the register-staged form. With few groups the group's cells are split into ns runs of
 // whole slices (grid z = group x ns) whose partial sums part[z][j][a] k_reduce_groups adds in order:
-// 4 groups of 20,000 cells x 2,000 genes (68 columns) took 0.94 ms as 64 blocks, 0.28 ms split.
+// 4 groups of 20,000 cells x 2,000 genes (68 columns) took 0.94 ms as 64 blocks, 0.28 ms split. MODE 2: as 0,
+// with Omega in rOmg's place and W / Omega by division (an OrderScope beyond 144 columns).
 template <int MODE, int MT>
 __global__ void __launch_bounds__(256, 1)
     k_group_sums_dmma(int m, int n, int n_grp, int ns, int ldN, const int* __restrict__ gstart,
@@ -657,7 +664,7 @@ __global__ void __launch_bounds__(256, 1)
       const int nb = (m0 + r < m && k < kend) ? 8 : 0;
       cp_async8(As + r * kZtS + kc, Dg + (size_t)min(m0 + r, m - 1) * ldN + min(k, last), nb);
     }
-    if (MODE == 0) {
+    if (MODE != 1) {
 #pragma unroll
       for (int q = 0; q < (kZtBN * kZtBK) / 256; q++) {
         const int e = tid + q * 256, cc = e >> 4, kc = e & 15, k = k0 + kc;
@@ -703,7 +710,8 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
       for (int y = 0; y < 2; y++) {
         const int e = (wn * 16 + y * 8 + g) * kZtS + kk;
-        b[y] = MODE == 0 ? Ws[e] * Rs[kk] : (kk < live && n0 + wn * 16 + y * 8 + g < n ? 1.0 * 1.0 : 0.0);
+        if (MODE == 2) b[y] = kk < live ? Ws[e] / Rs[kk] : 0.0;
+        else b[y] = MODE == 0 ? Ws[e] * Rs[kk] : (kk < live && n0 + wn * 16 + y * 8 + g < n ? 1.0 * 1.0 : 0.0);
       }
 #pragma unroll
       for (int x = 0; x < MT; x++)
@@ -748,17 +756,17 @@ static int group_runs(const Ctx* c, int J, int m, int rows) {
 }
 
 // c->gsum[j][g][a] = sum over group g of w_ij Dg_a (m columns in group order, ld ldN); w = W/Omega with
-// c->rOmg current (mode 0) or 1 for one gene (mode 1)
+// c->rOmg current (mode 0), 1 for one gene (mode 1) or W/Omega with Omega in c->rOmg (mode 2)
 static int group_sums(Ctx* c, int mode, const double* Dg, int m) {
   const int J = mode == 1 ? 1 : c->J;
   return with_row_tiles(m, [&](auto mt) -> int {
     constexpr int MT = decltype(mt)::value;
-    const int ns = group_runs(c, J, m, MT * 16);
+    const int ns = c->one_order ? 1 : group_runs(c, J, m, MT * 16);
     if (ns > 1) {
       const int rp = ensure_part(c, (size_t)c->n_grp * ns * J * m);
       if (rp) return rp;
     }
-    auto* fn = mode == 0 ? k_group_sums_dmma<0, MT> : k_group_sums_dmma<1, MT>;
+    auto* fn = mode == 0 ? k_group_sums_dmma<0, MT> : mode == 1 ? k_group_sums_dmma<1, MT> : k_group_sums_dmma<2, MT>;
     GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
     fn<<<dim3(div_up(m, MT * 16), div_up(J, kZtBN), c->n_grp * ns), 256, zt_smem(MT), c->stream>>>(
         m, J, c->n_grp, ns, c->ldN, c->gstart_d, Dg, c->Wg, c->rOmg, c->gsum, c->part);
@@ -783,6 +791,11 @@ int recip_omega_grouped(Ctx* c) {
 
 int dgen_group_sums(Ctx* c, int mode) {
   int rc;
+  if (mode == 0 && c->one_order && c->n_d > 144) {
+    mode = 2;
+    c->rOmg_done = false;
+    if ((rc = launch_group_order(c, c->Omega, 1, c->rOmg))) return rc;
+  }
   if (mode == 0 && (rc = recip_omega_grouped(c))) return rc;
   if (!c->Dg_done) {
     if ((rc = launch_group_order(c, c->Dm, c->n_d, c->Dg))) return rc;
@@ -1193,7 +1206,58 @@ static size_t part_bound(const Ctx* c) {
   return std::max(n, cell_sums_part(c));
 }
 
+// The same as one chain over the cells for every entry, within an OrderScope (gpl_internal.cuh): a warp per
+// 16 x 8 outputs, fragments straight from the columns, 32 cells' loads ahead of their products.
+__global__ void __launch_bounds__(32) k_gram_chain(int n, int N, int ldN, int P, const double* __restrict__ D,
+                                                   const int* __restrict__ dcol, const double* __restrict__ Dinv,
+                                                   double* __restrict__ Psi) {
+  const int a0 = blockIdx.x * 16, b0 = blockIdx.y * 8;
+  if (a0 > b0 + 7) return;  // below the diagonal
+  const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+  const double* ra = D + (size_t)min(a0 + g, n - 1) * ldN;
+  const double* rb = D + (size_t)min(a0 + g + 8, n - 1) * ldN;
+  const double* rc = D + (size_t)min(b0 + g, n - 1) * ldN;
+  constexpr int K = 8;  // steps of four cells
+  double x[K], y[K], z[K], acc[4] = {0.0, 0.0, 0.0, 0.0};
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < K; u++) {
+      const int k = k0 + 4 * u + t;
+      const bool in = k < N;
+      x[u] = in ? ra[k] : 0.0;
+      y[u] = in ? rb[k] : 0.0;
+      z[u] = in ? rc[k] : 0.0;
+    }
+  };
+  load(0);
+  for (int k0 = 0; k0 < N; k0 += 4 * K) {
+    double p[K], q[K], r[K];
+#pragma unroll
+    for (int u = 0; u < K; u++) p[u] = x[u], q[u] = y[u], r[u] = z[u];
+    load(k0 + 4 * K);
+#pragma unroll
+    for (int u = 0; u < K; u++) dmma_16x8x4(acc, p[u], q[u], r[u]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int a = a0 + g + 8 * h, b = b0 + 2 * t + e;
+      if (b >= n || a > b) continue;
+      const size_t mk = dcol[a], ml = dcol[b];
+      const double v = acc[2 * h + e] + Dinv[mk + ml * P];
+      Psi[mk + ml * P] = v;
+      Psi[ml + mk * P] = v;
+    }
+}
+
 int dgen_unweighted_gram(Ctx* c) {
+  if (c->one_order) {
+    k_gram_chain<<<dim3(div_up(c->n_d, 16), div_up(c->n_d, 8)), 32, 0, c->stream>>>(c->n_d, c->N, c->ldN, c->P, c->Dm,
+                                                                                  c->dcol_d, c->DeltaInv, c->Psi);
+    GPL_LAUNCHED(c, "k_gram_chain");
+    return GPL_OK;
+  }
   using T = TileSq;
   const int n = c->n_d, t = div_up(n, T::BM);
   const int S = gram_splits(c);

@@ -3,9 +3,10 @@
 // ggplvm.cu:46-53, choldc/cholsl chol.cu:19-97, initPsi init.cu:125-181).
 //
 //   k_chol_exact  one matrix in choldc's operation order (Kmm, the prior, the GLM Gram).
-//   k_chol      one matrix wider than that kernel's row slots, left-looking by columns: the
-//               update of column j reads row j of the factor (broadcast) and the rows below it
-//               (coalesced). A non-positive pivot zero-fills the matrix, as choldc does.
+//   k_chol      one matrix wider than that kernel's row slots, or a batch within an OrderScope,
+//               left-looking by columns: the update of column j reads row j of the factor
+//               (broadcast) and the rows below it (coalesced). A non-positive pivot zero-fills
+//               the matrix, as choldc does.
 //   k_solve     batched (L L^T) x = b, one warp per system: forward substitution column-
 //               oriented (coalesced), back substitution as warp dot products.
 //   k_trtri     V = L^{-1} (row-major scratch), one thread per column of V.
@@ -291,6 +292,11 @@ int launch_gram(Ctx* c, bool unweighted) {
 
 int launch_chol_batched(Ctx* c, double* A, int n, int batch, int64_t stride) {
   ProfScope ps(c, "chol");
+  if (c->one_order && n > kPotrfMaxP) {  // the row-block kernel takes its sums in another order
+    k_chol<<<batch, 256, 0, c->stream>>>(A, n, stride, 0);
+    GPL_LAUNCHED(c, "k_chol");
+    return GPL_OK;
+  }
   return launch_potrf_panels(c, A, n, batch, stride);
 }
 

@@ -52,6 +52,28 @@ __global__ void k_group_t(int ldN, int J, int n_grp, const int* __restrict__ gce
   if (lane == 0) T[(size_t)j * n_grp + g] = t;
 }
 
+// The same sums within an OrderScope (gpl_internal.cuh): a lane's cells in one chain, W / Omega by division.
+template <int MODE>
+__global__ void k_group_t_chain(int ldN, int J, int n_grp, const int* __restrict__ gcells,
+                                const int* __restrict__ gstart, const double* __restrict__ Wg,
+                                const double* __restrict__ Omega, const double* __restrict__ U,
+                                double* __restrict__ T) {
+  const int g = blockIdx.x;
+  const int j = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (j >= J) return;
+  const double *Wj = Wg + (size_t)j * ldN, *Uj = U + (size_t)j * ldN;
+  double s = 0.0;
+#pragma unroll 4
+  for (int k = gstart[g] + lane; k < gstart[g + 1]; k += 32) {
+    const int i = gcells[k];
+    if (MODE == 2) s += Uj[i];
+    else s += Wj[k] / Omega[i] * Uj[i];
+  }
+  s = warp_sum(s);
+  if (lane == 0) T[(size_t)j * n_grp + g] = s;
+}
+
 // mode 0: S with w = W/Omega (Gram of the objective and the IRLS); 1: S of gene 0 with w = 1
 // (GLM initialisation Gram); 2: T with w = 1, u = y0 (GLM initialisation right-hand side);
 // 3: T with w = W/Omega, u = nu (Z^T diag(W/Omega) nu).
@@ -63,6 +85,13 @@ int launch_group_sums(Ctx* c, int mode) {
   }
   ProfScope pt(c, "group_t");
   dim3 g(c->n_grp, div_up(c->J, 8));
+  if (c->one_order) {
+    auto fn = mode == 2 ? k_group_t_chain<2> : k_group_t_chain<0>;
+    fn<<<g, 256, 0, c->stream>>>(c->ldN, c->J, c->n_grp, c->gcells_d, c->gstart_d, c->Wg, c->Omega,
+                                 mode == 2 ? c->scratch : c->zt_u_src ? c->zt_u_src : c->Nu, c->gT);
+    GPL_LAUNCHED(c, "k_group_t_chain");
+    return GPL_OK;
+  }
   if (mode != 2) {
     const int rc = recip_omega_grouped(c);
     if (rc) return rc;

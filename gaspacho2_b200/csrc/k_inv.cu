@@ -35,10 +35,9 @@ constexpr int IB = 32;  // block size
 constexpr int IS = 36;  // shared row stride (doubles): conflict-free fragment loads
 constexpr int NB = 3;   // buffers of the inverse's block stream
 constexpr int CW = 8;   // finished columns per chunk of the Cholesky's panel update
-// Largest P each kernel is launched for. k_potrf_panel's update covers 256 rows of a panel
+// Largest P each kernel is launched for (kPotrfMaxP: gpl_internal.cuh). k_potrf_panel's update covers 256 rows of a panel
 // (8 warps x 2 row tiles of 16), so its panels below the first may hold at most 256 rows:
 // P <= 288. The inverse panels hold any P their shared memory admits (P <= 640 within 220 KiB).
-constexpr int kPotrfMaxP = 288;
 // With half the threads (128 rows below the first panel), up to four CTAs per SM hide more of a
 // panel's latency.
 constexpr int kPotrfHalfP = 160;

@@ -212,6 +212,27 @@ __global__ void __launch_bounds__(kSolveCells, 8)
   }
 }
 
+// The same in cholslg's order for any M, a row at a time, within an OrderScope (gpl_internal.cuh): 1.58 ms
+// at N = 100,000, M = 128.
+__global__ void k_kmm_solve_rows(int N, int ldN, int M, const double* __restrict__ L, const double* __restrict__ Knm,
+                                 double* __restrict__ Y, double* __restrict__ titsias) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  for (int r = 0; r < M; r++) {
+    double sum = Knm[i + (size_t)r * ldN];
+    for (int k = r - 1; k >= 0; k--) sum = __dsub_rn(sum, __dmul_rn(L[r + k * M], Y[i + (size_t)k * ldN]));
+    Y[i + (size_t)r * ldN] = __ddiv_rn(sum, L[r + r * M]);
+  }
+  for (int r = M - 1; r >= 0; r--) {
+    double sum = Y[i + (size_t)r * ldN];
+    for (int k = r + 1; k < M; k++) sum = __dsub_rn(sum, __dmul_rn(L[k + r * M], Y[i + (size_t)k * ldN]));
+    Y[i + (size_t)r * ldN] = __ddiv_rn(sum, L[r + r * M]);
+  }
+  double d = 0.0;
+  for (int k = 0; k < M; k++) d = __dadd_rn(d, __dmul_rn(Knm[i + (size_t)k * ldN], Y[i + (size_t)k * ldN]));
+  titsias[i] = (1.0 - d) / 2.0;
+}
+
 int launch_cholinv(Ctx* c, const double* L, int n, double* out) {
   auto fn = n <= 32 ? k_kmm_solve<true, true> : k_kmm_solve<true, false>;
   fn<<<div_up(n, kSolveCells), kSolveCells, 0, c->stream>>>(n, n, n, L, nullptr, out, nullptr);
@@ -264,6 +285,12 @@ int launch_kernel_cells(Ctx* c) {
     GPL_LAUNCHED(c, "k_knm");
   }
   ProfScope ps(c, "kinvkmn");
+  if (c->one_order && c->M > 32) {
+    k_kmm_solve_rows<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
+                                                               c->titsias);
+    GPL_LAUNCHED(c, "k_kmm_solve_rows");
+    return GPL_OK;
+  }
   auto fn = c->M <= 32 ? k_kmm_solve<false, true> : k_kmm_solve<false, false>;
   fn<<<div_up(c->N, kSolveCells), kSolveCells, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
                                                                c->titsias);
