@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(256) k_crt_conv_rows(const double* __restrict_
                                                        int64_t ldk, size_t plane, const double* __restrict__ sc,
                                                        int8_t* __restrict__ out, const int* __restrict__ flag) {
   if (*flag) return;
-  const int j = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 8;
+  const int j = blockIdx.x, i = (blockIdx.y * 256 + threadIdx.x) * 8;  // genes along x: more than 65,535
   if (i >= kpad) return;
   const double* r = src + (size_t)j * ld + i;
   double v[8];
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
                                                  double* __restrict__ acc, int64_t lda, int first, int last,
                                                  double* __restrict__ Psi, const int* __restrict__ flag) {
   if (*flag) return;
-  const int j = blockIdx.y, p0 = (blockIdx.x * 256 + threadIdx.x) * 4;
+  const int j = blockIdx.x, p0 = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (p0 >= n_pairs) return;
   double v[4];
   crt_values(in + (size_t)j * ldo + p0, plane, v);
@@ -831,7 +831,7 @@ int launch_crt_gram(Ctx* c) {
     GPL_LAUNCHED(c, "k_crt_norm_pairs");
     k_crt_scales<<<div_up(s.n_pairs, 256), 256, 0, c->stream>>>(s.n_pairs, ny, part, R, sc_p, inv_p, t.flag);
     GPL_LAUNCHED(c, "k_crt_scales");
-    k_crt_conv_rows<<<dim3(div_up(kpad, 2048), c->J), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad, t.gram_cells,
+    k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad, t.gram_cells,
                                                                           plane_a, sc_j, t.g_a, t.flag);
     GPL_LAUNCHED(c, "k_crt_conv_rows");
     k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(s.n_pairs, kConvPairs)), 256, 0, c->stream>>>(
@@ -839,7 +839,7 @@ int launch_crt_gram(Ctx* c) {
     GPL_LAUNCHED(c, "k_crt_conv_pairs");
     const int rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, s.n_pairs, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp);
     if (rc) return rc;
-    k_crt_psi<<<dim3(div_up(s.n_pairs, 1024), c->J), 256, 0, c->stream>>>(
+    k_crt_psi<<<dim3(c->J, div_up(s.n_pairs, 1024)), 256, 0, c->stream>>>(
         c->P, s.n_pairs, t.Pp, plane_o, t.g_out, inv_j, inv_p, s.pairs, c->dcol_d, c->DeltaInv, t.g_acc, t.Pp,
         c0 == 0, c0 + len >= c->N, c->Psi, t.flag);
     GPL_LAUNCHED(c, "k_crt_psi");
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(256) k_crt_t(int J, int P, int n_d, int rows, 
                                                const double* __restrict__ inv_p, const int* __restrict__ dcol,
                                                int first, double* __restrict__ T, const int* __restrict__ flag) {
   if (*flag) return;
-  const int j = blockIdx.y, r0 = (blockIdx.x * 256 + threadIdx.x) * 4;
+  const int j = blockIdx.x, r0 = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (r0 >= rows) return;
   double v[4];
   crt_values(in + (size_t)j * ldo + r0, plane, v);
@@ -967,14 +967,14 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
       GPL_LAUNCHED(c, "k_crt_norm_pairs");
       k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.flag);
       GPL_LAUNCHED(c, "k_crt_scales");
-      k_crt_conv_rows<<<dim3(div_up(kpad, 2048), c->J), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad,
+      k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad,
                                                                             t.gram_cells, plane_a, sc_j, t.g_a, t.flag);
       GPL_LAUNCHED(c, "k_crt_conv_rows");
       k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(rows, kConvPairs)), 256, 0, c->stream>>>(
           c->ldN, c0, len, kpad, t.gram_cells, plane_b, rows, pairs, D, rOm, sc_p, t.g_b, t.flag);
       GPL_LAUNCHED(c, "k_crt_conv_pairs");
       if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp))) return rc;
-      k_crt_t<<<dim3(div_up(rows, 1024), c->J), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
+      k_crt_t<<<dim3(c->J, div_up(rows, 1024)), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
                                                                     inv_j, inv_p, c->dcol_d, c0 == 0,
                                                                     T + (size_t)l0 * c->J * c->P, t.flag);
       GPL_LAUNCHED(c, "k_crt_t");
