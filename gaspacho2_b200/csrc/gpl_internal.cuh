@@ -60,8 +60,9 @@ struct CrtState {
   int Jp = 0, Pp = 0, Jk = 0;     // genes and pairs padded to tiles, genes padded to K chunks
   int gram_cells = 0, grad_cells = 0;  // 0: that product stays with the DMMA form
   size_t bytes = 0;
-  double* scales = nullptr;
+  double *scales = nullptr, *balance = nullptr, *lim = nullptr;
   int *flag = nullptr, *err = nullptr;  // operands out of range (the DMMA form runs); a wait gave up
+  int* cells = nullptr;  // the gradient's: [0] all cells, [1 + k] the k-th 128 cells go to the DMMA form
   int8_t *g_a = nullptr, *g_b = nullptr, *v_a = nullptr, *v_b = nullptr;
   uint8_t *g_out = nullptr, *v_out = nullptr;
   double* g_acc = nullptr;
@@ -389,7 +390,7 @@ int launch_quad(Ctx* c, int J, int V, const double* Psi, const double* T, size_t
 int dgen_unwhiten(Ctx* c, const double* Gt, double* Tt, const double* Lw);  // Psi_DD = L G L^T + DeltaInv
 int dgen_whiten_inverse(Ctx* c, const double* Lw, double* Tt, double* St);  // S~ = L^T S_DD L per gene
 int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D);  // U from the V rows of cells [c0, c1)
-int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* gate);  // given V, gated
+int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* cells);  // given V; cells: CrtState
 // k_crt.cu (the pair products on the INT8 tensor cores)
 void crt_plan(Ctx* c, size_t cap);
 int crt_prepare(Ctx* c);

@@ -110,7 +110,8 @@ static double crt_norm_limit() {
 }
 
 // The scale of a row from its squared norm: 2^s with norm 2^s <= R, and 2^-s. Rows below 1e-145 are
-// taken as zeros; a norm that is not finite or beyond 1e100 raises the flag.
+// taken as zeros; a norm that is not finite or beyond 1e100 raises the flag (the row's residues are then
+// those of no number in particular, and so is its product).
 __device__ __forceinline__ void crt_scale(double n2, double R, double* sc, double* inv, int* flag) {
   if (!(n2 < 1e200)) {
     atomicExch(flag, 1);
@@ -151,9 +152,10 @@ __global__ void __launch_bounds__(256) k_crt_norm_rows(const double* __restrict_
   if (threadIdx.x == 0) crt_scale(n2, R, sc + blockIdx.x, inv + blockIdx.x, flag);
 }
 
-// rows with K strided: src[k * ld + m], row m over k; partial sums over K ranges, then the scales
+// rows with K strided: src[k * ld + m] bal[k], row m over k; partial sums over K ranges, then the scales
 __global__ void __launch_bounds__(256) k_crt_norm_cols(const double* __restrict__ src, int64_t ld, int M, int K,
-                                                       int kper, double* __restrict__ part) {
+                                                       int kper, const double* __restrict__ bal,
+                                                       double* __restrict__ part) {
   const int m = blockIdx.x * 256 + threadIdx.x;
   if (m >= M) return;
   const int k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
@@ -162,11 +164,11 @@ __global__ void __launch_bounds__(256) k_crt_norm_cols(const double* __restrict_
   for (; k + 4 <= k1; k += 4)
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-      const double v = src[(size_t)(k + u) * ld + m];
+      const double v = src[(size_t)(k + u) * ld + m] * bal[k + u];
       s[u] = fma(v, v, s[u]);
     }
   for (; k < k1; k++) {
-    const double v = src[(size_t)k * ld + m];
+    const double v = src[(size_t)k * ld + m] * bal[k];
     s[0] = fma(v, v, s[0]);
   }
   part[(size_t)blockIdx.y * M + m] = (s[0] + s[1]) + (s[2] + s[3]);
@@ -214,13 +216,58 @@ __global__ void __launch_bounds__(256) k_crt_norm_pairs(int ldN, int n_d, int c0
   }
 }
 
+// flag[m >> shift] is raised for row m (shift 31: one flag for all rows)
 __global__ void k_crt_scales(int M, int n_part, const double* __restrict__ part, double R, double* __restrict__ sc,
-                             double* __restrict__ inv, int* __restrict__ flag) {
+                             double* __restrict__ inv, int* __restrict__ flag, int shift) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   double s = 0.0;
   for (int k = 0; k < n_part; k++) s += part[(size_t)k * M + m];
-  crt_scale(s, R, sc + m, inv + m, flag);
+  crt_scale(s, R, sc + m, inv + m, flag + (m >> shift));
+}
+
+// The gradient's contraction runs over the genes, and its operands run against each other there: a gene's
+// Psi_j^-1 falls as its weights grow. So each gene's row of W is multiplied by a power of two and its
+// pairs by the inverse, which changes no product and brings both to a like size: half the difference of
+// their mean exponents (over up to 1,024 cells, and over the diagonal of the dense block). Without it the
+// product of the norms, which sets the rounding, stood up to 300 u above the sum of the products at gene
+// means of log sd 1.2; with it at 0.4 to 3 u (u = 2^-53).
+constexpr int kBalanceCells = 1024;
+__global__ void __launch_bounds__(256) k_crt_balance(int N, int64_t ldN, int n_d, int64_t ldp,
+                                                     const double* __restrict__ W, const double* __restrict__ Sp,
+                                                     double* __restrict__ bal_w, double* __restrict__ bal_s) {
+  __shared__ double sh[32];
+  const int j = blockIdx.x;
+  const double *w = W + (size_t)j * ldN, *s = Sp + (size_t)j * ldp;
+  double sum[2] = {0.0, 0.0}, num[2] = {0.0, 0.0};
+  auto add = [&](int which, double v) {
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    if (e == 0 || e == 0x7ff) return;
+    sum[which] += e - 1023;
+    num[which] += 1.0;
+  };
+  const int n = min(N, kBalanceCells);
+  for (int k = threadIdx.x; k < n; k += 256) add(0, w[(int)((int64_t)k * N / n)]);
+  for (int a = threadIdx.x; a < n_d; a += 256) add(1, s[(int64_t)a * n_d - (int64_t)a * (a - 1) / 2]);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    sum[q] = block_sum(sum[q], sh);
+    num[q] = block_sum(num[q], sh);
+  }
+  if (threadIdx.x == 0) {
+    const double d = num[0] > 0.0 && num[1] > 0.0 ? (sum[1] / num[1] - sum[0] / num[0]) / 2.0 : 0.0;
+    const int e = (int)rint(fmin(fmax(d, -300.0), 300.0));
+    bal_w[j] = ldexp(1.0, e);
+    bal_s[j] = ldexp(1.0, -e);
+  }
+}
+
+// What a sum of two rows' products is off by, for rows at their scales: both operands' entries are off by
+// 0.29 of a unit (rms), so the sum by 0.41 R units at most, R bounding both norms. lim[a] is the least
+// value, before the row's own scale, of the diagonal pair (a, a) at which that is no more than `share`.
+__global__ void k_crt_limits(int n_d, double least, const double* __restrict__ inv_p, double* __restrict__ lim) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a < n_d) lim[a] = least * inv_p[(int64_t)a * n_d - (int64_t)a * (a - 1) / 2];
 }
 
 // ---- residues ------------------------------------------------------------------------------------
@@ -324,13 +371,14 @@ __global__ void __launch_bounds__(256) k_crt_conv_pairs(int ldN, int c0, int len
   }
 }
 
-// rows with K strided, src[k * ld + m]: planes [m][ldk], zeros in [K, kpad). Tiles of 32 rows x 128
+// rows with K strided, src[k * ld + m] bal[k]: planes [m][ldk], zeros in [K, kpad). Tiles of 32 rows x 128
 // K entries: lanes read along the rows, the packed residues turn through shared memory.
 constexpr int kTurnWords = 33;  // 32 words of 4 residues per row, padded
 template <bool kA>
 __global__ void __launch_bounds__(256) k_crt_conv_cols(const double* __restrict__ src, int64_t ld, int M, int K,
-                                                       int64_t ldk, size_t plane, const double* __restrict__ sc,
-                                                       int8_t* __restrict__ out, const int* __restrict__ flag) {
+                                                       int64_t ldk, size_t plane, const double* __restrict__ bal,
+                                                       const double* __restrict__ sc, int8_t* __restrict__ out,
+                                                       const int* __restrict__ flag) {
   extern __shared__ uint32_t turn[];  // [kMod][32][kTurnWords]
   if (*flag) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -343,7 +391,7 @@ __global__ void __launch_bounds__(256) k_crt_conv_cols(const double* __restrict_
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int k = k0 + kw * 4 + e;
-      crt_limbs(m < M && k < K ? src[(size_t)k * ld + m] : 0.0, s, l[e]);
+      crt_limbs(m < M && k < K ? src[(size_t)k * ld + m] * bal[k] : 0.0, s, l[e]);
     }
 #pragma unroll
     for (int q = 0; q < kMod; q++)
@@ -637,7 +685,10 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
 }
 
 // U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], W warps per cell: the
-// cell's row of V from its residues into shared memory (pair_rows.cuh).
+// cell's row of V from its residues into shared memory (pair_rows.cuh). A cell with a diagonal V[i, (a, a)]
+// below lim (k_crt_limits) sends its 128 cells to the DMMA form. The diagonal is enough: W_ij and the
+// S_j[a, a] are positive, |S_j[a, b]| <= sqrt(S_j[a, a] S_j[b, b]), and so by Cauchy-Schwarz the rounding of
+// V[i, (a, b)] stays within the same share of sqrt(V[i, (a, a)] V[i, (b, b)]).
 // Bound by the entries' arithmetic (crt_values) while 24 to 32 warps share an SM; without the limit on
 // registers the compiler keeps several entries' loads and all the digits in flight at half the warps
 // (50,000 cells x 132 columns x 1,000 genes: 6.0 against 2.9 ms).
@@ -645,24 +696,30 @@ template <int S, int W>
 __global__ void __launch_bounds__(256, S > 9 ? 2 : S > 5 ? 4 : 3) k_crt_u(int ldN, int n_d, int len, int c0, int64_t ldo, size_t plane,
                                                const uint8_t* __restrict__ in, const double* __restrict__ inv_i,
                                                const double* __restrict__ inv_p, const double* __restrict__ rOm,
-                                               const double* __restrict__ D, double* __restrict__ U,
-                                               const int* __restrict__ flag) {
+                                               const double* __restrict__ D, const double* __restrict__ lim,
+                                               double* __restrict__ U, int* __restrict__ cells) {
   extern __shared__ __align__(16) double vs[];
-  if (*flag) return;
+  if (cells[0]) return;
   const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g, i = c0 + r;
   if (r >= len) return;  // W = 1: a whole warp, no barrier of the block follows
   double* vc = vs + g * u_space<W>(n_d);
   const double s = inv_i[r] * rOm[i] * kUnit;
   const uint8_t* row_in = in + (size_t)r * ldo;
-  pair_rows_to_u<S, W>(i, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
-    for (int p = from + 4 * tid; p < p1; p += 4 * nt) {
-      double v[4];
-      crt_values(row_in + p, plane, v);
-      const double2 x = *reinterpret_cast<const double2*>(inv_p + p), y = *reinterpret_cast<const double2*>(inv_p + p + 2);
-      *reinterpret_cast<double2*>(vc + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
-      *reinterpret_cast<double2*>(vc + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
-    }
-  });
+  bool out = false;
+  pair_rows_to_u<S, W>(
+      i, ldN, n_d, vc, D, U,
+      [&](int from, int p1, int tid, int nt) {
+        for (int p = from + 4 * tid; p < p1; p += 4 * nt) {
+          double v[4];
+          crt_values(row_in + p, plane, v);
+          const double2 x = *reinterpret_cast<const double2*>(inv_p + p),
+                        y = *reinterpret_cast<const double2*>(inv_p + p + 2);
+          *reinterpret_cast<double2*>(vc + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
+          *reinterpret_cast<double2*>(vc + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
+        }
+      },
+      [&](int a, double v) { out |= !(v >= lim[a] * s); });
+  if (out && (threadIdx.x & 31) == 0) cells[1 + (i >> 7)] = 1;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -734,15 +791,18 @@ int crt_prepare(Ctx* c) {
   PairState& s = c->pr;
   CrtState& t = s.crt;
   if (!t.on) return GPL_OK;
-  const size_t rows = (size_t)2 * (t.Jp + t.Pp + t.grad_cells);
-  if (cudaMalloc((void**)&t.scales, sizeof(double) * rows) != cudaSuccess ||
-      cudaMalloc((void**)&t.flag, 2 * sizeof(int)) != cudaSuccess) {
+  const size_t rows = (size_t)2 * (t.Jp + t.Pp + t.grad_cells), tiles = div_up(c->N, 128);
+  if (cudaMalloc((void**)&t.scales, sizeof(double) * (rows + 2 * t.Jp + c->n_d)) != cudaSuccess ||
+      cudaMalloc((void**)&t.flag, (3 + tiles) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     c->err = "device allocation failed: scales of the integer pair products";
     return GPL_ERR_ALLOC;
   }
+  t.balance = t.scales + rows;  // of W, then of the pairs
+  t.lim = t.balance + 2 * t.Jp;
   t.err = t.flag + 1;
-  GPL_TRY(c, cudaMemset(t.flag, 0, 2 * sizeof(int)));
+  t.cells = t.flag + 2;
+  GPL_TRY(c, cudaMemset(t.flag, 0, (3 + tiles) * sizeof(int)));
   int8_t* pool = reinterpret_cast<int8_t*>(s.V);
   // Gram: gene planes, pair planes, residues out, partial sums over the ranges
   t.g_a = pool;
@@ -775,7 +835,7 @@ void crt_release(Ctx* c) {
 }
 
 static int crt_gemm(Ctx* c, const CUtensorMap& ma, const CUtensorMap& mb, int rows, int cols, int a_rows, int b_rows,
-                    int k, uint8_t* out, size_t plane, int64_t ldo) {
+                    int k, uint8_t* out, size_t plane, int64_t ldo, const int* flag) {
   I8Args a{};
   a.tiles_m = div_up(rows, kTile);
   a.tiles_n = div_up(cols, kTile);
@@ -786,7 +846,7 @@ static int crt_gemm(Ctx* c, const CUtensorMap& ma, const CUtensorMap& mb, int ro
   a.plane = plane;
   a.ldo = ldo;
   a.out = out;
-  a.flag = c->pr.crt.flag;
+  a.flag = flag;
   a.err = c->pr.crt.err;
   const int tiles = kMod * a.tiles_m * a.tiles_n;
   const int grid = 2 * std::min(tiles, c->sm_count / 2);
@@ -795,14 +855,22 @@ static int crt_gemm(Ctx* c, const CUtensorMap& ma, const CUtensorMap& mb, int ro
   return GPL_OK;
 }
 
-// scales of rows with K strided (src[k * ld + m]); `part` holds at least 16 sums per row
-static int crt_col_scales(Ctx* c, const double* src, int64_t ld, int M, int K, double* part, double* sc, double* inv) {
+// What the rounding of an integer product may be of the diagonal it is measured by (k_crt_limits), over K
+// terms: what a chain of K FP64 multiply-adds is off by, 0.15 sqrt(K) u (rms; 12 u measured at K = 6,001, 19 u
+// at 19,997), less a third, and 4 u at least.
+static double crt_share(double K) {
+  return 0x1p-53 * std::max(4.0, 0.1 * std::sqrt(K));
+}
+
+// scales of rows with K strided (src[k * ld + m] bal[k]); `part` holds at least 16 sums per row
+static int crt_col_scales(Ctx* c, const double* src, int64_t ld, int M, int K, const double* bal, double* part,
+                          double* sc, double* inv, int* flag, int shift) {
   const int nb = div_up(M, 256);
   const int ks = std::max(1, std::min({16, 1184 / std::max(1, nb), div_up(K, 64)}));
   const int kper = div_up(K, ks);
-  k_crt_norm_cols<<<dim3(nb, ks), 256, 0, c->stream>>>(src, ld, M, K, kper, part);
+  k_crt_norm_cols<<<dim3(nb, ks), 256, 0, c->stream>>>(src, ld, M, K, kper, bal, part);
   GPL_LAUNCHED(c, "k_crt_norm_cols");
-  k_crt_scales<<<nb, 256, 0, c->stream>>>(M, ks, part, crt_norm_limit(), sc, inv, c->pr.crt.flag);
+  k_crt_scales<<<nb, 256, 0, c->stream>>>(M, ks, part, crt_norm_limit(), sc, inv, flag, shift);
   GPL_LAUNCHED(c, "k_crt_scales");
   return GPL_OK;
 }
@@ -829,7 +897,7 @@ int launch_crt_gram(Ctx* c) {
     k_crt_norm_pairs<<<dim3(gx, ny), 256, sizeof(double) * 32 * (c->n_d + 1), c->stream>>>(
         c->ldN, c->n_d, c0, c0 + len, cper, s.n_pairs, s.pairs, c->Dm, s.rOm, part);
     GPL_LAUNCHED(c, "k_crt_norm_pairs");
-    k_crt_scales<<<div_up(s.n_pairs, 256), 256, 0, c->stream>>>(s.n_pairs, ny, part, R, sc_p, inv_p, t.flag);
+    k_crt_scales<<<div_up(s.n_pairs, 256), 256, 0, c->stream>>>(s.n_pairs, ny, part, R, sc_p, inv_p, t.flag, 31);
     GPL_LAUNCHED(c, "k_crt_scales");
     k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad, t.gram_cells,
                                                                           plane_a, sc_j, t.g_a, t.flag);
@@ -837,7 +905,7 @@ int launch_crt_gram(Ctx* c) {
     k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(s.n_pairs, kConvPairs)), 256, 0, c->stream>>>(
         c->ldN, c0, len, kpad, t.gram_cells, plane_b, s.n_pairs, s.pairs, c->Dm, s.rOm, sc_p, t.g_b, t.flag);
     GPL_LAUNCHED(c, "k_crt_conv_pairs");
-    const int rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, s.n_pairs, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp);
+    const int rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, s.n_pairs, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.flag);
     if (rc) return rc;
     k_crt_psi<<<dim3(c->J, div_up(s.n_pairs, 1024)), 256, 0, c->stream>>>(
         c->P, s.n_pairs, t.Pp, plane_o, t.g_out, inv_j, inv_p, s.pairs, c->dcol_d, c->DeltaInv, t.g_acc, t.Pp,
@@ -855,21 +923,31 @@ int launch_crt_uq(Ctx* c) {
   double* part = reinterpret_cast<double*>(t.v_out);
   const size_t plane_b = (size_t)t.Pp * t.Jk, plane_a = (size_t)t.grad_cells * t.Jk;
   const size_t plane_o = (size_t)t.grad_cells * t.Pp;
-  GPL_TRY(c, cudaMemsetAsync(t.flag, 0, sizeof(int), c->stream));
+  const double *bal_w = t.balance, *bal_s = bal_w + t.Jp;
+  GPL_TRY(c, cudaMemsetAsync(t.cells, 0, (1 + div_up(c->N, 128)) * sizeof(int), c->stream));
+  k_crt_balance<<<c->J, 256, 0, c->stream>>>(c->N, c->ldN, c->n_d, s.pairs_pad, c->W, s.Sp, t.balance,
+                                             t.balance + t.Jp);
+  GPL_LAUNCHED(c, "k_crt_balance");
   int rc;
-  if ((rc = crt_col_scales(c, s.Sp, s.pairs_pad, s.n_pairs, c->J, part, sc_p, inv_p))) return rc;
+  if ((rc = crt_col_scales(c, s.Sp, s.pairs_pad, s.n_pairs, c->J, bal_s, part, sc_p, inv_p, t.cells, 31))) return rc;
+  k_crt_limits<<<div_up(c->n_d, 128), 128, 0, c->stream>>>(
+      c->n_d, 0.41 * crt_norm_limit() / kUnit / crt_share(c->J), inv_p, t.lim);
+  GPL_LAUNCHED(c, "k_crt_limits");
   k_crt_conv_cols<false><<<dim3(div_up(s.n_pairs, 32), t.Jk / 128), 256, kSmemTurn, c->stream>>>(
-      s.Sp, s.pairs_pad, s.n_pairs, c->J, t.Jk, plane_b, sc_p, t.v_b, t.flag);
+      s.Sp, s.pairs_pad, s.n_pairs, c->J, t.Jk, plane_b, bal_s, sc_p, t.v_b, t.cells);
   GPL_LAUNCHED(c, "k_crt_conv_cols");
   for (int c0 = 0; c0 < c->N; c0 += t.grad_cells) {
     const int len = std::min(t.grad_cells, c->N - c0);
     {
       ProfScope ps(c, "uq");
-      if ((rc = crt_col_scales(c, c->W + c0, c->ldN, len, c->J, part, sc_i, inv_i))) return rc;
+      // c0 is a multiple of 256: the cells' own flags, of 128 each
+      if ((rc = crt_col_scales(c, c->W + c0, c->ldN, len, c->J, bal_w, part, sc_i, inv_i, t.cells + 1 + c0 / 128, 7)))
+        return rc;
       k_crt_conv_cols<true><<<dim3(div_up(len, 32), t.Jk / 128), 256, kSmemTurn, c->stream>>>(
-          c->W + c0, c->ldN, len, c->J, t.Jk, plane_a, sc_i, t.v_a, t.flag);
+          c->W + c0, c->ldN, len, c->J, t.Jk, plane_a, bal_w, sc_i, t.v_a, t.cells);
       GPL_LAUNCHED(c, "k_crt_conv_cols");
-      if ((rc = crt_gemm(c, t.map_va, t.map_vb, len, s.n_pairs, t.grad_cells, t.Pp, t.Jk, t.v_out, plane_o, t.Pp)))
+      if ((rc = crt_gemm(c, t.map_va, t.map_vb, len, s.n_pairs, t.grad_cells, t.Pp, t.Jk, t.v_out, plane_o, t.Pp,
+                         t.cells)))
         return rc;
     }
     ProfScope ps(c, "v_to_u");
@@ -877,7 +955,7 @@ int launch_crt_uq(Ctx* c) {
       constexpr int per = 8 / W;
       const int smem = (int)sizeof(double) * u_space<W>(c->n_d) * per;
       k_crt_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, len, c0, t.Pp, plane_o, t.v_out, inv_i,
-                                                               inv_p, s.rOm, c->Dm, c->U, t.flag);
+                                                               inv_p, s.rOm, c->Dm, t.lim, c->U, t.cells);
     });
     GPL_LAUNCHED(c, "k_crt_u");
   }
@@ -965,7 +1043,7 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
       k_crt_norm_pairs<<<dim3(gx, ny), 256, smem_n, c->stream>>>(c->ldN, cols, c0, c0 + len, cper, rows, pairs, D, rOm,
                                                                 part);
       GPL_LAUNCHED(c, "k_crt_norm_pairs");
-      k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.flag);
+      k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.flag, 31);
       GPL_LAUNCHED(c, "k_crt_scales");
       k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad,
                                                                             t.gram_cells, plane_a, sc_j, t.g_a, t.flag);
@@ -973,7 +1051,7 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
       k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(rows, kConvPairs)), 256, 0, c->stream>>>(
           c->ldN, c0, len, kpad, t.gram_cells, plane_b, rows, pairs, D, rOm, sc_p, t.g_b, t.flag);
       GPL_LAUNCHED(c, "k_crt_conv_pairs");
-      if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp))) return rc;
+      if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.flag))) return rc;
       k_crt_t<<<dim3(c->J, div_up(rows, 1024)), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
                                                                     inv_j, inv_p, c->dcol_d, c0 == 0,
                                                                     T + (size_t)l0 * c->J * c->P, t.flag);

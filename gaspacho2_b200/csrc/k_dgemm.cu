@@ -293,15 +293,15 @@ __global__ void k_gather_spair(int J, int P, int n_pairs, int pairs_pad, const i
 __global__ void __launch_bounds__(kThreads, 1)
     k_pair_v(int N, int ldN, int J, int c0, int c1, int pairs_pad, const double* __restrict__ W,
              const double* __restrict__ Sp, const double* __restrict__ rOm, double* __restrict__ V, int group_m,
-             const int* __restrict__ gate) {
+             const int* __restrict__ cells) {
   extern __shared__ __align__(16) double smem_d[];
-  if (gate && *gate == 0) return;
   double* As = smem_d;                // [3][BK][SA]  W rows (cells contiguous)
   double* Bs = smem_d + 3 * BK * SA;  // [3][BK][SBN] S pairs (pairs contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3, wm = warp >> 2, wn = warp & 3;
   const int2 tile = grouped_tile(blockIdx.x, (c1 - c0 + BM - 1) / BM, pairs_pad / BN, group_m);
   const int i0 = c0 + tile.x * BM, n0 = tile.y * BN;
+  if (cells && !cells[0] && !cells[1 + i0 / BM]) return;  // c0 is a multiple of BM
   const int nsl = (J + BK - 1) / BK;
 
   auto load = [&](int s, int buf) {
@@ -370,27 +370,26 @@ __global__ void __launch_bounds__(kThreads, 1)
 template <int S, int W>
 __global__ void __launch_bounds__(256, S > 9 ? 2 : 4) k_v_to_u(int ldN, int n_d, int pairs_pad, int c0, int c1,
                                                    const double* __restrict__ D, const double* __restrict__ V,
-                                                   double* __restrict__ U, const int* __restrict__ gate) {
+                                                   double* __restrict__ U, const int* __restrict__ cells) {
   extern __shared__ __align__(16) double vs[];
-  if (gate && *gate == 0) return;
   const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g;
   if (c0 + r >= c1) return;  // W = 1: a whole warp, no barrier of the block follows
+  if (cells && !cells[0] && !cells[1 + (c0 + r) / BM]) return;
   double* vc = vs + g * u_space<W>(n_d);
   const double* vr = V + (size_t)r * pairs_pad;
   pair_rows_to_u<S, W>(c0 + r, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
     for (int p = from + 2 * tid; p < p1; p += 2 * nt) cp_async16(vc + p - from, vr + p, 16);
     cp_async_commit();
     cp_async_wait<0>();
-  });
+  }, [](int, double) {});
 }
 
 // The same for more dense columns than that takes (512): the row is read from global memory (L1 / L2)
 // instead of staged, the dense row of the cell is staged.
 __global__ void __launch_bounds__(256) k_v_to_u_wide(int N, int ldN, int n_d, int pairs_pad, int c0, int c1,
                                                      const double* __restrict__ D, const double* __restrict__ V,
-                                                     double* __restrict__ U, const int* __restrict__ gate) {
+                                                     double* __restrict__ U) {
   extern __shared__ __align__(16) double ds[];  // D row of the cell
-  if (gate && *gate == 0) return;
   for (int i = c0 + blockIdx.x; i < c1 && i < N; i += gridDim.x) {
     const double* vr = V + (size_t)(i - c0) * pairs_pad;
     for (int e = threadIdx.x; e < n_d; e += blockDim.x) ds[e] = D[(size_t)e * ldN + i];
@@ -552,21 +551,22 @@ int launch_pair_uq(Ctx* c) {
                                              s.Sp);
     GPL_LAUNCHED(c, "k_gather_spair");
   }
-  const int* gate = s.crt.grad_cells ? s.crt.flag : nullptr;  // as in launch_pair_gram
-  if (gate && (rc = launch_crt_uq(c))) return rc;
+  // the integer form, where it is planned; the kernels below then run for the tiles of cells that it sent here
+  const int* cells = s.crt.grad_cells ? s.crt.cells : nullptr;
+  if (cells && (rc = launch_crt_uq(c))) return rc;
   for (int c0 = 0; c0 < c->N; c0 += s.v_cells) {
     const int c1 = std::min(c->N, c0 + s.v_cells);
     {
       ProfScope ps(c, "uq");
       const int g = div_up(c1 - c0, BM) * (s.pairs_pad / BN);
       Tunable* tu = nullptr;
-      const int gm = gate ? kGroupM : tune_pick(c, "pair_v", {8, 12, 16}, kGroupM, &tu);
+      const int gm = cells ? kGroupM : tune_pick(c, "pair_v", {8, 12, 16}, kGroupM, &tu);
       TuneScope ts(c, c1 - c0 == c->N ? tu : nullptr);
       k_pair_v<<<g, kThreads, s.smem_v, c->stream>>>(c->N, c->ldN, c->J, c0, c1, s.pairs_pad, c->W, s.Sp, s.rOm,
-                                                     s.V, gm, gate);
+                                                     s.V, gm, cells);
       GPL_LAUNCHED(c, "k_pair_v");
     }
-    if ((rc = launch_v_to_u_rows(c, c0, c1, c->Dm, s.V, gate))) return rc;
+    if ((rc = launch_v_to_u_rows(c, c0, c1, c->Dm, s.V, cells))) return rc;
   }
   return GPL_OK;
 }
@@ -575,13 +575,13 @@ int launch_v_to_u_cells(Ctx* c, int c0, int c1, const double* D) {
   return launch_v_to_u_rows(c, c0, c1, D, c->pr.V, nullptr);
 }
 
-int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* gate) {
+int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V, const int* cells) {
   PairState& s = c->pr;
   ProfScope ps(c, "v_to_u");
   if (c->n_d > kUMaxDense) {
     const int grid = std::min(c1 - c0, 148 * 8);
     k_v_to_u_wide<<<grid, 256, sizeof(double) * c->n_d, c->stream>>>(c->N, c->ldN, c->n_d, s.pairs_pad, c0, c1, D,
-                                                                    V, c->U, gate);
+                                                                    V, c->U);  // never gated: crt_plan
     GPL_LAUNCHED(c, "k_v_to_u_wide");
     return GPL_OK;
   }
@@ -592,7 +592,7 @@ int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V,
     if (smem > 48 * 1024)  // 97 or more columns, a warp per cell
       cudaFuncSetAttribute(k_v_to_u<S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k_v_to_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, s.pairs_pad, c0, c0 + len, D, V, c->U,
-                                                              gate);
+                                                              cells);
   });
   GPL_LAUNCHED(c, "k_v_to_u");
   return GPL_OK;

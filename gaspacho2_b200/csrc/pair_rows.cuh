@@ -46,10 +46,11 @@ void pair_rows_form(int n_d, int cells, int warp_dense, F f) {
 }
 
 // S: 32-column slots, n_d <= 32 S. vs: the cell's u_space doubles. fill(from, p1, t, n): the threads t of n
-// write V[from ..] to vs[0 ..], up to p1 (from: a multiple of four).
-template <int S, int W, class Fill>
+// write V[from ..] to vs[0 ..], up to p1 (from: a multiple of four). diag(a, v): called by lane 0 of a warp with
+// each diagonal V[pair(a, a)].
+template <int S, int W, class Fill, class Diag>
 __device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* vs, const double* __restrict__ D,
-                                               double* __restrict__ U, Fill fill) {
+                                               double* __restrict__ U, Fill fill, Diag diag) {
   constexpr int kThr = 32 * W, kOwn = (32 * S + kThr - 1) / kThr;
   double *ds = vs + u_entries<W>() + 4, *rs = ds + ((n_d + 1) & ~1);
   const int lane = threadIdx.x & 31, warp = W == 8 ? threadIdx.x >> 5 : 0, tid = W == 8 ? threadIdx.x : lane;
@@ -108,7 +109,11 @@ __device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* 
       sum2 = warp_sum(sum2);
       if (lane == 0) {
         rs[a] = sum;
-        if (two) rs[e] = sum2;
+        diag(a, row[a]);
+        if (two) {
+          rs[e] = sum2;
+          diag(e, row2[e]);
+        }
       }
     }
     a0 = a1;

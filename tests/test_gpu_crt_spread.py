@@ -1,0 +1,62 @@
+"""The integer pair products (k_crt.cu) where the operands' rows spread over many orders of magnitude: their
+rounding is relative to a row's norm, so they have to notice where that is more than the FP64 form's."""
+import numpy as np
+import pytest
+
+from gaspacho2_b200 import synth
+from gaspacho2_b200.model import GPLVM
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _share(K):
+    return U * max(4.0, 0.1 * np.sqrt(K))
+
+
+def _context(N, G, M, Q=5, config=0, seed=5):
+    ds = synth.make(config, seed, N=N, G=G, M=M, Q=Q, init=False)
+    ds.init.rho[:] = 3.0
+    ds.init.Omega[:] = np.exp(0.3 * np.random.default_rng(seed).standard_normal(N))
+    m = GPLVM.from_dataset(ds)
+    m.set_params(ds.init)
+    return ds, m
+
+
+# genes at one scale, and over seven orders of magnitude; one gene with a cell at e^30 of the others
+@pytest.mark.parametrize("lo,hi,outlier", [(0.0, 0.0, 0.0), (np.log(1e-4), np.log(1e3), 0.0),
+                                           (np.log(1e-4), np.log(1e3), 30.0)])
+def test_gradient_pairs_of_genes_far_apart(lo, hi, outlier):
+    N, G, M = 2500, 600, 64
+    ds, m = _context(N, G, M)
+    with m:
+        rng = np.random.default_rng(3)
+        beta = 0.2 * rng.standard_normal((m.P, G))
+        beta[0] = rng.uniform(lo, hi, G)
+        if outlier:
+            beta[-1, 7] = outlier  # the cells near one inducing point
+        m.set_beta(beta)
+        m.kernel_mats()
+        m.expand_delta()
+        m.irls_sweep(0, 0)
+        m.objective(0, 1)
+        got = []
+        for cells in (0, 128):  # 128 cells per range: the FP64 form, on the same factors
+            m.set_option("pair_range_cells", cells)
+            m.gradient()
+            assert m.get_option("pair_form") == (0 if cells else 3)
+            got.append(m.get("C1").reshape(M, N))
+        W = m.get("W").reshape(-1, N)[:G]
+        D = m.get("Dm").reshape(m.n_dense(), N)
+        P = m.P
+        cols = np.array([0] + list(range(P - D.shape[0] + 1, P)))
+        Sd = np.diagonal(m.get("PsiInv").reshape(G, P, P), axis1=1, axis2=2)[:, cols]
+    V = (W.T @ Sd) / ds.init.Omega[:, None]  # diagonal pairs, positive
+    # U_a = sum_b D_b V_ab, |V_ab| <= sqrt(V_aa V_bb): 8 times the rms rounding of either form (the integer
+    # form's share, the chain's 0.15 sqrt(G) u) and the sum over b of both; C1 = (terms common to both - U) D
+    size = np.sqrt(V) * (np.abs(D.T) * np.sqrt(V)).sum(1)[:, None]
+    tol = (8 * _share(G) + 1.2 * np.sqrt(G) * U + 2 * (D.shape[0] + 4) * U) * size
+    K = np.abs(D[-M:])
+    err = np.abs(got[0] - got[1])
+    assert np.all(err <= K * tol.T[-M:] + 4 * U * (np.abs(got[1]) + K * size.T[-M:])), \
+        float((err / (K * size.T[-M:])).max())
