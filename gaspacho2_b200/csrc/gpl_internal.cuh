@@ -60,9 +60,13 @@ struct CrtState {
   int Jp = 0, Pp = 0, Jk = 0;     // genes and pairs padded to tiles, genes padded to K chunks
   int gram_cells = 0, grad_cells = 0;  // 0: that product stays with the DMMA form
   size_t bytes = 0;
-  double *scales = nullptr, *balance = nullptr, *lim = nullptr;
+  double *scales = nullptr, *balance = nullptr;
   int *flag = nullptr, *err = nullptr;  // operands out of range (the DMMA form runs); a wait gave up
   int* cells = nullptr;  // the gradient's: [0] all cells, [1 + k] the k-th 128 cells go to the DMMA form
+  // the Gram's: [0] all genes, [1] how many, [2 + j] gene j go to the DMMA form, those genes, and over
+  // several ranges of cells the rounding of the diagonals so far (genes x dense columns)
+  int *genes = nullptr, *list = nullptr;
+  double* g_err = nullptr;
   int8_t *g_a = nullptr, *g_b = nullptr, *v_a = nullptr, *v_b = nullptr;
   uint8_t *g_out = nullptr, *v_out = nullptr;
   double* g_acc = nullptr;
@@ -371,6 +375,7 @@ int launch_kernel_mats_raw(cudaStream_t st, int N, int M, int Q, const double* X
 int launch_pair_gram(Ctx* c);             // dense block of every Psi_j, FP64 DMMA over column pairs
 int launch_pair_uq(Ctx* c);               // U = sum_j O_ij S_j[DD] d_i, FP64 DMMA over column pairs
 void pair_release(Ctx* c);
+double pair_gram_cost(const Ctx* c, int n_pairs);  // of the DMMA Gram, in clocks per 16 cells
 int pair_prepare(Ctx* c);                 // column-pair list, 1/Omega, gathered S pairs, V rows
 int recip_omega(Ctx* c, const double** rOm);  // 1/Omega (0 past N), refreshed on every call
 int dgen_zt_u(Ctx* c, int mode, const double* u, double* out);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);

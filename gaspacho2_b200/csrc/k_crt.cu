@@ -110,28 +110,38 @@ static double crt_norm_limit() {
 }
 
 // The scale of a row from its squared norm: 2^s with norm 2^s <= R, and 2^-s. Rows below 1e-145 are
-// taken as zeros; a norm that is not finite or beyond 1e100 raises the flag (the row's residues are then
+// taken as zeros; false for a norm that is not finite or beyond 1e100 (the row's residues are then
 // those of no number in particular, and so is its product).
-__device__ __forceinline__ void crt_scale(double n2, double R, double* sc, double* inv, int* flag) {
+__device__ __forceinline__ bool crt_scale(double n2, double R, double* sc, double* inv) {
   if (!(n2 < 1e200)) {
-    atomicExch(flag, 1);
     *sc = *inv = 0.0;
-    return;
+    return false;
   }
   if (n2 < 1e-290) {
     *sc = *inv = 0.0;
-    return;
+    return true;
   }
   const int s = ilogb(R / (sqrt(n2) * (1.0 + 1e-9)));
   *sc = ldexp(1.0, s);
   *inv = ldexp(1.0, -s);
+  return true;
 }
+
+// Where a gene goes that the integer form cannot take: onto the Gram's list (CrtState::genes), once, or
+// without a list into the flag for all.
+struct CrtGenes {
+  int *state, *list;
+  __device__ __forceinline__ void add(int j) const {
+    if (!list) atomicExch(state, 1);
+    else if (atomicExch(state + 2 + j, 1) == 0) list[atomicAdd(state + 1, 1)] = j;
+  }
+};
 
 // ---- norms -------------------------------------------------------------------------------------
 // rows with K contiguous: gene j over the cells [c0, c0 + len)
 __global__ void __launch_bounds__(256) k_crt_norm_rows(const double* __restrict__ src, int64_t ld, int len, double R,
                                                        double* __restrict__ sc, double* __restrict__ inv,
-                                                       int* __restrict__ flag) {
+                                                       CrtGenes genes) {
   __shared__ double sh[32];
   const double* r = src + (size_t)blockIdx.x * ld;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
@@ -149,7 +159,7 @@ __global__ void __launch_bounds__(256) k_crt_norm_rows(const double* __restrict_
     if (i + 1 < len) s1 = fma(r[i + 1], r[i + 1], s1);
   }
   const double n2 = block_sum((s0 + s1) + (s2 + s3), sh);
-  if (threadIdx.x == 0) crt_scale(n2, R, sc + blockIdx.x, inv + blockIdx.x, flag);
+  if (threadIdx.x == 0 && !crt_scale(n2, R, sc + blockIdx.x, inv + blockIdx.x)) genes.add(blockIdx.x);
 }
 
 // rows with K strided: src[k * ld + m] bal[k], row m over k; partial sums over K ranges, then the scales
@@ -161,12 +171,16 @@ __global__ void __launch_bounds__(256) k_crt_norm_cols(const double* __restrict_
   const int k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   int k = k0;
-  for (; k + 4 <= k1; k += 4)
+  for (; k + 8 <= k1; k += 8) {
+    double v[8];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const double v = src[(size_t)(k + u) * ld + m] * bal[k + u];
-      s[u] = fma(v, v, s[u]);
+    for (int u = 0; u < 8; u++) v[u] = src[(size_t)(k + u) * ld + m];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      v[u] *= bal[k + u];
+      s[u & 3] = fma(v[u], v[u], s[u & 3]);
     }
+  }
   for (; k < k1; k++) {
     const double v = src[(size_t)k * ld + m] * bal[k];
     s[0] = fma(v, v, s[0]);
@@ -223,16 +237,16 @@ __global__ void k_crt_scales(int M, int n_part, const double* __restrict__ part,
   if (m >= M) return;
   double s = 0.0;
   for (int k = 0; k < n_part; k++) s += part[(size_t)k * M + m];
-  crt_scale(s, R, sc + m, inv + m, flag + (m >> shift));
+  if (!crt_scale(s, R, sc + m, inv + m)) atomicExch(flag + (m >> shift), 1);
 }
 
 // The gradient's contraction runs over the genes, and its operands run against each other there: a gene's
 // Psi_j^-1 falls as its weights grow. So each gene's row of W is multiplied by a power of two and its
 // pairs by the inverse, which changes no product and brings both to a like size: half the difference of
-// their mean exponents (over up to 1,024 cells, and over the diagonal of the dense block). Without it the
+// their mean exponents (over up to 256 cells, and over the diagonal of the dense block). Without it the
 // product of the norms, which sets the rounding, stood up to 300 u above the sum of the products at gene
 // means of log sd 1.2; with it at 0.4 to 3 u (u = 2^-53).
-constexpr int kBalanceCells = 1024;
+constexpr int kBalanceCells = 256;
 __global__ void __launch_bounds__(256) k_crt_balance(int N, int64_t ldN, int n_d, int64_t ldp,
                                                      const double* __restrict__ W, const double* __restrict__ Sp,
                                                      double* __restrict__ bal_w, double* __restrict__ bal_s) {
@@ -260,14 +274,6 @@ __global__ void __launch_bounds__(256) k_crt_balance(int N, int64_t ldN, int n_d
     bal_w[j] = ldexp(1.0, e);
     bal_s[j] = ldexp(1.0, -e);
   }
-}
-
-// What a sum of two rows' products is off by, for rows at their scales: both operands' entries are off by
-// 0.29 of a unit (rms), so the sum by 0.41 R units at most, R bounding both norms. lim[a] is the least
-// value, before the row's own scale, of the diagonal pair (a, a) at which that is no more than `share`.
-__global__ void k_crt_limits(int n_d, double least, const double* __restrict__ inv_p, double* __restrict__ lim) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a < n_d) lim[a] = least * inv_p[(int64_t)a * n_d - (int64_t)a * (a - 1) / 2];
 }
 
 // ---- residues ------------------------------------------------------------------------------------
@@ -653,13 +659,20 @@ __device__ __forceinline__ void crt_values(const uint8_t* __restrict__ in, size_
 
 // Psi_j's dense block (both triangles, plus DeltaInv) from the residues of gene rows x pair columns;
 // over several ranges of cells the partial sums collect in acc (first / last: the range's place).
+// A gene's row of W cannot be balanced for all pairs at once: where its mass lies on other cells than a
+// column's, the sum is far below the product of the norms. So a gene goes on the list of the DMMA form
+// when the rounding of a diagonal entry, `unit` inv_j inv_p (0.41 R units; its ranges added up, in err), is
+// more than `share` of that entry. The diagonal is enough, as in k_crt_u: |p_ab|^2 <= |p_aa| |p_bb| by
+// Cauchy-Schwarz, so the rounding of entry (a, b) stays within that share of sqrt(Psi_aa Psi_bb), the
+// scale by which a factorization sees it.
 __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo, size_t plane,
                                                  const uint8_t* __restrict__ in, const double* __restrict__ inv_j,
                                                  const double* __restrict__ inv_p, const int2* __restrict__ pairs,
                                                  const int* __restrict__ dcol, const double* __restrict__ Dinv,
                                                  double* __restrict__ acc, int64_t lda, int first, int last,
-                                                 double* __restrict__ Psi, const int* __restrict__ flag) {
-  if (*flag) return;
+                                                 double* __restrict__ Psi, int n_d, double unit, double share,
+                                                 double* __restrict__ err, CrtGenes genes) {
+  if (*(const volatile int*)genes.state) return;
   const int j = blockIdx.x, p0 = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (p0 >= n_pairs) return;
   double v[4];
@@ -672,12 +685,19 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
     if (p >= n_pairs) break;
     double x = v[e] * inv_p[p] * sj;
     if (!first) x += acc[(size_t)j * lda + p];
+    const int2 q = pairs[p];
+    double off = 0.0;
+    if (q.x == q.y) {
+      off = unit * inv_j[j] * inv_p[p];
+      if (!first) off += err[(size_t)j * n_d + q.x];
+      if (!last) err[(size_t)j * n_d + q.x] = off;
+    }
     if (!last) {
       acc[(size_t)j * lda + p] = x;
     } else {
-      const int2 q = pairs[p];
       const size_t mk = dcol[q.x], ml = dcol[q.y];
       x += Dinv[mk + ml * P];
+      if (q.x == q.y && !(off <= share * x)) genes.add(j);
       Pj[mk + ml * P] = x;
       Pj[ml + mk * P] = x;
     }
@@ -685,8 +705,10 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
 }
 
 // U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], W warps per cell: the
-// cell's row of V from its residues into shared memory (pair_rows.cuh). A cell with a diagonal V[i, (a, a)]
-// below lim (k_crt_limits) sends its 128 cells to the DMMA form. The diagonal is enough: W_ij and the
+// cell's row of V from its residues into shared memory (pair_rows.cuh). The operands' entries are off by 0.29
+// of a unit (rms), so a sum by at most 0.41 R units, R bounding both rows' norms. Where that is more than its
+// share (crt_share) of a diagonal V[i, (a, a)], the value below `least` units, the cell's 128 cells go to the
+// DMMA form. The diagonal is enough: W_ij and the
 // S_j[a, a] are positive, |S_j[a, b]| <= sqrt(S_j[a, a] S_j[b, b]), and so by Cauchy-Schwarz the rounding of
 // V[i, (a, b)] stays within the same share of sqrt(V[i, (a, a)] V[i, (b, b)]).
 // Bound by the entries' arithmetic (crt_values) while 24 to 32 warps share an SM; without the limit on
@@ -696,30 +718,28 @@ template <int S, int W>
 __global__ void __launch_bounds__(256, S > 9 ? 2 : S > 5 ? 4 : 3) k_crt_u(int ldN, int n_d, int len, int c0, int64_t ldo, size_t plane,
                                                const uint8_t* __restrict__ in, const double* __restrict__ inv_i,
                                                const double* __restrict__ inv_p, const double* __restrict__ rOm,
-                                               const double* __restrict__ D, const double* __restrict__ lim,
-                                               double* __restrict__ U, int* __restrict__ cells) {
+                                               const double* __restrict__ D, double least, double* __restrict__ U,
+                                               int* __restrict__ cells) {
   extern __shared__ __align__(16) double vs[];
   if (cells[0]) return;
   const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g, i = c0 + r;
   if (r >= len) return;  // W = 1: a whole warp, no barrier of the block follows
-  double* vc = vs + g * u_space<W>(n_d);
+  double* vc = vs + g * u_space<W, true>(n_d);
   const double s = inv_i[r] * rOm[i] * kUnit;
   const uint8_t* row_in = in + (size_t)r * ldo;
+  const double* dv = pair_rows_to_u<S, W, true>(i, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
+    for (int p = from + 4 * tid; p < p1; p += 4 * nt) {
+      double v[4];
+      crt_values(row_in + p, plane, v);
+      const double2 x = *reinterpret_cast<const double2*>(inv_p + p), y = *reinterpret_cast<const double2*>(inv_p + p + 2);
+      *reinterpret_cast<double2*>(vc + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
+      *reinterpret_cast<double2*>(vc + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
+    }
+  });
   bool out = false;
-  pair_rows_to_u<S, W>(
-      i, ldN, n_d, vc, D, U,
-      [&](int from, int p1, int tid, int nt) {
-        for (int p = from + 4 * tid; p < p1; p += 4 * nt) {
-          double v[4];
-          crt_values(row_in + p, plane, v);
-          const double2 x = *reinterpret_cast<const double2*>(inv_p + p),
-                        y = *reinterpret_cast<const double2*>(inv_p + p + 2);
-          *reinterpret_cast<double2*>(vc + p - from) = make_double2(v[0] * x.x * s, v[1] * x.y * s);
-          *reinterpret_cast<double2*>(vc + p - from + 2) = make_double2(v[2] * y.x * s, v[3] * y.y * s);
-        }
-      },
-      [&](int a, double v) { out |= !(v >= lim[a] * s); });
-  if (out && (threadIdx.x & 31) == 0) cells[1 + (i >> 7)] = 1;
+  for (int a = W == 8 ? threadIdx.x : threadIdx.x & 31; a < n_d; a += 32 * W)
+    out |= !(dv[a] >= least * inv_p[a * n_d - a * (a - 1) / 2] * s);
+  if (out) cells[1 + (i >> 7)] = 1;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -734,19 +754,25 @@ constexpr int kGroupI8 = 8;
 int up(int64_t v, int m) { return (int)((v + m - 1) / m * m); }
 }  // namespace
 
-// Where the integer form is taken. The Gram: from 512 cells on. The DMMA form has one CTA per 128
-// pairs x 128 genes and takes 0.15 us for every cell in it (K in slices of 16), however few the tiles;
-// measured from 1,000 x 20 x 21 (cells, genes, pairs: 0.163 -> 0.071 ms) over 20,000 x 1,001 x 15 (2.98
-// -> 0.32) to 10,000 x 1,000 x 4,851 (4.64 -> 0.98) the integer form was 1.3 to 25 times as fast. A few
-// genes keep the DMMA form, whose tile order the autotuner can choose (2,000 cells: 0.2 ms lost).
-// The gradient pairs: the two forms' times as estimated by the costs measured over 1,000 to 30,000
-// cells, 20 to 1,000 genes and 21 to 4,851 pairs (us). DMMA: 0.165 per gene and wave of 148 tiles, and
-// the pair rows. Integer: the conversions of both operands, the way back to FP64, padded tiles and
-// chunks, and the products. E.g. 1,000 x 1,000 x 105: 169 / 65; 3,000 x 300 x 595: 74 / 107;
-// 30,000 x 300 x 105: 167 / 391; 30,000 x 300 x 4,851: 3,707 / 2,495.
-constexpr int kMinCells = 512, kMinGenes = 32;
-static bool crt_grad_faster(double N, double J, double pairs, double Jk, double Pp) {
-  const double waves = std::ceil(std::ceil(N / 128) * std::ceil(pairs / 128) / 148);
+// Where the integer form is taken: by both forms' times (us), as estimated by costs fitted to measurements.
+// The Gram, over 600 to 20,000 cells, 40 to 2,500 genes and 55 to 8,515 pairs (within 36%; the faster form
+// was missed by more than 5% at three of 86 sizes): the DMMA form's tiles (pair_gram_cost) and its pair products;
+// this one's 256 x 256 tiles of each modulus on 74 CTA pairs, the conversions and the way back. E.g. 2,000 cells
+// x 300 x 595: 154 integer, 111 DMMA; 5,000 x 1,000 x 595: 268 / 393; 20,000 x 1,000 x 8,515: 3,736 / 12,668.
+static bool crt_gram_faster(const Ctx* c, double N, double J, double pairs) {
+  const double dmma = 54 + pair_gram_cost(c, c->pr.n_pairs) * N / 16 / 1900 + N * (3.8e-6 * pairs + 1.7e-6 * J) +
+                      19e-6 * J * pairs;
+  const double tiles = kMod * std::ceil(J / kTile) * std::ceil(pairs / kTile);
+  const double integer = 126 + 0.40 * std::ceil(tiles / (c->sm_count / 2)) * std::ceil(N / kChunk) +
+                         N * (7.9e-6 * pairs + 10.4e-6 * J) + 24e-6 * J * pairs;
+  return integer < dmma;
+}
+// The gradient pairs, over 1,000 to 30,000 cells, 20 to 1,000 genes and 21 to 4,851 pairs. DMMA: 0.165 per
+// gene and wave of tiles, and the pair rows. Integer: the conversions of both operands, the way back to FP64,
+// padded tiles and chunks, and the products. E.g. 1,000 x 1,000 x 105: 169 / 65; 3,000 x 300 x 595: 74 / 107;
+// 30,000 x 300 x 105: 167 / 391; 30,000 x 300 x 4,851: 3,707 / 2,495 (DMMA / integer).
+static bool crt_grad_faster(const Ctx* c, double N, double J, double pairs, double Jk, double Pp) {
+  const double waves = std::ceil(std::ceil(N / 128) * std::ceil(pairs / 128) / c->sm_count);
   const double dmma = 10 + 0.165 * J * waves + 5e-6 * N * pairs;
   const double integer = 50 + N * (15e-6 * Pp + 10e-6 * Jk) + N * Jk * Pp * 2 * kMod / 2.9e9;
   return integer < dmma;
@@ -759,7 +785,7 @@ void crt_plan(Ctx* c, size_t cap) {
   t.Jp = up(J, kTile);
   t.Pp = up(s.n_pairs, kTile);
   t.Jk = up(J, kChunk);
-  if (N < kMinCells || J < kMinGenes || J > kMaxK || c->n_d > kUMaxDense) return;
+  if (J > kMaxK || c->n_d > kUMaxDense) return;
   int64_t most = std::min<int64_t>(up(N, kTile), kMaxK / kTile * kTile);
   if (c->pair_range_cells > 0) {  // ranges below a tile: the DMMA form
     if (c->pair_range_cells < kTile) return;
@@ -781,8 +807,8 @@ void crt_plan(Ctx* c, size_t cap) {
     const int64_t ranges = (N + n - 1) / n;  // ranges of one size
     return std::min<int64_t>(n, up((N + ranges - 1) / ranges, kTile));
   };
-  t.gram_cells = (int)cells(gram);
-  t.grad_cells = crt_grad_faster(N, J, s.n_pairs, t.Jk, t.Pp) ? (int)cells(grad) : 0;
+  t.gram_cells = crt_gram_faster(c, N, J, s.n_pairs) ? (int)cells(gram) : 0;
+  t.grad_cells = crt_grad_faster(c, N, J, s.n_pairs, t.Jk, t.Pp) ? (int)cells(grad) : 0;
   t.bytes = (size_t)std::max(t.gram_cells ? gram(t.gram_cells) : 0, t.grad_cells ? grad(t.grad_cells) : 0);
   t.on = t.gram_cells > 0 || t.grad_cells > 0;
 }
@@ -792,17 +818,20 @@ int crt_prepare(Ctx* c) {
   CrtState& t = s.crt;
   if (!t.on) return GPL_OK;
   const size_t rows = (size_t)2 * (t.Jp + t.Pp + t.grad_cells), tiles = div_up(c->N, 128);
-  if (cudaMalloc((void**)&t.scales, sizeof(double) * (rows + 2 * t.Jp + c->n_d)) != cudaSuccess ||
-      cudaMalloc((void**)&t.flag, (3 + tiles) * sizeof(int)) != cudaSuccess) {
+  const size_t ints = 5 + tiles + 2 * (size_t)c->J, errs = t.gram_cells < c->N ? (size_t)c->J * c->n_d : 0;
+  if (cudaMalloc((void**)&t.scales, sizeof(double) * (rows + 2 * t.Jp + errs)) != cudaSuccess ||
+      cudaMalloc((void**)&t.flag, ints * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     c->err = "device allocation failed: scales of the integer pair products";
     return GPL_ERR_ALLOC;
   }
   t.balance = t.scales + rows;  // of W, then of the pairs
-  t.lim = t.balance + 2 * t.Jp;
   t.err = t.flag + 1;
   t.cells = t.flag + 2;
-  GPL_TRY(c, cudaMemset(t.flag, 0, (3 + tiles) * sizeof(int)));
+  t.genes = t.cells + 1 + tiles;
+  t.list = t.genes + 2 + c->J;
+  t.g_err = t.balance + 2 * t.Jp;
+  GPL_TRY(c, cudaMemset(t.flag, 0, ints * sizeof(int)));
   int8_t* pool = reinterpret_cast<int8_t*>(s.V);
   // Gram: gene planes, pair planes, residues out, partial sums over the ranges
   t.g_a = pool;
@@ -855,7 +884,7 @@ static int crt_gemm(Ctx* c, const CUtensorMap& ma, const CUtensorMap& mb, int ro
   return GPL_OK;
 }
 
-// What the rounding of an integer product may be of the diagonal it is measured by (k_crt_limits), over K
+// What the rounding of an integer product may be of the diagonal it is measured by (k_crt_psi, k_crt_u), over K
 // terms: what a chain of K FP64 multiply-adds is off by, 0.15 sqrt(K) u (rms; 12 u measured at K = 6,001, 19 u
 // at 19,997), less a third, and 4 u at least.
 static double crt_share(double K) {
@@ -882,12 +911,13 @@ int launch_crt_gram(Ctx* c) {
   const double R = crt_norm_limit();
   double *sc_j = t.scales, *inv_j = sc_j + t.Jp, *sc_p = inv_j + t.Jp, *inv_p = sc_p + t.Pp;
   double* part = reinterpret_cast<double*>(t.g_out);
-  GPL_TRY(c, cudaMemsetAsync(t.flag, 0, sizeof(int), c->stream));
+  const CrtGenes genes{t.genes, t.list};
+  GPL_TRY(c, cudaMemsetAsync(t.genes, 0, (2 + c->J) * sizeof(int), c->stream));
   for (int c0 = 0; c0 < c->N; c0 += t.gram_cells) {
     const int len = std::min(t.gram_cells, c->N - c0), kpad = up(len, kChunk);
     const size_t plane_a = (size_t)t.Jp * t.gram_cells, plane_b = (size_t)t.Pp * t.gram_cells;
     const size_t plane_o = (size_t)t.Jp * t.Pp;
-    k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, t.flag);
+    k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, genes);
     GPL_LAUNCHED(c, "k_crt_norm_rows");
     const int gx = div_up(s.n_pairs, 256 * kNormPairs);
     // as many cell parts as fill the SMs, within the partial sums' space (14 bytes x 256 rows per pair)
@@ -897,19 +927,19 @@ int launch_crt_gram(Ctx* c) {
     k_crt_norm_pairs<<<dim3(gx, ny), 256, sizeof(double) * 32 * (c->n_d + 1), c->stream>>>(
         c->ldN, c->n_d, c0, c0 + len, cper, s.n_pairs, s.pairs, c->Dm, s.rOm, part);
     GPL_LAUNCHED(c, "k_crt_norm_pairs");
-    k_crt_scales<<<div_up(s.n_pairs, 256), 256, 0, c->stream>>>(s.n_pairs, ny, part, R, sc_p, inv_p, t.flag, 31);
+    k_crt_scales<<<div_up(s.n_pairs, 256), 256, 0, c->stream>>>(s.n_pairs, ny, part, R, sc_p, inv_p, t.genes, 31);
     GPL_LAUNCHED(c, "k_crt_scales");
     k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad, t.gram_cells,
-                                                                          plane_a, sc_j, t.g_a, t.flag);
+                                                                          plane_a, sc_j, t.g_a, t.genes);
     GPL_LAUNCHED(c, "k_crt_conv_rows");
     k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(s.n_pairs, kConvPairs)), 256, 0, c->stream>>>(
-        c->ldN, c0, len, kpad, t.gram_cells, plane_b, s.n_pairs, s.pairs, c->Dm, s.rOm, sc_p, t.g_b, t.flag);
+        c->ldN, c0, len, kpad, t.gram_cells, plane_b, s.n_pairs, s.pairs, c->Dm, s.rOm, sc_p, t.g_b, t.genes);
     GPL_LAUNCHED(c, "k_crt_conv_pairs");
-    const int rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, s.n_pairs, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.flag);
+    const int rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, s.n_pairs, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.genes);
     if (rc) return rc;
     k_crt_psi<<<dim3(c->J, div_up(s.n_pairs, 1024)), 256, 0, c->stream>>>(
         c->P, s.n_pairs, t.Pp, plane_o, t.g_out, inv_j, inv_p, s.pairs, c->dcol_d, c->DeltaInv, t.g_acc, t.Pp,
-        c0 == 0, c0 + len >= c->N, c->Psi, t.flag);
+        c0 == 0, c0 + len >= c->N, c->Psi, c->n_d, 0.41 * R, crt_share(c->N), t.g_err, genes);
     GPL_LAUNCHED(c, "k_crt_psi");
   }
   return GPL_OK;
@@ -930,9 +960,7 @@ int launch_crt_uq(Ctx* c) {
   GPL_LAUNCHED(c, "k_crt_balance");
   int rc;
   if ((rc = crt_col_scales(c, s.Sp, s.pairs_pad, s.n_pairs, c->J, bal_s, part, sc_p, inv_p, t.cells, 31))) return rc;
-  k_crt_limits<<<div_up(c->n_d, 128), 128, 0, c->stream>>>(
-      c->n_d, 0.41 * crt_norm_limit() / kUnit / crt_share(c->J), inv_p, t.lim);
-  GPL_LAUNCHED(c, "k_crt_limits");
+  const double least = 0.41 * crt_norm_limit() / crt_share(c->J) / kUnit;
   k_crt_conv_cols<false><<<dim3(div_up(s.n_pairs, 32), t.Jk / 128), 256, kSmemTurn, c->stream>>>(
       s.Sp, s.pairs_pad, s.n_pairs, c->J, t.Jk, plane_b, bal_s, sc_p, t.v_b, t.cells);
   GPL_LAUNCHED(c, "k_crt_conv_cols");
@@ -953,9 +981,11 @@ int launch_crt_uq(Ctx* c) {
     ProfScope ps(c, "v_to_u");
     pair_rows_form(c->n_d, len, 96, [&](auto S, auto W) {
       constexpr int per = 8 / W;
-      const int smem = (int)sizeof(double) * u_space<W>(c->n_d) * per;
+      const int smem = (int)sizeof(double) * u_space<W, true>(c->n_d) * per;
+      if (smem > 48 * 1024)  // 85 or more columns, a warp per cell
+        cudaFuncSetAttribute(k_crt_u<S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       k_crt_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, len, c0, t.Pp, plane_o, t.v_out, inv_i,
-                                                               inv_p, s.rOm, c->Dm, t.lim, c->U, t.cells);
+                                                               inv_p, s.rOm, c->Dm, least, c->U, t.cells);
     });
     GPL_LAUNCHED(c, "k_crt_u");
   }
@@ -1034,7 +1064,7 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
                                  sizeof(double) * c->N, nl, cudaMemcpyDeviceToDevice, c->stream));
     for (int c0 = 0; c0 < c->N; c0 += t.gram_cells) {
       const int len = std::min(t.gram_cells, c->N - c0), kpad = up(len, kChunk);
-      k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, t.flag);
+      k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, CrtGenes{t.flag, nullptr});
       GPL_LAUNCHED(c, "k_crt_norm_rows");
       const int gx = div_up(rows, 256 * kNormPairs);
       const int gy = std::max(1, std::min({div_up(len, 64), 592 / gx, 256}));

@@ -24,6 +24,7 @@
 // c0,c1 = C[g][2t, 2t+1], c2,c3 = C[g+8][2t, 2t+1]. Shared rows are padded so that the
 // 16 lanes of each half-warp hit 16 distinct 8-byte bank pairs.
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 
 #include "dmma_common.cuh"
@@ -90,31 +91,33 @@ constexpr int kProdCells = 8;
 __global__ void __launch_bounds__(256) k_pair_products(int ldN, int n_d, int c0, int c1, int n_pairs, int pairs_pad,
                                                        const int2* __restrict__ pairs, const double* __restrict__ D,
                                                        const double* __restrict__ rOm, double* __restrict__ A,
-                                                       const int* __restrict__ gate) {
+                                                       const int* __restrict__ state) {
   extern __shared__ double dsh[];  // [n_d][kProdCells] then rOm[kProdCells]
-  if (gate && *gate == 0) return;
-  const int i0 = c0 + blockIdx.x * kProdCells;
-  const int nc = min(kProdCells, c1 - i0);
-  for (int e = threadIdx.x; e < n_d * kProdCells; e += blockDim.x) {
-    const int a = e / kProdCells, r = e - a * kProdCells;
-    dsh[e] = r < nc ? D[(size_t)a * ldN + i0 + r] : 0.0;
-  }
-  if (threadIdx.x < kProdCells) dsh[n_d * kProdCells + threadIdx.x] = threadIdx.x < nc ? rOm[i0 + threadIdx.x] : 0.0;
-  __syncthreads();
-  const double* ro = dsh + n_d * kProdCells;
-  for (int p = threadIdx.x; p < pairs_pad; p += blockDim.x) {
-    double v[kProdCells];
-    if (p < n_pairs) {
-      const int2 q = pairs[p];
-      const double* da = dsh + q.x * kProdCells;
-      const double* db = dsh + q.y * kProdCells;
-#pragma unroll
-      for (int r = 0; r < kProdCells; r++) v[r] = da[r] * db[r] * ro[r];
-    } else {
-#pragma unroll
-      for (int r = 0; r < kProdCells; r++) v[r] = 0.0;
+  if (state && !state[0] && !state[1]) return;  // no gene on the list (GramGenes)
+  for (int i0 = c0 + blockIdx.x * kProdCells; i0 < c1; i0 += gridDim.x * kProdCells) {
+    __syncthreads();
+    const int nc = min(kProdCells, c1 - i0);
+    for (int e = threadIdx.x; e < n_d * kProdCells; e += blockDim.x) {
+      const int a = e / kProdCells, r = e - a * kProdCells;
+      dsh[e] = r < nc ? D[(size_t)a * ldN + i0 + r] : 0.0;
     }
-    for (int r = 0; r < nc; r++) A[(size_t)(i0 - c0 + r) * pairs_pad + p] = v[r];
+    if (threadIdx.x < kProdCells) dsh[n_d * kProdCells + threadIdx.x] = threadIdx.x < nc ? rOm[i0 + threadIdx.x] : 0.0;
+    __syncthreads();
+    const double* ro = dsh + n_d * kProdCells;
+    for (int p = threadIdx.x; p < pairs_pad; p += blockDim.x) {
+      double v[kProdCells];
+      if (p < n_pairs) {
+        const int2 q = pairs[p];
+        const double* da = dsh + q.x * kProdCells;
+        const double* db = dsh + q.y * kProdCells;
+#pragma unroll
+        for (int r = 0; r < kProdCells; r++) v[r] = da[r] * db[r] * ro[r];
+      } else {
+#pragma unroll
+        for (int r = 0; r < kProdCells; r++) v[r] = 0.0;
+      }
+      for (int r = 0; r < nc; r++) A[(size_t)(i0 - c0 + r) * pairs_pad + p] = v[r];
+    }
   }
 }
 
@@ -134,133 +137,154 @@ struct GramTile {
   static constexpr int smem = (int)sizeof(double) * 3 * (BK * SAm + TN * SBT);
 };
 
+// The genes that a launch takes: all of them, or those on the list that the integer form left (CrtState):
+// state[0] all, state[1] how many. Launches for few and for many of them stand one behind the other
+// (lo <= count < hi), as the count is not known to the host.
+struct GramGenes {
+  const int *state, *list;
+  int lo, hi;
+  __device__ __forceinline__ int count(int J) const { return !state || state[0] ? J : state[1]; }
+  __device__ __forceinline__ int gene(int k) const { return !state || state[0] ? k : list[k]; }
+};
+
 template <int TM, int TN>
 __global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
     k_pair_gram(int N, int ldN, int J, int P, int c0, int c1, int pairs_pad, int n_pairs, int mode,
                 const double* __restrict__ A, const int2* __restrict__ pairs, const int* __restrict__ dcol,
                 const double* __restrict__ W, const double* __restrict__ Dinv, double* __restrict__ Psi,
-                double* __restrict__ Gacc, int group_m, const int* __restrict__ gate) {
+                double* __restrict__ Gacc, int group_m, GramGenes genes) {
   using G = GramTile<TM, TN>;
   constexpr int SAm = G::SAm, MT = G::MT, NT = G::NT;
   extern __shared__ __align__(16) double smem_d[];
-  if (gate && *gate == 0) return;
+  const int n_j = genes.count(J);
+  if (n_j < genes.lo || n_j >= genes.hi) return;
   double* As = smem_d;               // [3][BK][SAm]  pair products (pairs contiguous)
   double* Bs = As + 3 * BK * SAm;    // [3][TN][SBT]  weights (cells contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3, wm = warp / G::WN, wn = warp % G::WN;
-  const int2 tile = grouped_tile(blockIdx.x, (n_pairs + TM - 1) / TM, (J + TN - 1) / TN, group_m);
-  const int p0 = tile.x * TM, j0 = tile.y * TN;
+  const int tm = (n_pairs + TM - 1) / TM, tn = (n_j + TN - 1) / TN;
   const int nsl = (c1 - c0 + BK - 1) / BK;
+  for (int id = blockIdx.x; id < tm * tn; id += gridDim.x) {
+    const int2 tile = grouped_tile(id, tm, tn, group_m);
+    const int p0 = tile.x * TM, j0 = tile.y * TN;
+    // the weights' rows that this thread copies
+    constexpr int kRowsB = (TN * BK / 2 + kThreads - 1) / kThreads;
+    const double* rows_b[kRowsB];
+#pragma unroll
+    for (int r = 0; r < kRowsB; r++)
+      rows_b[r] = W + (size_t)genes.gene(min(j0 + ((tid + r * kThreads) >> 3), n_j - 1)) * ldN;
+    __syncthreads();  // the last tile's slices are read
 
-  // slice s: cells [c0 + 16 s, c0 + 16 s + 16) of both operands (16-byte copies; rows of A
-  // past the range and weights past N arrive as zeros)
-  auto load = [&](int s, int st) {
-    const int kb = s * BK;
+    // slice s: cells [c0 + 16 s, c0 + 16 s + 16) of both operands (16-byte copies; rows of A
+    // past the range and weights past N arrive as zeros)
+    auto load = [&](int s, int st) {
+      const int kb = s * BK;
 #pragma unroll
-    for (int r = 0; r < (TM * BK / 2) / kThreads; r++) {
-      const int ch = tid + r * kThreads;
-      const int k = ch / (TM / 2), part = ch % (TM / 2);
-      const int row = kb + k;
-      const int nb = (c0 + row < c1) ? 16 : 0;
-      const double* src = A + (size_t)min(row, c1 - c0 - 1) * pairs_pad + p0 + part * 2;
-      cp_async16(As + st * BK * SAm + k * SAm + part * 2, src, nb);
-    }
+      for (int r = 0; r < (TM * BK / 2) / kThreads; r++) {
+        const int ch = tid + r * kThreads;
+        const int k = ch / (TM / 2), part = ch % (TM / 2);
+        const int row = kb + k;
+        const int nb = (c0 + row < c1) ? 16 : 0;
+        const double* src = A + (size_t)min(row, c1 - c0 - 1) * pairs_pad + p0 + part * 2;
+        cp_async16(As + st * BK * SAm + k * SAm + part * 2, src, nb);
+      }
 #pragma unroll
-    for (int r = 0; r < (TN * BK / 2 + kThreads - 1) / kThreads; r++) {
-      const int ch = tid + r * kThreads;
-      if (TN * BK / 2 < kThreads && ch >= TN * BK / 2) break;
-      const int n = ch >> 3, part = ch & 7;
-      const int j = j0 + n, i = c0 + kb + part * 2;
-      const int nb = (j < J) ? 8 * max(0, min(2, min(N, c1) - i)) : 0;
-      const double* src = W + (size_t)min(j, J - 1) * ldN + min(i, ldN - 2);
-      cp_async16(Bs + st * TN * SBT + n * SBT + part * 2, src, nb);
-    }
-  };
+      for (int r = 0; r < kRowsB; r++) {
+        const int ch = tid + r * kThreads;
+        if (TN * BK / 2 < kThreads && ch >= TN * BK / 2) break;
+        const int n = ch >> 3, part = ch & 7;
+        const int j = j0 + n, i = c0 + kb + part * 2;
+        const int nb = (j < n_j) ? 8 * max(0, min(2, min(N, c1) - i)) : 0;
+        const double* src = rows_b[r] + min(i, ldN - 2);
+        cp_async16(Bs + st * TN * SBT + n * SBT + part * 2, src, nb);
+      }
+    };
 
-  double acc[MT][NT][4];
+    double acc[MT][NT][4];
 #pragma unroll
-  for (int x = 0; x < MT; x++)
+    for (int x = 0; x < MT; x++)
 #pragma unroll
-    for (int y = 0; y < NT; y++)
+      for (int y = 0; y < NT; y++)
 #pragma unroll
-      for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
+        for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
 
-  // three stages, one barrier per slice (as k_pair_v)
-  load(0, 0);
-  cp_async_commit();
-  if (nsl > 1) load(1, 1);
-  cp_async_commit();
-  for (int s = 0; s < nsl; s++) {
-    cp_async_wait<1>();  // slice s landed
-    __syncthreads();
-    if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
+    // three stages, one barrier per slice (as k_pair_v)
+    load(0, 0);
     cp_async_commit();
-    const double* as = As + (s % 3) * BK * SAm;
-    const double* bs = Bs + (s % 3) * TN * SBT;
+    if (nsl > 1) load(1, 1);
+    cp_async_commit();
+    for (int s = 0; s < nsl; s++) {
+      cp_async_wait<1>();  // slice s landed
+      __syncthreads();
+      if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
+      cp_async_commit();
+      const double* as = As + (s % 3) * BK * SAm;
+      const double* bs = Bs + (s % 3) * TN * SBT;
 #pragma unroll
-    for (int kk = 0; kk < BK / 4; kk++) {
-      double a[MT][2], b[NT];
-      const double* ar = as + (kk * 4 + t) * SAm + wm * MT * 16 + g;
+      for (int kk = 0; kk < BK / 4; kk++) {
+        double a[MT][2], b[NT];
+        const double* ar = as + (kk * 4 + t) * SAm + wm * MT * 16 + g;
 #pragma unroll
-      for (int mt = 0; mt < MT; mt++) {
-        a[mt][0] = ar[mt * 16];
-        a[mt][1] = ar[mt * 16 + 8];
+        for (int mt = 0; mt < MT; mt++) {
+          a[mt][0] = ar[mt * 16];
+          a[mt][1] = ar[mt * 16 + 8];
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) b[nt] = bs[(wn * NT * 8 + nt * 8 + g) * SBT + kk * 4 + t];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+          for (int nt = 0; nt < NT; nt++) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
       }
-#pragma unroll
-      for (int nt = 0; nt < NT; nt++) b[nt] = bs[(wn * NT * 8 + nt * 8 + g) * SBT + kk * 4 + t];
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
     }
-  }
-  cp_async_wait<0>();
+    cp_async_wait<0>();
 
 #pragma unroll
-  for (int mt = 0; mt < MT; mt++)
+    for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int p = p0 + (wm * MT + mt) * 16 + g + h * 8;
-      if (p >= n_pairs) continue;
-      size_t mk = 0, ml = 0;
-      double dv = 0.0;
-      if (mode == kGramPsi) {
-        const int2 q = pairs[p];
-        mk = dcol[q.x];
-        ml = dcol[q.y];
-        dv = Dinv[mk + ml * P];
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int j = j0 + (wn * NT + nt) * 8 + 2 * t + e;
-          if (j >= J) continue;
-          const double v = acc[mt][nt][h * 2 + e];
-          if (mode == kGramPsi) {
-            double* Pj = Psi + (size_t)j * P * P;
-            Pj[mk + ml * P] = v + dv;
-            Pj[ml + mk * P] = v + dv;
-          } else if (mode == kGramSet) {
-            Gacc[(size_t)p * J + j] = v;
-          } else {
-            Gacc[(size_t)p * J + j] += v;
-          }
+      for (int h = 0; h < 2; h++) {
+        const int p = p0 + (wm * MT + mt) * 16 + g + h * 8;
+        if (p >= n_pairs) continue;
+        size_t mk = 0, ml = 0;
+        double dv = 0.0;
+        if (mode == kGramPsi) {
+          const int2 q = pairs[p];
+          mk = dcol[q.x];
+          ml = dcol[q.y];
+          dv = Dinv[mk + ml * P];
         }
-    }
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            if (j0 + (wn * NT + nt) * 8 + 2 * t + e >= n_j) continue;
+            const int j = genes.gene(j0 + (wn * NT + nt) * 8 + 2 * t + e);
+            const double v = acc[mt][nt][h * 2 + e];
+            if (mode == kGramPsi) {
+              double* Pj = Psi + (size_t)j * P * P;
+              Pj[mk + ml * P] = v + dv;
+              Pj[ml + mk * P] = v + dv;
+            } else if (mode == kGramSet) {
+              Gacc[(size_t)p * J + j] = v;
+            } else {
+              Gacc[(size_t)p * J + j] += v;
+            }
+          }
+      }
+  }
 }
 
 // Psi_j[mk, ml] = Psi_j[ml, mk] = Gacc[p * J + j] + DeltaInv[mk, ml] after several ranges
 __global__ void k_pair_scatter(int J, int P, int n_pairs, const int2* __restrict__ pairs,
                                const int* __restrict__ dcol, const double* __restrict__ Gacc,
-                               const double* __restrict__ Dinv, double* __restrict__ Psi,
-                               const int* __restrict__ gate) {
-  if (gate && *gate == 0) return;
-  const int p = blockIdx.x;
+                               const double* __restrict__ Dinv, double* __restrict__ Psi, GramGenes genes) {
+  const int n_j = genes.count(J), p = blockIdx.x;
+  if (n_j == 0) return;
   const int2 q = pairs[p];
   const size_t mk = dcol[q.x], ml = dcol[q.y];
   const double dv = Dinv[mk + ml * P];
-  for (int j = threadIdx.x; j < J; j += blockDim.x) {
+  for (int k = threadIdx.x; k < n_j; k += blockDim.x) {
+    const int j = genes.gene(k);
     const double v = Gacc[(size_t)p * J + j] + dv;
     double* Pj = Psi + (size_t)j * P * P;
     Pj[mk + ml * P] = v;
@@ -375,13 +399,13 @@ __global__ void __launch_bounds__(256, S > 9 ? 2 : 4) k_v_to_u(int ldN, int n_d,
   const int g = W == 8 ? 0 : threadIdx.x >> 5, r = blockIdx.x * (8 / W) + g;
   if (c0 + r >= c1) return;  // W = 1: a whole warp, no barrier of the block follows
   if (cells && !cells[0] && !cells[1 + (c0 + r) / BM]) return;
-  double* vc = vs + g * u_space<W>(n_d);
+  double* vc = vs + g * u_space<W, false>(n_d);
   const double* vr = V + (size_t)r * pairs_pad;
-  pair_rows_to_u<S, W>(c0 + r, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
+  pair_rows_to_u<S, W, false>(c0 + r, ldN, n_d, vc, D, U, [&](int from, int p1, int tid, int nt) {
     for (int p = from + 2 * tid; p < p1; p += 2 * nt) cp_async16(vc + p - from, vr + p, 16);
     cp_async_commit();
     cp_async_wait<0>();
-  }, [](int, double) {});
+  });
 }
 
 // The same for more dense columns than that takes (512): the row is read from global memory (L1 / L2)
@@ -488,13 +512,20 @@ int recip_omega(Ctx* c, const double** rOm) {
 // The Gram's tile for n_pairs x J outputs, by its time per 16 cells: the tile's multiply-adds (64 per clock
 // and SM) times the tiles an SM takes, at least 400 clocks of copies and barriers; the smaller tiles with a
 // tenth for their operands' traffic.
-static int gram_tile(const Ctx* c, int n_pairs) {
-  const auto cost = [&](int tm, int tn) {
-    const double tiles = (double)div_up(n_pairs, tm) * div_up(c->J, tn);
-    return std::ceil(tiles / c->sm_count) * std::max(tm * tn * 16 / 64, 400) * (tm < 128 ? 1.1 : 1.0);
-  };
-  const double big = cost(128, 128), mid = cost(64, 64), small = cost(64, 16);
+static double gram_tile_cost(const Ctx* c, int n_pairs, int tm, int tn) {
+  const double tiles = (double)div_up(n_pairs, tm) * div_up(c->J, tn);
+  return std::ceil(tiles / c->sm_count) * std::max(tm * tn * 16 / 64, 400) * (tm < 128 ? 1.1 : 1.0);
+}
+static int gram_tile(const Ctx* c, int n_pairs, double* cost) {
+  const double big = gram_tile_cost(c, n_pairs, 128, 128), mid = gram_tile_cost(c, n_pairs, 64, 64),
+               small = gram_tile_cost(c, n_pairs, 64, 16);
+  if (cost) *cost = std::min({big, mid, small});
   return big <= mid && big <= small ? 0 : mid <= small ? 1 : 2;
+}
+double pair_gram_cost(const Ctx* c, int n_pairs) {
+  double cost;
+  gram_tile(c, n_pairs, &cost);
+  return cost;
 }
 
 int launch_pair_gram(Ctx* c) {
@@ -503,37 +534,49 @@ int launch_pair_gram(Ctx* c) {
   if (rc) return rc;
   PairState& s = c->pr;
   ProfScope ps(c, "gram");
-  // the integer form, where it is planned; the kernels below then run only if it found operands out of
-  // its range (gate), as they do for non-finite values
-  const int* gate = s.crt.gram_cells && !c->one_order ? s.crt.flag : nullptr;
-  if (gate && (rc = launch_crt_gram(c))) return rc;
+  // the integer form, where it is planned; the kernels below then run for the genes that it left
+  const bool crt = s.crt.gram_cells && !c->one_order;
+  if (crt && (rc = launch_crt_gram(c))) return rc;
+  const int* state = crt ? s.crt.genes : nullptr;
   const bool one = s.v_cells >= c->N;
   for (int c0 = 0; c0 < c->N; c0 += s.v_cells) {
     const int c1 = std::min(c->N, c0 + s.v_cells);
     const int smem_p = (int)sizeof(double) * (c->n_d + 1) * kProdCells;
-    k_pair_products<<<div_up(c1 - c0, kProdCells), 256, smem_p, c->stream>>>(
-        c->ldN, c->n_d, c0, c1, s.n_pairs, s.pairs_pad, s.pairs, c->Dm, s.rOm, s.V, gate);
+    const int gp = div_up(c1 - c0, kProdCells);
+    k_pair_products<<<crt ? std::min(gp, 8 * c->sm_count) : gp, 256, smem_p, c->stream>>>(
+        c->ldN, c->n_d, c0, c1, s.n_pairs, s.pairs_pad, s.pairs, c->Dm, s.rOm, s.V, state);
     GPL_LAUNCHED(c, "k_pair_products");
     const int mode = one ? kGramPsi : (c0 == 0 ? kGramSet : kGramAdd);
     Tunable* tu = nullptr;
-    const int gm = gate ? kGroupM : tune_pick(c, "pair_gram", {8, 12, 16}, kGroupM, &tu);
+    const int gm = crt ? kGroupM : tune_pick(c, "pair_gram", {8, 12, 16}, kGroupM, &tu);
     TuneScope ts(c, one ? tu : nullptr);
-    auto run = [&](auto tm, auto tn) {
+    auto run = [&](auto tm, auto tn, int most, const GramGenes& genes) {
       constexpr int TM = decltype(tm)::value, TN = decltype(tn)::value;
-      k_pair_gram<TM, TN><<<div_up(s.n_pairs, TM) * div_up(c->J, TN), kThreads, GramTile<TM, TN>::smem, c->stream>>>(
-          c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs, mode, s.V, s.pairs, c->dcol_d, c->W, c->DeltaInv,
-          c->Psi, s.Gacc, gm, gate);
+      k_pair_gram<TM, TN><<<std::min(most, div_up(s.n_pairs, TM) * div_up(c->J, TN)), kThreads, GramTile<TM, TN>::smem,
+                            c->stream>>>(c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs, mode, s.V, s.pairs,
+                                         c->dcol_d, c->W, c->DeltaInv, c->Psi, s.Gacc, gm, genes);
     };
     using std::integral_constant;
-    const int form = gram_tile(c, s.n_pairs);
-    if (form == 0) run(integral_constant<int, 128>(), integral_constant<int, 128>());
-    else if (form == 1) run(integral_constant<int, 64>(), integral_constant<int, 64>());
-    else run(integral_constant<int, 64>(), integral_constant<int, 16>());
+    constexpr integral_constant<int, 128> n128;
+    constexpr integral_constant<int, 64> n64;
+    constexpr integral_constant<int, 16> n16;
+    const int all = INT_MAX, resident = 3 * c->sm_count;
+    if (crt) {  // up to 48 genes in tiles of 16
+      run(n64, n16, resident, GramGenes{state, s.crt.list, 1, 49});
+      GPL_LAUNCHED(c, "k_pair_gram");
+      run(n64, n64, resident, GramGenes{state, s.crt.list, 49, all});
+    } else {
+      const GramGenes genes{nullptr, nullptr, 0, all};
+      const int form = gram_tile(c, s.n_pairs, nullptr);
+      if (form == 0) run(n128, n128, all, genes);
+      else if (form == 1) run(n64, n64, all, genes);
+      else run(n64, n16, all, genes);
+    }
     GPL_LAUNCHED(c, "k_pair_gram");
   }
   if (!one) {
     k_pair_scatter<<<s.n_pairs, 256, 0, c->stream>>>(c->J, c->P, s.n_pairs, s.pairs, c->dcol_d, s.Gacc,
-                                                    c->DeltaInv, c->Psi, gate);
+                                                    c->DeltaInv, c->Psi, GramGenes{state, s.crt.list, 0, INT_MAX});
     GPL_LAUNCHED(c, "k_pair_scatter");
   }
   return GPL_OK;
@@ -588,7 +631,7 @@ int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V,
   const int len = std::min(c1, c->N) - c0;
   pair_rows_form(c->n_d, len, 160, [&](auto S, auto W) {
     constexpr int per = 8 / W;
-    const int smem = (int)sizeof(double) * u_space<W>(c->n_d) * per;
+    const int smem = (int)sizeof(double) * u_space<W, false>(c->n_d) * per;
     if (smem > 48 * 1024)  // 97 or more columns, a warp per cell
       cudaFuncSetAttribute(k_v_to_u<S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     k_v_to_u<S, W><<<div_up(len, per), 256, smem, c->stream>>>(c->ldN, c->n_d, s.pairs_pad, c0, c0 + len, D, V, c->U,

@@ -26,10 +26,10 @@ template <int W>
 constexpr int u_entries() {
   return W == 8 ? 4096 : 512;
 }
-// doubles of a cell's shared memory: V, the D row and the row sums
-template <int W>
+// doubles of a cell's shared memory: V, the D row, the row sums and, where they are asked for, the diagonals
+template <int W, bool kDiag>
 __host__ __device__ constexpr int u_space(int n_d) {
-  return u_entries<W>() + 4 + 2 * ((n_d + 1) & ~1);
+  return u_entries<W>() + 4 + (kDiag ? 3 : 2) * ((n_d + 1) & ~1);
 }
 
 // f(slots, warps): the form for n_d columns and `cells` cells, as two integral constants; a warp per
@@ -46,13 +46,14 @@ void pair_rows_form(int n_d, int cells, int warp_dense, F f) {
 }
 
 // S: 32-column slots, n_d <= 32 S. vs: the cell's u_space doubles. fill(from, p1, t, n): the threads t of n
-// write V[from ..] to vs[0 ..], up to p1 (from: a multiple of four). diag(a, v): called by lane 0 of a warp with
-// each diagonal V[pair(a, a)].
-template <int S, int W, class Fill, class Diag>
-__device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* vs, const double* __restrict__ D,
-                                               double* __restrict__ U, Fill fill, Diag diag) {
+// write V[from ..] to vs[0 ..], up to p1 (from: a multiple of four). kDiag: returns where the diagonals
+// V[pair(a, a)] lie in shared memory, complete for the threads of the cell.
+template <int S, int W, bool kDiag, class Fill>
+__device__ __forceinline__ const double* pair_rows_to_u(int i, int ldN, int n_d, double* vs,
+                                                        const double* __restrict__ D, double* __restrict__ U,
+                                                        Fill fill) {
   constexpr int kThr = 32 * W, kOwn = (32 * S + kThr - 1) / kThr;
-  double *ds = vs + u_entries<W>() + 4, *rs = ds + ((n_d + 1) & ~1);
+  double *ds = vs + u_entries<W>() + 4, *rs = ds + ((n_d + 1) & ~1), *dv = rs + ((n_d + 1) & ~1);
   const int lane = threadIdx.x & 31, warp = W == 8 ? threadIdx.x >> 5 : 0, tid = W == 8 ? threadIdx.x : lane;
   auto sync = [&]() {
     if (W == 8) __syncthreads();
@@ -109,10 +110,10 @@ __device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* 
       sum2 = warp_sum(sum2);
       if (lane == 0) {
         rs[a] = sum;
-        diag(a, row[a]);
+        if (kDiag) dv[a] = row[a];
         if (two) {
           rs[e] = sum2;
-          diag(e, row2[e]);
+          if (kDiag) dv[e] = row2[e];
         }
       }
     }
@@ -124,7 +125,7 @@ __device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* 
 #pragma unroll
     for (int t = 0; t < S; t++)
       if (32 * t + lane < n_d) U[i + (size_t)(32 * t + lane) * ldN] = rs[32 * t + lane] + col[t];
-    return;
+    return dv;
   }
   double* cs = vs;  // [8][n_d] the warps' column sums
 #pragma unroll
@@ -137,6 +138,7 @@ __device__ __forceinline__ void pair_rows_to_u(int i, int ldN, int n_d, double* 
     for (int w = 0; w < 8; w++) u += cs[w * n_d + a];
     U[i + (size_t)a * ldN] = u;
   }
+  return dv;
 }
 
 }  // namespace gpl

@@ -60,3 +60,59 @@ def test_gradient_pairs_of_genes_far_apart(lo, hi, outlier):
     err = np.abs(got[0] - got[1])
     assert np.all(err <= K * tol.T[-M:] + 4 * U * (np.abs(got[1]) + K * size.T[-M:])), \
         float((err / (K * size.T[-M:])).max())
+
+
+def _psi(m, ds, beta):
+    m.set_beta(beta)
+    m.kernel_mats()
+    m.expand_delta()
+    m.irls_sweep(0, 0)
+    m.gram()
+    assert m.get_option("pair_form") & 1
+    return m.get("Psi").reshape(m.J, m.P, m.P)
+
+
+# the log of a gene's weight near one inducing point over the others', the genes that have it of 600 (on the
+# list's small and large tiles), cells per range (0: one range)
+@pytest.mark.parametrize("spread,n_out,cells", [(6.0, 60, 0), (10.0, 3, 0), (14.0, 60, 0), (14.0, 48, 512), (30.0, 49, 0),
+                                                (40.0, 3, 512), (40.0, 600, 0)])
+def test_gram_of_spread_weights(spread, n_out, cells):
+    N, G, M = 2500, 600, 64
+    ds, m = _context(N, G, M, Q=2)
+    with m:
+        m.set_option("pair_range_cells", cells)
+        ds.init.rho[:] = 0.2  # columns of few cells each
+        m.set_params(ds.init)
+        beta = 0.2 * np.random.default_rng(3).standard_normal((m.P, G))
+        for j in range(n_out):
+            beta[m.P - M + j % M, j] = spread
+        psi = _psi(m, ds, beta)
+        nd, P = m.n_dense(), m.P
+        W = m.get("W").reshape(-1, N)[:G]
+        D = m.get("Dm").reshape(nd, N).astype(np.longdouble)
+        prior = np.triu(m.get("DeltaInv").reshape(P, P).T)
+    prior = prior + np.triu(prior, 1).T
+    cols = np.array([0] + list(range(P - nd + 1, P)))
+    om = ds.init.Omega.astype(np.longdouble)
+    # 8 times the rms rounding of either form (the integer form's share, the chain's 0.15 sqrt(N) u) and a few
+    # roundings of the entry, by the scale sqrt(Psi_aa Psi_bb) of both
+    tol = 8 * _share(N) + 1.2 * np.sqrt(N) * U + 8 * U
+    for j in (0, 1, 2, n_out - 1, G // 2, G - 1):
+        ref = (D * (W[j].astype(np.longdouble) / om)) @ D.T + prior[np.ix_(cols, cols)]
+        d = np.sqrt(np.diag(ref))
+        err = np.abs(psi[j][np.ix_(cols, cols)] - ref) / np.outer(d, d)
+        assert np.all(err <= tol), (j, float(err.max() / U))
+
+
+def test_non_finite_gene_leaves_the_others():
+    """A gene whose weights overflow takes the FP64 form alone: the others keep their bits."""
+    N, G, M = 2500, 600, 64
+    ds, m = _context(N, G, M, Q=2)
+    with m:
+        beta = 0.2 * np.random.default_rng(3).standard_normal((m.P, G))
+        a = _psi(m, ds, beta).copy()
+        beta[0, 5] = 800.0
+        b = _psi(m, ds, beta)
+    assert not np.all(np.isfinite(b[5]))
+    keep = np.arange(G) != 5
+    assert np.all(np.isfinite(b[keep])) and np.array_equal(a[keep], b[keep])
