@@ -61,12 +61,13 @@ struct CrtState {
   int gram_cells = 0, grad_cells = 0;  // 0: that product stays with the DMMA form
   size_t bytes = 0;
   double *scales = nullptr, *balance = nullptr;
-  int *flag = nullptr, *err = nullptr;  // operands out of range (the DMMA form runs); a wait gave up
+  int* err = nullptr;    // a wait gave up
   int* cells = nullptr;  // the gradient's: [0] all cells, [1 + k] the k-th 128 cells go to the DMMA form
   // the Gram's: [0] all genes, [1] how many, [2 + j] gene j go to the DMMA form, those genes, and over
   // several ranges of cells the rounding of the diagonals so far (genes x dense columns)
   int *genes = nullptr, *list = nullptr;
   double* g_err = nullptr;
+  int* cols = nullptr;   // the genotype columns': [0] all genes, [1 + k] the k-th 128 genes go to the DMMA form
   int8_t *g_a = nullptr, *g_b = nullptr, *v_a = nullptr, *v_b = nullptr;
   uint8_t *g_out = nullptr, *v_out = nullptr;
   double* g_acc = nullptr;
@@ -378,7 +379,7 @@ void pair_release(Ctx* c);
 double pair_gram_cost(const Ctx* c, int n_pairs);  // of the DMMA Gram, in clocks per 16 cells
 int pair_prepare(Ctx* c);                 // column-pair list, 1/Omega, gathered S pairs, V rows
 int recip_omega(Ctx* c, const double** rOm);  // 1/Omega (0 past N), refreshed on every call
-int dgen_zt_u(Ctx* c, int mode, const double* u, double* out);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);
+int dgen_zt_u(Ctx* c, int mode, const double* u, double* out, const int* tiles = nullptr);          // DMMA forms of the cell x gene GEMMs (k_dgen.cu);
 int dgen_c1_tn(Ctx* c);
 int dgen_resid_gp(Ctx* c, const double* R, const double* B, double* G);  // cells x genes against the GP coefficients
 int dgen_c2(Ctx* c);                      // C2 (M x M adjoint of Kmm) up to its final combination
@@ -405,7 +406,9 @@ int launch_crt_uq(Ctx* c);
 int crt_error_flag(Ctx* c);
 bool crt_columns_faster(const Ctx* c, int L);    // Z^T diag(W/Omega) g of L per-cell columns there
 size_t crt_columns_work(const Ctx* c, int L);    // doubles of scratch that takes
-int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, bool* done);
+// T of L columns; gg: J x L sums of W g^2 / Omega; *left: the genes that are not done, none (0), those of the
+// 128s in CrtState::cols (1) or all (2)
+int launch_crt_columns(Ctx* c, int L, const double* G, const double* gg, double* T, double* work, int* left);
 bool tc_map_u8(CUtensorMap* m, void* ptr, uint64_t cols, uint64_t rows);  // 128 x 128 byte boxes, swizzled
 int launch_tc_gram(Ctx* c);               // dense block of every Psi_j on tensor cores
 int launch_tc_grad(Ctx* c);               // U = sum_j O_ij S_j[DD] d_i on tensor cores

@@ -30,6 +30,7 @@
 // ranges that fit the buffer the DMMA form uses for its pair products (at most 8 GiB).
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "gpl_internal.cuh"
 #include "pair_rows.cuh"
@@ -128,11 +129,11 @@ __device__ __forceinline__ bool crt_scale(double n2, double R, double* sc, doubl
 }
 
 // Where a gene goes that the integer form cannot take: onto the Gram's list (CrtState::genes), once, or
-// without a list into the flag for all.
+// without a list into the flag of its 128 (CrtState::cols).
 struct CrtGenes {
   int *state, *list;
   __device__ __forceinline__ void add(int j) const {
-    if (!list) atomicExch(state, 1);
+    if (!list) state[1 + (j >> 7)] = 1;
     else if (atomicExch(state + 2 + j, 1) == 0) list[atomicAdd(state + 1, 1)] = j;
   }
 };
@@ -818,20 +819,20 @@ int crt_prepare(Ctx* c) {
   CrtState& t = s.crt;
   if (!t.on) return GPL_OK;
   const size_t rows = (size_t)2 * (t.Jp + t.Pp + t.grad_cells), tiles = div_up(c->N, 128);
-  const size_t ints = 5 + tiles + 2 * (size_t)c->J, errs = t.gram_cells < c->N ? (size_t)c->J * c->n_d : 0;
+  const size_t ints = 5 + tiles + 2 * (size_t)c->J + div_up(c->J, 128), errs = t.gram_cells < c->N ? (size_t)c->J * c->n_d : 0;
   if (cudaMalloc((void**)&t.scales, sizeof(double) * (rows + 2 * t.Jp + errs)) != cudaSuccess ||
-      cudaMalloc((void**)&t.flag, ints * sizeof(int)) != cudaSuccess) {
+      cudaMalloc((void**)&t.err, ints * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     c->err = "device allocation failed: scales of the integer pair products";
     return GPL_ERR_ALLOC;
   }
   t.balance = t.scales + rows;  // of W, then of the pairs
-  t.err = t.flag + 1;
-  t.cells = t.flag + 2;
+  t.cells = t.err + 1;
   t.genes = t.cells + 1 + tiles;
   t.list = t.genes + 2 + c->J;
+  t.cols = t.list + c->J;
   t.g_err = t.balance + 2 * t.Jp;
-  GPL_TRY(c, cudaMemset(t.flag, 0, ints * sizeof(int)));
+  GPL_TRY(c, cudaMemset(t.err, 0, ints * sizeof(int)));
   int8_t* pool = reinterpret_cast<int8_t*>(s.V);
   // Gram: gene planes, pair planes, residues out, partial sums over the ranges
   t.g_a = pool;
@@ -859,7 +860,7 @@ int crt_prepare(Ctx* c) {
 void crt_release(Ctx* c) {
   CrtState& t = c->pr.crt;
   if (t.scales) cudaFree(t.scales);
-  if (t.flag) cudaFree(t.flag);
+  if (t.err) cudaFree(t.err);
   t = CrtState();
 }
 
@@ -994,7 +995,9 @@ int launch_crt_uq(Ctx* c) {
 
 // T[l][j][dcol a] = sum_i D_ia g_il W_ij / Omega_i: the Gram's operands and kernels with the products of the
 // dense columns and the L per-cell columns in place of the dense pairs, as many columns at a time as
-// the pairs' space holds.
+// the pairs' space holds. An entry's rounding (as in k_crt_psi; each range of cells has its part of it) is held
+// against sqrt(Psi_aa g^T diag(W/Omega) g), which bounds the sum of its terms' sizes; a gene with one
+// beyond its share sends its 128 genes to the DMMA form.
 __global__ void k_crt_column_pairs(int n_d, int rows, int2* __restrict__ pairs) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < rows) pairs[r] = make_int2(r % n_d, n_d + r / n_d);
@@ -1002,8 +1005,9 @@ __global__ void k_crt_column_pairs(int n_d, int rows, int2* __restrict__ pairs) 
 __global__ void __launch_bounds__(256) k_crt_t(int J, int P, int n_d, int rows, int64_t ldo, size_t plane,
                                                const uint8_t* __restrict__ in, const double* __restrict__ inv_j,
                                                const double* __restrict__ inv_p, const int* __restrict__ dcol,
-                                               int first, double* __restrict__ T, const int* __restrict__ flag) {
-  if (*flag) return;
+                                               int first, double unit, const double* __restrict__ root,
+                                               const double* __restrict__ gg, double* __restrict__ T, int* cols) {
+  if (*(const volatile int*)cols) return;
   const int j = blockIdx.x, r0 = (blockIdx.y * 256 + threadIdx.x) * 4;
   if (r0 >= rows) return;
   double v[4];
@@ -1013,10 +1017,24 @@ __global__ void __launch_bounds__(256) k_crt_t(int J, int P, int n_d, int rows, 
   for (int e = 0; e < 4; e++) {
     const int r = r0 + e;
     if (r >= rows) break;
-    double* t = T + ((size_t)(r / n_d) * J + j) * P + dcol[r % n_d];
+    const int l = r / n_d, a = r % n_d;
+    double* t = T + ((size_t)l * J + j) * P + dcol[a];
     const double x = v[e] * inv_p[r] * sj;
     *t = first ? x : *t + x;
+    if (!(unit * inv_j[j] * inv_p[r] <= root[(size_t)j * n_d + a] * sqrt(gg[j + (size_t)l * J]))) cols[1 + (j >> 7)] = 1;
   }
+}
+// root[j][a] = sqrt(Psi_j[dcol a, dcol a]) from the rows of its factor
+__global__ void __launch_bounds__(160) k_crt_roots(int P, int n_d, const int* __restrict__ dcol,
+                                                   const double* __restrict__ Psi, double* __restrict__ root) {
+  const int a = threadIdx.x, j = blockIdx.x;
+  if (a >= n_d) return;
+  const int r = dcol[a];
+  const double* L = Psi + (size_t)j * P * P + r;
+  double s = 0.0;
+#pragma unroll 4
+  for (int k = 0; k <= r; k++) s = fma(L[(size_t)k * P], L[(size_t)k * P], s);
+  root[(size_t)j * n_d + a] = sqrt(s);
 }
 
 // The two forms' times (us), by the rates measured at 30,000 x 1,000 with 132 dense columns: 330 per
@@ -1033,11 +1051,10 @@ bool crt_columns_faster(const Ctx* c, int L) {
 }
 size_t crt_columns_work(const Ctx* c, int L) {
   const int per = crt_column_group(c, L);
-  return (size_t)(c->n_d + per) * c->ldN + (size_t)per * c->n_d + 2;
+  return (size_t)(c->n_d + per) * c->ldN + (size_t)per * c->n_d + (size_t)c->J * c->n_d + 2;
 }
 
-// *done is false where an operand is not finite (nothing of T is to be used then).
-int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, bool* done) {
+int launch_crt_columns(Ctx* c, int L, const double* G, const double* gg, double* T, double* work, int* left) {
   PairState& s = c->pr;
   CrtState& t = s.crt;
   const int per = crt_column_group(c, L);
@@ -1047,13 +1064,17 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
   ProfScope ps(c, "zt_u");
   double* D = work + (reinterpret_cast<uintptr_t>(work) / sizeof(double) & 1);  // 16-byte aligned columns
   int2* pairs = reinterpret_cast<int2*>(D + (size_t)(c->n_d + per) * c->ldN);
+  double* root = D + (size_t)(c->n_d + per) * c->ldN + (size_t)per * c->n_d;
   const double R = crt_norm_limit();
   double *sc_j = t.scales, *inv_j = sc_j + t.Jp, *sc_p = inv_j + t.Jp, *inv_p = sc_p + t.Pp;
   double* part = reinterpret_cast<double*>(t.g_out);
   const size_t plane_a = (size_t)t.Jp * t.gram_cells, plane_b = (size_t)t.Pp * t.gram_cells;
   const size_t plane_o = (size_t)t.Jp * t.Pp, col = sizeof(double) * c->ldN;
   const int smem_n = (int)sizeof(double) * 32 * (c->n_d + per + 1);
-  GPL_TRY(c, cudaMemsetAsync(t.flag, 0, sizeof(int), c->stream));
+  const int tiles = div_up(c->J, 128);
+  GPL_TRY(c, cudaMemsetAsync(t.cols, 0, (1 + tiles) * sizeof(int), c->stream));
+  k_crt_roots<<<c->J, 160, 0, c->stream>>>(c->P, c->n_d, c->dcol_d, c->Psi, root);  // at most 144 dense columns
+  GPL_LAUNCHED(c, "k_crt_roots");
   GPL_TRY(c, cudaMemcpyAsync(D, c->Dm, col * c->n_d, cudaMemcpyDeviceToDevice, c->stream));
   GPL_TRY(c, cudaMemsetAsync(D + (size_t)c->n_d * c->ldN, 0, col * per, c->stream));
   k_crt_column_pairs<<<div_up(per * c->n_d, 256), 256, 0, c->stream>>>(c->n_d, per * c->n_d, pairs);
@@ -1064,7 +1085,7 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
                                  sizeof(double) * c->N, nl, cudaMemcpyDeviceToDevice, c->stream));
     for (int c0 = 0; c0 < c->N; c0 += t.gram_cells) {
       const int len = std::min(t.gram_cells, c->N - c0), kpad = up(len, kChunk);
-      k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, CrtGenes{t.flag, nullptr});
+      k_crt_norm_rows<<<c->J, 256, 0, c->stream>>>(c->W + c0, c->ldN, len, R, sc_j, inv_j, CrtGenes{t.cols, nullptr});
       GPL_LAUNCHED(c, "k_crt_norm_rows");
       const int gx = div_up(rows, 256 * kNormPairs);
       const int gy = std::max(1, std::min({div_up(len, 64), 592 / gx, 256}));
@@ -1073,25 +1094,27 @@ int launch_crt_columns(Ctx* c, int L, const double* G, double* T, double* work, 
       k_crt_norm_pairs<<<dim3(gx, ny), 256, smem_n, c->stream>>>(c->ldN, cols, c0, c0 + len, cper, rows, pairs, D, rOm,
                                                                 part);
       GPL_LAUNCHED(c, "k_crt_norm_pairs");
-      k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.flag, 31);
+      k_crt_scales<<<div_up(rows, 256), 256, 0, c->stream>>>(rows, ny, part, R, sc_p, inv_p, t.cols, 31);
       GPL_LAUNCHED(c, "k_crt_scales");
       k_crt_conv_rows<<<dim3(c->J, div_up(kpad, 2048)), 256, 0, c->stream>>>(c->W + c0, c->ldN, len, kpad,
-                                                                            t.gram_cells, plane_a, sc_j, t.g_a, t.flag);
+                                                                            t.gram_cells, plane_a, sc_j, t.g_a, t.cols);
       GPL_LAUNCHED(c, "k_crt_conv_rows");
       k_crt_conv_pairs<<<dim3(div_up(kpad, 2048), div_up(rows, kConvPairs)), 256, 0, c->stream>>>(
-          c->ldN, c0, len, kpad, t.gram_cells, plane_b, rows, pairs, D, rOm, sc_p, t.g_b, t.flag);
+          c->ldN, c0, len, kpad, t.gram_cells, plane_b, rows, pairs, D, rOm, sc_p, t.g_b, t.cols);
       GPL_LAUNCHED(c, "k_crt_conv_pairs");
-      if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.flag))) return rc;
+      if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.cols))) return rc;
       k_crt_t<<<dim3(c->J, div_up(rows, 1024)), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
                                                                     inv_j, inv_p, c->dcol_d, c0 == 0,
-                                                                    T + (size_t)l0 * c->J * c->P, t.flag);
+                                                                    0.41 * R / crt_share(c->N) * c->N / len, root,
+                                                                    gg + (size_t)l0 * c->J,
+                                                                    T + (size_t)l0 * c->J * c->P, t.cols);
       GPL_LAUNCHED(c, "k_crt_t");
     }
   }
-  int flag = 0;
-  GPL_TRY(c, cudaMemcpyAsync(&flag, t.flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  std::vector<int> out(1 + tiles);
+  GPL_TRY(c, cudaMemcpyAsync(out.data(), t.cols, sizeof(int) * out.size(), cudaMemcpyDeviceToHost, c->stream));
   if ((rc = crt_error_flag(c))) return rc;  // waits for the stream
-  *done = flag == 0;
+  *left = out[0] ? 2 : std::find(out.begin(), out.end(), 1) != out.end() ? 1 : 0;
   return GPL_OK;
 }
 

@@ -338,10 +338,11 @@ struct EpPsiDD {  // Psi_z at (dcol r, dcol c) and its mirror, plus DeltaInv; r 
 
 // bvec[dcol[a] + j*P] = sum_z part[z][a][j]
 __global__ void k_reduce_bvec(int n_d, int J, int P, int nz, const int* __restrict__ dcol,
-                              const double* __restrict__ part, double* __restrict__ bvec) {
+                              const double* __restrict__ part, double* __restrict__ bvec,
+                              const int* __restrict__ tiles) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const int a = blockIdx.y;
-  if (j >= J) return;
+  if (j >= J || (tiles && !tiles[j >> 7])) return;
   double s = 0.0;
   for (int z = 0; z < nz; z++) s += part[((size_t)z * n_d + a) * J + j];
   bvec[dcol[a] + (size_t)j * P] = s;
@@ -439,8 +440,10 @@ int with_row_tiles(int rows, F f) {
 template <int MODE, int MT>
 __global__ void __launch_bounds__(256, 1)
     k_zt_u(int m, int n, int N, int ldN, int per, const double* __restrict__ D, const double* __restrict__ W,
-           const double* __restrict__ U, const double* __restrict__ rOm, double* __restrict__ part) {
+           const double* __restrict__ U, const double* __restrict__ rOm, double* __restrict__ part,
+           const int* __restrict__ tiles) {
   extern __shared__ __align__(16) double zs[];
+  if (tiles && !tiles[blockIdx.y]) return;  // gene tiles that are not asked for
   const int tid = threadIdx.x, wn = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   constexpr int kRows = MT * 16, kStage = zt_stage(MT);
   const int m0 = blockIdx.x * kRows, n0 = blockIdx.y * kZtBN, z = blockIdx.z;
@@ -541,7 +544,8 @@ static int zt_splits(const Ctx* c, int rows) {
   return split_count(div_up(c->J, kZtBN) * div_up(c->n_d, rows), c->sm_count);
 }
 
-int dgen_zt_u(Ctx* c, int mode, const double* u, double* out) {
+// tiles: a flag for every 128 genes (nullptr: all of them)
+int dgen_zt_u(Ctx* c, int mode, const double* u, double* out, const int* gene_tiles) {
   if (mode == 2 && c->n_d > 144) return GPL_ERR_ARG;
   const double* rOm = nullptr;
   if (mode != 1) {
@@ -562,10 +566,10 @@ int dgen_zt_u(Ctx* c, int mode, const double* u, double* out) {
     auto* fn = mode == 0 ? chain ? k_zt_u<3, MT> : k_zt_u<0, MT> : mode == 1 ? k_zt_u<1, MT> : k_zt_u<2, MT>;
     GPL_TRY(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, zt_smem(MT)));
     fn<<<dim3(mtiles, tiles, S), 256, zt_smem(MT), c->stream>>>(c->n_d, c->J, c->N, c->ldN, per, c->Dm, c->W, u, rOm,
-                                                               c->part);
+                                                               c->part, gene_tiles);
     GPL_LAUNCHED(c, "k_zt_u");
     dim3 g2(div_up(c->J, 256), c->n_d);
-    k_reduce_bvec<<<g2, 256, 0, c->stream>>>(c->n_d, c->J, c->P, S, c->dcol_d, c->part, out);
+    k_reduce_bvec<<<g2, 256, 0, c->stream>>>(c->n_d, c->J, c->P, S, c->dcol_d, c->part, out, gene_tiles);
     GPL_LAUNCHED(c, "k_reduce_bvec");
     return GPL_OK;
   });

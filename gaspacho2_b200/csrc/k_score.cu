@@ -221,10 +221,13 @@ int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratc
   double* T = Gg + (size_t)L * c->ldN;
   T += (T - scratch) & 1;
   int rc;
-  bool done = false;
-  if (crt && (rc = launch_crt_columns(c, L, G, T, scratch + score_work(c, L), &done))) return rc;
-  for (int l = 0; l < L && !done; l++)
-    if ((rc = dgen_zt_u(c, 2, G + (size_t)l * N, T + (size_t)l * J * P))) {
+  k_score_cols<<<dim3(div_up(c->N, 256), L), 256, 0, c->stream>>>(c->N, L, G, c->Omega, G2, Gt);
+  GPL_LAUNCHED(c, "k_score_cols");
+  if ((rc = dgen_weighted_colsums(c, G2, 2 * L, C))) return rc;
+  int left = 2;
+  if (crt && (rc = launch_crt_columns(c, L, G, C, T, scratch + score_work(c, L), &left))) return rc;
+  for (int l = 0; l < L && left; l++)
+    if ((rc = dgen_zt_u(c, 2, G + (size_t)l * N, T + (size_t)l * J * P, left == 1 ? c->pr.crt.cols + 1 : nullptr))) {
       if (rc == GPL_ERR_ARG) c->err = "per-cell Z^T u takes at most 144 dense columns";
       return rc;
     }
@@ -237,9 +240,6 @@ int launch_score_stats(Ctx* c, int L, const double* G, double* S, double* scratc
     GPL_LAUNCHED(c, "k_score_levels");
   }
   if ((rc = launch_quad(c, c->J, L, c->Psi, T, P, J * P, td))) return rc;
-  k_score_cols<<<dim3(div_up(c->N, 256), L), 256, 0, c->stream>>>(c->N, L, G, c->Omega, G2, Gt);
-  GPL_LAUNCHED(c, "k_score_cols");
-  if ((rc = dgen_weighted_colsums(c, G2, 2 * L, C))) return rc;
   k_score_counts<<<c->J, 256, 0, c->stream>>>(c->J, L, c->cell, c->gptr, c->gvalid, c->cnt, Gt, sp);
   GPL_LAUNCHED(c, "k_score_counts");
   k_score_final<<<dim3(div_up(c->J, 256), L), 256, 0, c->stream>>>(c->J, L, sp, C, td, c->phi, S);

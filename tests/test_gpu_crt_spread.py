@@ -116,3 +116,26 @@ def test_non_finite_gene_leaves_the_others():
     assert not np.all(np.isfinite(b[5]))
     keep = np.arange(G) != 5
     assert np.all(np.isfinite(b[keep])) and np.array_equal(a[keep], b[keep])
+
+
+@pytest.mark.parametrize("spread", [0.0, 14.0, 20.0, 23.0])
+def test_genotype_columns_of_spread_weights(spread):
+    """Columns that are zero where three genes have their mass: in one call (32 columns, the integer form) and
+    one by one (the FP64 form). The variance that is left of g^T diag(w) g is at least 1e-3 of it."""
+    N, G, M, L = 2500, 600, 64, 32
+    ds, m = _context(N, G, M, Q=2)
+    with m:
+        ds.init.rho[:] = 0.2
+        m.set_params(ds.init)
+        beta = 0.2 * np.random.default_rng(3).standard_normal((m.P, G))
+        beta[m.P - M, [5, 200, 599]] = spread
+        m.set_beta(beta)
+        m.kernel_mats()
+        m.expand_delta()
+        m.irls_sweep(0, 0)
+        K = m.get("Knm").reshape(M, N)[0]
+        geno = np.random.default_rng(7).normal(1.0, 0.7, (N, L)) * (K < 1e-3)[:, None]
+        S = m.score_stats(geno)
+        one = np.concatenate([m.score_stats(geno[:, k:k + 1]) for k in range(L)], 1)
+    assert np.all(np.isfinite(one))
+    assert np.all(np.abs(S - one) <= 1e-9 * (1.0 + np.abs(one)))
