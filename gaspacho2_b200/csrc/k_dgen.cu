@@ -1198,7 +1198,9 @@ static size_t part_bound(const Ctx* c) {
   size_t n = std::max(MM * (n1 + n2 + n3), (size_t)gram_splits(c) * n_d * n_d);
   with_row_tiles(c->n_d, [&](auto mt) -> int {
     n = std::max(n, (size_t)zt_splits(c, 16 * decltype(mt)::value) * n_d * J);
-    if (c->n_grp) n = std::max(n, (size_t)c->n_grp * group_runs(c, c->J, c->n_d, 16 * decltype(mt)::value) * J * n_d);
+    // unsplit group sums go straight to their place (with many groups that is gigabytes)
+    const int runs = c->n_grp ? group_runs(c, c->J, c->n_d, 16 * decltype(mt)::value) : 1;
+    if (runs > 1) n = std::max(n, (size_t)c->n_grp * runs * J * n_d);
     return GPL_OK;
   });
   with_row_tiles(c->n_d + 1, [&](auto mt) -> int {
