@@ -361,7 +361,6 @@ int launch_solve_batched(Ctx* c, const double* L, int n, int64_t lstride, const 
                          double* X, int64_t xstride, int batch);
 int launch_inverse_batched(Ctx* c);      // PsiInv from Psi's factor
 int launch_potrf_panels(Ctx* c, double* A, int n, int batch, int64_t stride);  // 32-column panels, DMMA
-constexpr int kPotrfMaxP = 288;           // widest matrix of the panel Cholesky
 int launch_inverse_panels(Ctx* c);       // the same in 32-column panels with DMMA block products
 int launch_irls_tail(Ctx* c, int jtr, int ctas_per_sm);  // persistent per-gene IRLS tail; GPL_ERR_ARG:
                                                           // P beyond the panel Cholesky's range

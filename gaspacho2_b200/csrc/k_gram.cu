@@ -292,12 +292,11 @@ int launch_gram(Ctx* c, bool unweighted) {
 
 int launch_chol_batched(Ctx* c, double* A, int n, int batch, int64_t stride) {
   ProfScope ps(c, "chol");
-  if (c->one_order && n > kPotrfMaxP) {  // the row-block kernel takes its sums in another order
-    k_chol<<<batch, 256, 0, c->stream>>>(A, n, stride, 0);
-    GPL_LAUNCHED(c, "k_chol");
-    return GPL_OK;
-  }
-  return launch_potrf_panels(c, A, n, batch, stride);
+  const int rc = launch_potrf_panels(c, A, n, batch, stride);
+  if (rc != GPL_ERR_ARG) return rc;
+  k_chol<<<batch, 256, 0, c->stream>>>(A, n, stride, 0);
+  GPL_LAUNCHED(c, "k_chol");
+  return GPL_OK;
 }
 
 int launch_chol_single(Ctx* c, double* A, int n) {

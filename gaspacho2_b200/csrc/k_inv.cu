@@ -35,9 +35,10 @@ constexpr int IB = 32;  // block size
 constexpr int IS = 36;  // shared row stride (doubles): conflict-free fragment loads
 constexpr int NB = 3;   // buffers of the inverse's block stream
 constexpr int CW = 8;   // finished columns per chunk of the Cholesky's panel update
-// Largest P each kernel is launched for (kPotrfMaxP: gpl_internal.cuh). k_potrf_panel's update covers 256 rows of a panel
+// Largest P each kernel is launched for. k_potrf_panel's update covers 256 rows of a panel
 // (8 warps x 2 row tiles of 16), so its panels below the first may hold at most 256 rows:
 // P <= 288. The inverse panels hold any P their shared memory admits (P <= 640 within 220 KiB).
+constexpr int kPotrfMaxP = 288;
 // With half the threads (128 rows below the first panel), up to four CTAs per SM hide more of a
 // panel's latency.
 constexpr int kPotrfHalfP = 160;
@@ -587,9 +588,12 @@ __global__ void __launch_bounds__(256, 2) k_potrf_rows(double* __restrict__ Psi,
     for (int e = tid; e < P * P; e += 256) A[e] = 0.0;
 }
 
+// GPL_ERR_ARG within an OrderScope beyond the panel kernel's range: the row-block kernel takes its sums in
+// another order than the entry-by-entry form.
 int launch_potrf_panels(Ctx* c, double* A, int n, int batch, int64_t stride) {
   const int ns = potrf_buffers(n, 0), smem = potrf_panel_smem(n, ns);
   if (n > kPotrfMaxP || smem > 220 * 1024) {
+    if (c->one_order) return GPL_ERR_ARG;
     GPL_TRY(c, cudaFuncSetAttribute(k_potrf_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem));
     GPL_TRY(c, cudaFuncSetAttribute(k_potrf_rows, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     k_potrf_rows<<<batch, 256, kRowsSmem, c->stream>>>(A, n, stride);
