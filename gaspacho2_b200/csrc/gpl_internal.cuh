@@ -301,8 +301,7 @@ int launch_kernel_cells(Ctx* c);         // Knm, KinvKmn and titsias at a new X,
 int launch_expand_delta(Ctx* c);         // DeltaInv (upper + diag)
 int launch_chol_single(Ctx* c, double* A, int n);  // choldc on one n x n matrix
 // k_groups.cu
-int launch_group_sums(Ctx* c, int mode);  // 0: S (W/Omega); 1: S unweighted (gene 0); 2: T of y0; 3: T of nu;
-                                          // 4: T of a per-cell u (zt_u_src)
+int launch_group_sums(Ctx* c, int mode);  // 0: S (W/Omega); 1: S unweighted (gene 0); 2: T of y0; 3: T of nu
 int launch_assemble_psi(Ctx* c, int J);   // categorical rows/columns of Psi from the group sums
 int launch_assemble_b(Ctx* c, double* out);  // categorical entries of Z^T u (P x J) from the group sums
 int launch_group_tables(Ctx* c);          // per (gene, group) categorical blocks of Psi^{-1}
@@ -346,8 +345,7 @@ int launch_eta_dmma(Ctx* c, const double* B, double* out);
 // row stride of the per-group level sums (groups x genes): J rounded up to even
 inline int lvt_ld(int J) { return J + (J & 1); }
 int launch_zt_u(Ctx* c, int mode);       // bvec = Z^T u; mode 0: u = W/Omega*Nu; 1: init response
-int launch_zt_u_ex(Ctx* c, int mode, const double* u, double* out);  // the same for another u / output;
-                                                                      // mode 2: u is one value per cell
+int launch_zt_u_ex(Ctx* c, int mode, const double* u, double* out);  // the same for another u / output
 int solve_refined(Ctx* c, const double* b, double* x, bool dinv_factored = false);  // Psi_j x = b; FP64-residual
                                                         // refinement in the precision form
 int launch_init_response(Ctx* c);        // scratch = log((y+0.05)/ls) or log(0.05/ls)
@@ -364,7 +362,6 @@ int launch_potrf_panels(Ctx* c, double* A, int n, int batch, int64_t stride);  /
 int launch_inverse_panels(Ctx* c);       // the same in 32-column panels with DMMA block products
 int launch_irls_tail(Ctx* c, int jtr, int ctas_per_sm);  // persistent per-gene IRLS tail; GPL_ERR_ARG:
                                                           // P beyond the panel Cholesky's range
-int launch_inverse_single(Ctx* c, const double* L, int n, double* tmp, double* out);
 int launch_cholinv(Ctx* c, const double* L, int n, double* out);  // (L L^T)^{-1}, k_kmats.cu
 // choldc's order on one matrix whose first `diag` rows are diagonal; the launch's own status
 cudaError_t launch_chol_exact_raw(cudaStream_t st, double* A, int n, int diag = 0);

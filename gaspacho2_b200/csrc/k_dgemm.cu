@@ -622,7 +622,7 @@ int launch_v_to_u_rows(Ctx* c, int c0, int c1, const double* D, const double* V,
   PairState& s = c->pr;
   ProfScope ps(c, "v_to_u");
   if (c->n_d > kUMaxDense) {
-    const int grid = std::min(c1 - c0, 148 * 8);
+    const int grid = std::min(c1 - c0, 8 * c->sm_count);
     k_v_to_u_wide<<<grid, 256, sizeof(double) * c->n_d, c->stream>>>(c->N, c->ldN, c->n_d, s.pairs_pad, c0, c1, D,
                                                                     V, c->U);  // never gated: crt_plan
     GPL_LAUNCHED(c, "k_v_to_u_wide");

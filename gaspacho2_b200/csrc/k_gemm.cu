@@ -346,11 +346,10 @@ int launch_zt_u_ex(Ctx* c, int mode, const double* u, double* out) {
   {
     ProfScope ps(c, "zt_u");
     const int rc = dgen_zt_u(c, mode, u, out);
-    if (rc == GPL_ERR_ARG) c->err = "per-cell Z^T u takes at most 144 dense columns";
     if (rc != GPL_OK) return rc;
   }
-  c->zt_u_src = (mode == 2 || (mode == 0 && u != c->Nu)) ? u : nullptr;
-  int rc = launch_group_sums(c, mode == 0 ? 3 : mode == 2 ? 4 : 2);
+  c->zt_u_src = mode == 0 && u != c->Nu ? u : nullptr;
+  int rc = launch_group_sums(c, mode == 0 ? 3 : 2);
   c->zt_u_src = nullptr;
   if (rc) return rc;
   return launch_assemble_b(c, out);

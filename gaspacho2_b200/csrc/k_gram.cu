@@ -358,12 +358,5 @@ int launch_inverse_batched(Ctx* c) {
   return GPL_OK;
 }
 
-int launch_inverse_single(Ctx* c, const double* L, int n, double* tmp, double* out) {
-  k_trtri<<<1, 256, 0, c->stream>>>(L, n, 0, tmp);
-  GPL_LAUNCHED(c, "k_trtri");
-  k_lauum<<<1, 256, 0, c->stream>>>(tmp, n, 0, out);
-  GPL_LAUNCHED(c, "k_lauum");
-  return GPL_OK;
-}
 
 }  // namespace gpl

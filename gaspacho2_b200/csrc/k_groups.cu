@@ -26,7 +26,7 @@
 namespace gpl {
 
 // T[j][g] = sum_{i in g} w_ij u_ij, one warp per (gene, group); mode 0: w = W/Omega, u = nu (W and
-// 1/Omega read in group order); mode 2: w = 1, u = y0 (scratch); mode 4: u one value per cell.
+// 1/Omega read in group order); mode 2: w = 1, u = y0 (scratch).
 template <int MODE>
 __global__ void k_group_t(int ldN, int J, int n_grp, const int* __restrict__ gcells, const int* __restrict__ gstart,
                           const double* __restrict__ Wg, const double* __restrict__ rOmg,
@@ -36,7 +36,7 @@ __global__ void k_group_t(int ldN, int J, int n_grp, const int* __restrict__ gce
   const int lane = threadIdx.x & 31;
   if (j >= J) return;
   const int c0 = gstart[g], c1 = gstart[g + 1];
-  const double *Wj = Wg + (size_t)j * ldN, *Uj = MODE == 4 ? U : U + (size_t)j * ldN;
+  const double *Wj = Wg + (size_t)j * ldN, *Uj = U + (size_t)j * ldN;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (int k0 = c0 + lane; k0 < c1; k0 += 128) {
     double v[4];
@@ -99,9 +99,6 @@ int launch_group_sums(Ctx* c, int mode) {
   if (mode == 2)
     k_group_t<2><<<g, 256, 0, c->stream>>>(c->ldN, c->J, c->n_grp, c->gcells_d, c->gstart_d, c->Wg, c->rOmg,
                                            c->scratch, c->gT);
-  else if (mode == 4)  // u per cell, the same for every gene
-    k_group_t<4><<<g, 256, 0, c->stream>>>(c->ldN, c->J, c->n_grp, c->gcells_d, c->gstart_d, c->Wg, c->rOmg,
-                                           c->zt_u_src, c->gT);
   else
     k_group_t<0><<<g, 256, 0, c->stream>>>(c->ldN, c->J, c->n_grp, c->gcells_d, c->gstart_d, c->Wg, c->rOmg,
                                            c->zt_u_src ? c->zt_u_src : c->Nu, c->gT);

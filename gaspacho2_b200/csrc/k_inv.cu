@@ -304,7 +304,7 @@ __device__ __forceinline__ bool factor_diagonal(double* Ap, int SP, int ncol, do
 // diagonal block. 3,000 matrices of P = 232: 3.1 -> 1.93 ms; 2,000 of 69: 0.28 -> 0.19 ms; 1,000 of
 // 285: 2.4 -> 1.01 ms. Each entry's operations and their order are the same.
 template <int T>
-__device__ __forceinline__ void potrf_panel_one(double* A, int P, int ns, double* sm, int& fail) {
+__device__ __forceinline__ void potrf_panel_one(double* A, int P, int ns, int sms, double* sm, int& fail) {
   const int rows_pad = max(IB, (P + 15) / 16 * 16);
   const int SP = rows_pad + 2, space = ns * CW * (rows_pad + 4);
   double* Ap = sm;                          // [32][SP]: the panel, column cc, row r
@@ -312,7 +312,7 @@ __device__ __forceinline__ void potrf_panel_one(double* A, int P, int ns, double
   double* Rd = La + space;                  // [32] reciprocals of the diagonal
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const bool pairs = (P & 1) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
-  const int dw = (blockIdx.x / 148) & 3;  // a CTA's neighbours on its SM were launched about 148 blocks apart
+  const int dw = (blockIdx.x / sms) & 3;  // a CTA's neighbours on its SM were launched about a block per SM apart
   if (tid == 0) fail = 0;
   // the panel that copies are issued for: its first row, the chunks' stride, columns and buffers that
   // the space holds at its height, and the next chunk to load
@@ -436,10 +436,11 @@ __device__ __forceinline__ void potrf_panel_one(double* A, int P, int ns, double
 }
 
 template <int T>
-__global__ void __launch_bounds__(T, 512 / T) k_potrf_panel(double* __restrict__ Psi, int P, int64_t stride, int ns) {
+__global__ void __launch_bounds__(T, 512 / T) k_potrf_panel(double* __restrict__ Psi, int P, int64_t stride, int ns,
+                                                             int sms) {
   extern __shared__ __align__(16) double sm[];
   __shared__ int fail;
-  potrf_panel_one<T>(Psi + (size_t)blockIdx.x * stride, P, ns, sm, fail);
+  potrf_panel_one<T>(Psi + (size_t)blockIdx.x * stride, P, ns, sms, sm, fail);
 }
 
 int potrf_panel_smem(int P, int ns) {
@@ -603,7 +604,7 @@ int launch_potrf_panels(Ctx* c, double* A, int n, int batch, int64_t stride) {
   auto* kernel = n <= kPotrfHalfP ? k_potrf_panel<128> : k_potrf_panel<256>;
   GPL_TRY(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   GPL_TRY(c, cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  kernel<<<batch, n <= kPotrfHalfP ? 128 : 256, smem, c->stream>>>(A, n, stride, ns);
+  kernel<<<batch, n <= kPotrfHalfP ? 128 : 256, smem, c->stream>>>(A, n, stride, ns, c->sm_count);
   GPL_LAUNCHED(c, "k_potrf_panel");
   return GPL_OK;
 }
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(256, 2)
                 const double* __restrict__ titsias, const int32_t* __restrict__ cell,
                 const int64_t* __restrict__ gptr, const int32_t* __restrict__ gvalid,
                 const double* __restrict__ cnt, double* __restrict__ lkhds, const int* __restrict__ order,
-                int* __restrict__ head, int ns) {
+                int* __restrict__ head, int ns, int sms) {
   extern __shared__ __align__(16) double sm[];
   __shared__ int fail, next;
   __shared__ double sh[32];
@@ -670,7 +671,7 @@ __global__ void __launch_bounds__(256, 2)
   double* sb = y + P;
   double* dg = sb + P;  // the factor's diagonal
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  const int sw = (blockIdx.x / 148) & 3;  // the solving warp: not on the same SM partition as the neighbour's
+  const int sw = (blockIdx.x / sms) & 3;  // the solving warp: not on the same SM partition as the neighbour's
   const int64_t PP = (int64_t)P * P;
   for (;;) {
     __syncthreads();  // the previous gene's shared values are no longer read
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(256, 2)
     if (q >= J) break;
     const int j = order[q];
     double* L = Psi + (size_t)j * PP;
-    potrf_panel_one<256>(L, P, ns, sm, fail);
+    potrf_panel_one<256>(L, P, ns, sms, sm, fail);
     __syncthreads();
     // 2. (L L^T) x = b_j, one warp, in k_solve's operation order (lane l updates the rows
     // k + 1 + l + 32 m of column k, and sums the rows i + 1 + l + 32 m of row i's column). The columns
@@ -832,7 +833,7 @@ int launch_irls_tail(Ctx* c, int jtr, int ctas_per_sm) {
   k_irls_tail<<<grid, 256, smem, c->stream>>>(c->J, c->N, c->ldN, P, c->p, r, c->vcomp ? 1.0 : kWt, c->Psi, c->bvec,
                                               c->sol, c->Beta, c->phi, c->W, c->Nu, c->Omega, c->delta,
                                               c->titsias, c->cell, c->gptr, c->gvalid, c->cnt, c->lkhds,
-                                              c->gene_order_d, c->queue_head_d, ns);
+                                              c->gene_order_d, c->queue_head_d, ns, c->sm_count);
   GPL_LAUNCHED(c, "k_irls_tail");
   return GPL_OK;
 }

@@ -102,7 +102,9 @@ GPL_API int gpl_set_precision(gpl_ctx* ctx, int precision);
  *   "graph_replays"     (read only) graph launches so far
  *   "pair_form"         (read only) the FP64 column-pair products that run in integer arithmetic
  *                       modulo fourteen moduli: 1 the Gram, 2 the gradient's, added (0 before
- *                       the first of them)
+ *                       the first of them). Genes and cells that it would lose digits of take the
+ *                       FP64 form by themselves, and so do the undamped sweeps of gpl_de_irls and
+ *                       gpl_vc_fit
  *   "fused_tail"        1: each IRLS sweep's per-gene tail (cholPsi, the solve and coefficient
  *                       update of getBetaPhi, getLkhdPois: ggplvm.cu:683-692, 418-464, 703-724)
  *                       runs as one persistent launch whose CTAs take genes from a queue ordered
@@ -115,6 +117,7 @@ GPL_API int gpl_set_precision(gpl_ctx* ctx, int precision);
  *                       each candidate on the context's own
  *                       launches (every candidate gives the same bits); the choices are kept for
  *                       the process per problem shape. Graphs are captured once all are chosen.
+ *                       Products in integer arithmetic (pair_form) have no such choice.
  *                       Default 0. */
 GPL_API int gpl_set_option(gpl_ctx* ctx, const char* name, int64_t value);
 GPL_API int gpl_get_option(const gpl_ctx* ctx, const char* name, int64_t* value);
