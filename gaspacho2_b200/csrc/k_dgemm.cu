@@ -126,9 +126,11 @@ constexpr int kGramPsi = 0;  // one range: Psi_j[mk, ml] = Psi_j[ml, mk] = G + D
 constexpr int kGramSet = 1;  // first of several ranges: Gacc[p * J + j] = G
 constexpr int kGramAdd = 2;  // later ranges: Gacc[p * J + j] += G
 
-// Output tiles of TM pairs x TN genes, WM x WN warps. An entry is one chain of DMMAs over the cells whatever
-// the tile, so the tile's size changes no bits; a CTA's time is its tile's multiply-adds for every cell,
-// so few pairs or genes, or a last wave that is nearly empty, want small tiles (launch_pair_gram).
+// Output tiles of TM pairs x TN genes, WM x WN warps. A CTA's time is its tile's multiply-adds for every cell,
+// so few pairs or genes, or a last wave that is nearly empty, want small tiles (launch_pair_gram). An entry is one
+// chain of DMMAs over the cells, whatever the tile, or (kRuns, the small tiles outside an OrderScope) the sum of
+// chains of 128 cells, whose rounding is what is left of the chain's: 4e-16 to 6e-16 of the diagonal (rms) at 1,274
+// to 2,000 cells, 6e-17 in runs, in the same time.
 template <int TM, int TN>
 struct GramTile {
   static constexpr int WM = TM / TN >= 4 ? 4 : 2, WN = 8 / WM;
@@ -147,8 +149,8 @@ struct GramGenes {
   __device__ __forceinline__ int gene(int k) const { return !state || state[0] ? k : list[k]; }
 };
 
-template <int TM, int TN>
-__global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
+template <int TM, int TN, bool kRuns>
+__global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : kRuns && TN == 64 ? 2 : 3)
     k_pair_gram(int N, int ldN, int J, int P, int c0, int c1, int pairs_pad, int n_pairs, int mode,
                 const double* __restrict__ A, const int2* __restrict__ pairs, const int* __restrict__ dcol,
                 const double* __restrict__ W, const double* __restrict__ Dinv, double* __restrict__ Psi,
@@ -200,13 +202,13 @@ __global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
       }
     };
 
-    double acc[MT][NT][4];
+    double acc[MT][NT][4], sum[MT][NT][4];
 #pragma unroll
     for (int x = 0; x < MT; x++)
 #pragma unroll
       for (int y = 0; y < NT; y++)
 #pragma unroll
-        for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
+        for (int z = 0; z < 4; z++) acc[x][y][z] = sum[x][y][z] = 0.0;
 
     // three stages, one barrier per slice (as k_pair_v)
     load(0, 0);
@@ -236,6 +238,17 @@ __global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
 #pragma unroll
           for (int nt = 0; nt < NT; nt++) dmma_16x8x4(acc[mt][nt], a[mt][0], a[mt][1], b[nt]);
       }
+      if (kRuns && ((s & 7) == 7 || s + 1 == nsl)) {
+#pragma unroll
+        for (int x = 0; x < MT; x++)
+#pragma unroll
+          for (int y = 0; y < NT; y++)
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+              sum[x][y][z] += acc[x][y][z];
+              acc[x][y][z] = 0.0;
+            }
+      }
     }
     cp_async_wait<0>();
 
@@ -259,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, TM == 128 ? 1 : 3)
           for (int e = 0; e < 2; e++) {
             if (j0 + (wn * NT + nt) * 8 + 2 * t + e >= n_j) continue;
             const int j = genes.gene(j0 + (wn * NT + nt) * 8 + 2 * t + e);
-            const double v = acc[mt][nt][h * 2 + e];
+            const double v = kRuns ? sum[mt][nt][h * 2 + e] : acc[mt][nt][h * 2 + e];
             if (mode == kGramPsi) {
               double* Pj = Psi + (size_t)j * P * P;
               Pj[mk + ml * P] = v + dv;
@@ -473,9 +486,11 @@ int pair_prepare(Ctx* c) {
     c->err = "device allocation failed: pair Gram accumulator";
     return GPL_ERR_ALLOC;
   }
-  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<128, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<128, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   GramTile<128, 128>::smem));
-  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<64, 64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  GramTile<64, 64>::smem));
+  GPL_TRY(c, cudaFuncSetAttribute(k_pair_gram<64, 64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   GramTile<64, 64>::smem));
   GPL_TRY(c, cudaFuncSetAttribute(k_pair_v, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_v));
   const int rc = crt_prepare(c);
@@ -552,7 +567,8 @@ int launch_pair_gram(Ctx* c) {
     TuneScope ts(c, one ? tu : nullptr);
     auto run = [&](auto tm, auto tn, int most, const GramGenes& genes) {
       constexpr int TM = decltype(tm)::value, TN = decltype(tn)::value;
-      k_pair_gram<TM, TN><<<std::min(most, div_up(s.n_pairs, TM) * div_up(c->J, TN)), kThreads, GramTile<TM, TN>::smem,
+      auto* fn = TM == 128 || c->one_order ? k_pair_gram<TM, TN, false> : k_pair_gram<TM, TN, TM != 128>;
+      fn<<<std::min(most, div_up(s.n_pairs, TM) * div_up(c->J, TN)), kThreads, GramTile<TM, TN>::smem,
                             c->stream>>>(c->N, c->ldN, c->J, c->P, c0, c1, s.pairs_pad, s.n_pairs, mode, s.V, s.pairs,
                                          c->dcol_d, c->W, c->DeltaInv, c->Psi, s.Gacc, gm, genes);
     };
