@@ -7,15 +7,20 @@
 // C[m, n] = sum_k A[m, k] B[n, k] in FP64. Row m of A is scaled by a power of two 2^s so that its
 // 2-norm is at most R = sqrt(0.48 P), P the product of the moduli (2^110.5), and rounded to integers;
 // rows of B the same way. By Cauchy-Schwarz the integer sum lies within +-0.48 P, so its residues
-// modulo the p_l determine it exactly: the only error of the whole sum is the rounding of the
-// operands, 2^-55 of a row's norm per entry, and of the final value to FP64. A chain of FP64
-// multiply-adds (the DMMA form) rounds at every step, 2^-53 of the partial sum each time. Measured
-// against extended precision over the cells of four genes (6,001 cells, M = 128: 132 dense columns;
-// 19,997 cells, M = 64), relative to the diagonal: 4e-17 to 7e-17 rms, DMMA 1.3e-15 to 2.1e-15.
+// modulo the p_l determine it exactly: the error of the whole sum is the rounding of the operands and of
+// the final value to FP64. The operands' is relative to the rows' norms: an entry is off by up to half of
+// 2^-s, |a| / R <= 2^-s < 2 |a| / R, so the sum by 0.41 R units of both rows (rms; 2^-55.4 |a| |b| on average, at
+// most 0.5 sqrt(K) 2^-53.7 |a| |b|). A chain of FP64 multiply-adds (the DMMA form) rounds at every step, by
+// 0.15 sqrt(K) 2^-53 sum |a_k b_k| in all (rms). Measured against extended precision, relative to the diagonal
+// of the Gram (14 shapes of 1,274 to 75,034 cells, rms): 5e-17 to 7e-17, DMMA 3e-16 to 5e-15. Where the norms'
+// product stands far above the sum (weights over many orders of magnitude, on other cells than a column) it
+// would be the other way round: k_crt_psi, k_crt_u and k_crt_t hold the rounding against the result, and the
+// DMMA kernels run for the genes or cells where it is more than theirs (crt_share).
 //
 //   k_crt_norm_*   2-norms of the operand rows and their scales; a row that is not finite (or whose
-//                  norm leaves the range where the scaling is exact) raises a flag, on which every
-//                  kernel of this file returns at once and the DMMA kernels run in its place.
+//                  norm leaves the range where the scaling is exact) goes the same way: a gene or a cell by
+//                  itself, all of them for a pair of columns.
+//   k_crt_balance  powers of two per gene that bring the gradient's operands to a like size.
 //   k_crt_conv_*   operand rows -> one INT8 plane per modulus (symmetric residues), K contiguous:
 //                  the scaled integer in four signed 16-bit limbs, each residue as an FP32 dot
 //                  product of the limbs with 2^(16 l) mod p (exact below 2^24), reduced by one
