@@ -336,70 +336,73 @@ __global__ void __launch_bounds__(kThreads, 1)
   double* Bs = smem_d + 3 * BK * SA;  // [3][BK][SBN] S pairs (pairs contiguous)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3, wm = warp >> 2, wn = warp & 3;
-  const int2 tile = grouped_tile(blockIdx.x, (c1 - c0 + BM - 1) / BM, pairs_pad / BN, group_m);
-  const int i0 = c0 + tile.x * BM, n0 = tile.y * BN;
-  if (cells && !cells[0] && !cells[1 + i0 / BM]) return;  // c0 is a multiple of BM
-  const int nsl = (J + BK - 1) / BK;
+  const int nsl = (J + BK - 1) / BK, tm = (c1 - c0 + BM - 1) / BM, tn = pairs_pad / BN;
+  for (int id = blockIdx.x; id < tm * tn; id += gridDim.x) {
+    const int2 tile = grouped_tile(id, tm, tn, group_m);
+    const int i0 = c0 + tile.x * BM, n0 = tile.y * BN;
+    if (cells && !cells[0] && !cells[1 + i0 / BM]) continue;  // c0 is a multiple of BM
+    __syncthreads();  // the last tile's slices are read
 
-  auto load = [&](int s, int buf) {
-    const int jb = s * BK;
+    auto load = [&](int s, int buf) {
+      const int jb = s * BK;
 #pragma unroll
-    for (int r = 0; r < (BM * BK / 2) / kThreads; r++) {
-      const int ch = tid + r * kThreads;
-      const int k = ch >> 6, part = ch & 63;
-      const int j = jb + k, i = i0 + part * 2;
-      const int nb = (j < J) ? 8 * max(0, min(2, min(N, c1) - i)) : 0;
-      const double* src = W + (size_t)min(j, J - 1) * ldN + min(max(i, 0), ldN - 2);
-      cp_async16(As + buf * BK * SA + k * SA + part * 2, src, nb);
-    }
-#pragma unroll
-    for (int r = 0; r < (BN * BK / 2) / kThreads; r++) {
-      const int ch = tid + r * kThreads;
-      const int k = ch >> 6, part = ch & 63;
-      const int j = jb + k;
-      const int nb = (j < J) ? 16 : 0;
-      const double* src = Sp + (size_t)min(j, J - 1) * pairs_pad + n0 + part * 2;
-      cp_async16(Bs + buf * BK * SBN + k * SBN + part * 2, src, nb);
-    }
-  };
-
-  double acc[4][4][4];
-#pragma unroll
-  for (int x = 0; x < 4; x++)
-#pragma unroll
-    for (int y = 0; y < 4; y++)
-#pragma unroll
-      for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
-
-  // three stages, one barrier per slice: after the barrier of iteration s every warp is done
-  // with slice s - 1, whose stage (s + 2) % 3 is refilled while slice s is multiplied
-  load(0, 0);
-  cp_async_commit();
-  if (nsl > 1) load(1, 1);
-  cp_async_commit();
-  for (int s = 0; s < nsl; s++) {
-    cp_async_wait<1>();  // slice s landed
-    __syncthreads();
-    if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
-    cp_async_commit();
-    warp_slice(As + (s % 3) * BK * SA, Bs + (s % 3) * BK * SBN, wm, wn, g, t, acc);
-  }
-  cp_async_wait<0>();
-
-#pragma unroll
-  for (int mt = 0; mt < 4; mt++)
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int i = i0 + wm * 64 + mt * 16 + g + h * 8;
-      if (i >= N || i >= c1) continue;
-      const double r = rOm[i];
-      double* vrow = V + (size_t)(i - c0) * pairs_pad + n0 + wn * 32 + 2 * t;
-#pragma unroll
-      for (int nt = 0; nt < 4; nt++) {
-        double2 v = make_double2(acc[mt][nt][h * 2] * r, acc[mt][nt][h * 2 + 1] * r);
-        *reinterpret_cast<double2*>(vrow + nt * 8) = v;
+      for (int r = 0; r < (BM * BK / 2) / kThreads; r++) {
+        const int ch = tid + r * kThreads;
+        const int k = ch >> 6, part = ch & 63;
+        const int j = jb + k, i = i0 + part * 2;
+        const int nb = (j < J) ? 8 * max(0, min(2, min(N, c1) - i)) : 0;
+        const double* src = W + (size_t)min(j, J - 1) * ldN + min(max(i, 0), ldN - 2);
+        cp_async16(As + buf * BK * SA + k * SA + part * 2, src, nb);
       }
+#pragma unroll
+      for (int r = 0; r < (BN * BK / 2) / kThreads; r++) {
+        const int ch = tid + r * kThreads;
+        const int k = ch >> 6, part = ch & 63;
+        const int j = jb + k;
+        const int nb = (j < J) ? 16 : 0;
+        const double* src = Sp + (size_t)min(j, J - 1) * pairs_pad + n0 + part * 2;
+        cp_async16(Bs + buf * BK * SBN + k * SBN + part * 2, src, nb);
+      }
+    };
+
+    double acc[4][4][4];
+#pragma unroll
+    for (int x = 0; x < 4; x++)
+#pragma unroll
+      for (int y = 0; y < 4; y++)
+#pragma unroll
+        for (int z = 0; z < 4; z++) acc[x][y][z] = 0.0;
+
+    // three stages, one barrier per slice: after the barrier of iteration s every warp is done
+    // with slice s - 1, whose stage (s + 2) % 3 is refilled while slice s is multiplied
+    load(0, 0);
+    cp_async_commit();
+    if (nsl > 1) load(1, 1);
+    cp_async_commit();
+    for (int s = 0; s < nsl; s++) {
+      cp_async_wait<1>();  // slice s landed
+      __syncthreads();
+      if (s + 2 < nsl) load(s + 2, (s + 2) % 3);
+      cp_async_commit();
+      warp_slice(As + (s % 3) * BK * SA, Bs + (s % 3) * BK * SBN, wm, wn, g, t, acc);
     }
+    cp_async_wait<0>();
+
+#pragma unroll
+    for (int mt = 0; mt < 4; mt++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int i = i0 + wm * 64 + mt * 16 + g + h * 8;
+        if (i >= N || i >= c1) continue;
+        const double r = rOm[i];
+        double* vrow = V + (size_t)(i - c0) * pairs_pad + n0 + wn * 32 + 2 * t;
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++) {
+          double2 v = make_double2(acc[mt][nt][h * 2] * r, acc[mt][nt][h * 2 + 1] * r);
+          *reinterpret_cast<double2*>(vrow + nt * 8) = v;
+        }
+      }
+  }
 }
 
 // U[i, a] = sum_b D_ib V[i, pair(min(a,b), max(a,b))], W warps per cell (pair_rows.cuh), the cell's V row
@@ -617,7 +620,9 @@ int launch_pair_uq(Ctx* c) {
     const int c1 = std::min(c->N, c0 + s.v_cells);
     {
       ProfScope ps(c, "uq");
-      const int g = div_up(c1 - c0, BM) * (s.pairs_pad / BN);
+      // behind the integer form most tiles have nothing to do: a block per SM walks them (thousands of blocks
+      // that return at once took 0.19 ms at 100,000 cells x 8,778 pairs)
+      const int tiles = div_up(c1 - c0, BM) * (s.pairs_pad / BN), g = cells ? std::min(tiles, c->sm_count) : tiles;
       Tunable* tu = nullptr;
       const int gm = cells ? kGroupM : tune_pick(c, "pair_v", {8, 12, 16}, kGroupM, &tu);
       TuneScope ts(c, c1 - c0 == c->N ? tu : nullptr);
