@@ -1363,10 +1363,7 @@ int gpl_de_model(gpl_ctx* h, int model) {
   GPL_RUN(de_loader_value(c, model == GPL_DE_NULL));
   c->de = true;
   c->kernel_lv = model == GPL_DE_NULL ? kLvNone : (model == GPL_DE_FULL ? kLvAll : model);
-  {
-    OrderScope order(c);
-    GPL_RUN(launch_kernel_mats(c));
-  }
+  GPL_RUN(launch_kernel_mats(c));
   GPL_TRY(c, cudaStreamSynchronize(c->stream));
   return GPL_OK;
 }

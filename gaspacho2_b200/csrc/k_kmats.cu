@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kSolveCells, 8)
   }
 }
 
-// The same in cholslg's order for any M, a row at a time, within an OrderScope (gpl_internal.cuh): 1.58 ms
-// at N = 100,000, M = 128.
+// The same in cholslg's order for any M, a row at a time, for the undamped drivers (OrderScope,
+// gpl_internal.cuh): 1.58 ms at N = 100,000, M = 128.
 __global__ void k_kmm_solve_rows(int N, int ldN, int M, const double* __restrict__ L, const double* __restrict__ Knm,
                                  double* __restrict__ Y, double* __restrict__ titsias) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -285,7 +285,7 @@ int launch_kernel_cells(Ctx* c) {
     GPL_LAUNCHED(c, "k_knm");
   }
   ProfScope ps(c, "kinvkmn");
-  if (c->one_order && c->M > 32) {
+  if ((c->one_order || c->de) && c->M > 32) {  // the undamped drivers' contexts
     k_kmm_solve_rows<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
                                                                c->titsias);
     GPL_LAUNCHED(c, "k_kmm_solve_rows");

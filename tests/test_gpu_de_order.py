@@ -45,6 +45,18 @@ def test_table_keeps_its_order(name):
     assert np.array_equal(r["phi"], z["phi"])
 
 
+def test_kernel_matrices_of_a_selected_model():
+    """Forming the kernel matrices again by gpl_kernel_mats keeps the order too (M = 40, beyond the sizes whose
+    substitution has the reference's order anyway)."""
+    z, y, d, p, (Q, reduced, M, sweeps) = _load("a")
+    with GPLVM(y, d, z["s"], z["X"], M, Q) as m:
+        m.set_params(p)
+        m.de_model("full")
+        t, k = m.get("titsias"), m.get("KinvKmn")
+        m.kernel_mats()
+        assert np.array_equal(m.get("titsias"), t) and np.array_equal(m.get("KinvKmn"), k)
+
+
 def test_gram_tiles_give_the_same_bits():
     """4,656 pairs x 512, 100 and 40 genes take the Gram's three tile sizes (128 x 128, 64 x 64, 64 x 16): an
     entry is the same chain of multiply-adds in each. 128 cells per range select the FP64 form."""
