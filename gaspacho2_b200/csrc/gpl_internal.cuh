@@ -320,8 +320,9 @@ struct PhaseScope {
   PhaseScope(const PhaseScope&) = delete;
   PhaseScope& operator=(const PhaseScope&) = delete;
 };
-// Within one, every sum of a sweep is taken in one order that no split, tile or form of a product changes:
-// the undamped IRLS of the model comparison and of the variance-component driver. A gene whose coefficients
+// Within one, every sum is taken in one order that no split, tile or form of a product changes: the undamped
+// IRLS of the model comparison and of the variance-component driver, and the placement's evaluations, whose
+// L-BFGS carries a rounding 1e8 times as far. In the IRLS, a gene whose coefficients
 // overshoot there reaches weights of 1e20 times the median, its system is singular to working precision,
 // and its entries lead the table: 2,227 cells x 1,553 genes, Q = 5, three sweeps, gave a table that
 // differed by 13 times its norm between two orders of the same sums, and other entries that were not

@@ -11,6 +11,7 @@
 //   k_expand     DeltaInv = blockdiag(1/delta_k I, Kmm/delta_GP), upper + diagonal.
 #include <algorithm>
 
+#include "dmma_common.cuh"
 #include "gpl_internal.cuh"
 
 namespace gpl {
@@ -212,10 +213,61 @@ __global__ void __launch_bounds__(kSolveCells, 8)
   }
 }
 
-// The same in cholslg's order for any M, a row at a time, for the undamped drivers (OrderScope,
-// gpl_internal.cuh): 1.58 ms at N = 100,000, M = 128.
-__global__ void k_kmm_solve_rows(int N, int ldN, int M, const double* __restrict__ L, const double* __restrict__ Knm,
-                                 double* __restrict__ Y, double* __restrict__ titsias) {
+// The same in cholslg's order for any M, a row at a time, where the order is kept (OrderScope,
+// gpl_internal.cuh). A cell per thread, its solution in shared memory, the factor's next row (forward) or column
+// (backward) copied there while the last one is used. Bound: the chain of M^2 subtractions per cell with few
+// cells, the reads of the solution (two wavefronts a step and warp) with many. At N = 20,003, M = 128: 1.04 ms from
+// global memory throughout, 0.33 ms so (k_kmm_solve: 0.15).
+constexpr int kRowsCells = 64;
+__global__ void __launch_bounds__(kRowsCells) k_kmm_solve_rows(int N, int ldN, int M, const double* __restrict__ L,
+                                                               const double* __restrict__ Knm, double* __restrict__ Y,
+                                                               double* __restrict__ titsias) {
+  extern __shared__ __align__(16) double rows_sm[];
+  double* ys = rows_sm + threadIdx.x;                // [M][kRowsCells]
+  double* Ls = rows_sm + (size_t)M * kRowsCells;     // [2][M]
+  const int i = blockIdx.x * kRowsCells + threadIdx.x;
+  const bool on = i < N;
+  const double* b = Knm + min(i, N - 1);
+  // row r: L[r, 0 .. r]; column r: L[r .. M - 1, r] at its own rows
+  auto stage = [&](int r, bool forward, int buf) {
+    double* d = Ls + (size_t)buf * M;
+    if (forward) {
+      for (int k = threadIdx.x; k <= r; k += kRowsCells) cp_async8(d + k, L + r + (size_t)k * M, 8);
+    } else {
+      for (int k = r + threadIdx.x; k < M; k += kRowsCells) cp_async8(d + k, L + k + (size_t)r * M, 8);
+    }
+  };
+  stage(0, true, 0);
+  cp_async_commit();
+  for (int step = 0; step < 2 * M; step++) {
+    const bool forward = step < M;
+    const int r = forward ? step : 2 * M - 1 - step;
+    cp_async_wait<0>();
+    __syncthreads();  // this row is there, and the buffer loaded next is no longer read
+    if (step + 1 < 2 * M) stage(step + 1 < M ? step + 1 : 2 * M - 2 - step, step + 1 < M, (step + 1) & 1);
+    cp_async_commit();
+    const double* l = Ls + (size_t)(step & 1) * M;
+    double sum = forward ? b[(size_t)r * ldN] : ys[(size_t)r * kRowsCells];
+    if (forward) {
+#pragma unroll 8
+      for (int k = r - 1; k >= 0; k--) sum = __dsub_rn(sum, __dmul_rn(l[k], ys[(size_t)k * kRowsCells]));
+    } else {
+#pragma unroll 8
+      for (int k = r + 1; k < M; k++) sum = __dsub_rn(sum, __dmul_rn(l[k], ys[(size_t)k * kRowsCells]));
+    }
+    sum = __ddiv_rn(sum, l[r]);
+    ys[(size_t)r * kRowsCells] = sum;
+    if (!forward && on) Y[i + (size_t)r * ldN] = sum;
+  }
+  if (!on) return;
+  double d = 0.0;
+  for (int k = 0; k < M; k++) d = __dadd_rn(d, __dmul_rn(b[(size_t)k * ldN], ys[(size_t)k * kRowsCells]));
+  titsias[i] = (1.0 - d) / 2.0;
+}
+// The same with the solution in global memory, for more inducing points than that one holds.
+__global__ void k_kmm_solve_rows_any(int N, int ldN, int M, const double* __restrict__ L,
+                                     const double* __restrict__ Knm, double* __restrict__ Y,
+                                     double* __restrict__ titsias) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   for (int r = 0; r < M; r++) {
@@ -286,8 +338,16 @@ int launch_kernel_cells(Ctx* c) {
   }
   ProfScope ps(c, "kinvkmn");
   if ((c->one_order || c->de) && c->M > 32) {  // the undamped drivers' contexts
-    k_kmm_solve_rows<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
-                                                               c->titsias);
+    const size_t smem = sizeof(double) * c->M * (kRowsCells + 2);
+    if (smem > 220 * 1024) {  // more than 426 inducing points
+      k_kmm_solve_rows_any<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm, c->KinvKmn,
+                                                                     c->titsias);
+      GPL_LAUNCHED(c, "k_kmm_solve_rows_any");
+      return GPL_OK;
+    }
+    GPL_TRY(c, cudaFuncSetAttribute(k_kmm_solve_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_kmm_solve_rows<<<div_up(c->N, kRowsCells), kRowsCells, smem, c->stream>>>(c->N, c->ldN, c->M, c->Kinv, Knm,
+                                                                               c->KinvKmn, c->titsias);
     GPL_LAUNCHED(c, "k_kmm_solve_rows");
     return GPL_OK;
   }

@@ -50,73 +50,58 @@ __global__ void k_place_counts(int ldN, const int32_t* __restrict__ cell, const 
   for (int64_t l = b + threadIdx.x; l < e; l += blockDim.x) Y[(size_t)j * ldN + cell[l]] = cnt[l];
 }
 
-// Residuals and per-cell sums over the genes: a block takes 64 cells (two per lane, 16-byte accesses)
-// and its eight warps every eighth gene of the range of grid y, log(y!) of small counts from a table.
-// Parts per range: part[range][cell] of l_i and of sum_j W (ldN apart), added up by k_place_sums. Bound:
-// eta and the counts read, R written, one exp() per entry (a thread per cell over all genes, with an
-// lgamma() per count, took 1.77 ms at 20,003 cells x 2,000 genes; 0.27 ms so).
-constexpr int kFactorials = 256;
-__global__ void __launch_bounds__(256) k_place_resid(int N, int ldN, int J, int jper, int pvars,
-                                                     const double* __restrict__ E, const double* __restrict__ Y,
-                                                     const double* __restrict__ ls, const double* __restrict__ delta,
-                                                     const double* __restrict__ titsias, double* __restrict__ R,
-                                                     double* __restrict__ part) {
+// Residuals and per-cell sums over the genes, a thread per cell: its genes in order in one chain (the L-BFGS
+// of a cell divides by differences of gradients and carries a rounding 1e8 times as far, so the placement keeps
+// the order of its sums), kAhead genes' loads and exponentials ahead of their additions, log(y!) of small
+// counts from a table. Bound: eta and the counts read, R written, one exp() per entry; with an lgamma() per
+// count and nothing ahead it took 1.77 ms at 20,003 cells x 2,000 genes, 0.43 ms so (0.27 ms with the genes split
+// over warps, whose sums are other bits).
+constexpr int kFactorials = 256, kAhead = 8, kResidCells = 64;
+__global__ void __launch_bounds__(kResidCells) k_place_resid(int N, int ldN, int J, int Q, int pvars,
+                                                             const double* __restrict__ E, const double* __restrict__ Y,
+                                                             const double* __restrict__ ls,
+                                                             const double* __restrict__ delta,
+                                                             const double* __restrict__ titsias,
+                                                             const double* __restrict__ X, double* __restrict__ R,
+                                                             double* __restrict__ obj, double* __restrict__ wsum) {
   __shared__ double lf[kFactorials];
-  __shared__ double sh[2][8][64];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  lf[threadIdx.x] = lgamma((double)threadIdx.x + 1.0);
+  for (int k = threadIdx.x; k < kFactorials; k += kResidCells) lf[k] = lgamma((double)k + 1.0);
   __syncthreads();
-  const int i = blockIdx.x * 64 + 2 * lane;  // even; ldN is a multiple of 32
-  const int j1 = min(J, (int)(blockIdx.y + 1) * jper);
-  double2 l = make_double2(0.0, 0.0), ws = l;
-  if (i < N) {
-    const bool two = i + 1 < N;
-    const double dgp = delta[pvars - 1] * kWt;
-    const double s0 = ls[i], s1 = two ? ls[i + 1] : 1.0;
-    const double f0 = s0 * exp(dgp * titsias[i]), f1 = two ? s1 * exp(dgp * titsias[i + 1]) : 0.0;
-    const double g0 = log(s0), g1 = log(s1);
-    auto logfact = [&](double y) {  // log(y!) of a count
-      const int k = (int)y;
-      return k < kFactorials && (double)k == y ? lf[k] : lgamma(y + 1.0);
-    };
-#pragma unroll 2
-    for (int j = blockIdx.y * jper + warp; j < j1; j += 8) {
-      const size_t e = (size_t)j * ldN + i;
-      const double2 eta = *reinterpret_cast<const double2*>(E + e), y = *reinterpret_cast<const double2*>(Y + e);
-      const double w0 = exp(eta.x) * f0, w1 = exp(eta.y) * f1;
-      if (R) *reinterpret_cast<double2*>(R + e) = make_double2(y.x - w0, y.y - w1);
-      l.x += y.x * (eta.x + g0) - w0;
-      if (y.x > 0.0) l.x -= logfact(y.x);  // the full Poisson log-probability (constant in x)
-      ws.x += w0;
-      if (two) {
-        l.y += y.y * (eta.y + g1) - w1;
-        if (y.y > 0.0) l.y -= logfact(y.y);
-        ws.y += w1;
+  const int i = blockIdx.x * kResidCells + threadIdx.x;
+  if (i >= N) return;
+  const double lsi = ls[i], lls = log(lsi), ett = exp(delta[pvars - 1] * titsias[i] * kWt);
+  double l = 0.0, ws = 0.0;
+  double eta[kAhead], y[kAhead];
+  auto load = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) {
+      const size_t e = (size_t)min(j0 + u, J - 1) * ldN + i;
+      eta[u] = E[e];
+      y[u] = Y[e];
+    }
+  };
+  load(0);
+  for (int j0 = 0; j0 < J; j0 += kAhead) {
+    double w[kAhead], t[kAhead], c[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) {
+      w[u] = exp(eta[u]) * lsi * ett;
+      t[u] = y[u] * (eta[u] + lls) - w[u];
+      c[u] = y[u];
+    }
+    if (j0 + kAhead < J) load(j0 + kAhead);
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) {
+      if (j0 + u < J) {
+        if (R) R[(size_t)(j0 + u) * ldN + i] = c[u] - w[u];
+        l += t[u];
+        if (c[u] > 0.0) {  // the full Poisson log-probability (constant in x)
+          const int k = (int)c[u];
+          l -= k < kFactorials && (double)k == c[u] ? lf[k] : lgamma(c[u] + 1.0);
+        }
+        ws += w[u];
       }
     }
-  }
-  sh[0][warp][2 * lane] = l.x;
-  sh[0][warp][2 * lane + 1] = l.y;
-  sh[1][warp][2 * lane] = ws.x;
-  sh[1][warp][2 * lane + 1] = ws.y;
-  __syncthreads();
-  if (threadIdx.x < 128) {
-    const int q = threadIdx.x >> 6, c = threadIdx.x & 63;
-    double t = 0.0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) t += sh[q][k][c];
-    if (blockIdx.x * 64 + c < N) part[((size_t)blockIdx.y * 2 + q) * ldN + blockIdx.x * 64 + c] = t;
-  }
-}
-
-__global__ void k_place_sums(int N, int ldN, int Q, int ns, const double* __restrict__ part,
-                             const double* __restrict__ X, double* __restrict__ obj, double* __restrict__ wsum) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  double l = 0.0, ws = 0.0;
-  for (int k = 0; k < ns; k++) {
-    l += part[(size_t)k * 2 * ldN + i];
-    ws += part[((size_t)k * 2 + 1) * ldN + i];
   }
   for (int q = 1; q < Q; q++) {  // N(0, 1) prior on the ARD dimensions
     const double x = X[i + (size_t)q * N];
@@ -126,49 +111,28 @@ __global__ void k_place_sums(int N, int ldN, int Q, int ns, const double* __rest
   wsum[i] = ws;
 }
 
-// d l_i / d x_iq (stored as g[i + q N], the ascent direction of l): 32 cells per block (a lane each),
-// its eight warps every eighth inducing point, their sums added in order.
-__global__ void __launch_bounds__(256) k_place_grad(int N, int ldN, int M, int Q, int pvars,
+// d l_i / d x_iq (stored as g[i + q N], the ascent direction of l): 32 cells per block, a lane each, a warp per
+// dimension q, whose sum over the inducing points is one chain in their order.
+__global__ void __launch_bounds__(512) k_place_grad(int N, int ldN, int M, int Q, int pvars,
                                                     const double* __restrict__ X, const double* __restrict__ T,
                                                     const double* __restrict__ rho, const double* __restrict__ Knm,
                                                     const double* __restrict__ KinvKmn, const double* __restrict__ G,
                                                     const double* __restrict__ wsum, const double* __restrict__ delta,
                                                     double* __restrict__ g) {
-  extern __shared__ double sums[];  // [8][Q][32]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
-  double acc[16];
-#pragma unroll
-  for (int q = 0; q < 16; q++) acc[q] = 0.0;
-  if (i < N) {
-    const double tw = kWt * delta[pvars - 1] * wsum[i];
-    double x[16], ir[16];
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      x[q] = q < Q ? X[i + (size_t)q * N] : 0.0;
-      ir[q] = q < Q ? 1.0 / rho[q] : 0.0;
-    }
-    for (int k = warp; k < M; k += 8) {
-      const double K = Knm[(size_t)k * ldN + i];
-      const double C = (G[(size_t)k * ldN + i] + tw * KinvKmn[(size_t)k * ldN + i]) * K;
-      acc[0] -= C * sin(x[0] - T[k]) * (0.5 * ir[0]);
-#pragma unroll
-      for (int q = 1; q < 16; q++)
-        if (q < Q) acc[q] -= C * (x[q] - T[k + (size_t)q * M]) * ir[q];
-    }
+  const int q = threadIdx.x >> 5, i = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (i >= N) return;
+  const double tw = kWt * delta[pvars - 1] * wsum[i];
+  const double x = X[i + (size_t)q * N], r = rho[q];
+  double acc = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < M; k++) {
+    const double K = Knm[(size_t)k * ldN + i];
+    const double C = (G[(size_t)k * ldN + i] + tw * KinvKmn[(size_t)k * ldN + i]) * K;
+    if (q == 0) acc -= C * sin(x - T[k]) / (2.0 * r);
+    else acc -= C * (x - T[k + (size_t)q * M]) / r;
   }
-#pragma unroll
-  for (int q = 0; q < 16; q++)
-    if (q < Q) sums[(warp * Q + q) * 32 + lane] = acc[q];
-  __syncthreads();
-  for (int q = warp; q < Q; q += 8) {
-    if (i >= N) continue;
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) s += sums[(k * Q + q) * 32 + lane];
-    if (q > 0) s -= X[i + (size_t)q * N];  // the prior's gradient
-    g[i + (size_t)q * N] = s;
-  }
+  if (q > 0) acc -= x;  // the prior's gradient
+  g[i + (size_t)q * N] = acc;
 }
 
 // The step of cell i on f = -l (gradient gf = -g): the first iteration -gf/1e5, then the two-loop
@@ -305,17 +269,14 @@ static int place_eval(Ctx* c, PlaceBufs& pb, double* f, bool grad, bool first) {
   int rc = first ? launch_kernel_mats(c) : launch_kernel_cells(c);
   if (rc) return rc;
   if ((rc = launch_zbeta(c, c->Beta, c->scratch))) return rc;  // eta
-  const int bx = div_up(c->N, 64), ns = cell_sum_ranges(c);
-  if ((rc = ensure_part(c, (size_t)2 * ns * c->ldN))) return rc;
-  k_place_resid<<<dim3(bx, ns), 256, 0, c->stream>>>(c->N, c->ldN, c->J, div_up(c->J, ns), c->p, c->scratch, c->Nu,
-                                                     c->ls, c->delta, c->titsias, grad ? c->W : nullptr, c->part);
+  k_place_resid<<<div_up(c->N, kResidCells), kResidCells, 0, c->stream>>>(c->N, c->ldN, c->J, c->Q, c->p, c->scratch,
+                                                                         c->Nu, c->ls, c->delta, c->titsias, c->X,
+                                                                         grad ? c->W : nullptr, f, pb.wsum);
   GPL_LAUNCHED(c, "k_place_resid");
-  k_place_sums<<<div_up(c->N, 128), 128, 0, c->stream>>>(c->N, c->ldN, c->Q, ns, c->part, c->X, f, pb.wsum);
-  GPL_LAUNCHED(c, "k_place_sums");
   if (!grad) return GPL_OK;
   if ((rc = dgen_resid_gp(c, c->W, c->Beta, c->C1))) return rc;
   const double* Knm = c->Dm + (size_t)c->dg0 * c->ldN;
-  k_place_grad<<<div_up(c->N, 32), 256, sizeof(double) * 8 * 32 * c->Q, c->stream>>>(
+  k_place_grad<<<div_up(c->N, 32), 32 * c->Q, 0, c->stream>>>(
       c->N, c->ldN, c->M, c->Q, c->p, c->X, c->T, c->rho, Knm, c->KinvKmn, c->C1, pb.wsum, c->delta, pb.g);
   GPL_LAUNCHED(c, "k_place_grad");
   return GPL_OK;
@@ -327,6 +288,7 @@ int place_cells(Ctx* c, int iters, double* X_host, double* obj_host, int32_t* st
     c->err = "placement needs Q <= 16 and the full GP model";
     return GPL_ERR_ARG;
   }
+  OrderScope order(c);
   PlaceBufs pb;
   const size_t nq = (size_t)N * Q;
   int rc = place_bufs(c, &pb);
@@ -386,6 +348,7 @@ int cell_objective(Ctx* c, const double* X_host, double* obj_host, double* grad_
     c->err = "placement needs Q <= 16 and the full GP model";
     return GPL_ERR_ARG;
   }
+  OrderScope order(c);
   PlaceBufs pb;
   int rc = place_bufs(c, &pb);
   if (rc) return rc;

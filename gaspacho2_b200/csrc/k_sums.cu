@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) k_state_sums(int N, const double* __restr
 }
 }  // namespace
 
-size_t cell_sums_part(const Ctx* c) { return (size_t)2 * cell_sum_ranges(c) * c->ldN; }  // two sums: the placement's
+size_t cell_sums_part(const Ctx* c) { return (size_t)cell_sum_ranges(c) * c->ldN; }
 
 int launch_oinvt(Ctx* c) {
   ProfScope ps(c, "oinvt");
