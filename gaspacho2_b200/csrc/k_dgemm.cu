@@ -12,14 +12,15 @@
 //                 (dcol a, dcol b) when one range covers all cells: the dense block of getPsi
 //                 (ggplvm.cu:621-680); otherwise added up range by range in a pairs x genes
 //                 buffer that k_pair_scatter moves into Psi. Work: N*J*n_d*(n_d+1) flops.
+//                 Behind the integer form (k_crt.cu) these three run for the genes that it left.
 //   k_pair_v      V[i, p] = (1/Omega_i) sum_j W_ij S_j[a, b] for a cell range, S_j = Psi_j^{-1}
 //                 gathered per pair (k_gather_spair). M = cells, N = pairs, K = genes; both
 //                 operands by cp.async. Work: N*J*n_d*(n_d+1) flops.
 //   k_v_to_u      U[i, a] = sum_b D_ib V[i, pair(a, b)]: the gradient contraction
 //                 sum_j O_ij S_j[DD] d_i of getGradLogOmega (ggplvm.cu:301-376) from V.
 //
-// CTA tile 128 x 128 x 16 (K), 8 warps as 2 (M) x 4 (N), warp tile 64 x 32 (4 x 4 DMMA tiles
-// of 16 x 8), three-stage cp.async pipelines with one barrier per slice. m16n8k4 fragments (lane = 4*g + t):
+// CTA tile 128 x 128 x 16 (K; the Gram also 64 x 64 and 64 x 16), 8 warps as 2 (M) x 4 (N), warp tile 64 x 32
+// (4 x 4 DMMA tiles of 16 x 8), three-stage cp.async pipelines with one barrier per slice. m16n8k4 fragments (lane = 4*g + t):
 // A 16x4 row-major a0 = A[g][t], a1 = A[g+8][t]; B 4x8 b0 = B[t][g]; C 16x8
 // c0,c1 = C[g][2t, 2t+1], c2,c3 = C[g+8][2t, 2t+1]. Shared rows are padded so that the
 // 16 lanes of each half-warp hit 16 distinct 8-byte bank pairs.
