@@ -8,9 +8,9 @@
 // 2-norm is at most R = sqrt(0.48 P), P the product of the moduli (2^110.5), and rounded to integers;
 // rows of B the same way. By Cauchy-Schwarz the integer sum lies within +-0.48 P, so its residues
 // modulo the p_l determine it exactly: the error of the whole sum is the rounding of the operands and of
-// the final value to FP64. The operands' is relative to the rows' norms: an entry is off by up to half of
-// 2^-s, |a| / R <= 2^-s < 2 |a| / R, so the sum by 0.41 R units of both rows (rms; 2^-55.4 |a| |b| on average, at
-// most 0.5 sqrt(K) 2^-53.7 |a| |b|). A chain of FP64 multiply-adds (the DMMA form) rounds at every step, by
+// the final value to FP64. The operands' is relative to the rows' norms: an entry is off by less than
+// 2^-s, |a| / R <= 2^-s < 2 |a| / R, and by nothing on average (crt_dither), so the sum by 0.58 R units of both
+// rows at most (rms; 2^-54.9 |a| |b| on average). A chain of FP64 multiply-adds (the DMMA form) rounds at every step, by
 // 0.15 sqrt(K) 2^-53 sum |a_k b_k| in all (rms). Measured against extended precision, relative to the diagonal
 // of the Gram (14 shapes of 1,274 to 75,034 cells, rms): 5e-17 to 7e-17, DMMA 3e-16 to 5e-15. Where the norms'
 // product stands far above the sum (weights over many orders of magnitude, on other cells than a column) it
@@ -283,9 +283,21 @@ __global__ void __launch_bounds__(256) k_crt_balance(int N, int64_t ldN, int n_d
 }
 
 // ---- residues ------------------------------------------------------------------------------------
-// the four signed 16-bit limbs of rint(v sc), |v sc| < 2^60
-__device__ __forceinline__ void crt_limbs(double v, double sc, float (&l)[4]) {
-  long long x = __double2ll_rn(v * sc);
+// Entries are rounded down after a number in [0, 1) has been added, one per contraction index k and operand,
+// as if drawn at random (a multiplicative hash): an entry is off by 0.41 of a unit (rms; 0.29 rounded to
+// nearest) and by nothing on average, and integers stay as they are. Rounded to nearest, a row of one value
+// (1/Omega of cells that share it, equal weights) is off by the same fraction everywhere, and its sums by
+// that: up to 103 u at 100,000 cells, where an entry has 46 bits and a chain of FP64 additions is off by 47 u.
+template <bool kA>
+__device__ __forceinline__ double crt_dither(uint32_t k) {
+  uint32_t h = k * 0x9e3779b1u + (kA ? 0x7f4a7c15u : 0x1ce4e5b9u);
+  h = (h ^ (h >> 15)) * 0x2c9277b5u;
+  h = (h ^ (h >> 13)) * 0xac564b05u;
+  return __hiloint2double((int)(0x3ff00000u | (h >> 12)), (int)(h << 20)) - 1.0;
+}
+// the four signed 16-bit limbs of floor(v sc + u), |v sc| < 2^60
+__device__ __forceinline__ void crt_limbs(double v, double sc, double u, float (&l)[4]) {
+  long long x = __double2ll_rd(__dadd_rd(__dmul_rn(v, sc), u));
   const int l0 = (int)(short)x;
   x = (x - l0) >> 16;
   const int l1 = (int)(short)x;
@@ -315,10 +327,11 @@ __device__ __forceinline__ uint32_t crt_pack(uint32_t a, uint32_t b, uint32_t c,
 
 // eight consecutive K entries v (scaled by sc) of row `row`: 8 bytes into every plane
 template <bool kA>
-__device__ __forceinline__ void crt_store8(const double (&v)[8], double sc, int8_t* __restrict__ out, size_t plane) {
+__device__ __forceinline__ void crt_store8(const double (&v)[8], double sc, const double (&u)[8],
+                                           int8_t* __restrict__ out, size_t plane) {
   float l[8][4];
 #pragma unroll
-  for (int e = 0; e < 8; e++) crt_limbs(v[e], sc, l[e]);
+  for (int e = 0; e < 8; e++) crt_limbs(v[e], sc, u[e], l[e]);
 #pragma unroll
   for (int m = 0; m < kMod; m++) {
     uint32_t r[8];
@@ -349,7 +362,10 @@ __global__ void __launch_bounds__(256) k_crt_conv_rows(const double* __restrict_
 #pragma unroll
     for (int e = 0; e < 8; e++) v[e] = i + e < len ? r[e] : 0.0;
   }
-  crt_store8<true>(v, sc[j], out + (size_t)j * ldk + i, plane);
+  double u[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) u[e] = crt_dither<true>(i + e);
+  crt_store8<true>(v, sc[j], u, out + (size_t)j * ldk + i, plane);
 }
 
 // the pair products of a range of cells: planes [pair][ldk]; kConvPairs pairs per block, which share
@@ -367,6 +383,9 @@ __global__ void __launch_bounds__(256) k_crt_conv_pairs(int ldN, int c0, int len
   // [0, len) can be read whole; products past the range are dropped
   const bool any = i < len;
   const int at = any ? c0 + i : c0;
+  double u[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) u[e] = crt_dither<false>(i + e);
   for (int p = blockIdx.y * kConvPairs; p < min(n_pairs, (int)(blockIdx.y + 1) * kConvPairs); p++) {
     const int2 q = pairs[p];
     const double *da = D + (size_t)q.x * ldN + at, *db = D + (size_t)q.y * ldN + at;
@@ -379,7 +398,7 @@ __global__ void __launch_bounds__(256) k_crt_conv_pairs(int ldN, int c0, int len
       v[2 * e] = i + 2 * e < len ? a.x * b.x * o.x : 0.0;
       v[2 * e + 1] = i + 2 * e + 1 < len ? a.y * b.y * o.y : 0.0;
     }
-    crt_store8<false>(v, sc[p], out + (size_t)p * ldk + i, plane);
+    crt_store8<false>(v, sc[p], u, out + (size_t)p * ldk + i, plane);
   }
 }
 
@@ -392,9 +411,12 @@ __global__ void __launch_bounds__(256) k_crt_conv_cols(const double* __restrict_
                                                        const double* __restrict__ sc, int8_t* __restrict__ out,
                                                        const int* __restrict__ flag) {
   extern __shared__ uint32_t turn[];  // [kMod][32][kTurnWords]
+  __shared__ double u[128];
   if (*flag) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m = blockIdx.x * 32 + lane, k0 = blockIdx.y * 128;
+  if (threadIdx.x < 128) u[threadIdx.x] = crt_dither<kA>(k0 + threadIdx.x);
+  __syncthreads();
   const double s = m < M ? sc[m] : 0.0;
 #pragma unroll 1
   for (int g = 0; g < 4; g++) {
@@ -403,7 +425,7 @@ __global__ void __launch_bounds__(256) k_crt_conv_cols(const double* __restrict_
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int k = k0 + kw * 4 + e;
-      crt_limbs(m < M && k < K ? src[(size_t)k * ld + m] * bal[k] : 0.0, s, l[e]);
+      crt_limbs(m < M && k < K ? src[(size_t)k * ld + m] * bal[k] : 0.0, s, u[kw * 4 + e], l[e]);
     }
 #pragma unroll
     for (int q = 0; q < kMod; q++)
@@ -667,7 +689,7 @@ __device__ __forceinline__ void crt_values(const uint8_t* __restrict__ in, size_
 // over several ranges of cells the partial sums collect in acc (first / last: the range's place).
 // A gene's row of W cannot be balanced for all pairs at once: where its mass lies on other cells than a
 // column's, the sum is far below the product of the norms. So a gene goes on the list of the DMMA form
-// when the rounding of a diagonal entry, `unit` inv_j inv_p (0.41 R units; its ranges added up, in err), is
+// when the rounding of a diagonal entry, `unit` inv_j inv_p (0.58 R units; its ranges added up, in err), is
 // more than `share` of that entry. The diagonal is enough, as in k_crt_u: |p_ab|^2 <= |p_aa| |p_bb| by
 // Cauchy-Schwarz, so the rounding of entry (a, b) stays within that share of sqrt(Psi_aa Psi_bb), the
 // scale by which a factorization sees it.
@@ -711,8 +733,8 @@ __global__ void __launch_bounds__(256) k_crt_psi(int P, int n_pairs, int64_t ldo
 }
 
 // U_i = sum_b D_ib V[i, pair(a, b)], V[i, p] = (1/Omega_i) sum_j W_ij S_j[p], W warps per cell: the
-// cell's row of V from its residues into shared memory (pair_rows.cuh). The operands' entries are off by 0.29
-// of a unit (rms), so a sum by at most 0.41 R units, R bounding both rows' norms. Where that is more than its
+// cell's row of V from its residues into shared memory (pair_rows.cuh). The operands' entries are off by 0.41
+// of a unit (rms), so a sum by at most 0.58 R units, R bounding both rows' norms. Where that is more than its
 // share (crt_share) of a diagonal V[i, (a, a)], the value below `least` units, the cell's 128 cells go to the
 // DMMA form. The diagonal is enough: W_ij and the
 // S_j[a, a] are positive, |S_j[a, b]| <= sqrt(S_j[a, a] S_j[b, b]), and so by Cauchy-Schwarz the rounding of
@@ -892,9 +914,9 @@ static int crt_gemm(Ctx* c, const CUtensorMap& ma, const CUtensorMap& mb, int ro
 
 // What the rounding of an integer product may be of the diagonal it is measured by (k_crt_psi, k_crt_u), over K
 // terms: what a chain of K FP64 multiply-adds is off by, 0.15 sqrt(K) u (rms; 12 u measured at K = 6,001, 19 u
-// at 19,997), less a third, and 4 u at least.
+// at 19,997), and 4 u at least. The rounding is taken at its bound, which lies up to twice above its rms.
 static double crt_share(double K) {
-  return 0x1p-53 * std::max(4.0, 0.1 * std::sqrt(K));
+  return 0x1p-53 * std::max(4.0, 0.15 * std::sqrt(K));
 }
 
 // scales of rows with K strided (src[k * ld + m] bal[k]); `part` holds at least 16 sums per row
@@ -945,7 +967,7 @@ int launch_crt_gram(Ctx* c) {
     if (rc) return rc;
     k_crt_psi<<<dim3(c->J, div_up(s.n_pairs, 1024)), 256, 0, c->stream>>>(
         c->P, s.n_pairs, t.Pp, plane_o, t.g_out, inv_j, inv_p, s.pairs, c->dcol_d, c->DeltaInv, t.g_acc, t.Pp,
-        c0 == 0, c0 + len >= c->N, c->Psi, c->n_d, 0.41 * R, crt_share(c->N), t.g_err, genes);
+        c0 == 0, c0 + len >= c->N, c->Psi, c->n_d, 0.58 * R, crt_share(c->N), t.g_err, genes);
     GPL_LAUNCHED(c, "k_crt_psi");
   }
   return GPL_OK;
@@ -966,7 +988,7 @@ int launch_crt_uq(Ctx* c) {
   GPL_LAUNCHED(c, "k_crt_balance");
   int rc;
   if ((rc = crt_col_scales(c, s.Sp, s.pairs_pad, s.n_pairs, c->J, bal_s, part, sc_p, inv_p, t.cells, 31))) return rc;
-  const double least = 0.41 * crt_norm_limit() / crt_share(c->J) / kUnit;
+  const double least = 0.58 * crt_norm_limit() / crt_share(c->J) / kUnit;
   k_crt_conv_cols<false><<<dim3(div_up(s.n_pairs, 32), t.Jk / 128), 256, kSmemTurn, c->stream>>>(
       s.Sp, s.pairs_pad, s.n_pairs, c->J, t.Jk, plane_b, bal_s, sc_p, t.v_b, t.cells);
   GPL_LAUNCHED(c, "k_crt_conv_cols");
@@ -1110,7 +1132,7 @@ int launch_crt_columns(Ctx* c, int L, const double* G, const double* gg, double*
       if ((rc = crt_gemm(c, t.map_ga, t.map_gb, c->J, rows, t.Jp, t.Pp, len, t.g_out, plane_o, t.Pp, t.cols))) return rc;
       k_crt_t<<<dim3(c->J, div_up(rows, 1024)), 256, 0, c->stream>>>(c->J, c->P, c->n_d, rows, t.Pp, plane_o, t.g_out,
                                                                     inv_j, inv_p, c->dcol_d, c0 == 0,
-                                                                    0.41 * R / crt_share(c->N) * c->N / len, root,
+                                                                    0.58 * R / crt_share(c->N) * c->N / len, root,
                                                                     gg + (size_t)l0 * c->J,
                                                                     T + (size_t)l0 * c->J * c->P, t.cols);
       GPL_LAUNCHED(c, "k_crt_t");

@@ -139,3 +139,21 @@ def test_genotype_columns_of_spread_weights(spread):
         one = np.concatenate([m.score_stats(geno[:, k:k + 1]) for k in range(L)], 1)
     assert np.all(np.isfinite(one))
     assert np.all(np.abs(S - one) <= 1e-9 * (1.0 + np.abs(one)))
+
+
+@pytest.mark.parametrize("N,om", [(20000, 1.423), (60000, 1.2225)])
+def test_equal_entries_round_to_nothing_on_average(N, om):
+    """Cells that share one Omega: the intercept's row is one value whose nearest integer is off by 45 u and 77 u
+    here, and a sum rounded to nearest by as much; a random rounding averages out over the cells. The diagonal
+    stays within the share that the form allows itself (14 u and 24 u)."""
+    G, M = 300, 30
+    ds = synth.make(0, 5, N=N, G=G, M=M, Q=5, init=False)
+    ds.init.rho[:] = 3.0
+    ds.init.Omega[:] = om
+    with GPLVM.from_dataset(ds) as m:
+        m.set_params(ds.init)
+        psi = _psi(m, ds, 0.2 * np.random.default_rng(3).standard_normal((m.P, G)))
+        W = m.get("W").reshape(-1, N)[:G]
+        prior = m.get("DeltaInv").reshape(m.P, m.P)[0, 0]
+    ref = W.astype(np.longdouble).sum(1) / np.longdouble(om) + prior
+    assert np.all(np.abs(psi[:, 0, 0] - ref) <= (_share(N) + 2 * U) * ref)
