@@ -846,7 +846,8 @@ int crt_prepare(Ctx* c) {
   CrtState& t = s.crt;
   if (!t.on) return GPL_OK;
   const size_t rows = (size_t)2 * (t.Jp + t.Pp + t.grad_cells), tiles = div_up(c->N, 128);
-  const size_t ints = 5 + tiles + 2 * (size_t)c->J + div_up(c->J, 128), errs = t.gram_cells < c->N ? (size_t)c->J * c->n_d : 0;
+  const size_t ints = 5 + tiles + 2 * (size_t)c->J + div_up(c->J, 128);
+  const size_t errs = t.gram_cells && t.gram_cells < c->N ? (size_t)c->J * c->n_d : 0;
   if (cudaMalloc((void**)&t.scales, sizeof(double) * (rows + 2 * t.Jp + errs)) != cudaSuccess ||
       cudaMalloc((void**)&t.err, ints * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
